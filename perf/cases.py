@@ -171,3 +171,43 @@ def tolerance(case):
     # against the same path in fp32 (bf16 cases) or fp64 (fp32 cases) sums the largest relative error of
     # any output is 3.6e-3 and 1.6e-6
     return {"rel": 1.2e-2} if case["dtype"] == "bf16" else {"rel": 7e-6}
+
+
+def _exact_expert(x, gate_up, gate_up_bias, down, down_bias):
+    pre = x @ gate_up + gate_up_bias
+    gate, up = pre[:, 0::2].clamp(max=7.0), pre[:, 1::2].clamp(-7.0, 7.0)
+    return ((up + 1) * gate * torch.sigmoid(1.702 * gate)) @ down + down_bias
+
+
+def exact(case, seed):
+    """`run`'s outputs in 64 bits.  The layer picks its experts by rounded logits, near ties and the
+    capacity among them, so that its outputs have no value apart from that rounding."""
+    if case["op"] == "layer":
+        return None
+    state = prepare(case, seed)
+    hidden, indices, routing, *p = [t.detach() for t in state["args"]]
+    x, routing64 = hidden.double(), routing.double()
+    w_of = routing64.gather(1, indices) if case["dense"] else routing64
+    out, d_hidden, d_w = torch.zeros_like(x), torch.zeros_like(x), torch.zeros_like(w_of)
+    with_grad = case["op"] != "experts"
+    d = [torch.zeros(t.shape, dtype=torch.float64, device=t.device) for t in p] if with_grad else []
+    for e in range(case["E"]):
+        tok, slot = torch.nonzero(indices == e, as_tuple=True)
+        if tok.numel() == 0:
+            continue
+        w = w_of[tok, slot, None]
+        leaves = [t.requires_grad_(with_grad) for t in (x[tok], *(t[e].double() for t in p))]
+        y = _exact_expert(*leaves)
+        out.index_add_(0, tok, y.detach() * w)
+        if with_grad:
+            gy = state["grad"][tok].double()
+            grads = torch.autograd.grad(y, leaves, gy * w)
+            d_hidden.index_add_(0, tok, grads[0])
+            d_w[tok, slot] = (y.detach() * gy).sum(-1)
+            for whole, part in zip(d, grads[1:]):
+                whole[e] = part
+    if not with_grad:
+        return out
+    d_routing = torch.zeros_like(routing64).scatter_(1, indices, d_w) if case["dense"] else d_w
+    grads = [d_hidden, d_routing, *d]
+    return grads if case["op"] == "backward" else [out, *grads]
