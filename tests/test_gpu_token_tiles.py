@@ -1,0 +1,95 @@
+"""The grouped GEMMs at the numbers of rows per expert where a tile or a k-block ends, the routing of many
+assignments, and special values in fp32: against the CPU oracle, with the tolerances of the other tests."""
+import pytest
+import torch
+
+from oracle import experts_oracle as orc
+from helpers import REL_L2_BF16, RTOL_BF16, RTOL_F32
+
+pytestmark = pytest.mark.gpu
+GRADS = ["d_hidden", "d_routing", "d_wgu", "d_bgu", "d_wd", "d_bd"]
+#: rows per expert: none, around the 16-row step, a 64-deep k-block, the 96 / 128 / 256-row boxes and tiles
+COUNTS = [0, 1, 15, 16, 17, 63, 64, 65, 97, 129, 193, 255, 256, 257, 300, 513]
+
+
+def _problem(counts, H, dtype, seed):
+    g = torch.Generator().manual_seed(seed)
+    E, T = len(counts), sum(counts)
+    ridx = torch.repeat_interleave(torch.arange(E), torch.tensor(counts))[torch.randperm(T, generator=g)][:, None]
+
+    def normal(*shape, std):
+        return (torch.randn(*shape, generator=g) * std).to(dtype)
+
+    args = [normal(T, H, std=1.0), ridx, torch.rand(T, 1, generator=g).to(dtype) + 0.25, normal(E, H, 2 * H, std=0.1),
+            normal(E, 2 * H, std=0.2), normal(E, H, H, std=0.1), normal(E, H, std=0.2)]
+    return args, normal(T, H, std=1.0), T, E
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32], ids=["bf16", "fp32"])
+@pytest.mark.parametrize("H", [64, 192, 320])
+@pytest.mark.parametrize("capacity", [10000, 130])
+def test_rows_per_expert_at_tile_edges(dtype, H, capacity):
+    import yamoe_b200
+    from yamoe_b200.layers import experts_autograd
+    args, grad, T, E = _problem(COUNTS, H, dtype, seed=H + capacity)
+    rtol, l2 = (RTOL_BF16, REL_L2_BF16) if dtype == torch.bfloat16 else (RTOL_F32, RTOL_F32)
+    dev = [a.cuda() for a in args]
+    ref = orc.experts_forward_oracle(*args, capacity, E, 1)
+    orc.check_close(yamoe_b200.experts(*dev, capacity, E, 1).float().cpu(), ref, rtol, "forward", rel_l2=l2)
+    ref_g = orc.experts_backward_oracle(grad, *args, capacity, E, 1)
+    got = yamoe_b200.experts_backward(grad.cuda(), *dev, capacity, E, 1)
+    for a, b, n in zip(got, ref_g, GRADS):
+        orc.check_close(a.float().cpu(), b, rtol, n)
+    leaves = [t.requires_grad_(True) for t in dev if t.is_floating_point()]
+    out = experts_autograd(*dev, capacity, E, 1, save_activations=True)
+    orc.check_close(out.detach().float().cpu(), ref, rtol, "saving forward", rel_l2=l2)
+    for a, i in zip(torch.autograd.grad(out, leaves, grad.cuda()), [0, 1, 2, 3, 4, 5]):
+        orc.check_close(a.float().cpu(), ref_g[i], rtol, GRADS[i] + " (saved activations)")
+
+
+@pytest.mark.parametrize("T,E,K", [(8193, 7, 4), (8191, 300, 4), (9001, 16, 4), (2731, 33, 3)])
+def test_routing_of_many_assignments(T, E, K):
+    """Around 32768 assignments, with ids outside [0, E) and a capacity that drops."""
+    import yamoe_b200
+    H = 64
+    g = torch.Generator().manual_seed(T)
+    ridx = torch.stack([torch.randperm(E, generator=g)[:K] for _ in range(64)]).repeat((T + 63) // 64, 1)[:T]
+    ridx[5, 0], ridx[T - 1, K - 1] = -3, E + 2
+    rw = torch.rand(T, K, generator=g)
+    args = [torch.randn(T, H, generator=g), ridx, rw] + [torch.randn(*s, generator=g) * 0.1 for s in
+                                                         ((E, H, 2 * H), (E, 2 * H), (E, H, H), (E, H))]
+    cap = max(1, T * K // E - 3)
+    # an id out of range contributes nothing: the oracle gets expert 0 with weight zero, behind everybody else
+    rank = torch.zeros_like(ridx)
+    seen = torch.zeros(E, dtype=torch.long)
+    for p, e in enumerate(ridx.reshape(-1).tolist()):
+        if 0 <= e < E:
+            rank.view(-1)[p] = seen[e]
+            seen[e] += 1
+    keep = (rank < cap) & (ridx >= 0) & (ridx < E)
+    w = torch.where(keep, rw, torch.zeros_like(rw))
+    ref = orc.experts_forward_oracle(args[0], ridx.clamp(0, E - 1), w, *args[3:], T * K, E, K)
+    out = yamoe_b200.experts(*[a.cuda() for a in args], cap, E, K)
+    orc.check_close(out.cpu(), ref, RTOL_F32, "forward")
+
+
+@pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan"), 3.0e38])
+def test_fp32_parts_of_special_values(value):
+    """Every output is NaN, infinite or finite where the CUDA-core kernel's is; weights are multiples of
+    1/64, whose lower parts vanish."""
+    import yamoe_b200
+    args, grad, T, E = _problem([20, 33, 0, 70], 128, torch.float32, seed=5)
+    for i in (3, 5):
+        args[i] = (args[i] * 64).round() / 64
+    args[0][7, 3], args[3][1, 5, 11], args[5][3, 9, 2] = value, value, -value
+    dev = [a.cuda() for a in args]
+    res = {}
+    for path in ("auto", "simt"):
+        yamoe_b200.set_path(path)
+        try:
+            res[path] = [yamoe_b200.experts(*dev, T, E, 1), *yamoe_b200.experts_backward(grad.cuda(), *dev, T, E, 1)]
+        finally:
+            yamoe_b200.set_path("auto")
+    for a, b in zip(res["auto"], res["simt"]):
+        assert torch.equal(a.isnan(), b.isnan())
+        assert torch.equal(a.isinf() & (a > 0), b.isinf() & (b > 0)) and torch.equal(a.isinf(), b.isinf())

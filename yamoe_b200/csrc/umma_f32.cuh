@@ -1,0 +1,741 @@
+// fp32 grouped GEMM on the tensor cores (sm_100a): every fp32 operand is the exact sum of three bf16
+// parts of eight significant bits each, and six of the nine partial products are multiplied with
+// tcgen05.mma (bf16, fp32 accumulation).  The three that are left out are below 2^-24 of the product.
+//
+//   arrangement   M operand (128), fp32, split on the way       N operand (up to 128), three bf16 planes
+//   kFwd          W[e][k][m]   weight columns                   rows of the expert, K-major
+//   kDgrad        W[e][m][k]   weight rows                      rows of the expert, K-major
+//   kWgrad        grad[r][m]   columns, k = rows                act[r][n] columns, MN-major
+//
+// Why this split.  The CUDA cores bound the previous kernel (128 x 128 tile, FFMA) at 33 of 74.5
+// TFLOP/s; six bf16 products cost a sixth of the tensor rate, some 270 TFLOP/s.  Splitting costs
+// about ten instructions per element, so each side is split where it is cheapest: activations once, by
+// the kernel that produces them (three planes instead of one fp32 matrix); weights, which are far
+// larger and read by few tiles, by the GEMM itself.  The weight tile arrives as fp32 by TMA, eight
+// converter warps read it from shared memory, and write the three parts straight into TMEM, from where
+// tcgen05.mma takes its A operand: the parts never touch shared memory, whose bandwidth the B operand
+// and the fp32 tile already need.
+//
+// Precision.  The tensor core adds to an accumulator by truncation, whose errors would add up over a
+// long reduction.  Each 64-deep k-block therefore starts a fresh accumulator, takes the small
+// products first and the leading one last, and the block's sum is added to a running sum in registers
+// with round-to-nearest.  Against 64 bits the README forward is 3.9e-7 off where the FFMA kernel's serial
+// sum is 1.6e-6, the gradients of 600 tokens (H = 1024) at most 3.5e-7 against 1.1e-6.
+//
+// Measured: gate_up of the README forward (T = 512, H = 2880, E = 8, K = 2) 281 us = 121 TFLOP/s of the
+// original product; the whole forward 524 us against 1913, a training step of 600 tokens 466 against 1191.
+//
+// Infinities and NaN behave as in fp32 arithmetic: see split3_mag.
+//
+// A CTA has 20 warps: TMA producer, MMA issuer, two that only complete the warpgroup, eight
+// converters (two per TMEM lane quarter, 32 k each) and eight accumulator / epilogue warps (two per
+// lane quarter, 64 columns each).  Shared
+// memory: three stages of weights (32 KB) and two of activations (48 KB); TMEM: two accumulators of
+// 128 columns, two A operands of 96.  Every wait is bounded as in umma_gemm.cuh.
+#pragma once
+#include "misc_kernels.cuh"
+#include "umma_gemm.cuh"
+
+namespace yb {
+
+constexpr int kF32Threads = 640;
+constexpr int kF32ConvWarps = 8, kF32AccWarps = 8;
+constexpr int kF32M = 128, kF32N = 128, kF32K = 64;
+constexpr int kF32WBytes = kF32M * kF32K * 4;            // 32 KB: fp32 tile of the M operand
+constexpr int kF32PlaneBytes = kF32N * kF32K * 2;        // 16 KB: one part of the N operand
+constexpr int kF32BBytes = 3 * kF32PlaneBytes;
+constexpr int kF32WStages = 3, kF32BStages = 2;
+constexpr int kF32Smem = kF32WStages * kF32WBytes + kF32BStages * kF32BBytes + 1024;
+constexpr int kF32TmemA = 256;                           // first TMEM column of the A operands
+constexpr int kF32TmemAStride = 96;                      // 3 parts x 32 columns (64 bf16)
+
+// The three parts of |x| (value bits in the upper half of the words; the sign is put back by the
+// caller): a, b, c with a + b + c = |x|, exactly for normal numbers.  A part that would be zero is
+// |x| * 2^-40 instead (zero for x = 0): an infinite operand then meets no zero part of a finite
+// non-zero one, so that inf * y is inf and not NaN; for x = inf all parts are inf, for NaN b and c are.
+__device__ __forceinline__ void split3_mag(float x, uint32_t& b, uint32_t& c) {
+  const float ax = fabsf(x);
+  const float tiny = ax * 9.094947017729282e-13f;        // 2^-40
+  const float a = __uint_as_float(__float_as_uint(ax) & 0xffff0000u);
+  const float r = ax - a;
+  const float bf = __uint_as_float(__float_as_uint(r) & 0xffff0000u);
+  b = __float_as_uint(fmaxf(bf, tiny));
+  c = __float_as_uint(fmaxf(r - bf, tiny));
+}
+
+// bf16 pairs (x0 in the low half) of the three parts of two numbers
+__device__ __forceinline__ void split3_pair(float x0, float x1, uint32_t& p0, uint32_t& p1, uint32_t& p2) {
+  uint32_t b0, c0, b1, c1;
+  split3_mag(x0, b0, c0);
+  split3_mag(x1, b1, c1);
+  p0 = __byte_perm(__float_as_uint(x0), __float_as_uint(x1), 0x7632);
+  const uint32_t sign = p0 & 0x80008000u;
+  p1 = __byte_perm(b0, b1, 0x7632) | sign;
+  p2 = __byte_perm(c0, c1, 0x7632) | sign;
+}
+
+// Where an activation matrix is kept as three bf16 planes: [3][rows][ld].
+struct Planes {
+  __nv_bfloat16* p;
+  int64_t stride;                   // elements between planes
+  int ld;
+  __device__ __forceinline__ void store1(size_t row, int col, float x) const {
+    uint32_t p0, p1, p2;
+    split3_pair(x, 0.f, p0, p1, p2);
+    unsigned short* d = reinterpret_cast<unsigned short*>(p) + row * ld + col;
+    d[0] = (unsigned short)p0;
+    d[stride] = (unsigned short)p1;
+    d[2 * stride] = (unsigned short)p2;
+  }
+  // two adjacent columns, col even
+  __device__ __forceinline__ void store2(size_t row, int col, float x0, float x1) const {
+    uint32_t q0, q1, q2;
+    split3_pair(x0, x1, q0, q1, q2);
+    __nv_bfloat16* d = p + row * ld + col;
+    *reinterpret_cast<uint32_t*>(d) = q0;
+    *reinterpret_cast<uint32_t*>(d + stride) = q1;
+    *reinterpret_cast<uint32_t*>(d + 2 * stride) = q2;
+  }
+};
+
+// Gather of the token rows into the padded layout, as planes (see gather_rows_kernel; the columns
+// from H to ld are (1, 0, 0, ...) for token rows).
+__global__ void __launch_bounds__(kRowWarps * 32)
+gather_split_kernel(const float* __restrict__ src, Planes dst, const int32_t* __restrict__ row_token,
+                    const int32_t* __restrict__ header, int H) {
+  const int row = blockIdx.x * kRowWarps + (threadIdx.x >> 5);
+  if (row >= header[kHdrRowsUsed]) return;
+  const int lane = threadIdx.x & 31;
+  const int tok = row_token[row];
+  const float4* s = reinterpret_cast<const float4*>(src + (size_t)(tok < 0 ? 0 : tok) * H);
+  for (int i = lane; i < dst.ld / 4; i += 32) {
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (tok >= 0) {
+      if (4 * i < H) v = __ldg(s + i);
+      else if (4 * i == H) v.x = 1.f;
+    }
+    uint2 q[3];
+    split3_pair(v.x, v.y, q[0].x, q[1].x, q[2].x);
+    split3_pair(v.z, v.w, q[0].y, q[1].y, q[2].y);
+    __nv_bfloat16* d = dst.p + (size_t)row * dst.ld + 4 * i;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) *reinterpret_cast<uint2*>(d + k * dst.stride) = q[k];
+  }
+}
+
+// Gather of the upstream gradient: fp32 rows (M operand of the down weight gradient) and planes (N
+// operand of the data gradient); seeds the routing-weight gradient as gather_grad_kernel does.
+__global__ void __launch_bounds__(kRowWarps * 32)
+gather_grad_split_kernel(const float* __restrict__ grad_out, int slots, const float* __restrict__ down_bias,
+                         float* __restrict__ gys, Planes dst, float* __restrict__ gw_row,
+                         const int32_t* __restrict__ row_token, const int32_t* __restrict__ tile_expert,
+                         const int32_t* __restrict__ header, int H) {
+  const int row = blockIdx.x * kRowWarps + (threadIdx.x >> 5);
+  if (row >= header[kHdrRowsUsed]) return;
+  const int lane = threadIdx.x & 31;
+  const int tok = row_token[row];
+  const float* bias = down_bias + (size_t)tile_expert[row / kTileM] * H;
+  float dot = 0.f;
+  for (int i = lane; i < H / 4; i += 32) {
+    float g[4] = {0.f, 0.f, 0.f, 0.f};
+    if (tok >= 0) {
+      float g2[4], b[4];
+      for (int s = 0; s < slots; ++s) {
+        load_vec<float, 4>(grad_out + ((size_t)tok * slots + s) * H + 4 * (size_t)i, g2);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) g[j] = s == 0 ? g2[j] : g[j] + g2[j];
+      }
+      load_vec<float, 4>(bias + 4 * (size_t)i, b);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) dot += g[j] * b[j];
+    }
+    store_vec<float, 4>(gys + (size_t)row * H + 4 * (size_t)i, g);
+    dst.store2(row, 4 * i, g[0], g[1]);
+    dst.store2(row, 4 * i + 2, g[2], g[3]);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+  if (lane == 0) gw_row[row] = dot;
+}
+
+// ---------------------------------------------------------------------------------------------
+// Epilogues: a warp holds 32 consecutive M indices (lane L: m) for 16 consecutive N indices,
+//     epi.apply(e, m, row, nvalid, lane, v)      v[i] = C[row + i][m]; only i < nvalid exist
+// ---------------------------------------------------------------------------------------------
+// Neighbouring columns to one lane: the even lane gets (m, m+1) of rows 0..7, the odd lane
+// (m-1, m) of rows 8..15.
+__device__ __forceinline__ void pair_columns16(const float (&v)[16], bool odd, float (&lo)[8], float (&hi)[8]) {
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const float got = __shfl_xor_sync(0xffffffffu, odd ? v[i] : v[8 + i], 1);
+    lo[i] = odd ? got : v[i];
+    hi[i] = odd ? v[8 + i] : got;
+  }
+}
+
+// routing weight of row `row + lane` (0 for padding and beyond nvalid) and the ballot of token rows
+__device__ __forceinline__ unsigned row_info(const int32_t* row_token, const float* row_weight, int row, int nvalid,
+                                             int lane, float& w_lane) {
+  bool real = false;
+  w_lane = 0.f;
+  if (lane < nvalid) {
+    real = row_token[row + lane] >= 0;
+    if (real && row_weight != nullptr) w_lane = row_weight[row + lane];
+  }
+  return __ballot_sync(0xffffffffu, real);
+}
+
+template <bool TRAIN>
+struct F32Glu {                     // see PairGlu
+  const float* bias;               // [E, 2H]
+  Planes act;                      // [3][rows][H] or null (TRAIN)
+  Planes actw;                     // TRAIN: [3][rows][ld]
+  float* pre;                      // TRAIN: [rows, 2H]
+  const int32_t* row_token;
+  const float* row_weight;         // TRAIN
+  int H;
+
+  __device__ __forceinline__ void apply(int e, int m, int row, int nvalid, int lane, const float (&v)[16]) const {
+    const bool odd = lane & 1;
+    const float b = bias[(size_t)e * 2 * H + m];
+    float x[16], g[8], u[8];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) x[i] = v[i] + b;
+    pair_columns16(x, odd, g, u);
+    const int t0 = odd ? 8 : 0, j = m >> 1;
+    float w_lane;
+    const unsigned have = row_info(row_token, TRAIN ? row_weight : nullptr, row, nvalid, lane, w_lane);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int t = t0 + i;
+      const bool ok = (have >> t) & 1u;
+      const float w = TRAIN ? __shfl_sync(0xffffffffu, w_lane, t) : 0.f;
+      const float a = ok ? glu_act(g[i], u[i]) : 0.f;
+      if (t < nvalid) {
+        if (act.p != nullptr) act.store1(row + t, j, a);
+        if constexpr (TRAIN) {
+          *reinterpret_cast<float2*>(pre + (size_t)(row + t) * 2 * H + (m & ~1)) =
+              ok ? make_float2(g[i], u[i]) : make_float2(0.f, 0.f);
+          actw.store1(row + t, j, a * w);
+        }
+      }
+    }
+    if constexpr (TRAIN) {
+      if (m == lane)               // columns 0..31: this warp also fills the columns behind H with (w, 0, 0, ...)
+        for (int t = 0; t < nvalid; ++t) {
+          const float w = __shfl_sync(0xffffffffu, w_lane, t);
+          for (int c = H + 2 * lane; c < actw.ld; c += 64) actw.store2(row + t, c, c == H ? w : 0.f, 0.f);
+        }
+    }
+  }
+};
+
+struct F32WeightedRows {            // see PairWeightedRows
+  const float* bias;
+  float* y;
+  const int32_t* row_token;
+  const float* row_weight;
+  int N;
+
+  __device__ __forceinline__ void apply(int e, int m, int row, int nvalid, int lane, const float (&v)[16]) const {
+    const float b = bias[(size_t)e * N + m];
+    float w_lane;
+    const unsigned have = row_info(row_token, row_weight, row, nvalid, lane, w_lane);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const float w = __shfl_sync(0xffffffffu, w_lane, i);
+      if ((have >> i) & 1u) y[(size_t)(row + i) * N + m] = w * (b + v[i]);
+    }
+  }
+};
+
+struct F32ScatterAdd {              // see PairScatterAdd
+  float* dst;
+  const int32_t* row_token;
+  int N;
+
+  __device__ __forceinline__ void apply(int, int m, int row, int nvalid, int lane, const float (&v)[16]) const {
+    const bool odd = lane & 1;
+    const int tok_lane = lane < nvalid ? row_token[row + lane] : -1;
+    float lo[8], hi[8];
+    pair_columns16(v, odd, lo, hi);
+    const int t0 = odd ? 8 : 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int tok = __shfl_sync(0xffffffffu, tok_lane, t0 + i);
+      if (tok >= 0) atomicAdd(reinterpret_cast<float2*>(dst + (size_t)tok * N + (m & ~1)), make_float2(lo[i], hi[i]));
+    }
+  }
+};
+
+struct F32GluBackward {             // see PairGluBackward; the gradient leaves as fp32 rows and as planes
+  const float* pre;                // [rows, 2H]
+  float* g_pre;                    // [rows, 2H]
+  Planes g_planes;                 // [3][rows][2H]
+  float* gw_row;
+  const int32_t* row_token;
+  const float* row_weight;
+  int H;
+
+  __device__ __forceinline__ void apply(int, int m, int row, int nvalid, int lane, const float (&v)[16]) const {
+    float w_lane, dot[16];
+    const unsigned have = row_info(row_token, row_weight, row, nvalid, lane, w_lane);
+    const float2* src = reinterpret_cast<const float2*>(pre) + (size_t)row * H + m;
+    float2* dst = reinterpret_cast<float2*>(g_pre) + (size_t)row * H + m;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const bool ok = (have >> i) & 1u;
+      const float2 q = ok ? __ldg(src + (size_t)i * H) : make_float2(0.f, 0.f);
+      const float w = __shfl_sync(0xffffffffu, w_lane, i);
+      const float pg = q.x, pu = q.y;
+      const float gc = fminf(pg, kLimit);
+      const float uc = fminf(fmaxf(pu, -kLimit), kLimit);
+      const float s = __fdividef(1.0f, 1.0f + __expf(-kAlpha * gc));
+      const float gate_act = gc * s;
+      dot[i] = ok ? v[i] * (uc + 1.0f) * gate_act : 0.f;
+      const float gi = w * v[i];
+      float gu = gi * gate_act;
+      float gg = gi * (uc + 1.0f) * (s + gc * s * (1.0f - s) * kAlpha);
+      if (pg > kLimit || !ok) gg = 0.f;
+      if (pu > kLimit || pu < -kLimit || !ok) gu = 0.f;
+      if (i < nvalid) {
+        dst[(size_t)i * H] = make_float2(gg, gu);
+        g_planes.store2(row + i, 2 * m, gg, gu);
+      }
+    }
+    // lane L ends with half the sum of row L & 15, its partner L ^ 16 with the other half
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) {
+      const bool up = lane & o;
+#pragma unroll
+      for (int i = 0; i < o; ++i) {
+        const float got = __shfl_xor_sync(0xffffffffu, up ? dot[i] : dot[i + o], o);
+        dot[i] = (up ? dot[i + o] : dot[i]) + got;
+      }
+    }
+    dot[0] += __shfl_xor_sync(0xffffffffu, dot[0], 16);
+    if (lane < 16 && ((have >> lane) & 1u)) atomicAdd(gw_row + row + lane, dot[0]);
+  }
+};
+
+struct F32StoreBias {               // see PairStoreBias
+  float* C;
+  float* bias_out;
+  int H, ld;
+
+  __device__ __forceinline__ void apply(int e, int m, int row, int, int, const float (&v)[16]) const {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const int n = row + i;
+      if (n < H) C[((size_t)e * H + n) * ld + m] = v[i];
+      else if (n == H) bias_out[(size_t)e * ld + m] = v[i];
+    }
+  }
+};
+
+struct F32Params {
+  int M, N, K, E;
+  int row_round;                   // see PairParams
+  const int32_t* tile_expert;
+  const int32_t* pad_off;
+  const int32_t* counts;
+  int32_t* header;
+};
+
+// tcgen05.mma with the A operand in TMEM
+__device__ __forceinline__ void tc_mma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
+                                               uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %6, %7, %8}, p;\n\t}"
+      ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(0u), "r"(0u), "r"(0u), "r"(0u)
+      : "memory");
+}
+__device__ __forceinline__ void tc_st_32x8(uint32_t taddr, const uint32_t (&r)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%8], {%0, %1, %2, %3, %4, %5, %6, %7};"
+               ::"r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(taddr)
+               : "memory");
+}
+__device__ __forceinline__ void tc_ld_32x16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n\t"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void tc_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+template <int MODE, class Epi>
+__global__ void __launch_bounds__(kF32Threads, 1)
+umma_f32_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__ CUtensorMap tmN,
+                const __grid_constant__ CUtensorMap tmNsmall, const F32Params p, const Epi epi) {
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ __align__(8) uint64_t bar_w_full[kF32WStages], bar_w_empty[kF32WStages];
+  __shared__ __align__(8) uint64_t bar_b_full[kF32BStages], bar_b_empty[kF32BStages];
+  __shared__ __align__(8) uint64_t bar_a_full[2], bar_a_empty[2];
+  __shared__ __align__(8) uint64_t bar_acc_full[2], bar_acc_empty[2];
+  __shared__ uint32_t tmem_base_slot;
+  __shared__ int abort_flag;
+  __shared__ int32_t s_pad[kUmmaMaxExperts + 1];
+  __shared__ int32_t s_rows[kUmmaMaxExperts];
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  const uint32_t smem_b = smem_base + kF32WStages * kF32WBytes;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kF32WStages; ++s) {
+      mbar_init(smem_u32(&bar_w_full[s]), 1);
+      mbar_init(smem_u32(&bar_w_empty[s]), kF32ConvWarps);
+    }
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(smem_u32(&bar_b_full[s]), 1);
+      mbar_init(smem_u32(&bar_b_empty[s]), 1);
+      mbar_init(smem_u32(&bar_a_full[s]), kF32ConvWarps);
+      mbar_init(smem_u32(&bar_a_empty[s]), 1);
+      mbar_init(smem_u32(&bar_acc_full[s]), 1);
+      mbar_init(smem_u32(&bar_acc_empty[s]), kF32AccWarps);
+    }
+    abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+                 ::"r"(smem_u32(&tmem_base_slot)), "r"(512u) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  for (int i = threadIdx.x; i <= p.E; i += kF32Threads) {
+    const int p0 = p.pad_off[i];
+    s_pad[i] = p0;
+    if (i < p.E) {
+      const int have = min(p.counts[i], p.pad_off[i + 1] - p0);
+      s_rows[i] = (have + p.row_round - 1) & ~(p.row_round - 1);
+    }
+  }
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = tmem_base_slot;
+
+  const int MT = (p.M + kF32M - 1) / kF32M;
+  const int NT = (p.N + kF32N - 1) / kF32N;       // kWgrad
+  const int total = MODE == kWgrad ? p.E * MT * NT : p.header[kHdrRowTiles] * MT;
+  auto expert_of = [&](int id) -> int {
+    if constexpr (MODE == kWgrad) return 0;
+    return id < total ? __ldg(p.tile_expert + id / MT) : 0;
+  };
+  // as in umma_pair.cuh, with tiles of up to 128 rows / columns
+  auto decode = [&](int id, int e_hint, int& e, int& m0, int& n0, int& width, int& kblocks) {
+    if constexpr (MODE == kWgrad) {
+      e = id / (MT * NT);
+      const int rem = id - e * (MT * NT);
+      const int nt = rem / MT;
+      m0 = (rem - nt * MT) * kF32M;
+      n0 = nt * kF32N;
+      width = (min(kF32N, p.N - n0) + 15) & ~15;
+      kblocks = s_rows[e] / kF32K;
+    } else {
+      e = e_hint;
+      const int first = s_pad[e] / kTileM;
+      const int cnt = s_pad[e + 1] / kTileM - first;
+      const int local = id - first * MT;
+      const int mt = local / cnt;
+      const int rows = s_rows[e];
+      const int step = ((rows + cnt - 1) / cnt + 15) & ~15;
+      const int off = (local - mt * cnt) * step;
+      m0 = mt * kF32M;
+      n0 = s_pad[e] + off;
+      width = min(step, rows - off);
+      kblocks = p.K / kF32K;
+    }
+  };
+  auto give_up = [&](int status) {
+    abort_flag = 1;
+    atomicMax(p.header + kHdrStatus, status);
+  };
+
+  if (warp < 4) {
+  if (warp == 0) {
+    // =========================== TMA producer ================================================
+    if (lane == 0) {
+      int ws = 0, bs = 0;
+      uint32_t wph = 0, bph = 0;
+      bool ok = true;
+      // weights run one k-block ahead of the activations (they are released earlier)
+      int w_id = blockIdx.x, w_kb = 0;
+      int w_e = 0, w_m0 = 0, w_n0 = 0, w_width = 0, w_kblocks = 0;
+      auto w_open = [&]() {                         // next work item that has k-blocks
+        while (w_id < total) {
+          decode(w_id, expert_of(w_id), w_e, w_m0, w_n0, w_width, w_kblocks);
+          if (w_kblocks > 0) return;
+          w_id += gridDim.x;
+        }
+      };
+      auto w_issue = [&]() -> bool {
+        if (w_id >= total) return true;
+        if (!mbar_wait(smem_u32(&bar_w_empty[ws]), wph ^ 1u, &abort_flag)) return false;
+        const uint32_t full = smem_u32(&bar_w_full[ws]);
+        const uint32_t sw = smem_base + ws * kF32WBytes;
+        const int k0 = w_kb * kF32K;
+        mbar_expect_tx(full, kF32WBytes);
+        if constexpr (MODE == kFwd) {
+          tma_load_3d(sw, &tmM, w_m0, k0, w_e, full);
+        } else if constexpr (MODE == kDgrad) {
+          tma_load_3d(sw, &tmM, k0, w_m0, w_e, full);
+          tma_load_3d(sw + kF32WBytes / 2, &tmM, k0 + 32, w_m0, w_e, full);
+        } else {
+          tma_load_2d(sw, &tmM, w_m0, s_pad[w_e] + k0, full);
+        }
+        if (++ws == kF32WStages) { ws = 0; wph ^= 1u; }
+        if (++w_kb == w_kblocks) {
+          w_kb = 0;
+          w_id += gridDim.x;
+          w_open();
+        }
+        return true;
+      };
+      w_open();
+      ok = w_issue();
+      for (int id = blockIdx.x; id < total && ok; id += gridDim.x) {
+        int e, m0, n0, width, kblocks;
+        decode(id, expert_of(id), e, m0, n0, width, kblocks);
+        const bool big = width > 64;
+        const uint32_t bytes = big ? kF32BBytes : kF32BBytes / 2;
+        for (int kb = 0; kb < kblocks; ++kb) {
+          ok = w_issue() && mbar_wait(smem_u32(&bar_b_empty[bs]), bph ^ 1u, &abort_flag);
+          if (!ok) break;
+          const uint32_t full = smem_u32(&bar_b_full[bs]);
+          const uint32_t sb = smem_b + bs * kF32BBytes;
+          const CUtensorMap* map = big ? &tmN : &tmNsmall;
+          mbar_expect_tx(full, bytes);
+          if constexpr (MODE == kWgrad) tma_load_4d(sb, map, 0, s_pad[e] + kb * kF32K, n0 >> 6, 0, full);
+          else tma_load_3d(sb, map, kb * kF32K, n0, 0, full);
+          if (++bs == kF32BStages) { bs = 0; bph ^= 1u; }
+        }
+      }
+      if (!ok) give_up(kStatusProducerTimeout);
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    // =========================== MMA issuer ==================================================
+    if (lane == 0) {
+      constexpr bool kBMn = MODE == kWgrad;
+      constexpr uint32_t idesc_base = (1u << 4) | (1u << 7) | (1u << 10) | ((kBMn ? 1u : 0u) << 16) |
+                                      ((uint32_t)(kF32M >> 4) << 24);
+      constexpr uint32_t b_kstep = kBMn ? (16 * 128) >> 4 : 32 >> 4;
+      // parts (of M operand, of N operand), smallest products first
+      constexpr int kPartA[6] = {0, 2, 1, 0, 1, 0}, kPartB[6] = {2, 0, 1, 1, 0, 0};
+      int slot = 0;                                  // A operand, B stage and accumulator alike: two of each
+      uint32_t phase = 0;
+      bool ok = true;
+      int e_next = expert_of(blockIdx.x);
+      for (int id = blockIdx.x; id < total && ok; id += gridDim.x) {
+        int e, m0, n0, width, kblocks;
+        decode(id, e_next, e, m0, n0, width, kblocks);
+        e_next = expert_of(id + gridDim.x);
+        const uint32_t idesc = idesc_base | ((uint32_t)(width >> 3) << 17);
+        const uint32_t plane = width > 64 ? kF32PlaneBytes : kF32PlaneBytes / 2;
+        for (int kb = 0; kb < kblocks; ++kb) {
+          ok = mbar_wait(smem_u32(&bar_acc_empty[slot]), phase ^ 1u, &abort_flag) &&
+               mbar_wait(smem_u32(&bar_b_full[slot]), phase, &abort_flag) &&
+               mbar_wait(smem_u32(&bar_a_full[slot]), phase, &abort_flag);
+          if (!ok) break;
+          tc_fence_after();
+          const uint32_t d = tmem_base + slot * kF32N;
+          const uint32_t a0 = tmem_base + kF32TmemA + slot * kF32TmemAStride;
+          const uint32_t sb = smem_b + slot * kF32BBytes;
+#pragma unroll
+          for (int q = 0; q < 6; ++q) {
+            const uint32_t addr = sb + kPartB[q] * plane;
+            const uint64_t bdesc = kBMn ? make_smem_desc(addr, 8192, 1024) : make_smem_desc(addr, 16, 1024);
+#pragma unroll
+            for (int k = 0; k < kF32K / 16; ++k)
+              tc_mma_bf16_ts(d, a0 + kPartA[q] * 32 + k * 8, bdesc + (uint64_t)(k * b_kstep), idesc,
+                             (uint32_t)((q | k) != 0));
+          }
+          tc_commit(smem_u32(&bar_a_empty[slot]));
+          tc_commit(smem_u32(&bar_b_empty[slot]));
+          tc_commit(smem_u32(&bar_acc_full[slot]));
+          slot ^= 1;
+          if (slot == 0) phase ^= 1u;
+        }
+      }
+      if (!ok) give_up(kStatusMmaTimeout);
+    }
+    __syncwarp();
+  }
+  } else if (warp < 4 + kF32ConvWarps) {
+    // =========================== converters: fp32 tile -> three parts in TMEM ================
+    const int q = warp & 3, khalf = (warp - 4) >> 2;
+    const int mrow = q * 32 + lane;
+    int ws = 0, slot = 0;
+    uint32_t wph = 0, phase = 0;
+    bool ok = true;
+    int e_next = expert_of(blockIdx.x);
+    for (int id = blockIdx.x; id < total && ok; id += gridDim.x) {
+      int e, m0, n0, width, kblocks;
+      decode(id, e_next, e, m0, n0, width, kblocks);
+      e_next = expert_of(id + gridDim.x);
+      for (int kb = 0; kb < kblocks; ++kb) {
+        ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_w_full[ws]), wph, &abort_flag));
+        if (!ok) break;
+        ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_a_empty[slot]), phase ^ 1u, &abort_flag));
+        if (!ok) break;
+        tc_fence_after();
+        const uint8_t* tile = smem_raw + (smem_base - smem_u32(smem_raw)) + ws * kF32WBytes;
+        const uint32_t t = tmem_base + kF32TmemA + slot * kF32TmemAStride + khalf * 16 + ((uint32_t)(q * 32) << 16);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {                // 16 k at a time
+          uint32_t p0[8], p1[8], p2[8];
+          if constexpr (MODE == kDgrad) {
+            // 32 k of row mrow: 128 bytes, 16-byte pieces swizzled by the row
+            const uint8_t* rowp = tile + khalf * (kF32WBytes / 2) + mrow * 128;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const float4 x = *reinterpret_cast<const float4*>(rowp + (((h * 4 + i) ^ (mrow & 7)) << 4));
+              split3_pair(x.x, x.y, p0[2 * i], p1[2 * i], p2[2 * i]);
+              split3_pair(x.z, x.w, p0[2 * i + 1], p1[2 * i + 1], p2[2 * i + 1]);
+            }
+          } else {
+            const float* colp = reinterpret_cast<const float*>(tile) + (khalf * 32 + h * 16) * kF32M + mrow;
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+              split3_pair(colp[2 * i * kF32M], colp[(2 * i + 1) * kF32M], p0[i], p1[i], p2[i]);
+          }
+          tc_st_32x8(t + h * 8, p0);
+          tc_st_32x8(t + h * 8 + 32, p1);
+          tc_st_32x8(t + h * 8 + 64, p2);
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&bar_w_empty[ws]));
+        if (++ws == kF32WStages) { ws = 0; wph ^= 1u; }
+        tc_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&bar_a_full[slot]));
+        slot ^= 1;
+        if (slot == 0) phase ^= 1u;
+      }
+    }
+    if (!ok) give_up(kStatusMmaTimeout);
+    __syncwarp();
+  } else {
+    // =========================== accumulators and epilogue ===================================
+    const int q = warp & 3, nhalf = (warp - 4 - kF32ConvWarps) >> 2;
+    int slot = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    int e_next = expert_of(blockIdx.x);
+    for (int id = blockIdx.x; id < total && ok; id += gridDim.x) {
+      int e, m0, n0, width, kblocks;
+      decode(id, e_next, e, m0, n0, width, kblocks);
+      e_next = expert_of(id + gridDim.x);
+      const int cols = min(64, width - nhalf * 64);  // of this warp; <= 0: none
+      float acc[64];
+#pragma unroll
+      for (int i = 0; i < 64; ++i) acc[i] = 0.f;
+      for (int kb = 0; kb < kblocks; ++kb) {
+        ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_acc_full[slot]), phase, &abort_flag));
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t t = tmem_base + slot * kF32N + nhalf * 64 + ((uint32_t)(q * 32) << 16);
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+          if (c * 16 < cols) {
+            uint32_t r[16];
+            tc_ld_32x16(t + c * 16, r);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) acc[c * 16 + i] += __uint_as_float(r[i]);
+          }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&bar_acc_empty[slot]));
+        slot ^= 1;
+        if (slot == 0) phase ^= 1u;
+      }
+      if (!ok) break;
+      const int m = m0 + q * 32 + lane;
+      if (m - lane < p.M) {                          // M is a multiple of 32
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+          if (c * 16 < cols) {
+            float v[16];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) v[i] = acc[c * 16 + i];
+            epi.apply(e, m, n0 + nhalf * 64 + c * 16, min(16, cols - c * 16), lane, v);
+          }
+      }
+    }
+    if (!ok) give_up(kStatusEpilogueTimeout);
+    __syncwarp();
+  }
+
+  // ---- teardown ---------------------------------------------------------------------------
+  tc_fence_before();
+  __syncthreads();
+  if (abort_flag != 0) {
+    // give copies that may still be in flight time to land before the shared memory is released
+    const uint64_t t0 = global_timer_ns();
+    while (global_timer_ns() - t0 < 2000000ull) __nanosleep(1000);
+    __syncthreads();
+  }
+  if (warp == 1) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
+  }
+}
+
+// GemmArgs as for launch_umma_pair: A / lda describe the planes (N operand; `a_plane` elements
+// between planes), B / ldb the fp32 operand.  All widths and pitches are multiples of 64.
+template <int MODE, class Epi>
+inline int launch_umma_f32(const GemmArgs& g, int64_t a_plane, const Epi& epi, int64_t max_rows, int64_t max_tiles,
+                           int row_round, cudaStream_t stream) {
+  if (!umma_available() || g.E > kUmmaMaxExperts) return YAMOE_ERR_UNSUPPORTED;
+  CUtensorMap tmM, tmN, tmNs;
+  bool ok = true;
+  if (MODE == kWgrad) {
+    const uint64_t dn[4] = {64, (uint64_t)max_rows, (uint64_t)g.lda / 64, 3};
+    const uint64_t sn[3] = {(uint64_t)g.lda * 2, 128, (uint64_t)a_plane * 2};
+    const uint32_t b2[4] = {64, 64, 2, 3}, b1[4] = {64, 64, 1, 3};
+    ok = make_map(&tmN, g.A, 4, dn, sn, b2) && make_map(&tmNs, g.A, 4, dn, sn, b1);
+    const uint64_t dm[2] = {(uint64_t)g.N, (uint64_t)max_rows}, sm[1] = {(uint64_t)g.ldb * 4};
+    const uint32_t bm[2] = {kF32M, kF32K};
+    ok = ok && make_map(&tmM, g.B, 2, dm, sm, bm, kMapF32);
+  } else {
+    const uint64_t dn[3] = {(uint64_t)g.K, (uint64_t)max_rows, 3};
+    const uint64_t sn[2] = {(uint64_t)g.lda * 2, (uint64_t)a_plane * 2};
+    const uint32_t b128[3] = {64, 128, 3}, b64[3] = {64, 64, 3};
+    ok = make_map(&tmN, g.A, 3, dn, sn, b128) && make_map(&tmNs, g.A, 3, dn, sn, b64);
+    const uint64_t sm[2] = {(uint64_t)g.ldb * 4, (uint64_t)g.b_expert_stride * 4};
+    if (MODE == kFwd) {
+      const uint64_t dm[3] = {(uint64_t)g.N, (uint64_t)g.K, (uint64_t)g.E};
+      const uint32_t bm[3] = {kF32M, kF32K, 1};
+      ok = ok && make_map(&tmM, g.B, 3, dm, sm, bm, kMapF32);
+    } else {
+      const uint64_t dm[3] = {(uint64_t)g.K, (uint64_t)g.N, (uint64_t)g.E};
+      const uint32_t bm[3] = {32, kF32M, 1};
+      ok = ok && make_map(&tmM, g.B, 3, dm, sm, bm, kMapF32Swizzled);
+    }
+  }
+  if (!ok) return YAMOE_ERR_CUDA;
+  auto kern = umma_f32_kernel<MODE, Epi>;
+  static PerDevice<int> attr_done;   // per template instantiation and device
+  const int dev = current_device_index();
+  if (!attr_done.get(dev)) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kF32Smem) != cudaSuccess)
+      return YAMOE_ERR_CUDA;
+    attr_done.set(dev, 1);
+  }
+  const F32Params p{g.N, g.M, g.K, g.E, row_round, g.tile_expert, g.pad_off, g.counts, const_cast<int32_t*>(g.header)};
+  const int64_t MT = ceil_div(g.N, kF32M);
+  const int64_t total_max = MODE == kWgrad ? (int64_t)g.E * MT * ceil_div(g.M, kF32N) : max_tiles * MT;
+  const int grid = (int)std::min<int64_t>(total_max, umma_sm_count());
+  if (grid <= 0) return YAMOE_OK;
+  kern<<<grid, kF32Threads, kF32Smem, stream>>>(tmM, tmN, tmNs, p, epi);
+  return cudaGetLastError() == cudaSuccess ? YAMOE_OK : YAMOE_ERR_CUDA;
+}
+
+}  // namespace yb

@@ -786,17 +786,18 @@ inline bool umma_available() {
   return m - 1 == 10;
 }
 
-// bf16 tensor map with 128-byte swizzle; dims / box innermost first, strides in bytes for dims 1...
+// Tensor map (bf16 with 128-byte swizzle, or see MapKind); dims / box innermost first, strides in bytes for dims 1...
 // Encoding a map is a driver call that costs some tens of microseconds of host time; the same
 // (pointer, shape, box) comes back call after call (weights, persistent buffers, workspaces that the
 // caching allocator hands out again), so the last maps are kept in a small table.
+enum MapKind { kMapBf16 = 0, kMapF32 = 1, kMapF32Swizzled = 2 };   // fp32 tiles: plain, or 128-byte swizzle
 struct TensorMapKey {
   const void* base;
-  int rank;
+  int rank, kind;
   uint64_t dims[4], strides[3];
   uint32_t box[4];
   bool operator==(const TensorMapKey& o) const {
-    if (base != o.base || rank != o.rank) return false;
+    if (base != o.base || rank != o.rank || kind != o.kind) return false;
     for (int i = 0; i < rank; ++i)
       if (dims[i] != o.dims[i] || box[i] != o.box[i]) return false;
     for (int i = 0; i + 1 < rank; ++i)
@@ -806,8 +807,8 @@ struct TensorMapKey {
 };
 
 inline bool make_map(CUtensorMap* m, const void* base, int rank, const uint64_t* dims, const uint64_t* strides,
-                     const uint32_t* box) {
-  constexpr int kSlots = 32;
+                     const uint32_t* box, int kind = kMapBf16) {
+  constexpr int kSlots = 64;
   static TensorMapKey keys[kSlots];
   static CUtensorMap maps[kSlots];
   static int used = 0, next = 0;
@@ -815,6 +816,7 @@ inline bool make_map(CUtensorMap* m, const void* base, int rank, const uint64_t*
   TensorMapKey key{};
   key.base = base;
   key.rank = rank;
+  key.kind = kind;
   for (int i = 0; i < rank; ++i) { key.dims[i] = dims[i]; key.box[i] = box[i]; }
   for (int i = 0; i + 1 < rank; ++i) key.strides[i] = strides[i];
   {
@@ -827,8 +829,9 @@ inline bool make_map(CUtensorMap* m, const void* base, int rank, const uint64_t*
   cuuint32_t bx[4], es[4] = {1, 1, 1, 1};
   for (int i = 0; i < rank; ++i) { gd[i] = dims[i]; bx[i] = box[i]; }
   for (int i = 0; i + 1 < rank; ++i) gs[i] = strides[i];
-  CUresult r = encode_tiled_fn()(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)rank, const_cast<void*>(base), gd,
-                                 gs, bx, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+  CUresult r = encode_tiled_fn()(m, kind == kMapBf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32,
+                                 (cuuint32_t)rank, const_cast<void*>(base), gd, gs, bx, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                 kind == kMapF32 ? CU_TENSOR_MAP_SWIZZLE_NONE : CU_TENSOR_MAP_SWIZZLE_128B,
                                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return false;
   std::lock_guard<std::mutex> lock(mu);
