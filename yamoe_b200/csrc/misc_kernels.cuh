@@ -165,33 +165,46 @@ __global__ void routing_grad_kernel(const float* __restrict__ gw_row, const int3
 // out[t, :] = sum over the kept slots k of y[flat_row[t*K + k], :]   (rows already weighted).
 // Second half of the combine (reference: csrc/scatter.cu:67-108): fp32 accumulation in slot
 // order, one rounding, every output element written exactly once (no zero-fill, no atomics).
-template <typename T>
+// One warp per token and 32 16-byte pieces of its row, with the loads of up to KB slots in flight: latency bounds the
+// few-token calls (a warp per token left most SMs idle and walked the columns one after the
+// other: 30 us at T = 64 and 512 with H = 2880, now about 5).
+template <typename T, int KB>
 __global__ void __launch_bounds__(kRowWarps * 32)
 combine_padded_kernel(const T* __restrict__ y, const int32_t* __restrict__ flat_row, T* __restrict__ out,
                       int64_t Tn, int H, int K) {
   pdl_wait();
-  const int64_t t = (int64_t)blockIdx.x * kRowWarps + (threadIdx.x >> 5);
-  if (t >= Tn) return;
-  const int lane = threadIdx.x & 31;
   constexpr int VE = 16 / (int)sizeof(T);
-  const int nvec = H / VE;
-  int32_t r[8];
-  const int kk = K < 8 ? K : 8;
-  for (int k = 0; k < kk; ++k) r[k] = flat_row[t * K + k];
-  for (int i = lane; i < nvec; i += 32) {
-    float acc[VE];
+  const int64_t t = (int64_t)blockIdx.x * kRowWarps + (threadIdx.x >> 5);
+  const int i = blockIdx.y * 32 + (threadIdx.x & 31);
+  if (t >= Tn || i >= H / VE) return;
+  float acc[VE];
 #pragma unroll
-    for (int j = 0; j < VE; ++j) acc[j] = 0.f;
-    for (int k = 0; k < K; ++k) {
-      const int32_t row = k < 8 ? r[k] : flat_row[t * K + k];
-      if (row < 0) continue;
-      float v[VE];
-      load_vec<T, VE>(y + (size_t)row * H + (size_t)i * VE, v);
+  for (int j = 0; j < VE; ++j) acc[j] = 0.f;
+  for (int k0 = 0; k0 < K; k0 += KB) {
+    int32_t r[KB];
+    float v[KB][VE];
 #pragma unroll
-      for (int j = 0; j < VE; ++j) acc[j] += v[j];
-    }
-    store_vec<T, VE>(out + (size_t)t * H + (size_t)i * VE, acc);
+    for (int k = 0; k < KB; ++k) r[k] = k0 + k < K ? __ldg(flat_row + t * K + k0 + k) : -1;
+#pragma unroll
+    for (int k = 0; k < KB; ++k)
+      if (r[k] >= 0) load_vec<T, VE>(y + (size_t)r[k] * H + (size_t)i * VE, v[k]);
+#pragma unroll
+    for (int k = 0; k < KB; ++k)
+      if (r[k] >= 0) {
+#pragma unroll
+        for (int j = 0; j < VE; ++j) acc[j] += v[k][j];
+      }
   }
+  store_vec<T, VE>(out + (size_t)t * H + (size_t)i * VE, acc);
+}
+
+template <typename T>
+inline int launch_combine(const T* y, const int32_t* flat_row, T* out, int64_t Tn, int H, int K, cudaStream_t st) {
+  const dim3 grid((unsigned)ceil_div(Tn, kRowWarps), (unsigned)ceil_div(H, 32 * (16 / (int)sizeof(T))));
+  const cudaError_t rc =
+      K <= 4 ? launch_pdl_opt(true, combine_padded_kernel<T, 4>, grid, dim3(kRowWarps * 32), 0, st, y, flat_row, out, Tn, H, K)
+             : launch_pdl_opt(true, combine_padded_kernel<T, 8>, grid, dim3(kRowWarps * 32), 0, st, y, flat_row, out, Tn, H, K);
+  return rc == cudaSuccess && cudaGetLastError() == cudaSuccess ? YAMOE_OK : YAMOE_ERR_CUDA;
 }
 
 // ---- expert-parallel helpers ---------------------------------------------------------------

@@ -285,10 +285,10 @@ inline int launch_router_forward(const void* x, const void* w_router, const void
   int32_t* header = reinterpret_cast<int32_t*>(ws);
   int32_t* tickets = reinterpret_cast<int32_t*>(reinterpret_cast<char*>(ws) + 256);
   float* logits = reinterpret_cast<float*>(reinterpret_cast<char*>(ws) + 512);
-  YB_CUDA_OK(cudaMemsetAsync(header, 0, 16 * sizeof(int32_t), st));
+  static_assert(256 + kRouterSmallMaxT * sizeof(int32_t) <= 512, "header and tickets are cleared together");
+  YB_CUDA_OK(cudaMemsetAsync(header, 0, 512, st));
   if (Tn == 0) return YAMOE_OK;
   if (Tn <= kRouterSmallMaxT) {
-    YB_CUDA_OK(cudaMemsetAsync(tickets, 0, kRouterSmallMaxT * sizeof(int32_t), st));
     router_small_kernel<T><<<dim3((unsigned)Tn, (unsigned)ceil_div(E, 8)), 256, 0, st>>>(
         reinterpret_cast<const T*>(x), reinterpret_cast<const T*>(w_router), reinterpret_cast<const T*>(b_router),
         reinterpret_cast<T*>(logits), tickets, indices, reinterpret_cast<T*>(scores), H, E, K);

@@ -169,12 +169,6 @@ static int check_common(int64_t T, int H, int E, int K, int dtype) {
   return YAMOE_OK;
 }
 
-static int prepare_routing(const Plan& p, cudaStream_t st) {
-  YB_CUDA_OK(cudaMemsetAsync(p.rt.header, 0, 16 * sizeof(int32_t), st));
-  if (p.rt.row_token) YB_CUDA_OK(cudaMemsetAsync(p.rt.row_token, 0xFF, p.row_tables_bytes, st));
-  return YAMOE_OK;
-}
-
 // YAMOE_B200_FUSED_GATHER=1 lets the gate_up GEMM of the forward fetch its A rows straight from
 // hidden_states (four extra warps per CTA copy them into the swizzled A stage with cp.async), so
 // that the permuted activations are never written to global memory.  Off by default: the GEMM fed
@@ -234,9 +228,7 @@ static int forward_f32_split(const Plan& p, const float* hidden, const float* wg
   }
   if (rc) return rc;
   StageTimer tm(kStageCombine, st);
-  combine_padded_kernel<float><<<(unsigned)ceil_div(Tn, kRowWarps), kRowWarps * 32, 0, st>>>(
-      reinterpret_cast<const float*>(p.yrows), p.rt.flat_row, out, Tn, H, K);
-  return cudaGetLastError() == cudaSuccess ? YAMOE_OK : YAMOE_ERR_CUDA;
+  return launch_combine<float>(reinterpret_cast<const float*>(p.yrows), p.rt.flat_row, out, Tn, H, K, st);
 }
 
 template <typename T>
@@ -257,11 +249,10 @@ static int forward_impl(const void* hidden, const int64_t* ridx, const void* rw,
   const bool split = dtype == YAMOE_F32 && use_split_f32(path, H, wgu, wd);
   if (!tc && !split) YB_CUDA_OK(cudaMemsetAsync(acc, 0, (size_t)Tn * H * sizeof(float), st));
 
-  int rc = prepare_routing(p, st);
-  if (rc) return rc;
+  int rc;
   {
     StageTimer tm(kStageRoute, st);
-    rc = launch_route<T>(ridx, reinterpret_cast<const T*>(rw), rcols, Tn, E, K, cap, p.rt, st);
+    rc = launch_route_rows<T>(ridx, reinterpret_cast<const T*>(rw), rcols, Tn, E, K, cap, p.rt, p.row_tables_bytes, st);
   }
   if (rc) return rc;
   if constexpr (sizeof(T) == 4) {
@@ -309,11 +300,7 @@ static int forward_impl(const void* hidden, const int64_t* ridx, const void* rw,
       }
       if (rc) return rc;
       StageTimer tm(kStageCombine, st);
-      if (launch_pdl(combine_padded_kernel<T>, dim3((unsigned)ceil_div(Tn, kRowWarps)), dim3(kRowWarps * 32), 0, st,
-                     reinterpret_cast<const T*>(p.yrows), (const int32_t*)p.rt.flat_row, reinterpret_cast<T*>(out),
-                     Tn, H, K) != cudaSuccess)
-        return YAMOE_ERR_CUDA;
-      return cudaGetLastError() == cudaSuccess ? YAMOE_OK : YAMOE_ERR_CUDA;
+      return launch_combine<T>(reinterpret_cast<const T*>(p.yrows), p.rt.flat_row, reinterpret_cast<T*>(out), Tn, H, K, st);
     }
   } else {
     {
@@ -343,9 +330,7 @@ static int forward_train_impl(const void* hidden, const int64_t* ridx, const voi
                               int K, int64_t cap, int dtype, void* ws, cudaStream_t st) {
   Plan p = plan_backward(ws, Tn, H, E, K, dtype);
   if (Tn == 0) return YAMOE_OK;
-  int rc = prepare_routing(p, st);
-  if (rc) return rc;
-  rc = launch_route<T>(ridx, reinterpret_cast<const T*>(rw), rcols, Tn, E, K, cap, p.rt, st);
+  int rc = launch_route_rows<T>(ridx, reinterpret_cast<const T*>(rw), rcols, Tn, E, K, cap, p.rt, p.row_tables_bytes, st);
   if (rc) return rc;
   const unsigned row_blocks = (unsigned)ceil_div(p.max_rows, kRowWarps);
   const int Hp = H + kBiasCols;
@@ -365,9 +350,7 @@ static int forward_train_impl(const void* hidden, const int64_t* ridx, const voi
       if ((rc = launch_umma_f32<kFwd>(pair_args(p, act.p, H, wd, H, (int64_t)H * H, 0, H, H, E), act.stride, wrows,
                                       p.max_rows, p.max_tiles, 16, st)))
         return rc;
-      combine_padded_kernel<T><<<(unsigned)ceil_div(Tn, kRowWarps), kRowWarps * 32, 0, st>>>(
-          yrows, p.rt.flat_row, reinterpret_cast<T*>(out), Tn, H, K);
-      return cudaGetLastError() == cudaSuccess ? YAMOE_OK : YAMOE_ERR_CUDA;
+      return launch_combine<T>(yrows, p.rt.flat_row, reinterpret_cast<T*>(out), Tn, H, K, st);
     }
   }
   gather_rows_kernel<T><<<row_blocks, kRowWarps * 32, 0, st>>>(reinterpret_cast<const T*>(hidden),
@@ -392,9 +375,7 @@ static int forward_train_impl(const void* hidden, const int64_t* ridx, const voi
     launch_simt_gemm<T, kFwd>(g1, glu, p.max_rows, st);
     launch_simt_gemm<T, kFwd>(g2, wrows, p.max_rows, st);
   }
-  combine_padded_kernel<T><<<(unsigned)ceil_div(Tn, kRowWarps), kRowWarps * 32, 0, st>>>(
-      yrows, p.rt.flat_row, reinterpret_cast<T*>(out), Tn, H, K);
-  return cudaGetLastError() == cudaSuccess ? YAMOE_OK : YAMOE_ERR_CUDA;
+  return launch_combine<T>(yrows, p.rt.flat_row, reinterpret_cast<T*>(out), Tn, H, K, st);
 }
 
 // Input, weight and bias gradients in fp32 (the routing-weight gradients are left in p.gw_row); `acc` is zeroed.
@@ -459,9 +440,7 @@ static int backward_impl(const void* grad_out, int per_slot, const void* hidden,
   const int Hp = H + kBiasCols;     // row pitch of xs and actw (see kBiasCols)
   const unsigned row_blocks = (unsigned)ceil_div(p.max_rows, kRowWarps);
   if (!saved) {
-    rc = prepare_routing(p, st);
-    if (rc) return rc;
-    rc = launch_route<T>(ridx, reinterpret_cast<const T*>(rw), rcols, Tn, E, K, cap, p.rt, st);
+    rc = launch_route_rows<T>(ridx, reinterpret_cast<const T*>(rw), rcols, Tn, E, K, cap, p.rt, p.row_tables_bytes, st);
     if (rc) return rc;
   }
   if constexpr (sizeof(T) == 4) {
