@@ -42,10 +42,6 @@ struct GemmArgs {
   const int32_t* pair_expert = nullptr;   // tile-pair tables (256-row tcgen05 kernel only)
   const int32_t* pair_off = nullptr;
   const int32_t* counts = nullptr;        // rows present per expert: lets the CUDA-core kernel skip all-padding tiles
-  // tcgen05 kFwd only: A is the UN-permuted source [gather_src_rows, K]; row r of the padded layout
-  // is source row gather_rows[r] (negative = padding), fetched by TMA gather
-  const int32_t* gather_rows = nullptr;
-  int64_t gather_src_rows = 0;
   // row-tiled arrangements without tables (tile_expert == nullptr): one group (expert 0) owns the
   // a_rows rows of A; rows at and beyond a_rows read as zeros
   int64_t a_rows = 0;

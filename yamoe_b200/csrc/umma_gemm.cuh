@@ -47,7 +47,6 @@ namespace yb {
 constexpr int kUmmaBM = 128;
 constexpr int kUmmaBK = 64;            // 64 bf16 = one 128-byte swizzle row
 constexpr int kUmmaThreads = 192;          // TMA producer, MMA issuer, four epilogue warps
-constexpr int kUmmaGatherThreads = 128;    // four more warps that gather the A rows when the gather is fused
 constexpr int kUmmaAccStride = 256;    // TMEM columns between the two accumulators
 constexpr int kUmmaMaxExperts = 1024;  // padded row offsets of up to this many experts are cached in shared memory
 constexpr uint64_t kWaitLimitNs = 2000000000ull;
@@ -137,15 +136,6 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map
       "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
       ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2) : "memory");
 }
-// 16-byte asynchronous copy global -> shared (L2 only); src_bytes = 0 writes zeros instead.
-__device__ __forceinline__ void cp_async_16(uint32_t dst, const void* src, uint32_t src_bytes) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-// makes this thread's completed generic-proxy writes to shared memory visible to the async proxy (tcgen05.mma)
-__device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, int c3,
                                             uint32_t bar) {
   asm volatile(
@@ -220,13 +210,6 @@ struct epi_prefetches : std::false_type {};
 template <class E>
 struct epi_prefetches<E, std::enable_if_t<E::kPrefetchTile>> : std::true_type {};
 
-// Forward epilogues that declare `static constexpr bool kMayGather = true` also get the kernel
-// instantiation whose extra warps gather the A rows (one more kernel per such functor).
-template <class E, class = void>
-struct epi_gathers : std::false_type {};
-template <class E>
-struct epi_gathers<E, std::enable_if_t<E::kMayGather>> : std::true_type {};
-
 template <class E, class = void>
 struct epi_staged : std::false_type {};
 template <class E>
@@ -239,9 +222,6 @@ struct UmmaParams {
   const int32_t* pad_off;
   int uniform_tiles;
   int32_t* header;
-  const int32_t* gather_rows;   // kFwd: source row of every padded row (gather fused into the A operand), or null
-  const void* gather_src;       //       the un-permuted source rows [*, gather_ld]
-  int64_t gather_ld;
   GemmGate gate;                // see GemmGate
   // MN-major operands whose width is a multiple of 64 are described as (64 columns, rows, column
   // block[, expert]) so that ONE copy brings all the 64-column boxes of a stage (box 64 x 64 x BN/64):
@@ -263,10 +243,8 @@ struct UmmaSmem {
   static constexpr int kTotal = kStages * kStageBytes + 1024;       // + slack for 1024-byte alignment
 };
 
-// GATHER (kFwd only): the kernel is launched with four more warps that fetch the A rows themselves
-// (see "A-row gather" below); without it the kernel has six warps and no trace of that role.
-template <int MODE, int BN, class Epi, bool GATHER = false>
-__global__ void __launch_bounds__(kUmmaThreads + (GATHER ? kUmmaGatherThreads : 0), 1)
+template <int MODE, int BN, class Epi>
+__global__ void __launch_bounds__(kUmmaThreads, 1)
 umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const UmmaParams p, const Epi epi) {
   using SM = UmmaSmem<BN>;
@@ -285,13 +263,9 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
 
-  // Gather fused into the A operand: four extra warps copy the tile's rows straight from the
-  // un-permuted source into the swizzled A stage (cp.async), the TMA producer loads only B, and a
-  // stage is full after the producer's arrival plus one per gather warp.
-  constexpr bool gather = GATHER && MODE == kFwd;
   if (threadIdx.x == 0) {
     for (int s = 0; s < kUmmaStages; ++s) {
-      mbar_init(smem_u32(&bar_full[s]), gather ? 1 + kUmmaGatherThreads / 32 : 1);
+      mbar_init(smem_u32(&bar_full[s]), 1);
       mbar_init(smem_u32(&bar_empty[s]), 1);
     }
     for (int a = 0; a < 2; ++a) {
@@ -409,7 +383,7 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         // MN-major B arrives as 64-column boxes: the last column tile asks only for those it has.
         // (The K-major B of the data gradients is one box of BN rows; rows past N read as zeros.)
         const int nboxes = MODE == kDgrad ? BN / 64 : (min(BN, p.N - n0) + 63) >> 6;
-        const uint32_t stage_tx = (gather ? 0 : SM::kABytes) + (p.b_wide ? BN / 64 : nboxes) * 8192;
+        const uint32_t stage_tx = SM::kABytes + (p.b_wide ? BN / 64 : nboxes) * 8192;
         if (MODE == kFwd && p.gate.arrived != nullptr && e != gate_done) {
           // the A rows of this group come from other GPUs: all of them must have landed
           const int need = p.gate.needed[e];
@@ -462,7 +436,7 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                 if (i < nboxes) tma_load_2d(sb + i * 8192, &tmB, n0 + i * 64, r, full);
             }
           } else {
-            if (!gather) tma_load_2d(sa, &tmA, kb * kUmmaBK, row0, full);
+            tma_load_2d(sa, &tmA, kb * kUmmaBK, row0, full);
             if constexpr (MODE == kFwd) {
               if (p.b_wide) {
                 tma_load_4d(sb, &tmB, 0, kb * kUmmaBK, n0 >> 6, e, full);
@@ -553,76 +527,6 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       YB_PROF_FLUSH(2, prof_full)
       YB_PROF_FLUSH(3, prof_tmem)
       YB_PROF_FLUSH(4, prof_all)
-    }
-    __syncwarp();
-  } else if (gather && warp >= kUmmaThreads / 32) {
-    // =========================== A-row gather (warps 6..9, only launched when gathering) ========
-    // Warp g copies rows 32g .. 32g+31 of the tile: eight lanes cover the 128 bytes one row
-    // contributes to a 64-deep k-block, so an instruction fetches four full 128-byte lines.  The
-    // 16-byte piece c of row r lands at piece (c ^ (r & 7)) of that row: the 128-byte swizzle
-    // the MMA's descriptor expects (what a tiled TMA load would have produced).  Copies are
-    // asynchronous; three k-blocks are kept in flight per warp, and a k-block is announced on the
-    // stage's full barrier once its copies have completed and a proxy fence has made them visible
-    // to the tensor core.
-    if constexpr (gather) {
-      {
-        constexpr int kInFlight = 3;
-        const int gw = warp - kUmmaThreads / 32;
-        const int piece = lane & 7, sub = lane >> 3;
-        const char* src = reinterpret_cast<const char*>(p.gather_src);
-        const size_t row_bytes = (size_t)p.gather_ld * 2;
-        int stage = 0, arr_stage = 0, pending = 0;
-        uint32_t phase = 0;
-        bool ok = true;
-        int e_next = expert_of(blockIdx.x);
-        for (int id = blockIdx.x; id < total && ok; id += gridDim.x) {
-          int e, row0, n0, krow, kblocks;
-          decode(id, e_next, e, row0, n0, krow, kblocks);
-          e_next = expert_of(id + gridDim.x);
-          int tok[8];
-#pragma unroll
-          for (int i = 0; i < 8; ++i) tok[i] = __ldg(p.gather_rows + row0 + gw * 32 + i * 4 + sub);
-          for (int kb = 0; kb < kblocks; ++kb) {
-            int good = 1;
-            if (lane == 0) good = mbar_wait(smem_u32(&bar_empty[stage]), phase ^ 1u, &abort_flag) ? 1 : 0;
-            good = __shfl_sync(0xffffffffu, good, 0);
-            if (!good) {
-              if (lane == 0) {
-                abort_flag = 1;
-                atomicMax(p.header + kHdrStatus, (int)kStatusProducerTimeout);
-              }
-              ok = false;
-              break;
-            }
-            const uint32_t sa = smem_base + stage * SM::kStageBytes;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              const int r = gw * 32 + i * 4 + sub;
-              const bool real = tok[i] >= 0;                       // padding rows are written as zeros
-              cp_async_16(sa + r * 128 + ((piece ^ (r & 7)) << 4),
-                          src + (real ? (size_t)tok[i] * row_bytes + (size_t)kb * 128 + piece * 16 : 0), real ? 16u : 0u);
-            }
-            cp_async_commit();
-            if (++pending == kInFlight) {
-              cp_async_wait<kInFlight - 1>();
-              fence_proxy_async_smem();
-              __syncwarp();
-              if (lane == 0) mbar_arrive(smem_u32(&bar_full[arr_stage]));
-              if (++arr_stage == kUmmaStages) arr_stage = 0;
-              --pending;
-            }
-            if (++stage == kUmmaStages) { stage = 0; phase ^= 1u; }
-          }
-        }
-        cp_async_wait<0>();                 // nothing of this warp is in flight past this point
-        fence_proxy_async_smem();
-        __syncwarp();
-        if (ok && lane == 0)
-          for (; pending > 0; --pending) {
-            mbar_arrive(smem_u32(&bar_full[arr_stage]));
-            if (++arr_stage == kUmmaStages) arr_stage = 0;
-          }
-      }
     }
     __syncwarp();
   } else {
@@ -790,7 +694,7 @@ inline bool umma_available() {
 // Encoding a map is a driver call that costs some tens of microseconds of host time; the same
 // (pointer, shape, box) comes back call after call (weights, persistent buffers, workspaces that the
 // caching allocator hands out again), so the last maps are kept in a small table.
-enum MapKind { kMapBf16 = 0, kMapF32 = 1, kMapF32Swizzled = 2 };   // fp32 tiles: plain, or 128-byte swizzle
+enum MapKind { kMapBf16 = 0, kMapF32 = 1, kMapF32Swizzled = 2, kMapBf16Plain = 3 };   // plain: no swizzle
 struct TensorMapKey {
   const void* base;
   int rank, kind;
@@ -829,9 +733,9 @@ inline bool make_map(CUtensorMap* m, const void* base, int rank, const uint64_t*
   cuuint32_t bx[4], es[4] = {1, 1, 1, 1};
   for (int i = 0; i < rank; ++i) { gd[i] = dims[i]; bx[i] = box[i]; }
   for (int i = 0; i + 1 < rank; ++i) gs[i] = strides[i];
-  CUresult r = encode_tiled_fn()(m, kind == kMapBf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32,
+  CUresult r = encode_tiled_fn()(m, kind == kMapBf16 || kind == kMapBf16Plain ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32,
                                  (cuuint32_t)rank, const_cast<void*>(base), gd, gs, bx, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                                 kind == kMapF32 ? CU_TENSOR_MAP_SWIZZLE_NONE : CU_TENSOR_MAP_SWIZZLE_128B,
+                                 kind == kMapF32 || kind == kMapBf16Plain ? CU_TENSOR_MAP_SWIZZLE_NONE : CU_TENSOR_MAP_SWIZZLE_128B,
                                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return false;
   std::lock_guard<std::mutex> lock(mu);
@@ -862,17 +766,12 @@ inline int umma_tile_n() {
   return bn;
 }
 
-template <int MODE, int BN, class Epi, bool GATHER>
-inline int launch_umma_kernel(const GemmArgs& g, const Epi& epi, const CUtensorMap& tmA, const CUtensorMap& tmB,
-                              int64_t max_tiles, bool a_wide, bool b_wide, cudaStream_t stream);
-
 template <int MODE, int BN, class Epi>
 inline int launch_umma_gemm_bn(const GemmArgs& g, const Epi& epi, int64_t max_rows, int64_t max_tiles,
                                cudaStream_t stream) {
   if (!umma_available()) return YAMOE_ERR_UNSUPPORTED;
   CUtensorMap tmA, tmB;
   bool ok = true;
-  const bool gather = MODE == kFwd && g.gather_rows != nullptr;
   // one copy per operand and k-block where the MN-major operand's width allows the blocked view
   // (YAMOE_B200_WIDE_TMA=0 keeps one copy per 64-column box)
   static const bool wide_on = []() {
@@ -905,8 +804,7 @@ inline int launch_umma_gemm_bn(const GemmArgs& g, const Epi& epi, int64_t max_ro
     const uint64_t da[2] = {(uint64_t)g.K, (uint64_t)max_rows};
     const uint64_t sa[1] = {(uint64_t)g.lda * 2};
     const uint32_t ba[2] = {64, 128u};
-    // with the gather fused, A is read by the gather warps: no map of it is needed
-    if (!gather) ok = ok && make_map(&tmA, g.A, 2, da, sa, ba);
+    ok = ok && make_map(&tmA, g.A, 2, da, sa, ba);
     if (MODE == kFwd && b_wide) {
       const uint64_t db[4] = {64, (uint64_t)g.K, (uint64_t)g.N / 64, (uint64_t)g.E};
       const uint64_t sb[3] = {(uint64_t)g.ldb * 2, 128, (uint64_t)g.b_expert_stride * 2};
@@ -925,21 +823,8 @@ inline int launch_umma_gemm_bn(const GemmArgs& g, const Epi& epi, int64_t max_ro
     }
   }
   if (!ok) return YAMOE_ERR_CUDA;
-  if (gather) tmA = tmB;              // placeholder for the unused kernel parameter
-  if constexpr (MODE == kFwd && epi_gathers<Epi>::value) {
-    if (gather) return launch_umma_kernel<MODE, BN, Epi, true>(g, epi, tmA, tmB, max_tiles, a_wide, b_wide, stream);
-  } else {
-    if (gather) return YAMOE_ERR_UNSUPPORTED;     // no gathering instantiation for this epilogue
-  }
-  return launch_umma_kernel<MODE, BN, Epi, false>(g, epi, tmA, tmB, max_tiles, a_wide, b_wide, stream);
-}
-
-template <int MODE, int BN, class Epi, bool GATHER>
-inline int launch_umma_kernel(const GemmArgs& g, const Epi& epi, const CUtensorMap& tmA, const CUtensorMap& tmB,
-                              int64_t max_tiles, bool a_wide, bool b_wide, cudaStream_t stream) {
+  auto kern = umma_gemm_kernel<MODE, BN, Epi>;
   using SM = UmmaSmem<BN>;
-  constexpr bool gather = GATHER;
-  auto kern = umma_gemm_kernel<MODE, BN, Epi, GATHER>;
   static PerDevice<int> attr_done;   // per template instantiation and device
   const int dev = current_device_index();
   if (!attr_done.get(dev)) {
@@ -947,15 +832,14 @@ inline int launch_umma_kernel(const GemmArgs& g, const Epi& epi, const CUtensorM
       return YAMOE_ERR_CUDA;
     attr_done.set(dev, 1);
   }
-  UmmaParams p{g.M, g.N, g.K, g.E, g.tile_expert, g.pad_off, (int)max_tiles, const_cast<int32_t*>(g.header),
-               gather ? g.gather_rows : nullptr, g.A, g.lda, g.gate, a_wide ? 1 : 0, b_wide ? 1 : 0};
+  UmmaParams p{g.M, g.N, g.K, g.E, g.tile_expert, g.pad_off, (int)max_tiles, const_cast<int32_t*>(g.header), g.gate,
+               a_wide ? 1 : 0, b_wide ? 1 : 0};
   const int NT = (int)ceil_div(g.N, BN);
   int64_t total_max = MODE == kWgrad ? (int64_t)g.E * ceil_div(g.M, kUmmaBM) * NT : max_tiles * NT;
   int grid = (int)std::min<int64_t>(total_max, umma_sm_count());
   if (grid <= 0) return YAMOE_OK;
   // a gated GEMM is meant to start while its predecessor on the stream still runs
-  const int threads = kUmmaThreads + (gather ? kUmmaGatherThreads : 0);
-  if (launch_pdl_opt(g.gate.prep != nullptr, kern, dim3(grid), dim3(threads), SM::kTotal, stream, tmA, tmB, p, epi) !=
+  if (launch_pdl_opt(g.gate.prep != nullptr, kern, dim3(grid), dim3(kUmmaThreads), SM::kTotal, stream, tmA, tmB, p, epi) !=
       cudaSuccess)
     return YAMOE_ERR_CUDA;
   return cudaGetLastError() == cudaSuccess ? YAMOE_OK : YAMOE_ERR_CUDA;

@@ -16,7 +16,7 @@
 #include "routing.cuh"
 #include "simt_gemm.cuh"
 #include "umma_gemm.cuh"
-#include "umma_gemm_2cta.cuh"
+#include "umma_pair.cuh"
 #include "umma_f32.cuh"
 #include "gemv.cuh"
 #include "ep_fused.cuh"
@@ -169,19 +169,6 @@ static int check_common(int64_t T, int H, int E, int K, int dtype) {
   return YAMOE_OK;
 }
 
-// YAMOE_B200_FUSED_GATHER=1 lets the gate_up GEMM of the forward fetch its A rows straight from
-// hidden_states (four extra warps per CTA copy them into the swizzled A stage with cp.async), so
-// that the permuted activations are never written to global memory.  Off by default: the GEMM fed
-// that way measures 518 us against 457 us for the TMA-fed one, more than the 27 us gather kernel
-// it saves (0.841 against 0.814 ms per forward at T = 4096).
-static bool fused_gather_enabled() {
-  static int on = []() {
-    const char* env = std::getenv("YAMOE_B200_FUSED_GATHER");
-    return env ? std::atoi(env) : 0;
-  }();
-  return on != 0;
-}
-
 static bool use_tcgen05(int path, int dtype, int H) {
   if (dtype != YAMOE_BF16 || !umma_available()) return false;
   if (H % 64 != 0) return false;
@@ -261,13 +248,10 @@ static int forward_impl(const void* hidden, const int64_t* ridx, const void* rw,
                                reinterpret_cast<const T*>(bgu), reinterpret_cast<const T*>(wd),
                                reinterpret_cast<const T*>(bd), reinterpret_cast<T*>(out), Tn, H, E, K, st);
   }
-  // With the gather fused the gate_up GEMM reads its A rows from hidden_states itself; otherwise
-  // gather_rows_kernel materialises the permuted copy first.
-  const bool fused_gather = tc && fused_gather_enabled() && !umma_2cta_enabled();
   const unsigned row_blocks = (unsigned)ceil_div(p.max_rows, kRowWarps);
-  if (!fused_gather) {
+  {
     StageTimer tm(kStageGather, st);
-    if (launch_pdl(gather_rows_kernel<T>, dim3(row_blocks), dim3(kRowWarps * 32), 0, st,
+    if (launch_pdl_opt(true, gather_rows_kernel<T>, dim3(row_blocks), dim3(kRowWarps * 32), 0, st,
                    reinterpret_cast<const T*>(hidden), reinterpret_cast<T*>(p.xs),
                    (const int32_t*)p.rt.row_token, (const int32_t*)p.rt.header, H, H) != cudaSuccess)
       return YAMOE_ERR_CUDA;
@@ -279,24 +263,21 @@ static int forward_impl(const void* hidden, const int64_t* ridx, const void* rw,
   g1.pair_expert = p.rt.pair_expert; g1.pair_off = p.rt.pair_off; g1.counts = p.rt.counts;
   GemmArgs g2{p.act, H, wd, H, (int64_t)H * H, 0, H, H, E, p.rt.tile_expert, p.rt.pad_off, p.rt.header};
   g2.pair_expert = p.rt.pair_expert; g2.pair_off = p.rt.pair_off; g2.counts = p.rt.counts;
-  if (fused_gather) {
-    g1.A = hidden;
-    g1.gather_rows = p.rt.row_token;
-    g1.gather_src_rows = Tn;
-  }
   if (tc) {
     if constexpr (sizeof(T) == 2) {
       {
         StageTimer tm(kStageGateUp, st);
-        rc = launch_umma<kFwd>(g1, glu, p.max_rows, p.max_tiles, st);
+        const PairGlu<false> pglu{reinterpret_cast<const T*>(bgu), reinterpret_cast<T*>(p.act), nullptr, nullptr,
+                                  nullptr, nullptr, H, 0};
+        rc = launch_umma_pair<kFwd>(g1, pglu, p.max_rows, p.max_tiles, 16, st);
       }
       if (rc) return rc;
       // two-step combine: weighted rows out of the GEMM epilogue, then one gather-sum pass
-      EpiWeightedRows<T> wrows{reinterpret_cast<const T*>(bd), reinterpret_cast<T*>(p.yrows), p.rt.row_token,
-                               p.rt.row_weight, H};
+      const PairWeightedRows wrows{reinterpret_cast<const T*>(bd), reinterpret_cast<T*>(p.yrows), p.rt.row_token,
+                                   p.rt.row_weight, H};
       {
         StageTimer tm(kStageDown, st);
-        rc = launch_umma<kFwd>(g2, wrows, p.max_rows, p.max_tiles, st);
+        rc = launch_umma_pair<kFwd>(g2, wrows, p.max_rows, p.max_tiles, 16, st);
       }
       if (rc) return rc;
       StageTimer tm(kStageCombine, st);
@@ -368,8 +349,10 @@ static int forward_train_impl(const void* hidden, const int64_t* ridx, const voi
   g2.pair_expert = p.rt.pair_expert; g2.pair_off = p.rt.pair_off; g2.counts = p.rt.counts;
   if (use_tcgen05(current_path(), dtype, H)) {
     if constexpr (sizeof(T) == 2) {
-      if ((rc = launch_umma<kFwd>(g1, glu, p.max_rows, p.max_tiles, st))) return rc;
-      if ((rc = launch_umma<kFwd>(g2, wrows, p.max_rows, p.max_tiles, st))) return rc;
+      const PairGlu<true> pglu{glu.bias, act, glu.actw, glu.pre, p.rt.row_token, p.rt.row_weight, H, Hp};
+      const PairWeightedRows pw{wrows.bias, yrows, p.rt.row_token, p.rt.row_weight, H};
+      if ((rc = launch_umma_pair<kFwd>(g1, pglu, p.max_rows, p.max_tiles, 64, st))) return rc;
+      if ((rc = launch_umma_pair<kFwd>(g2, pw, p.max_rows, p.max_tiles, 16, st))) return rc;
     }
   } else {
     launch_simt_gemm<T, kFwd>(g1, glu, p.max_rows, st);
@@ -492,11 +475,15 @@ static int backward_impl(const void* grad_out, int per_slot, const void* hidden,
 
   if (use_tcgen05(path, dtype, H)) {
     if constexpr (sizeof(T) == 2) {
-      if (!saved && (rc = launch_umma<kFwd>(g1, glu, p.max_rows, p.max_tiles, st))) return rc;
-      if ((rc = launch_umma<kDgrad>(g2, glub, p.max_rows, p.max_tiles, st))) return rc;
-      if ((rc = launch_umma<kWgrad>(g3, st_wd, p.max_rows, p.max_tiles, st))) return rc;
-      if ((rc = launch_umma<kDgrad>(g4, sc_dh, p.max_rows, p.max_tiles, st))) return rc;
-      if ((rc = launch_umma<kWgrad>(g5, st_wgu, p.max_rows, p.max_tiles, st))) return rc;
+      const PairGlu<true> pglu{glu.bias, nullptr, glu.actw, glu.pre, p.rt.row_token, p.rt.row_weight, H, Hp};
+      const PairGluBackward pglub{glub.pre, glub.g_pre, p.gw_row, p.rt.row_token, p.rt.row_weight, H};
+      const PairStoreBias pwd{st_wd.C, st_wd.bias_out, H, H}, pwgu{st_wgu.C, st_wgu.bias_out, H, 2 * H};
+      const PairScatterAdd pdh{acc, p.rt.row_token, H};
+      if (!saved && (rc = launch_umma_pair<kFwd>(g1, pglu, p.max_rows, p.max_tiles, 64, st))) return rc;
+      if ((rc = launch_umma_pair<kDgrad>(g2, pglub, p.max_rows, p.max_tiles, 64, st))) return rc;
+      if ((rc = launch_umma_pair<kWgrad>(g3, pwd, p.max_rows, p.max_tiles, 64, st))) return rc;
+      if ((rc = launch_umma_pair<kDgrad>(g4, pdh, p.max_rows, p.max_tiles, 16, st))) return rc;
+      if ((rc = launch_umma_pair<kWgrad>(g5, pwgu, p.max_rows, p.max_tiles, 64, st))) return rc;
     }
   } else {
     if (!saved) launch_simt_gemm<T, kFwd>(g1, glu, p.max_rows, st);
@@ -550,19 +537,19 @@ static int batch_mm_impl(const void* x, const void* w, void* out, int E, int C, 
     EpiStore<T> epi{reinterpret_cast<T*>(out), M, N};
     GemmArgs g{x, M, w, N, 0, M, N, 0, E, p.rt.tile_expert, p.rt.pad_off, p.rt.header};
       g.pair_expert = p.rt.pair_expert; g.pair_off = p.rt.pair_off;
-    if (tc) { if constexpr (sizeof(T) == 2) rc = launch_umma<kWgrad>(g, epi, rows, rows / kTileM, st); }
+    if (tc) { if constexpr (sizeof(T) == 2) rc = launch_umma_gemm<kWgrad>(g, epi, rows, rows / kTileM, st); }
     else launch_simt_gemm<T, kWgrad>(g, epi, rows, st);
   } else {
     EpiStoreRows<T> epi{reinterpret_cast<T*>(out), N};
     if (mode == kFwd) {
       GemmArgs g{x, K, w, N, (int64_t)K * N, 0, N, K, E, p.rt.tile_expert, p.rt.pad_off, p.rt.header};
       g.pair_expert = p.rt.pair_expert; g.pair_off = p.rt.pair_off;
-      if (tc) { if constexpr (sizeof(T) == 2) rc = launch_umma<kFwd>(g, epi, rows, rows / kTileM, st); }
+      if (tc) { if constexpr (sizeof(T) == 2) rc = launch_umma_gemm<kFwd>(g, epi, rows, rows / kTileM, st); }
       else launch_simt_gemm<T, kFwd>(g, epi, rows, st);
     } else {
       GemmArgs g{x, K, w, K, (int64_t)K * N, 0, N, K, E, p.rt.tile_expert, p.rt.pad_off, p.rt.header};
       g.pair_expert = p.rt.pair_expert; g.pair_off = p.rt.pair_off;
-      if (tc) { if constexpr (sizeof(T) == 2) rc = launch_umma<kDgrad>(g, epi, rows, rows / kTileM, st); }
+      if (tc) { if constexpr (sizeof(T) == 2) rc = launch_umma_gemm<kDgrad>(g, epi, rows, rows / kTileM, st); }
       else launch_simt_gemm<T, kDgrad>(g, epi, rows, st);
     }
   }
@@ -645,12 +632,12 @@ static int ep_local_forward_impl(const void* recv_x, const void* wgu, const void
         StageTimer tm(kStageGateUp, st);
         // the gate is a feature of the one-CTA kernel
         rc = gate.prep != nullptr ? launch_umma_gemm<kFwd>(g1, glu, max_rows, max_tiles, st)
-                                  : launch_umma<kFwd>(g1, glu, max_rows, max_tiles, st);
+                                  : launch_umma_gemm<kFwd>(g1, glu, max_rows, max_tiles, st);
       }
       if (rc) return rc;
       StageTimer tm(kStageDown, st);
-      rc = fused ? launch_umma<kFwd>(g2, prows, max_rows, max_tiles, st)
-                 : launch_umma<kFwd>(g2, wrows, max_rows, max_tiles, st);
+      rc = fused ? launch_umma_gemm<kFwd>(g2, prows, max_rows, max_tiles, st)
+                 : launch_umma_gemm<kFwd>(g2, wrows, max_rows, max_tiles, st);
       if (rc) return rc;
     }
   } else {
@@ -701,7 +688,7 @@ static int ep_local_backward_impl(const void* recv_x, const void* recv_g, const 
   // every row of this rank (token, gradient, weight) has arrived.
   if (tc) {
     if constexpr (sizeof(T) == 2) {
-      if ((rc = launch_umma<kFwd>(g1, glu, max_rows, max_tiles, st))) return rc;
+      if ((rc = launch_umma_gemm<kFwd>(g1, glu, max_rows, max_tiles, st))) return rc;
     }
   } else {
     launch_simt_gemm<T, kFwd>(g1, glu, max_rows, st);
@@ -712,10 +699,10 @@ static int ep_local_backward_impl(const void* recv_x, const void* recv_g, const 
       rt.row_token, rt.tile_expert, rt.header, H);
   if (tc) {
     if constexpr (sizeof(T) == 2) {
-      if ((rc = launch_umma<kDgrad>(g2, glub, max_rows, max_tiles, st))) return rc;
-      if ((rc = launch_umma<kWgrad>(g3, st_wd, max_rows, max_tiles, st))) return rc;
-      if ((rc = launch_umma<kDgrad>(g4, prows, max_rows, max_tiles, st))) return rc;
-      if ((rc = launch_umma<kWgrad>(g5, st_wgu, max_rows, max_tiles, st))) return rc;
+      if ((rc = launch_umma_gemm<kDgrad>(g2, glub, max_rows, max_tiles, st))) return rc;
+      if ((rc = launch_umma_gemm<kWgrad>(g3, st_wd, max_rows, max_tiles, st))) return rc;
+      if ((rc = launch_umma_gemm<kDgrad>(g4, prows, max_rows, max_tiles, st))) return rc;
+      if ((rc = launch_umma_gemm<kWgrad>(g5, st_wgu, max_rows, max_tiles, st))) return rc;
     }
   } else {
     launch_simt_gemm<T, kDgrad>(g2, glub, max_rows, st);
