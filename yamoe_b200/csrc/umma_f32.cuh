@@ -2,7 +2,7 @@
 // parts of eight significant bits each, and six of the nine partial products are multiplied with
 // tcgen05.mma (bf16, fp32 accumulation).  The three that are left out are below 2^-24 of the product.
 //
-//   arrangement   M operand (128), fp32, split on the way       N operand (up to 128), three bf16 planes
+//   arrangement   M operand (256), fp32, split on the way       N operand (up to 128), three bf16 planes
 //   kFwd          W[e][k][m]   weight columns                   rows of the expert, K-major
 //   kDgrad        W[e][m][k]   weight rows                      rows of the expert, K-major
 //   kWgrad        grad[r][m]   columns, k = rows                act[r][n] columns, MN-major
@@ -22,29 +22,33 @@
 // with round-to-nearest.  Against 64 bits the README forward is 3.9e-7 off where the FFMA kernel's serial
 // sum is 1.6e-6, the gradients of 600 tokens (H = 1024) at most 3.5e-7 against 1.1e-6.
 //
-// Measured: gate_up of the README forward (T = 512, H = 2880, E = 8, K = 2) 281 us = 121 TFLOP/s of the
-// original product; the whole forward 524 us against 1913, a training step of 600 tokens 466 against 1191.
+// Measured: gate_up of the README forward (T = 512, H = 2880, E = 8, K = 2) 190 us = 180 TFLOP/s of the
+// original product; the whole forward 422 us against 1797, a training step of 600 tokens 405 against 1191.
 //
 // Infinities and NaN behave as in fp32 arithmetic: see split3_mag.
 //
-// A CTA has 20 warps: TMA producer, MMA issuer, two that only complete the warpgroup, eight
-// converters (two per TMEM lane quarter, 32 k each) and eight accumulator / epilogue warps (two per
-// lane quarter, 64 columns each).  Shared
-// memory: three stages of weights (32 KB) and two of activations (48 KB); TMEM: two accumulators of
-// 128 columns, two A operands of 96.  Every wait is bounded as in umma_gemm.cuh.
+// Two CTAs share a tile (cta_group::2), 128 weight columns each: the planes are the larger half of what
+// L2 has to deliver (48 KB per 64-deep block against 32 KB of weights), and a pair needs them once.
+// With one CTA per tile the README forward took 485 us and the training step 463; now 422 and 405.
+//
+// A CTA has 20 warps: TMA producer, MMA issuer (of the leader only), two that only complete the
+// warpgroup, eight converters (two per TMEM lane quarter, 32 k each) and eight accumulator / epilogue
+// warps (two per lane quarter, 64 columns each).  Shared memory: three stages of weights (32 KB) and four
+// of activations (24 KB); TMEM: two accumulators of 128 columns, two A operands of 96.  Signals between
+// the CTAs as in umma_pair.cuh, every wait bounded as in umma_gemm.cuh.
 #pragma once
 #include "misc_kernels.cuh"
-#include "umma_gemm.cuh"
+#include "umma_pair.cuh"
 
 namespace yb {
 
 constexpr int kF32Threads = 640;
 constexpr int kF32ConvWarps = 8, kF32AccWarps = 8;
-constexpr int kF32M = 128, kF32N = 128, kF32K = 64;
+constexpr int kF32M = 128, kF32N = 128, kF32K = 64;      // M per CTA, N per pair
 constexpr int kF32WBytes = kF32M * kF32K * 4;            // 32 KB: fp32 tile of the M operand
-constexpr int kF32PlaneBytes = kF32N * kF32K * 2;        // 16 KB: one part of the N operand
+constexpr int kF32PlaneBytes = kF32N / 2 * kF32K * 2;    // 8 KB: this CTA's half of one part of the N operand
 constexpr int kF32BBytes = 3 * kF32PlaneBytes;
-constexpr int kF32WStages = 3, kF32BStages = 2;
+constexpr int kF32WStages = 3, kF32BStages = 4;
 constexpr int kF32Smem = kF32WStages * kF32WBytes + kF32BStages * kF32BBytes + 1024;
 constexpr int kF32TmemA = 256;                           // first TMEM column of the A operands
 constexpr int kF32TmemAStride = 96;                      // 3 parts x 32 columns (64 bf16)
@@ -342,15 +346,14 @@ struct F32Params {
   int32_t* header;
 };
 
-// tcgen05.mma with the A operand in TMEM
-__device__ __forceinline__ void tc_mma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
-                                               uint32_t accumulate) {
+// tcgen05.mma with the A operand in TMEM (each CTA of the pair holds its own 128 rows)
+__device__ __forceinline__ void tc2_mma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
+                                                uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %6, %7, %8}, p;\n\t}"
-      ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(0u), "r"(0u), "r"(0u), "r"(0u)
-      : "memory");
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
 __device__ __forceinline__ void tc_st_32x8(uint32_t taddr, const uint32_t (&r)[8]) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%8], {%0, %1, %2, %3, %4, %5, %6, %7};"
@@ -369,7 +372,7 @@ __device__ __forceinline__ void tc_ld_32x16(uint32_t taddr, uint32_t (&r)[16]) {
 __device__ __forceinline__ void tc_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 template <int MODE, class Epi>
-__global__ void __launch_bounds__(kF32Threads, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kF32Threads, 1)
 umma_f32_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__ CUtensorMap tmN,
                 const __grid_constant__ CUtensorMap tmNsmall, const F32Params p, const Epi epi) {
   extern __shared__ uint8_t smem_raw[];
@@ -383,6 +386,8 @@ umma_f32_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__
   __shared__ int32_t s_rows[kUmmaMaxExperts];
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t rank = cluster_ctarank();
+  const bool leader = rank == 0;
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t smem_b = smem_base + kF32WStages * kF32WBytes;
 
@@ -391,23 +396,30 @@ umma_f32_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__
       mbar_init(smem_u32(&bar_w_full[s]), 1);
       mbar_init(smem_u32(&bar_w_empty[s]), kF32ConvWarps);
     }
-    for (int s = 0; s < 2; ++s) {
-      mbar_init(smem_u32(&bar_b_full[s]), 1);
+    for (int s = 0; s < kF32BStages; ++s) {
+      mbar_init(smem_u32(&bar_b_full[s]), 2);                    // leader's: both producers
       mbar_init(smem_u32(&bar_b_empty[s]), 1);
-      mbar_init(smem_u32(&bar_a_full[s]), kF32ConvWarps);
+    }
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(smem_u32(&bar_a_full[s]), 2 * kF32ConvWarps);    // leader's
       mbar_init(smem_u32(&bar_a_empty[s]), 1);
       mbar_init(smem_u32(&bar_acc_full[s]), 1);
-      mbar_init(smem_u32(&bar_acc_empty[s]), kF32AccWarps);
+      mbar_init(smem_u32(&bar_acc_empty[s]), 2 * kF32AccWarps);  // leader's
     }
     abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;"
                  ::"r"(smem_u32(&tmem_base_slot)), "r"(512u) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
   tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();          // the peer's barriers exist before any remote signal is sent
+  tc_fence_after();
+  pdl_trigger();
+  pdl_wait();
   for (int i = threadIdx.x; i <= p.E; i += kF32Threads) {
     const int p0 = p.pad_off[i];
     s_pad[i] = p0;
@@ -417,12 +429,12 @@ umma_f32_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__
     }
   }
   __syncthreads();
-  tc_fence_after();
   const uint32_t tmem_base = tmem_base_slot;
 
-  const int MT = (p.M + kF32M - 1) / kF32M;
+  const int MT = (p.M + 2 * kF32M - 1) / (2 * kF32M);
   const int NT = (p.N + kF32N - 1) / kF32N;       // kWgrad
   const int total = MODE == kWgrad ? p.E * MT * NT : p.header[kHdrRowTiles] * MT;
+  const int cluster_id = blockIdx.x >> 1, n_clusters = gridDim.x >> 1;
   auto expert_of = [&](int id) -> int {
     if constexpr (MODE == kWgrad) return 0;
     return id < total ? __ldg(p.tile_expert + id / MT) : 0;
@@ -433,9 +445,10 @@ umma_f32_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__
       e = id / (MT * NT);
       const int rem = id - e * (MT * NT);
       const int nt = rem / MT;
-      m0 = (rem - nt * MT) * kF32M;
+      m0 = (rem - nt * MT) * 2 * kF32M + (int)rank * kF32M;
       n0 = nt * kF32N;
-      width = (min(kF32N, p.N - n0) + 15) & ~15;
+      const int left = p.N - n0;
+      width = left > 64 ? kF32N : (left + 15) & ~15;        // a 64-column box per CTA, or both halves in one box
       kblocks = s_rows[e] / kF32K;
     } else {
       e = e_hint;
@@ -446,7 +459,7 @@ umma_f32_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__
       const int rows = s_rows[e];
       const int step = ((rows + cnt - 1) / cnt + 15) & ~15;
       const int off = (local - mt * cnt) * step;
-      m0 = mt * kF32M;
+      m0 = mt * 2 * kF32M + (int)rank * kF32M;
       n0 = s_pad[e] + off;
       width = min(step, rows - off);
       kblocks = p.K / kF32K;
@@ -465,13 +478,13 @@ umma_f32_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__
       uint32_t wph = 0, bph = 0;
       bool ok = true;
       // weights run one k-block ahead of the activations (they are released earlier)
-      int w_id = blockIdx.x, w_kb = 0;
+      int w_id = cluster_id, w_kb = 0;
       int w_e = 0, w_m0 = 0, w_n0 = 0, w_width = 0, w_kblocks = 0;
       auto w_open = [&]() {                         // next work item that has k-blocks
         while (w_id < total) {
           decode(w_id, expert_of(w_id), w_e, w_m0, w_n0, w_width, w_kblocks);
           if (w_kblocks > 0) return;
-          w_id += gridDim.x;
+          w_id += n_clusters;
         }
       };
       auto w_issue = [&]() -> bool {
@@ -492,78 +505,89 @@ umma_f32_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__
         if (++ws == kF32WStages) { ws = 0; wph ^= 1u; }
         if (++w_kb == w_kblocks) {
           w_kb = 0;
-          w_id += gridDim.x;
+          w_id += n_clusters;
           w_open();
         }
         return true;
       };
       w_open();
       ok = w_issue();
-      for (int id = blockIdx.x; id < total && ok; id += gridDim.x) {
+      for (int id = cluster_id; id < total && ok; id += n_clusters) {
         int e, m0, n0, width, kblocks;
         decode(id, expert_of(id), e, m0, n0, width, kblocks);
-        const bool big = width > 64;
+        const int half = width >> 1;
+        // this CTA's rows (columns) of the N operand: one box of 64, or of 32
+        const bool big = MODE == kWgrad || half > 32;
         const uint32_t bytes = big ? kF32BBytes : kF32BBytes / 2;
+        const int my_n = n0 + (int)rank * half;
         for (int kb = 0; kb < kblocks; ++kb) {
           ok = w_issue() && mbar_wait(smem_u32(&bar_b_empty[bs]), bph ^ 1u, &abort_flag);
           if (!ok) break;
-          const uint32_t full = smem_u32(&bar_b_full[bs]);
+          const uint32_t full = mapa_u32(smem_u32(&bar_b_full[bs]), 0);
           const uint32_t sb = smem_b + bs * kF32BBytes;
-          const CUtensorMap* map = big ? &tmN : &tmNsmall;
-          mbar_expect_tx(full, bytes);
-          if constexpr (MODE == kWgrad) tma_load_4d(sb, map, 0, s_pad[e] + kb * kF32K, n0 >> 6, 0, full);
-          else tma_load_3d(sb, map, kb * kF32K, n0, 0, full);
+          mbar_expect_tx_cluster(full, bytes);
+          if constexpr (MODE == kWgrad) tma2_load_4d(sb, &tmN, my_n & 63, s_pad[e] + kb * kF32K, my_n >> 6, 0, full);
+          else tma2_load_3d(sb, big ? &tmN : &tmNsmall, kb * kF32K, my_n, 0, full);
           if (++bs == kF32BStages) { bs = 0; bph ^= 1u; }
         }
+      }
+      // the commits that free the last stages must have arrived here before this CTA ends
+      for (int g = 0; g < kF32BStages && ok; ++g) {
+        ok = mbar_wait(smem_u32(&bar_b_empty[bs]), bph ^ 1u, &abort_flag);
+        if (++bs == kF32BStages) { bs = 0; bph ^= 1u; }
       }
       if (!ok) give_up(kStatusProducerTimeout);
     }
     __syncwarp();
   } else if (warp == 1) {
-    // =========================== MMA issuer ==================================================
-    if (lane == 0) {
+    // =========================== MMA issuer (leader CTA only; see umma_pair.cuh) ==============
+    if (leader) {
       constexpr bool kBMn = MODE == kWgrad;
       constexpr uint32_t idesc_base = (1u << 4) | (1u << 7) | (1u << 10) | ((kBMn ? 1u : 0u) << 16) |
-                                      ((uint32_t)(kF32M >> 4) << 24);
+                                      ((uint32_t)(2 * kF32M >> 4) << 24);
       constexpr uint32_t b_kstep = kBMn ? (16 * 128) >> 4 : 32 >> 4;
       // parts (of M operand, of N operand), smallest products first
       constexpr int kPartA[6] = {0, 2, 1, 0, 1, 0}, kPartB[6] = {2, 0, 1, 1, 0, 0};
-      int slot = 0;                                  // A operand, B stage and accumulator alike: two of each
-      uint32_t phase = 0;
+      const uint64_t bdesc0 = make_smem_desc(smem_b, kBMn ? 8192 : 16, 1024);
+      const bool elected = elect_one();
+      int slot = 0, bs = 0;                          // A operand and accumulator: two of each; B stage
+      uint32_t phase = 0, bph = 0;
       bool ok = true;
-      int e_next = expert_of(blockIdx.x);
-      for (int id = blockIdx.x; id < total && ok; id += gridDim.x) {
+      int e_next = expert_of(cluster_id);
+      for (int id = cluster_id; id < total && ok; id += n_clusters) {
         int e, m0, n0, width, kblocks;
         decode(id, e_next, e, m0, n0, width, kblocks);
-        e_next = expert_of(id + gridDim.x);
+        e_next = expert_of(id + n_clusters);
         const uint32_t idesc = idesc_base | ((uint32_t)(width >> 3) << 17);
-        const uint32_t plane = width > 64 ? kF32PlaneBytes : kF32PlaneBytes / 2;
+        const uint32_t plane = (MODE == kWgrad || width > 64 ? kF32PlaneBytes : kF32PlaneBytes / 2) >> 4;
         for (int kb = 0; kb < kblocks; ++kb) {
           ok = mbar_wait(smem_u32(&bar_acc_empty[slot]), phase ^ 1u, &abort_flag) &&
-               mbar_wait(smem_u32(&bar_b_full[slot]), phase, &abort_flag) &&
+               mbar_wait(smem_u32(&bar_b_full[bs]), bph, &abort_flag) &&
                mbar_wait(smem_u32(&bar_a_full[slot]), phase, &abort_flag);
+          ok = __all_sync(0xffffffffu, ok);
           if (!ok) break;
           tc_fence_after();
-          const uint32_t d = tmem_base + slot * kF32N;
-          const uint32_t a0 = tmem_base + kF32TmemA + slot * kF32TmemAStride;
-          const uint32_t sb = smem_b + slot * kF32BBytes;
+          if (elected) {
+            const uint32_t d = tmem_base + slot * kF32N;
+            const uint32_t a0 = tmem_base + kF32TmemA + slot * kF32TmemAStride;
+            const uint64_t bdesc = bdesc0 + (uint64_t)(bs * (kF32BBytes >> 4));
 #pragma unroll
-          for (int q = 0; q < 6; ++q) {
-            const uint32_t addr = sb + kPartB[q] * plane;
-            const uint64_t bdesc = kBMn ? make_smem_desc(addr, 8192, 1024) : make_smem_desc(addr, 16, 1024);
+            for (int q = 0; q < 6; ++q)
 #pragma unroll
-            for (int k = 0; k < kF32K / 16; ++k)
-              tc_mma_bf16_ts(d, a0 + kPartA[q] * 32 + k * 8, bdesc + (uint64_t)(k * b_kstep), idesc,
-                             (uint32_t)((q | k) != 0));
+              for (int k = 0; k < kF32K / 16; ++k)
+                tc2_mma_bf16_ts(d, a0 + kPartA[q] * 32 + k * 8, bdesc + (uint64_t)(kPartB[q] * plane + k * b_kstep), idesc,
+                                (uint32_t)((q | k) != 0));
+            tc2_commit_pair(smem_u32(&bar_a_empty[slot]));
+            tc2_commit_pair(smem_u32(&bar_b_empty[bs]));
+            tc2_commit_pair(smem_u32(&bar_acc_full[slot]));
           }
-          tc_commit(smem_u32(&bar_a_empty[slot]));
-          tc_commit(smem_u32(&bar_b_empty[slot]));
-          tc_commit(smem_u32(&bar_acc_full[slot]));
+          __syncwarp();
           slot ^= 1;
           if (slot == 0) phase ^= 1u;
+          if (++bs == kF32BStages) { bs = 0; bph ^= 1u; }
         }
       }
-      if (!ok) give_up(kStatusMmaTimeout);
+      if (!ok && lane == 0) give_up(kStatusMmaTimeout);
     }
     __syncwarp();
   }
@@ -574,11 +598,11 @@ umma_f32_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__
     int ws = 0, slot = 0;
     uint32_t wph = 0, phase = 0;
     bool ok = true;
-    int e_next = expert_of(blockIdx.x);
-    for (int id = blockIdx.x; id < total && ok; id += gridDim.x) {
+    int e_next = expert_of(cluster_id);
+    for (int id = cluster_id; id < total && ok; id += n_clusters) {
       int e, m0, n0, width, kblocks;
       decode(id, e_next, e, m0, n0, width, kblocks);
-      e_next = expert_of(id + gridDim.x);
+      e_next = expert_of(id + n_clusters);
       for (int kb = 0; kb < kblocks; ++kb) {
         ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_w_full[ws]), wph, &abort_flag));
         if (!ok) break;
@@ -615,7 +639,7 @@ umma_f32_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__
         tc_st_wait();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(&bar_a_full[slot]));
+        if (lane == 0) mbar_arrive_cluster(mapa_u32(smem_u32(&bar_a_full[slot]), 0));
         slot ^= 1;
         if (slot == 0) phase ^= 1u;
       }
@@ -628,11 +652,11 @@ umma_f32_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__
     int slot = 0;
     uint32_t phase = 0;
     bool ok = true;
-    int e_next = expert_of(blockIdx.x);
-    for (int id = blockIdx.x; id < total && ok; id += gridDim.x) {
+    int e_next = expert_of(cluster_id);
+    for (int id = cluster_id; id < total && ok; id += n_clusters) {
       int e, m0, n0, width, kblocks;
       decode(id, e_next, e, m0, n0, width, kblocks);
-      e_next = expert_of(id + gridDim.x);
+      e_next = expert_of(id + n_clusters);
       const int cols = min(64, width - nhalf * 64);  // of this warp; <= 0: none
       float acc[64];
 #pragma unroll
@@ -652,7 +676,7 @@ umma_f32_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__
           }
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(&bar_acc_empty[slot]));
+        if (lane == 0) mbar_arrive_cluster(mapa_u32(smem_u32(&bar_acc_empty[slot]), 0));
         slot ^= 1;
         if (slot == 0) phase ^= 1u;
       }
@@ -682,9 +706,10 @@ umma_f32_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__
     while (global_timer_ns() - t0 < 2000000ull) __nanosleep(1000);
     __syncthreads();
   }
+  cluster_sync_all();          // neither CTA releases shared memory or TMEM the pair may still use
   if (warp == 1) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
   }
 }
 
@@ -699,16 +724,17 @@ inline int launch_umma_f32(const GemmArgs& g, int64_t a_plane, const Epi& epi, i
   if (MODE == kWgrad) {
     const uint64_t dn[4] = {64, (uint64_t)max_rows, (uint64_t)g.lda / 64, 3};
     const uint64_t sn[3] = {(uint64_t)g.lda * 2, 128, (uint64_t)a_plane * 2};
-    const uint32_t b2[4] = {64, 64, 2, 3}, b1[4] = {64, 64, 1, 3};
-    ok = make_map(&tmN, g.A, 4, dn, sn, b2) && make_map(&tmNs, g.A, 4, dn, sn, b1);
+    const uint32_t b1[4] = {64, 64, 1, 3};
+    ok = make_map(&tmN, g.A, 4, dn, sn, b1);
+    tmNs = tmN;                          // not used
     const uint64_t dm[2] = {(uint64_t)g.N, (uint64_t)max_rows}, sm[1] = {(uint64_t)g.ldb * 4};
     const uint32_t bm[2] = {kF32M, kF32K};
     ok = ok && make_map(&tmM, g.B, 2, dm, sm, bm, kMapF32);
   } else {
     const uint64_t dn[3] = {(uint64_t)g.K, (uint64_t)max_rows, 3};
     const uint64_t sn[2] = {(uint64_t)g.lda * 2, (uint64_t)a_plane * 2};
-    const uint32_t b128[3] = {64, 128, 3}, b64[3] = {64, 64, 3};
-    ok = make_map(&tmN, g.A, 3, dn, sn, b128) && make_map(&tmNs, g.A, 3, dn, sn, b64);
+    const uint32_t b64[3] = {64, 64, 3}, b32[3] = {64, 32, 3};
+    ok = make_map(&tmN, g.A, 3, dn, sn, b64) && make_map(&tmNs, g.A, 3, dn, sn, b32);
     const uint64_t sm[2] = {(uint64_t)g.ldb * 4, (uint64_t)g.b_expert_stride * 4};
     if (MODE == kFwd) {
       const uint64_t dm[3] = {(uint64_t)g.N, (uint64_t)g.K, (uint64_t)g.E};
@@ -722,19 +748,16 @@ inline int launch_umma_f32(const GemmArgs& g, int64_t a_plane, const Epi& epi, i
   }
   if (!ok) return YAMOE_ERR_CUDA;
   auto kern = umma_f32_kernel<MODE, Epi>;
-  static PerDevice<int> attr_done;   // per template instantiation and device
-  const int dev = current_device_index();
-  if (!attr_done.get(dev)) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kF32Smem) != cudaSuccess)
-      return YAMOE_ERR_CUDA;
-    attr_done.set(dev, 1);
-  }
+  static PerDevice<int> resident;    // per template instantiation and device
+  const int pairs = resident_pairs(kern, kF32Threads, kF32Smem, resident);
+  if (pairs <= 0) return YAMOE_ERR_CUDA;
   const F32Params p{g.N, g.M, g.K, g.E, row_round, g.tile_expert, g.pad_off, g.counts, const_cast<int32_t*>(g.header)};
-  const int64_t MT = ceil_div(g.N, kF32M);
+  const int64_t MT = ceil_div(g.N, 2 * kF32M);
   const int64_t total_max = MODE == kWgrad ? (int64_t)g.E * MT * ceil_div(g.M, kF32N) : max_tiles * MT;
-  const int grid = (int)std::min<int64_t>(total_max, umma_sm_count());
+  const int grid = (int)(2 * std::min<int64_t>(total_max, pairs));
   if (grid <= 0) return YAMOE_OK;
-  kern<<<grid, kF32Threads, kF32Smem, stream>>>(tmM, tmN, tmNs, p, epi);
+  if (launch_pdl_opt(true, kern, dim3(grid), dim3(kF32Threads), kF32Smem, stream, tmM, tmN, tmNs, p, epi) != cudaSuccess)
+    return YAMOE_ERR_CUDA;
   return cudaGetLastError() == cudaSuccess ? YAMOE_OK : YAMOE_ERR_CUDA;
 }
 
