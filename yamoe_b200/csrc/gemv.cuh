@@ -337,9 +337,15 @@ inline int gemv_down_ksplit(int64_t S, int E, int N) {
   return ctas <= 2 * 148 ? 2 : 1;     // measured: 53.6 / 55.0 / 55.6 us with 2 / 1 / 4 parts at T = 1; no gain beyond
 }
 
-inline bool gemv_preferred(int64_t T, int E, int K) {
+// At most about 4 rows per expert: the kernels read an expert's weights once per 4 rows.  Where the
+// tensor-core GEMM (umma_pair.cuh) can take the call, it does from S * H = 80 K on: it needs some 25 us
+// for routing, gather and combine, and then reads every expert once whatever its number of rows.  Measured
+// per call, gemv / grouped:  H = 2880: S = 16 138 / 145 us (E = 32), S = 32 240 / 243 (E = 128) and
+// 224 / 196 (E = 32), S = 64 429 / 417;  H = 2048: S = 32 118 / 130, S = 64 186 / 186, S = 128 282 / 256;
+// H = 1024: S = 64 56 / 59, S = 128 76 / 60.
+inline bool gemv_preferred(int64_t T, int H, int E, int K, bool tensor_cores) {
   const int64_t S = T * K;
-  return S <= kGemvMaxS && S <= 4 * (int64_t)E;   // at most ~4 rows per expert on average
+  return S <= kGemvMaxS && S <= 4 * (int64_t)E && (!tensor_cores || S * H <= 80 * 1024);
 }
 
 template <int STAGE, int NB>

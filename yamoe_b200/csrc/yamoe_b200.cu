@@ -227,7 +227,7 @@ static int forward_impl(const void* hidden, const int64_t* ridx, const void* rw,
   float* acc = p.acc32 ? p.acc32 : reinterpret_cast<float*>(out);
   if (Tn == 0) return YAMOE_OK;
 
-  if (dtype == YAMOE_BF16 && (path == YAMOE_PATH_GEMV || (path == YAMOE_PATH_AUTO && gemv_preferred(Tn, E, K)))) {
+  if (dtype == YAMOE_BF16 && (path == YAMOE_PATH_GEMV || (path == YAMOE_PATH_AUTO && gemv_preferred(Tn, H, E, K, use_tcgen05(path, dtype, H))))) {
     int rc = launch_gemv_forward(hidden, ridx, rw, rcols, wgu, bgu, wd, bd, out, Tn, H, E, K, cap, p.act, acc,
                                  p.slab_done, st);
     if (rc != YAMOE_ERR_UNSUPPORTED) return rc;
