@@ -68,17 +68,19 @@ WORKLOADS = {
 # DRAM bytes (read + write) of one launch of the dominant kernel, from ncu captures of that kernel;
 # keyed by workload and output-tile width.  The source names the summary that holds the capture.
 TRAFFIC = {
-    ("gptoss20b_fwd_t4096", 256): (1.270e9, "ncu dram__bytes_read.sum + dram__bytes_write.sum of one gate_up launch, "
-                                            "profiles/umma_gemm_gptoss20b_fwd_t4096.md"),
+    ("gptoss20b_fwd_t4096", 256): (1.256e9, "ncu dram__bytes_read.sum + dram__bytes_write.sum of one gate_up launch, "
+                                            "profiles/umma_pair_gptoss20b_fwd_t4096.md"),
 }
 
 # kernels of this library launched by one call (memsets not counted):
-#   fwd     2 routing + row gather + gate_up GEMM + down GEMM + combine
-#   bwd     2 routing + 2 gathers + 5 GEMMs (bias gradients ride along) + routing gradient + cast
+#   fwd     routing + row gather + gate_up GEMM + down GEMM + combine
+#   bwd     routing + 2 gathers + 5 GEMMs (bias gradients ride along) + routing gradient + cast
+#           (one more in either where more than 32768 assignments take the two-launch routing)
+#   decode  2 GEMV kernels, or the kernels of fwd where the grouped GEMM takes the call
 #   ep_fwd  2 routing + publish + dispatch + 2 GEMMs + signal + combine
 #   ep_bwd  2 routing + publish + dispatch + weights + gather + 5 GEMMs + 2 column sums +
 #           scalar return + signal + combine + routing gradient
-LAUNCHES = {"fwd": 6, "fwd_fp32": 6, "bwd": 11, "train": 17, "decode": 2, "ep_fwd": 8, "ep_bwd": 17}
+LAUNCHES = {"fwd": 5, "fwd_fp32": 5, "bwd": 10, "train": 15, "decode": 2, "ep_fwd": 8, "ep_bwd": 17}
 
 
 def measured_peaks():
@@ -465,13 +467,15 @@ class Case:
         return self.T * self.K
 
     def launches(self):
-        if self.decode:
+        if self.decode and self.T * self.K * self.H <= 80 * 1024:
             return LAUNCHES["decode"]
         if self.use_ep and self.peer_ctx is not None:
             return LAUNCHES["ep_" + self.mode]
         if self.mode == "fwd" and self.w.get("fp32"):
             return LAUNCHES["fwd_fp32"]
-        return LAUNCHES[self.mode]
+        saved = self.mode == "train" and self.w.get("saved")     # its backward skips routing, gather and gate_up
+        routings = 2 if self.mode == "train" and not saved else 1
+        return LAUNCHES[self.mode] - (3 if saved else 0) + (routings if self.T * self.K > 32768 else 0)
 
 
 def time_resident(case: Case, steps: int, warmup: int, sample_clocks: bool = True):
@@ -689,25 +693,25 @@ def roofline_of(case: Case, res, peaks, rows):
     if case.decode:
         kbytes = case.distinct * (H * 2 * H * 2 + 2 * H * 2)          # gate_up weights + bias of the touched experts
         achieved = kbytes / (mean_ms * 1e-3) / 1e9
-        return {"bound": "hbm", "kernel": "gemv_kernel<gate_up + bias + clamped SwiGLU>",
+        grouped = case.T * case.K * H > 80 * 1024
+        return {"bound": "hbm", "kernel": ("umma_pair_kernel" if grouped else "gemv_kernel") + "<gate_up + bias + clamped SwiGLU>",
                 "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                 "frac": achieved / peaks["hbm_gbs"], "traffic": None, "kernel_ms": mean_ms,
                 "peak_source": peaks["source"] + " (copy bandwidth)",
                 "frac_of_nominal_8000": achieved / 8000.0, "distinct_experts": case.distinct,
                 "whole_op_gbs": case.distinct * 49783680 / (res["ms_step"] * 1e-3) / 1e9}
     if case.dtype == torch.float32:
-        # fp32 runs on the CUDA cores (FFMA): no measured peak exists for that pipe, so the
-        # fraction is against the nominal 148 SMs x 128 FMA x 2 x 1.965 GHz
+        # fp32 runs as six bf16 products of three-part operands on the tensor cores
         achieved = 4.0 * rows * H * H / (mean_ms * 1e-3) / 1e12
-        ffma_peak = 148 * 128 * 2 * 1.965e9 / 1e12
-        return {"bound": "tensor", "kernel": "simt_gemm_kernel<gate_up + bias + clamped SwiGLU> (fp32 FFMA)",
-                "achieved": achieved, "peak": ffma_peak, "unit": "TFLOP/s", "frac": achieved / ffma_peak,
+        peak = peaks["bf16_tflops"] / 6
+        return {"bound": "tensor", "kernel": "umma_f32_kernel<gate_up + bias + clamped SwiGLU> (three bf16 parts)",
+                "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
                 "traffic": None, "kernel_ms": mean_ms,
-                "peak_source": "nominal fp32 FFMA rate (CUDA cores; the tensor pipe is not used in fp32)"}
+                "peak_source": peaks["source"] + " (burst bf16 matmul, a sixth of it)"}
     achieved = 4.0 * rows * H * H / (mean_ms * 1e-3) / 1e12
     tile_n = int(os.environ.get("YAMOE_B200_BN", "256") or 256)
     traffic, source = TRAFFIC.get((case.name, tile_n), (None, None)) if not case.use_ep else (None, None)
-    out = {"bound": "tensor", "kernel": "umma_gemm_kernel<gate_up + bias + clamped SwiGLU>",
+    out = {"bound": "tensor", "kernel": ("umma_gemm_kernel" if case.use_ep else "umma_pair_kernel") + "<gate_up + bias + clamped SwiGLU>",
            "achieved": achieved, "peak": peaks["bf16_tflops"], "unit": "TFLOP/s",
            "frac": achieved / peaks["bf16_tflops"], "traffic": traffic, "traffic_source": source,
            "kernel_ms": mean_ms, "peak_source": peaks["source"] + " (burst bf16 matmul)",
