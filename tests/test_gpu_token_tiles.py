@@ -51,6 +51,28 @@ def test_rows_per_expert_at_tile_edges(dtype, H, capacity):
         orc.check_close(a.float().cpu(), ref_g[i], rtol, GRADS[i] + " (saved activations)")
 
 
+@pytest.mark.parametrize("first,second", [("auto", "simt"), ("simt", "auto")])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32], ids=["bf16", "fp32"])
+def test_saved_activations_survive_a_change_of_path(first, second, dtype):
+    """The buffer of the saving forward is consumed by the kernels of another path."""
+    import yamoe_b200
+    from yamoe_b200.layers import experts_autograd
+    args, grad, T, E = _problem([0, 5, 70, 130], 64, dtype, seed=3)
+    torch.full((1 << 24,), float("nan"), device="cuda")          # what the allocator hands out next is not zero
+    dev = [a.cuda() for a in args]
+    leaves = [t.requires_grad_(True) for t in dev if t.is_floating_point()]
+    try:
+        yamoe_b200.set_path(first)
+        out = experts_autograd(*dev, T, E, 1, save_activations=True)
+        yamoe_b200.set_path(second)
+        got = torch.autograd.grad(out, leaves, grad.cuda())
+    finally:
+        yamoe_b200.set_path("auto")
+    ref = orc.experts_backward_oracle(grad, *args, T, E, 1)
+    for a, b, n in zip(got, ref, GRADS):
+        orc.check_close(a.float().cpu(), b, RTOL_BF16 if dtype == torch.bfloat16 else RTOL_F32, n)
+
+
 @pytest.mark.parametrize("T,E,K", [(8193, 7, 4), (8191, 300, 4), (9001, 16, 4), (2731, 33, 3)])
 def test_routing_of_many_assignments(T, E, K):
     """Around 32768 assignments, with ids outside [0, E) and a capacity that drops."""

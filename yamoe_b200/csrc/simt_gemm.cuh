@@ -85,6 +85,9 @@ simt_gemm_kernel(GemmArgs g, Epi epi) {
     row0 = blockIdx.y * BM;                 // m0 within the expert's output
     k_begin = g.pad_off[e];
     k_end = g.pad_off[e + 1];
+    // padding rows add nothing, and the tensor-core kernels that may have left these operands (a buffer of
+    // the saving forward) write only part of them
+    if (g.counts != nullptr) k_end = min(k_end, k_begin + g.counts[e]);
     m_limit = g.M;
   } else {
     row0 = blockIdx.y * BM;                 // padded row
