@@ -83,8 +83,9 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // Measured on B200: between the two decode GEMV kernels it saves about 2 us per call (T = 1: 52.0 us
-// against 53.8 us as a CUDA-graph replay), so that pair uses it by default; between the kernels of
-// the grouped-GEMM forward it did not help (0.843 ms with, 0.814 ms without) and stays off.
+// against 53.8 us as a CUDA-graph replay).  The kernels of the expert pass use it as well (gather, the
+// grouped GEMMs of umma_pair.cuh and umma_f32.cuh, combine): their barrier and TMEM set-up and the launch
+// latency fall into the predecessor's tail.  The one-CTA GEMM does so only where it is gated.
 // YAMOE_B200_PDL=1 turns it on everywhere, YAMOE_B200_PDL=0 off everywhere.
 inline int pdl_setting() {
   static int v = []() {
