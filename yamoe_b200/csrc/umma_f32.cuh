@@ -22,7 +22,7 @@
 // with round-to-nearest.  Against 64 bits the README forward is 3.9e-7 off where the FFMA kernel's serial
 // sum is 1.6e-6, the gradients of 600 tokens (H = 1024) at most 3.5e-7 against 1.1e-6.
 //
-// Measured: gate_up of the README forward (T = 512, H = 2880, E = 8, K = 2) 190 us = 180 TFLOP/s of the
+// Measured: gate_up of the README forward (T = 512, H = 2880, E = 8, K = 2) 213 us = 160 TFLOP/s of the
 // original product; the whole forward 422 us against 1797, a training step of 600 tokens 405 against 1191.
 //
 // Infinities and NaN behave as in fp32 arithmetic: see split3_mag.
