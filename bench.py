@@ -466,8 +466,13 @@ class Case:
             return int(self.ep_stats.get("rows_received", self.T * self.K))
         return self.T * self.K
 
+    def uses_gemv(self):
+        """The library's rule for decode-sized bf16 calls of these widths (gemv_preferred in csrc/gemv.cuh)."""
+        S = self.T * self.K
+        return self.decode and S <= min(256, 4 * self.E) and (S < 2 * self.E or S * self.H <= 80 * 1024)
+
     def launches(self):
-        if self.decode and self.T * self.K * self.H <= 80 * 1024:
+        if self.uses_gemv():
             return LAUNCHES["decode"]
         if self.use_ep and self.peer_ctx is not None:
             return LAUNCHES["ep_" + self.mode]
@@ -693,8 +698,7 @@ def roofline_of(case: Case, res, peaks, rows):
     if case.decode:
         kbytes = case.distinct * (H * 2 * H * 2 + 2 * H * 2)          # gate_up weights + bias of the touched experts
         achieved = kbytes / (mean_ms * 1e-3) / 1e9
-        grouped = case.T * case.K * H > 80 * 1024
-        return {"bound": "hbm", "kernel": ("umma_pair_kernel" if grouped else "gemv_kernel") + "<gate_up + bias + clamped SwiGLU>",
+        return {"bound": "hbm", "kernel": ("gemv_kernel" if case.uses_gemv() else "umma_pair_kernel") + "<gate_up + bias + clamped SwiGLU>",
                 "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                 "frac": achieved / peaks["hbm_gbs"], "traffic": None, "kernel_ms": mean_ms,
                 "peak_source": peaks["source"] + " (copy bandwidth)",

@@ -43,3 +43,18 @@ def test_decode_gemv_topk_weights():
     args[2] = torch.gather(inp["routing_weights"], 1, inp["router_indices"])
     out = run_experts(args, T, E, K, path="gemv")
     orc.check_close(out.float(), ref, RTOL_BF16, "gemv per-slot weights", rel_l2=REL_L2_BF16)
+
+
+@pytest.mark.parametrize("T,H,E,K", [(16, 2880, 128, 4), (32, 2880, 128, 4), (16, 2880, 32, 4), (32, 2880, 32, 4),
+                                     (16, 2048, 64, 8), (32, 2048, 64, 8), (31, 1024, 32, 4), (43, 2048, 64, 3)])
+def test_decode_rows_are_summed_in_fp32(T, H, E, K):
+    """Whichever kernels `auto` picks for a decode-sized call, no result is rounded to bf16 more often than on the
+    weight-streaming path: activations and output, not the K rows of a token.  Then the errors against 64 bits
+    agree but for elements whose fp32 sums fall on different sides of a rounding boundary (a row
+    rounding raises the error by a fifth)."""
+    inp = orc.make_inputs(T, H, E, K, seed=T + E, weight_std=0.02, bias_std=0.02, dtype=torch.bfloat16, weights_on="cuda")
+    args = [inp[k] for k in KEYS]
+    ref = orc.experts_forward_oracle(*[a.cpu() for a in args], T, E, K, compute_dtype=torch.float64)
+    gemv, auto = run_experts(args, T, E, K, path="gemv"), run_experts(args, T, E, K, path="auto")
+    err = [((o.double() - ref).norm() / ref.norm()).item() for o in (gemv, auto)]
+    assert err[1] <= 1.02 * err[0], err

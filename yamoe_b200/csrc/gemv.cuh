@@ -337,15 +337,20 @@ inline int gemv_down_ksplit(int64_t S, int E, int N) {
   return ctas <= 2 * 148 ? 2 : 1;     // measured: 53.6 / 55.0 / 55.6 us with 2 / 1 / 4 parts at T = 1; no gain beyond
 }
 
-// At most about 4 rows per expert: the kernels read an expert's weights once per 4 rows.  Where the
-// tensor-core GEMM (umma_pair.cuh) can take the call, it does from S * H = 80 K on: it needs some 25 us
-// for routing, gather and combine, and then reads every expert once whatever its number of rows.  Measured
-// per call, gemv / grouped:  H = 2880: S = 16 138 / 145 us (E = 32), S = 32 240 / 243 (E = 128) and
-// 224 / 196 (E = 32), S = 64 429 / 417;  H = 2048: S = 32 118 / 130, S = 64 186 / 186, S = 128 282 / 256;
-// H = 1024: S = 64 56 / 59, S = 128 76 / 60.
+// Decode-sized calls, at most about 4 rows per expert.  A token's K weighted rows are summed in fp32 there,
+// whichever kernels compute them: by atomics here, as fp32 rows (PairWeightedFlat) in the grouped GEMM.
+inline bool decode_sized(int64_t S, int E) { return S <= kGemvMaxS && S <= 4 * (int64_t)E; }
+
+// These kernels read an expert's weights once per 4 rows, the grouped GEMM (umma_pair.cuh) once whatever
+// its number of rows, after some 25 us of routing, gather and combine.  So the grouped GEMM takes the calls
+// with two or more rows per expert, from S * H = 80 K on.  Measured per call with L2 flushed, gemv / grouped,
+// H = 2880: E = 32 T = 16 298 / 266 us, T = 32 466 / 287, E = 128 T = 64 1004 / 870;  H = 2048, E = 64, K = 8:
+// T = 16 298 / 264, T = 32 446 / 283;  H = 1024, E = 32: T = 16 60 / 64, T = 32 85 / 72.  Between one and two
+// rows per expert it would be 5 to 9 % faster too (E = 128 T = 32 718 / 662, E = 32 T = 8 224 / 205); there the
+// sums keep the order that they have in these kernels.
 inline bool gemv_preferred(int64_t T, int H, int E, int K, bool tensor_cores) {
   const int64_t S = T * K;
-  return S <= kGemvMaxS && S <= 4 * (int64_t)E && (!tensor_cores || S * H <= 80 * 1024);
+  return decode_sized(S, E) && (!tensor_cores || S < 2 * (int64_t)E || S * H <= 80 * 1024);
 }
 
 template <int STAGE, int NB>

@@ -168,12 +168,14 @@ __global__ void routing_grad_kernel(const float* __restrict__ gw_row, const int3
 // One warp per token and 32 16-byte pieces of its row, with the loads of up to KB slots in flight: latency bounds the
 // few-token calls (a warp per token left most SMs idle and walked the columns one after the
 // other: 30 us at T = 64 and 512 with H = 2880, now about 5).
-template <typename T, int KB>
+// Rows of another type than the output (fp32 rows of a bf16 call) lie at their flat positions p = t*K + k.
+template <typename TY, typename T, int KB>
 __global__ void __launch_bounds__(kRowWarps * 32)
-combine_padded_kernel(const T* __restrict__ y, const int32_t* __restrict__ flat_row, T* __restrict__ out,
+combine_padded_kernel(const TY* __restrict__ y, const int32_t* __restrict__ flat_row, T* __restrict__ out,
                       int64_t Tn, int H, int K) {
   pdl_wait();
-  constexpr int VE = 16 / (int)sizeof(T);
+  constexpr bool kFlat = !std::is_same<TY, T>::value;
+  constexpr int VE = 16 / (int)sizeof(TY);
   const int64_t t = (int64_t)blockIdx.x * kRowWarps + (threadIdx.x >> 5);
   const int i = blockIdx.y * 32 + (threadIdx.x & 31);
   if (t >= Tn || i >= H / VE) return;
@@ -187,7 +189,7 @@ combine_padded_kernel(const T* __restrict__ y, const int32_t* __restrict__ flat_
     for (int k = 0; k < KB; ++k) r[k] = k0 + k < K ? __ldg(flat_row + t * K + k0 + k) : -1;
 #pragma unroll
     for (int k = 0; k < KB; ++k)
-      if (r[k] >= 0) load_vec<T, VE>(y + (size_t)r[k] * H + (size_t)i * VE, v[k]);
+      if (r[k] >= 0) load_vec<TY, VE>(y + (kFlat ? (size_t)(t * K + k0 + k) : (size_t)r[k]) * H + (size_t)i * VE, v[k]);
 #pragma unroll
     for (int k = 0; k < KB; ++k)
       if (r[k] >= 0) {
@@ -198,12 +200,11 @@ combine_padded_kernel(const T* __restrict__ y, const int32_t* __restrict__ flat_
   store_vec<T, VE>(out + (size_t)t * H + (size_t)i * VE, acc);
 }
 
-template <typename T>
-inline int launch_combine(const T* y, const int32_t* flat_row, T* out, int64_t Tn, int H, int K, cudaStream_t st) {
-  const dim3 grid((unsigned)ceil_div(Tn, kRowWarps), (unsigned)ceil_div(H, 32 * (16 / (int)sizeof(T))));
-  const cudaError_t rc =
-      K <= 4 ? launch_pdl_opt(true, combine_padded_kernel<T, 4>, grid, dim3(kRowWarps * 32), 0, st, y, flat_row, out, Tn, H, K)
-             : launch_pdl_opt(true, combine_padded_kernel<T, 8>, grid, dim3(kRowWarps * 32), 0, st, y, flat_row, out, Tn, H, K);
+template <typename TY, typename T>
+inline int launch_combine(const TY* y, const int32_t* flat_row, T* out, int64_t Tn, int H, int K, cudaStream_t st) {
+  const dim3 grid((unsigned)ceil_div(Tn, kRowWarps), (unsigned)ceil_div(H, 32 * (16 / (int)sizeof(TY))));
+  auto kern = K <= 4 ? combine_padded_kernel<TY, T, 4> : combine_padded_kernel<TY, T, 8>;
+  const cudaError_t rc = launch_pdl_opt(true, kern, grid, dim3(kRowWarps * 32), 0, st, y, flat_row, out, Tn, H, K);
   return rc == cudaSuccess && cudaGetLastError() == cudaSuccess ? YAMOE_OK : YAMOE_ERR_CUDA;
 }
 

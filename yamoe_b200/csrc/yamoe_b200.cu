@@ -215,7 +215,7 @@ static int forward_f32_split(const Plan& p, const float* hidden, const float* wg
   }
   if (rc) return rc;
   StageTimer tm(kStageCombine, st);
-  return launch_combine<float>(reinterpret_cast<const float*>(p.yrows), p.rt.flat_row, out, Tn, H, K, st);
+  return launch_combine(reinterpret_cast<const float*>(p.yrows), p.rt.flat_row, out, Tn, H, K, st);
 }
 
 template <typename T>
@@ -272,16 +272,26 @@ static int forward_impl(const void* hidden, const int64_t* ridx, const void* rw,
         rc = launch_umma_pair<kFwd>(g1, pglu, p.max_rows, p.max_tiles, 16, st);
       }
       if (rc) return rc;
-      // two-step combine: weighted rows out of the GEMM epilogue, then one gather-sum pass
-      const PairWeightedRows wrows{reinterpret_cast<const T*>(bd), reinterpret_cast<T*>(p.yrows), p.rt.row_token,
-                                   p.rt.row_weight, H};
+      // two-step combine: weighted rows out of the GEMM epilogue, then one gather-sum pass; decode-sized calls
+      // keep the rows in fp32 (4 S H bytes: at least 32 S padded rows of H bf16 exist there, see plan_forward)
+      const bool flat = decode_sized(p.S, E);
       {
         StageTimer tm(kStageDown, st);
-        rc = launch_umma_pair<kFwd>(g2, wrows, p.max_rows, p.max_tiles, 16, st);
+        if (flat) {
+          const PairWeightedFlat wflat{reinterpret_cast<const T*>(bd), reinterpret_cast<float*>(p.yrows), p.rt.row_token,
+                                       p.rt.row_flat, p.rt.row_weight, H};
+          rc = launch_umma_pair<kFwd>(g2, wflat, p.max_rows, p.max_tiles, 16, st);
+        } else {
+          const PairWeightedRows wrows{reinterpret_cast<const T*>(bd), reinterpret_cast<T*>(p.yrows), p.rt.row_token,
+                                       p.rt.row_weight, H};
+          rc = launch_umma_pair<kFwd>(g2, wrows, p.max_rows, p.max_tiles, 16, st);
+        }
       }
       if (rc) return rc;
       StageTimer tm(kStageCombine, st);
-      return launch_combine<T>(reinterpret_cast<const T*>(p.yrows), p.rt.flat_row, reinterpret_cast<T*>(out), Tn, H, K, st);
+      if (flat)
+        return launch_combine(reinterpret_cast<const float*>(p.yrows), p.rt.flat_row, reinterpret_cast<T*>(out), Tn, H, K, st);
+      return launch_combine(reinterpret_cast<const T*>(p.yrows), p.rt.flat_row, reinterpret_cast<T*>(out), Tn, H, K, st);
     }
   } else {
     {
@@ -331,7 +341,7 @@ static int forward_train_impl(const void* hidden, const int64_t* ridx, const voi
       if ((rc = launch_umma_f32<kFwd>(pair_args(p, act.p, H, wd, H, (int64_t)H * H, 0, H, H, E), act.stride, wrows,
                                       p.max_rows, p.max_tiles, 16, st)))
         return rc;
-      return launch_combine<T>(yrows, p.rt.flat_row, reinterpret_cast<T*>(out), Tn, H, K, st);
+      return launch_combine(yrows, p.rt.flat_row, reinterpret_cast<T*>(out), Tn, H, K, st);
     }
   }
   gather_rows_kernel<T><<<row_blocks, kRowWarps * 32, 0, st>>>(reinterpret_cast<const T*>(hidden),
@@ -358,7 +368,7 @@ static int forward_train_impl(const void* hidden, const int64_t* ridx, const voi
     launch_simt_gemm<T, kFwd>(g1, glu, p.max_rows, st);
     launch_simt_gemm<T, kFwd>(g2, wrows, p.max_rows, st);
   }
-  return launch_combine<T>(yrows, p.rt.flat_row, reinterpret_cast<T*>(out), Tn, H, K, st);
+  return launch_combine(yrows, p.rt.flat_row, reinterpret_cast<T*>(out), Tn, H, K, st);
 }
 
 // Input, weight and bias gradients in fp32 (the routing-weight gradients are left in p.gw_row); `acc` is zeroed.
