@@ -302,8 +302,9 @@ int yamoe_b200_router_forward(const void *hidden_states, const void *router_weig
  *       gathered rows, the biased pre-activations and the weighted activations
  *   yamoe_b200_experts_backward_saved   same gradients as yamoe_b200_experts_backward, reading them
  *       from `saved` instead of running routing, gather and the gate_up GEMM again.  `saved` must
- *       be untouched since the matching forward call with the same T, H, E, K, capacity and dtype;
- *       it is also the scratch of this call and is consumed by it.
+ *       be untouched since the matching forward call with the same T, H, E, K, capacity and dtype
+ *       (the selected path and the addresses of the weights may differ); it is also the scratch of
+ *       this call and is consumed by it.
  * ------------------------------------------------------------------------------------------- */
 int yamoe_b200_experts_forward_saving(const void *hidden_states, const int64_t *router_indices,
                                       const void *routing_weights, int routing_cols, const void *gate_up_proj,

@@ -73,6 +73,48 @@ def test_saved_activations_survive_a_change_of_path(first, second, dtype):
         orc.check_close(a.float().cpu(), b, RTOL_BF16 if dtype == torch.bfloat16 else RTOL_F32, n)
 
 
+def _moved(t, floats):
+    """A contiguous copy that starts `floats` elements behind a 16-byte boundary."""
+    buf = torch.empty(t.numel() + 4, dtype=t.dtype, device="cuda")
+    assert buf.data_ptr() % 16 == 0
+    return buf[floats:floats + t.numel()].view(t.shape).copy_(t)
+
+
+@pytest.mark.parametrize("H", [64, 192])
+@pytest.mark.parametrize("forward,backward", [(1, 0), (0, 1), (1, 1), (0, 0)])
+def test_saved_activations_survive_weights_that_move(H, forward, backward):
+    """fp32 weights at 4-byte alignment run on the CUDA cores, aligned ones on the tensor cores: the saved buffer
+    does not depend on which, so the weights may lie elsewhere in the backward pass."""
+    import yamoe_b200
+    args, grad, T, E = _problem([0, 5, 70, 130], H, torch.float32, seed=3)
+    dev = [a.cuda() for a in args]
+    out, saved = yamoe_b200.ops.experts_forward_saving(*dev[:3], _moved(dev[3], forward), dev[4],
+                                                       _moved(dev[5], forward), dev[6], T, E, 1)
+    got = yamoe_b200.ops.experts_backward_saved(grad.cuda(), saved, dev[2], _moved(dev[3], backward),
+                                                _moved(dev[5], backward), dev[6], T, E, 1)
+    orc.check_close(out.cpu(), orc.experts_forward_oracle(*args, T, E, 1), RTOL_F32, "saving forward")
+    for a, b, n in zip(got, orc.experts_backward_oracle(grad, *args, T, E, 1), GRADS):
+        orc.check_close(a.cpu(), b, RTOL_F32, n)
+
+
+@pytest.mark.parametrize("path", ["simt", "auto"])
+def test_saving_forward_runs_on_the_selected_path(path):
+    """K = 1: one product sum per output, so that the same kernels give the same bits."""
+    import yamoe_b200
+    args, grad, T, E = _problem([0, 5, 70, 130], 192, torch.float32, seed=4)
+    dev = [a.cuda() for a in args]
+    yamoe_b200.set_path(path)
+    try:
+        plain, (out, saved) = yamoe_b200.experts(*dev, T, E, 1), yamoe_b200.ops.experts_forward_saving(*dev, T, E, 1)
+        got = yamoe_b200.ops.experts_backward_saved(grad.cuda(), saved, dev[2], dev[3], dev[5], dev[6], T, E, 1)
+        ref = yamoe_b200.experts_backward(grad.cuda(), *dev, T, E, 1)
+    finally:
+        yamoe_b200.set_path("auto")
+    assert torch.equal(out, plain)
+    for i in (2, 3, 4, 5):                    # the other two are sums of atomics
+        assert torch.equal(got[i], ref[i]), GRADS[i]
+
+
 @pytest.mark.parametrize("T,E,K", [(8193, 7, 4), (8191, 300, 4), (9001, 16, 4), (2731, 33, 3)])
 def test_routing_of_many_assignments(T, E, K):
     """Around 32768 assignments, with ids outside [0, E) and a capacity that drops."""

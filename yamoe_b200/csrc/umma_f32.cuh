@@ -127,6 +127,35 @@ gather_split_kernel(const float* __restrict__ src, Planes dst, const int32_t* __
   }
 }
 
+// Between fp32 rows and planes of the same pitch: the buffer of the saving forward holds planes whichever kernels
+// fill and read it, and the CUDA-core kernels (weights that TMA cannot address, the validation path) work on rows.
+__global__ void __launch_bounds__(kRowWarps * 32)
+split_rows_kernel(const float* __restrict__ src, Planes dst, const int32_t* __restrict__ header) {
+  const int row = blockIdx.x * kRowWarps + (threadIdx.x >> 5);
+  if (row >= header[kHdrRowsUsed]) return;
+  for (int i = 4 * (threadIdx.x & 31); i < dst.ld; i += 128) {
+    const float4 v = *reinterpret_cast<const float4*>(src + (size_t)row * dst.ld + i);
+    dst.store2(row, i, v.x, v.y);
+    dst.store2(row, i + 2, v.z, v.w);
+  }
+}
+
+__global__ void __launch_bounds__(kRowWarps * 32)
+join_rows_kernel(Planes src, float* __restrict__ dst, const int32_t* __restrict__ header) {
+  const int row = blockIdx.x * kRowWarps + (threadIdx.x >> 5);
+  if (row >= header[kHdrRowsUsed]) return;
+  for (int i = 4 * (threadIdx.x & 31); i < src.ld; i += 128) {
+    const __nv_bfloat16* s = src.p + (size_t)row * src.ld + i;
+    float a[4], b[4], c[4];
+    load_vec<__nv_bfloat16, 4>(s, a);
+    load_vec<__nv_bfloat16, 4>(s + src.stride, b);
+    load_vec<__nv_bfloat16, 4>(s + 2 * src.stride, c);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) a[j] += b[j] + c[j];          // exact: see split3_mag
+    store_vec<float, 4>(dst + (size_t)row * src.ld + i, a);
+  }
+}
+
 // Gather of the upstream gradient: fp32 rows (M operand of the down weight gradient) and planes (N
 // operand of the data gradient); seeds the routing-weight gradient as gather_grad_kernel does.
 __global__ void __launch_bounds__(kRowWarps * 32)

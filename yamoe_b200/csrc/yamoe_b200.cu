@@ -151,7 +151,8 @@ static Plan plan_backward(void* ws, int64_t T, int H, int E, int K, int dtype) {
   p.actw = b.take<char>((size_t)p.max_rows * (H + kBiasCols) * nsize);
   p.gpre = b.take<char>((size_t)p.max_rows * 2 * H * p.esize);
   if (dtype == YAMOE_F32) {
-    p.gys_planes = b.take<char>((size_t)p.max_rows * H * nsize);
+    // (or the fp32 rows of actw, see saved_actw_rows)
+    p.gys_planes = b.take<char>((size_t)p.max_rows * std::max(H * 6, (H + kBiasCols) * 4));
     p.gpre_planes = b.take<char>((size_t)p.max_rows * 2 * H * nsize);
   }
   p.gw_row = b.take<float>(p.max_rows);
@@ -183,6 +184,16 @@ static bool use_split_f32(int path, int H, const void* wgu, const void* wd) {
   return umma_available() && H % 64 == 0 && ((reinterpret_cast<uintptr_t>(wgu) | reinterpret_cast<uintptr_t>(wd)) & 15) == 0 &&
          (path == YAMOE_PATH_AUTO || path == YAMOE_PATH_TCGEN05);
 }
+
+// Layout of xs and actw in the buffer that the saving forward hands to the backward pass: planes for the widths
+// that umma_f32.cuh serves, rows otherwise.  Only the shape decides, since path, weight pointers and their
+// alignment may differ between the two calls; CUDA-core kernels convert (saved_xs_rows).
+static bool saves_planes(int dtype, int H) { return dtype == YAMOE_F32 && umma_available() && H % 64 == 0; }
+
+// Scratch for xs and actw as fp32 rows [max_rows, H + kBiasCols], in regions that only the tensor-core kernels use
+// (12 H and max(6 H, 4 H + 4 kBiasCols) bytes per row, H >= 64).
+static float* saved_xs_rows(const Plan& p) { return reinterpret_cast<float*>(p.gpre_planes); }
+static float* saved_actw_rows(const Plan& p) { return reinterpret_cast<float*>(p.gys_planes); }
 
 static GemmArgs pair_args(const Plan& p, const void* A, int64_t lda, const void* B, int64_t ldb, int64_t stride, int M,
                           int N, int K, int E) {
@@ -326,8 +337,7 @@ static int forward_train_impl(const void* hidden, const int64_t* ridx, const voi
   const unsigned row_blocks = (unsigned)ceil_div(p.max_rows, kRowWarps);
   const int Hp = H + kBiasCols;
   if constexpr (sizeof(T) == 4) {
-    // (whatever path is selected: the backward pass has to find the layout that the forward left)
-    if (use_split_f32(YAMOE_PATH_AUTO, H, wgu, wd)) {
+    if (use_split_f32(current_path(), H, wgu, wd)) {
       const Planes xs = p.planes(p.xs, Hp), actw = p.planes(p.actw, Hp), act = p.planes(p.gpre_planes, H);
       gather_split_kernel<<<row_blocks, kRowWarps * 32, 0, st>>>(reinterpret_cast<const T*>(hidden), xs, p.rt.row_token,
                                                                  p.rt.header, H);
@@ -344,15 +354,17 @@ static int forward_train_impl(const void* hidden, const int64_t* ridx, const voi
       return launch_combine(yrows, p.rt.flat_row, reinterpret_cast<T*>(out), Tn, H, K, st);
     }
   }
-  gather_rows_kernel<T><<<row_blocks, kRowWarps * 32, 0, st>>>(reinterpret_cast<const T*>(hidden),
-                                                              reinterpret_cast<T*>(p.xs), p.rt.row_token,
+  const bool convert = saves_planes(dtype, H);
+  T* xs = reinterpret_cast<T*>(convert ? (void*)saved_xs_rows(p) : p.xs);
+  T* actw = reinterpret_cast<T*>(convert ? (void*)saved_actw_rows(p) : p.actw);
+  gather_rows_kernel<T><<<row_blocks, kRowWarps * 32, 0, st>>>(reinterpret_cast<const T*>(hidden), xs, p.rt.row_token,
                                                               p.rt.header, H, Hp);
   T* act = reinterpret_cast<T*>(p.gpre);
   T* yrows = reinterpret_cast<T*>(p.gys);
-  EpiGlu<T> glu{reinterpret_cast<const T*>(bgu), act, reinterpret_cast<T*>(p.actw), reinterpret_cast<T*>(p.pre),
+  EpiGlu<T> glu{reinterpret_cast<const T*>(bgu), act, actw, reinterpret_cast<T*>(p.pre),
                 p.rt.row_token, p.rt.row_weight, H, Hp};
   EpiWeightedRows<T> wrows{reinterpret_cast<const T*>(bd), yrows, p.rt.row_token, p.rt.row_weight, H};
-  GemmArgs g1{p.xs, Hp, wgu, 2 * (int64_t)H, (int64_t)H * 2 * H, 0, 2 * H, H, E,
+  GemmArgs g1{xs, Hp, wgu, 2 * (int64_t)H, (int64_t)H * 2 * H, 0, 2 * H, H, E,
               p.rt.tile_expert, p.rt.pad_off, p.rt.header};
   g1.pair_expert = p.rt.pair_expert; g1.pair_off = p.rt.pair_off; g1.counts = p.rt.counts;
   GemmArgs g2{act, H, wd, H, (int64_t)H * H, 0, H, H, E, p.rt.tile_expert, p.rt.pad_off, p.rt.header};
@@ -367,6 +379,12 @@ static int forward_train_impl(const void* hidden, const int64_t* ridx, const voi
   } else {
     launch_simt_gemm<T, kFwd>(g1, glu, p.max_rows, st);
     launch_simt_gemm<T, kFwd>(g2, wrows, p.max_rows, st);
+  }
+  if constexpr (sizeof(T) == 4) {
+    if (convert) {
+      split_rows_kernel<<<row_blocks, kRowWarps * 32, 0, st>>>(xs, p.planes(p.xs, Hp), p.rt.header);
+      split_rows_kernel<<<row_blocks, kRowWarps * 32, 0, st>>>(actw, p.planes(p.actw, Hp), p.rt.header);
+    }
   }
   return launch_combine(yrows, p.rt.flat_row, reinterpret_cast<T*>(out), Tn, H, K, st);
 }
@@ -437,7 +455,7 @@ static int backward_impl(const void* grad_out, int per_slot, const void* hidden,
     if (rc) return rc;
   }
   if constexpr (sizeof(T) == 4) {
-    if (use_split_f32(saved ? YAMOE_PATH_AUTO : path, H, wgu, wd)) {
+    if (use_split_f32(path, H, wgu, wd)) {
       rc = backward_f32_split(p, reinterpret_cast<const T*>(grad_out), per_slot ? K : 1, reinterpret_cast<const T*>(hidden),
                               reinterpret_cast<const T*>(wgu), reinterpret_cast<const T*>(bgu),
                               reinterpret_cast<const T*>(wd), reinterpret_cast<const T*>(bd), acc,
@@ -450,18 +468,27 @@ static int backward_impl(const void* grad_out, int per_slot, const void* hidden,
       return cudaGetLastError() == cudaSuccess ? YAMOE_OK : YAMOE_ERR_CUDA;
     }
   }
+  T* xs = reinterpret_cast<T*>(p.xs);
+  T* actw = reinterpret_cast<T*>(p.actw);
+  if constexpr (sizeof(T) == 4) {
+    if (saved && saves_planes(dtype, H)) {
+      xs = saved_xs_rows(p);
+      actw = saved_actw_rows(p);
+      join_rows_kernel<<<row_blocks, kRowWarps * 32, 0, st>>>(p.planes(p.xs, Hp), xs, p.rt.header);
+      join_rows_kernel<<<row_blocks, kRowWarps * 32, 0, st>>>(p.planes(p.actw, Hp), actw, p.rt.header);
+    }
+  }
   if (!saved)
-    gather_rows_kernel<T><<<row_blocks, kRowWarps * 32, 0, st>>>(reinterpret_cast<const T*>(hidden),
-                                                                reinterpret_cast<T*>(p.xs), p.rt.row_token,
-                                                                p.rt.header, H, Hp);
+    gather_rows_kernel<T><<<row_blocks, kRowWarps * 32, 0, st>>>(reinterpret_cast<const T*>(hidden), xs,
+                                                                p.rt.row_token, p.rt.header, H, Hp);
   gather_grad_kernel<T><<<row_blocks, kRowWarps * 32, 0, st>>>(
       reinterpret_cast<const T*>(grad_out), per_slot ? K : 1, reinterpret_cast<const T*>(bd),
       reinterpret_cast<T*>(p.gys), p.gw_row, p.rt.row_token, p.rt.tile_expert, p.rt.header, H);
 
   // 1. recompute: pre = xs W_gu + b_gu,  actw = w * glu(pre)
-  EpiGlu<T> glu{reinterpret_cast<const T*>(bgu), nullptr, reinterpret_cast<T*>(p.actw),
-                reinterpret_cast<T*>(p.pre), p.rt.row_token, p.rt.row_weight, H, Hp};
-  GemmArgs g1{p.xs, Hp, wgu, 2 * (int64_t)H, (int64_t)H * 2 * H, 0, 2 * H, H, E,
+  EpiGlu<T> glu{reinterpret_cast<const T*>(bgu), nullptr, actw, reinterpret_cast<T*>(p.pre), p.rt.row_token,
+                p.rt.row_weight, H, Hp};
+  GemmArgs g1{xs, Hp, wgu, 2 * (int64_t)H, (int64_t)H * 2 * H, 0, 2 * H, H, E,
               p.rt.tile_expert, p.rt.pad_off, p.rt.header};
   g1.pair_expert = p.rt.pair_expert; g1.pair_off = p.rt.pair_off; g1.counts = p.rt.counts;
   // 2. gI' = gys W_d^T; fused GLU backward -> gpre, routing-weight gradient -> gw_row
@@ -471,7 +498,7 @@ static int backward_impl(const void* grad_out, int per_slot, const void* hidden,
   g2.pair_expert = p.rt.pair_expert; g2.pair_off = p.rt.pair_off; g2.counts = p.rt.counts;
   // 3. dW_d[e] = actw_e^T gys_e; the column of routing weights behind actw adds db_d[e] as output row H
   EpiStoreBias<T> st_wd{reinterpret_cast<T*>(d_wd), reinterpret_cast<T*>(d_bd), H, H};
-  GemmArgs g3{p.actw, Hp, p.gys, H, 0, H + 1, H, 0, E, p.rt.tile_expert, p.rt.pad_off, p.rt.header};
+  GemmArgs g3{actw, Hp, p.gys, H, 0, H + 1, H, 0, E, p.rt.tile_expert, p.rt.pad_off, p.rt.header};
   g3.pair_expert = p.rt.pair_expert; g3.pair_off = p.rt.pair_off; g3.counts = p.rt.counts;
   // 4. dHidden[token] += gpre W_gu^T
   EpiScatterAdd<T, false, false> sc_dh{nullptr, acc, p.rt.row_token, p.rt.row_weight, H};
@@ -480,7 +507,7 @@ static int backward_impl(const void* grad_out, int per_slot, const void* hidden,
   g4.pair_expert = p.rt.pair_expert; g4.pair_off = p.rt.pair_off; g4.counts = p.rt.counts;
   // 5. dW_gu[e] = xs_e^T gpre_e; the column of ones behind xs adds db_gu[e] as output row H
   EpiStoreBias<T> st_wgu{reinterpret_cast<T*>(d_wgu), reinterpret_cast<T*>(d_bgu), H, 2 * H};
-  GemmArgs g5{p.xs, Hp, p.gpre, 2 * (int64_t)H, 0, H + 1, 2 * H, 0, E, p.rt.tile_expert, p.rt.pad_off, p.rt.header};
+  GemmArgs g5{xs, Hp, p.gpre, 2 * (int64_t)H, 0, H + 1, 2 * H, 0, E, p.rt.tile_expert, p.rt.pad_off, p.rt.header};
   g5.pair_expert = p.rt.pair_expert; g5.pair_off = p.rt.pair_off; g5.counts = p.rt.counts;
 
   if (use_tcgen05(path, dtype, H)) {
