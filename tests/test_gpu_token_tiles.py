@@ -141,10 +141,44 @@ def test_routing_of_many_assignments(T, E, K):
     orc.check_close(out.cpu(), ref, RTOL_F32, "forward")
 
 
-@pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan"), 3.0e38])
+def test_fp32_products_keep_24_bits():
+    """One token: the gate_up weight gradient is a single product x_i * g_j, the bias gradient g_j itself (x = 1).
+    The bf16 parts that are multiplied leave out at most 2^-24 of a product, and the accumulator is cut off
+    once at its full magnitude (2^-23) and five times at 2^-7 of it or less."""
+    import yamoe_b200
+    H, g = 64, torch.Generator().manual_seed(8)
+    worst = [0x3f80ffff, 0x3f817fff, 0x3f807fff, 0x3f80ff7f, 0x3f8080ff, 0x3fffffff, 0x3f7fffff, 0x3f808080]
+    bits = torch.tensor(worst * 4 + [0] * 32, dtype=torch.int32)
+    x = torch.where(bits != 0, bits.view(torch.float32), torch.randn(H, generator=g))
+    x = (x * 2.0 ** torch.randint(-9, 3, (H,), generator=g) * (1 - 2 * torch.randint(0, 2, (H,), generator=g))).view(1, H)
+    args = [x, torch.zeros(1, 1, dtype=torch.long), torch.ones(1, 1)] + [
+        torch.randn(*s, generator=g) * 0.1 for s in ((1, H, 2 * H), (1, 2 * H), (1, H, H), (1, H))]
+    grads = yamoe_b200.experts_backward(torch.randn(1, H, generator=g).cuda(), *[a.cuda() for a in args], 1, 1, 1)
+    got, bias = grads[2][0].cpu().double(), grads[3][0].cpu().double()
+    want = x[0].double()[:, None] * bias[None, :]
+    assert (want != 0).all()
+    assert ((got - want) / want).abs().max().item() <= 2.0 ** -24 + 2.0 ** -23 + 5 * 2.0 ** -30
+
+
+@pytest.mark.parametrize("H", [64, 320, 1024])
+def test_fp32_against_64_bits(H):
+    """Relative error in the 2-norm.  A GEMM's 64-deep blocks are cut off about four times at full magnitude
+    (4 * 2^-23) and their sums rounded; a forward is two of them and the activation's few units of 2^-23, a
+    gradient one more: 16 * 2^-23.  Without the third parts of the operands it is about 1e-5."""
+    import yamoe_b200
+    args, grad, T, E = _problem([0, 5, 70, 130, 33], H, torch.float32, seed=9)
+    dev = [a.cuda() for a in args]
+    got = [yamoe_b200.experts(*dev, T, E, 1), *yamoe_b200.experts_backward(grad.cuda(), *dev, T, E, 1)]
+    ref = [orc.experts_forward_oracle(*args, T, E, 1, compute_dtype=torch.float64),
+           *orc.experts_backward_oracle(grad, *args, T, E, 1, compute_dtype=torch.float64)]
+    for a, b, n in zip(got, ref, ["out"] + GRADS):
+        assert ((a.cpu().double() - b).norm() / b.norm()).item() <= 16 * 2.0 ** -23, n
+
+
+@pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan"), 3.0e38, 3.395e38])
 def test_fp32_parts_of_special_values(value):
     """Every output is NaN, infinite or finite where the CUDA-core kernel's is; weights are multiples of
-    1/64, whose lower parts vanish."""
+    1/64, whose lower parts vanish.  bf16 rounds 3.395e38 to infinity."""
     import yamoe_b200
     args, grad, T, E = _problem([20, 33, 0, 70], 128, torch.float32, seed=5)
     for i in (3, 5):
@@ -156,6 +190,9 @@ def test_fp32_parts_of_special_values(value):
         yamoe_b200.set_path(path)
         try:
             res[path] = [yamoe_b200.experts(*dev, T, E, 1), *yamoe_b200.experts_backward(grad.cuda(), *dev, T, E, 1)]
+            out, saved = yamoe_b200.ops.experts_forward_saving(*dev, T, E, 1)
+            res[path] += [out, *yamoe_b200.ops.experts_backward_saved(grad.cuda(), saved, dev[2], dev[3], dev[5], dev[6],
+                                                                      T, E, 1)]
         finally:
             yamoe_b200.set_path("auto")
     for a, b in zip(res["auto"], res["simt"]):

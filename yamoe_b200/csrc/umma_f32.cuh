@@ -1,6 +1,9 @@
-// fp32 grouped GEMM on the tensor cores (sm_100a): every fp32 operand is the exact sum of three bf16
-// parts of eight significant bits each, and six of the nine partial products are multiplied with
-// tcgen05.mma (bf16, fp32 accumulation).  The three that are left out are below 2^-24 of the product.
+// fp32 grouped GEMM on the tensor cores (sm_100a): every fp32 operand is the sum of three bf16 parts (split3),
+// and six of the nine partial products are multiplied with tcgen05.mma (bf16, fp32 accumulation).  The three that
+// are left out amount to at most 2^-24 of the product, of either sign, like the rounding of an FFMA: the
+// parts are rounded to nearest.  (Cut off instead, all of one sign, they reached 2^-21 and shrank
+// every product.)  Splitting into bf16 parts for the tensor cores: G. Henry, P. T. P. Tang and A. Heinecke,
+// "Leveraging the bfloat16 artificial intelligence datatype for higher-precision computations", ARITH 2019.
 //
 //   arrangement   M operand (256), fp32, split on the way       N operand (up to 128), three bf16 planes
 //   kFwd          W[e][k][m]   weight columns                   rows of the expert, K-major
@@ -19,13 +22,14 @@
 // Precision.  The tensor core adds to an accumulator by truncation, whose errors would add up over a
 // long reduction.  Each 64-deep k-block therefore starts a fresh accumulator, takes the small
 // products first and the leading one last, and the block's sum is added to a running sum in registers
-// with round-to-nearest.  Against 64 bits the README forward is 3.9e-7 off where the FFMA kernel's serial
-// sum is 1.6e-6, the gradients of 600 tokens (H = 1024) at most 3.5e-7 against 1.1e-6.
+// with round-to-nearest.  Against 64 bits the README forward is 3.0e-7 off where the FFMA kernel's serial
+// sum is 1.6e-6, the gradients of 600 tokens (H = 1024) at most 2.7e-7 against 1.1e-6; at H = 64, where the serial sum
+// is short, 2.1e-7 against 2.5e-7.
 //
 // Measured: gate_up of the README forward (T = 512, H = 2880, E = 8, K = 2) 213 us = 160 TFLOP/s of the
-// original product; the whole forward 422 us against 1797, a training step of 600 tokens 405 against 1191.
+// original product; the whole forward 412 us against 1797, a training step of 600 tokens 412 against 1191.
 //
-// Infinities and NaN behave as in fp32 arithmetic: see split3_mag.
+// Infinities and NaN behave as in fp32 arithmetic: see split3_special.
 //
 // Two CTAs share a tile (cta_group::2), 128 weight columns each: the planes are the larger half of what
 // L2 has to deliver (48 KB per 64-deep block against 32 KB of weights), and a pair needs them once.
@@ -53,29 +57,58 @@ constexpr int kF32Smem = kF32WStages * kF32WBytes + kF32BStages * kF32BBytes + 1
 constexpr int kF32TmemA = 256;                           // first TMEM column of the A operands
 constexpr int kF32TmemAStride = 96;                      // 3 parts x 32 columns (64 bf16)
 
-// The three parts of |x| (value bits in the upper half of the words; the sign is put back by the
-// caller): a, b, c with a + b + c = |x|, exactly for normal numbers.  A part that would be zero is
-// |x| * 2^-40 instead (zero for x = 0): an infinite operand then meets no zero part of a finite
-// non-zero one, so that inf * y is inf and not NaN; for x = inf all parts are inf, for NaN b and c are.
-__device__ __forceinline__ void split3_mag(float x, uint32_t& b, uint32_t& c) {
-  const float ax = fabsf(x);
-  const float tiny = ax * 9.094947017729282e-13f;        // 2^-40
-  const float a = __uint_as_float(__float_as_uint(ax) & 0xffff0000u);
-  const float r = ax - a;
-  const float bf = __uint_as_float(__float_as_uint(r) & 0xffff0000u);
-  b = __float_as_uint(fmaxf(bf, tiny));
-  c = __float_as_uint(fmaxf(r - bf, tiny));
+// The three parts of a number: a = bf16(x), b = bf16(x - a), c = x - a - b, each rounded to nearest (halves away from
+// zero).  They sum to x exactly for |x| >= 2^-110 (below that c falls short of the last bits), with |b| <= 2^-8
+// and |c| <= 2^-17 of the power of two below |x|.
+//
+// Zero parts would turn inf * y into NaN, and parts of mixed signs inf into NaN as well.  So an infinity or NaN is
+// (+-1, 0, x): x meets nothing but the leading part of the other factor, and inf * inf stays infinite.
+// The finite numbers that bf16 rounds to infinity (the last 0.4 % of the range) are truncated instead.
+__device__ __forceinline__ uint32_t round_bf16_bits(float x) { return __float_as_uint(x) + 0x8000u; }   // upper half
+__device__ __forceinline__ float upper_half(uint32_t u) { return __uint_as_float(u & 0xffff0000u); }
+
+__device__ __forceinline__ uint3 split3_special(float x) {
+  const uint32_t u = __float_as_uint(x);
+  if (!(fabsf(x) <= 3.402823466e38f)) return make_uint3((u & 0x80000000u) | 0x3f800000u, 0u, x != x ? 0x7fff0000u : u);
+  uint32_t a = u + 0x8000u;
+  if ((a & 0x7f800000u) == 0x7f800000u) a = u;
+  const float r = x - upper_half(a);
+  const uint32_t b = round_bf16_bits(r);
+  return make_uint3(a, b, __float_as_uint(r - upper_half(b)));
 }
 
-// bf16 pairs (x0 in the low half) of the three parts of two numbers
-__device__ __forceinline__ void split3_pair(float x0, float x1, uint32_t& p0, uint32_t& p1, uint32_t& p2) {
-  uint32_t b0, c0, b1, c1;
-  split3_mag(x0, b0, c0);
-  split3_mag(x1, b1, c1);
-  p0 = __byte_perm(__float_as_uint(x0), __float_as_uint(x1), 0x7632);
-  const uint32_t sign = p0 & 0x80008000u;
-  p1 = __byte_perm(b0, b1, 0x7632) | sign;
-  p2 = __byte_perm(c0, c1, 0x7632) | sign;
+// The parts of N numbers as bf16 pairs (the first of a pair in the low half).  Returns NaN where one of them is special;
+// the caller then has it done again.  One look at all N: a branch for each pair keeps the loads of the next from
+// being issued ahead (README forward 513 us, now 412; 511 with cvt.rn.bf16x2 instead of integer arithmetic).
+template <int N>
+__device__ __forceinline__ float split3_finite(const float (&x)[N], uint32_t (&p0)[N / 2], uint32_t (&p1)[N / 2],
+                                               uint32_t (&p2)[N / 2]) {
+  float bad = 0.f;
+#pragma unroll
+  for (int i = 0; i < N; i += 2) {
+    const uint32_t a0 = round_bf16_bits(x[i]), a1 = round_bf16_bits(x[i + 1]);
+    const float r0 = x[i] - upper_half(a0), r1 = x[i + 1] - upper_half(a1);
+    const uint32_t b0 = round_bf16_bits(r0), b1 = round_bf16_bits(r1);
+    const float c0 = r0 - upper_half(b0), c1 = r1 - upper_half(b1);
+    p0[i / 2] = __byte_perm(a0, a1, 0x7632);
+    p1[i / 2] = __byte_perm(b0, b1, 0x7632);
+    p2[i / 2] = __byte_perm(__float_as_uint(c0), __float_as_uint(c1), 0x7632);
+    bad += c0 + c1;                          // NaN where a leading part is not finite
+  }
+  return bad;
+}
+template <int N>
+__device__ __forceinline__ void split3(const float (&x)[N], uint32_t (&p0)[N / 2], uint32_t (&p1)[N / 2], uint32_t (&p2)[N / 2]) {
+  const float bad = split3_finite<N>(x, p0, p1, p2);
+  if (bad != bad) {
+#pragma unroll
+    for (int i = 0; i < N; i += 2) {
+      const uint3 s0 = split3_special(x[i]), s1 = split3_special(x[i + 1]);
+      p0[i / 2] = __byte_perm(s0.x, s1.x, 0x7632);
+      p1[i / 2] = __byte_perm(s0.y, s1.y, 0x7632);
+      p2[i / 2] = __byte_perm(s0.z, s1.z, 0x7632);
+    }
+  }
 }
 
 // Where an activation matrix is kept as three bf16 planes: [3][rows][ld].
@@ -83,22 +116,50 @@ struct Planes {
   __nv_bfloat16* p;
   int64_t stride;                   // elements between planes
   int ld;
-  __device__ __forceinline__ void store1(size_t row, int col, float x) const {
-    uint32_t p0, p1, p2;
-    split3_pair(x, 0.f, p0, p1, p2);
+  // four adjacent columns, col a multiple of four
+  __device__ __forceinline__ void store4(size_t row, int col, const float (&x)[4]) const {
+    uint32_t q0[2], q1[2], q2[2];
+    split3<4>(x, q0, q1, q2);
+    __nv_bfloat16* d = p + row * ld + col;
+    *reinterpret_cast<uint2*>(d) = make_uint2(q0[0], q0[1]);
+    *reinterpret_cast<uint2*>(d + stride) = make_uint2(q1[0], q1[1]);
+    *reinterpret_cast<uint2*>(d + 2 * stride) = make_uint2(q2[0], q2[1]);
+  }
+  __device__ __forceinline__ void store1(size_t row, int col, float x) const {        // special or not
+    const uint3 s = split3_special(x);
     unsigned short* d = reinterpret_cast<unsigned short*>(p) + row * ld + col;
-    d[0] = (unsigned short)p0;
-    d[stride] = (unsigned short)p1;
-    d[2 * stride] = (unsigned short)p2;
+    d[0] = (unsigned short)(s.x >> 16);
+    d[stride] = (unsigned short)(s.y >> 16);
+    d[2 * stride] = (unsigned short)(s.z >> 16);
+  }
+  // For epilogues: what the functions below return is NaN where a number was special; the caller then stores again with
+  // store1, from values that it reads back (kept in registers for that, they cost more than the splitting).
+  // One column of two adjacent rows, of which `rows` exist
+  __device__ __forceinline__ float store_rows2(size_t row, int col, int rows, const float (&x)[2]) const {
+    uint32_t q0[1], q1[1], q2[1];
+    const float bad = split3_finite<2>(x, q0, q1, q2);
+    unsigned short* d = reinterpret_cast<unsigned short*>(p) + row * ld + col;
+    if (rows > 0) {
+      d[0] = (unsigned short)q0[0];
+      d[stride] = (unsigned short)q1[0];
+      d[2 * stride] = (unsigned short)q2[0];
+    }
+    if (rows > 1) {
+      d[ld] = (unsigned short)(q0[0] >> 16);
+      d[ld + stride] = (unsigned short)(q1[0] >> 16);
+      d[ld + 2 * stride] = (unsigned short)(q2[0] >> 16);
+    }
+    return bad;
   }
   // two adjacent columns, col even
-  __device__ __forceinline__ void store2(size_t row, int col, float x0, float x1) const {
-    uint32_t q0, q1, q2;
-    split3_pair(x0, x1, q0, q1, q2);
+  __device__ __forceinline__ float store2(size_t row, int col, float x0, float x1) const {
+    uint32_t q0[1], q1[1], q2[1];
+    const float bad = split3_finite<2>({x0, x1}, q0, q1, q2);
     __nv_bfloat16* d = p + row * ld + col;
-    *reinterpret_cast<uint32_t*>(d) = q0;
-    *reinterpret_cast<uint32_t*>(d + stride) = q1;
-    *reinterpret_cast<uint32_t*>(d + 2 * stride) = q2;
+    *reinterpret_cast<uint32_t*>(d) = q0[0];
+    *reinterpret_cast<uint32_t*>(d + stride) = q1[0];
+    *reinterpret_cast<uint32_t*>(d + 2 * stride) = q2[0];
+    return bad;
   }
 };
 
@@ -118,12 +179,7 @@ gather_split_kernel(const float* __restrict__ src, Planes dst, const int32_t* __
       if (4 * i < H) v = __ldg(s + i);
       else if (4 * i == H) v.x = 1.f;
     }
-    uint2 q[3];
-    split3_pair(v.x, v.y, q[0].x, q[1].x, q[2].x);
-    split3_pair(v.z, v.w, q[0].y, q[1].y, q[2].y);
-    __nv_bfloat16* d = dst.p + (size_t)row * dst.ld + 4 * i;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) *reinterpret_cast<uint2*>(d + k * dst.stride) = q[k];
+    dst.store4(row, 4 * i, {v.x, v.y, v.z, v.w});
   }
 }
 
@@ -135,8 +191,7 @@ split_rows_kernel(const float* __restrict__ src, Planes dst, const int32_t* __re
   if (row >= header[kHdrRowsUsed]) return;
   for (int i = 4 * (threadIdx.x & 31); i < dst.ld; i += 128) {
     const float4 v = *reinterpret_cast<const float4*>(src + (size_t)row * dst.ld + i);
-    dst.store2(row, i, v.x, v.y);
-    dst.store2(row, i + 2, v.z, v.w);
+    dst.store4(row, i, {v.x, v.y, v.z, v.w});
   }
 }
 
@@ -151,7 +206,7 @@ join_rows_kernel(Planes src, float* __restrict__ dst, const int32_t* __restrict_
     load_vec<__nv_bfloat16, 4>(s + src.stride, b);
     load_vec<__nv_bfloat16, 4>(s + 2 * src.stride, c);
 #pragma unroll
-    for (int j = 0; j < 4; ++j) a[j] += b[j] + c[j];          // exact: see split3_mag
+    for (int j = 0; j < 4; ++j) a[j] += b[j] + c[j];          // exact: see split3_special
     store_vec<float, 4>(dst + (size_t)row * src.ld + i, a);
   }
 }
@@ -183,8 +238,7 @@ gather_grad_split_kernel(const float* __restrict__ grad_out, int slots, const fl
       for (int j = 0; j < 4; ++j) dot += g[j] * b[j];
     }
     store_vec<float, 4>(gys + (size_t)row * H + 4 * (size_t)i, g);
-    dst.store2(row, 4 * i, g[0], g[1]);
-    dst.store2(row, 4 * i + 2, g[2], g[3]);
+    dst.store4(row, 4 * i, g);
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
@@ -238,26 +292,44 @@ struct F32Glu {                     // see PairGlu
     const int t0 = odd ? 8 : 0, j = m >> 1;
     float w_lane;
     const unsigned have = row_info(row_token, TRAIN ? row_weight : nullptr, row, nvalid, lane, w_lane);
+    float bad = 0.f;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int t = t0 + i;
-      const bool ok = (have >> t) & 1u;
-      const float w = TRAIN ? __shfl_sync(0xffffffffu, w_lane, t) : 0.f;
-      const float a = ok ? glu_act(g[i], u[i]) : 0.f;
-      if (t < nvalid) {
-        if (act.p != nullptr) act.store1(row + t, j, a);
-        if constexpr (TRAIN) {
+    for (int i = 0; i < 8; i += 2) {
+      float a[2], aw[2];
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const int t = t0 + i + k;
+        const bool ok = (have >> t) & 1u;
+        const float w = TRAIN ? __shfl_sync(0xffffffffu, w_lane, t) : 0.f;
+        a[k] = ok ? glu_act(g[i + k], u[i + k]) : 0.f;
+        aw[k] = a[k] * w;
+        if (TRAIN && t < nvalid)
           *reinterpret_cast<float2*>(pre + (size_t)(row + t) * 2 * H + (m & ~1)) =
-              ok ? make_float2(g[i], u[i]) : make_float2(0.f, 0.f);
-          actw.store1(row + t, j, a * w);
+              ok ? make_float2(g[i + k], u[i + k]) : make_float2(0.f, 0.f);
+      }
+      if (act.p != nullptr) bad += act.store_rows2(row + t0 + i, j, nvalid - t0 - i, a);
+      if constexpr (TRAIN) bad += actw.store_rows2(row + t0 + i, j, nvalid - t0 - i, aw);
+    }
+    if (bad != bad) {
+      if constexpr (TRAIN) {
+#pragma unroll 1
+        for (int t = t0; t < min(t0 + 8, nvalid); ++t) {
+          const float2 q = *reinterpret_cast<const float2*>(pre + (size_t)(row + t) * 2 * H + (m & ~1));
+          const float x = glu_act(q.x, q.y);       // 0 for the (0, 0) of a padding row
+          if (act.p != nullptr) act.store1(row + t, j, x);
+          actw.store1(row + t, j, row_token[row + t] >= 0 ? x * row_weight[row + t] : 0.f);
         }
+      } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+          if (t0 + i < nvalid) act.store1(row + t0 + i, j, (have >> (t0 + i)) & 1u ? glu_act(g[i], u[i]) : 0.f);
       }
     }
     if constexpr (TRAIN) {
       if (m == lane)               // columns 0..31: this warp also fills the columns behind H with (w, 0, 0, ...)
         for (int t = 0; t < nvalid; ++t) {
           const float w = __shfl_sync(0xffffffffu, w_lane, t);
-          for (int c = H + 2 * lane; c < actw.ld; c += 64) actw.store2(row + t, c, c == H ? w : 0.f, 0.f);
+          for (int c = H + 4 * lane; c < actw.ld; c += 128) actw.store4(row + t, c, {c == H ? w : 0.f, 0.f, 0.f, 0.f});
         }
     }
   }
@@ -315,6 +387,7 @@ struct F32GluBackward {             // see PairGluBackward; the gradient leaves 
     const unsigned have = row_info(row_token, row_weight, row, nvalid, lane, w_lane);
     const float2* src = reinterpret_cast<const float2*>(pre) + (size_t)row * H + m;
     float2* dst = reinterpret_cast<float2*>(g_pre) + (size_t)row * H + m;
+    float bad = 0.f;
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
       const bool ok = (have >> i) & 1u;
@@ -333,7 +406,15 @@ struct F32GluBackward {             // see PairGluBackward; the gradient leaves 
       if (pu > kLimit || pu < -kLimit || !ok) gu = 0.f;
       if (i < nvalid) {
         dst[(size_t)i * H] = make_float2(gg, gu);
-        g_planes.store2(row + i, 2 * m, gg, gu);
+        bad += g_planes.store2(row + i, 2 * m, gg, gu);
+      }
+    }
+    if (bad != bad) {
+#pragma unroll 1
+      for (int i = 0; i < nvalid; ++i) {
+        const float2 q = dst[(size_t)i * H];
+        g_planes.store1(row + i, 2 * m, q.x);
+        g_planes.store1(row + i, 2 * m + 1, q.y);
       }
     }
     // lane L ends with half the sum of row L & 15, its partner L ^ 16 with the other half
@@ -388,6 +469,9 @@ __device__ __forceinline__ void tc_st_32x8(uint32_t taddr, const uint32_t (&r)[8
   asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%8], {%0, %1, %2, %3, %4, %5, %6, %7};"
                ::"r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(taddr)
                : "memory");
+}
+__device__ __forceinline__ void tc_st_32x1(uint32_t taddr, uint32_t r) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%1], {%0};" ::"r"(r), "r"(taddr) : "memory");
 }
 __device__ __forceinline__ void tc_ld_32x16(uint32_t taddr, uint32_t (&r)[16]) {
   asm volatile(
@@ -642,25 +726,44 @@ umma_f32_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__
         const uint32_t t = tmem_base + kF32TmemA + slot * kF32TmemAStride + khalf * 16 + ((uint32_t)(q * 32) << 16);
 #pragma unroll
         for (int h = 0; h < 2; ++h) {                // 16 k at a time
-          uint32_t p0[8], p1[8], p2[8];
+          // MODE kDgrad: 32 k of row mrow are 128 bytes, 16-byte pieces swizzled by the row
+          const uint8_t* rowp = tile + khalf * (kF32WBytes / 2) + mrow * 128;
+          const float* colp = reinterpret_cast<const float*>(tile) + (khalf * 32 + h * 16) * kF32M + mrow;
+          float x[16];
           if constexpr (MODE == kDgrad) {
-            // 32 k of row mrow: 128 bytes, 16-byte pieces swizzled by the row
-            const uint8_t* rowp = tile + khalf * (kF32WBytes / 2) + mrow * 128;
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-              const float4 x = *reinterpret_cast<const float4*>(rowp + (((h * 4 + i) ^ (mrow & 7)) << 4));
-              split3_pair(x.x, x.y, p0[2 * i], p1[2 * i], p2[2 * i]);
-              split3_pair(x.z, x.w, p0[2 * i + 1], p1[2 * i + 1], p2[2 * i + 1]);
+              const float4 f = *reinterpret_cast<const float4*>(rowp + (((h * 4 + i) ^ (mrow & 7)) << 4));
+              x[4 * i] = f.x; x[4 * i + 1] = f.y; x[4 * i + 2] = f.z; x[4 * i + 3] = f.w;
             }
           } else {
-            const float* colp = reinterpret_cast<const float*>(tile) + (khalf * 32 + h * 16) * kF32M + mrow;
 #pragma unroll
-            for (int i = 0; i < 8; ++i)
-              split3_pair(colp[2 * i * kF32M], colp[(2 * i + 1) * kF32M], p0[i], p1[i], p2[i]);
+            for (int i = 0; i < 16; ++i) x[i] = colp[i * kF32M];
           }
+          uint32_t p0[8], p1[8], p2[8];
+          const float bad = split3_finite<16>(x, p0, p1, p2);
           tc_st_32x8(t + h * 8, p0);
           tc_st_32x8(t + h * 8 + 32, p1);
           tc_st_32x8(t + h * 8 + 64, p2);
+          if (__any_sync(0xffffffffu, bad != bad)) {
+            tc_st_wait();
+#pragma unroll 1
+            for (int i = 0; i < 8; ++i) {            // rolled, from memory again: rare, and hot code stays short
+              float y0, y1;
+              if constexpr (MODE == kDgrad) {
+                const uint8_t* q = rowp + (((h * 4 + (i >> 1)) ^ (mrow & 7)) << 4) + 8 * (i & 1);
+                y0 = *reinterpret_cast<const float*>(q);
+                y1 = *reinterpret_cast<const float*>(q + 4);
+              } else {
+                y0 = colp[2 * i * kF32M];
+                y1 = colp[(2 * i + 1) * kF32M];
+              }
+              const uint3 s0 = split3_special(y0), s1 = split3_special(y1);
+              tc_st_32x1(t + h * 8 + i, __byte_perm(s0.x, s1.x, 0x7632));
+              tc_st_32x1(t + h * 8 + i + 32, __byte_perm(s0.y, s1.y, 0x7632));
+              tc_st_32x1(t + h * 8 + i + 64, __byte_perm(s0.z, s1.z, 0x7632));
+            }
+          }
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&bar_w_empty[ws]));
