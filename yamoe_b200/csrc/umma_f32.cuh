@@ -717,9 +717,9 @@ umma_f32_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__
       decode(id, e_next, e, m0, n0, width, kblocks);
       e_next = expert_of(id + n_clusters);
       for (int kb = 0; kb < kblocks; ++kb) {
-        ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_w_full[ws]), wph, &abort_flag));
+        ok = mbar_wait_warp(smem_u32(&bar_w_full[ws]), wph, &abort_flag);
         if (!ok) break;
-        ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_a_empty[slot]), phase ^ 1u, &abort_flag));
+        ok = mbar_wait_warp(smem_u32(&bar_a_empty[slot]), phase ^ 1u, &abort_flag);
         if (!ok) break;
         tc_fence_after();
         const uint8_t* tile = smem_raw + (smem_base - smem_u32(smem_raw)) + ws * kF32WBytes;
@@ -794,7 +794,7 @@ umma_f32_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__
 #pragma unroll
       for (int i = 0; i < 64; ++i) acc[i] = 0.f;
       for (int kb = 0; kb < kblocks; ++kb) {
-        ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_acc_full[slot]), phase, &abort_flag));
+        ok = mbar_wait_warp(smem_u32(&bar_acc_full[slot]), phase, &abort_flag);
         if (!ok) break;
         tc_fence_after();
         const uint32_t t = tmem_base + slot * kF32N + nhalf * 64 + ((uint32_t)(q * 32) << 16);

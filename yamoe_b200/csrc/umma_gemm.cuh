@@ -109,6 +109,12 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   }
 }
 
+// The same by a whole warp, with one outcome for all its lanes.  Each lane has a clock of its own: where some gave up
+// and others got through, those would wait for the missing lanes in the next warp-wide instruction.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
+}
+
 // Test aid: one thread waits, with the given limit, on a barrier that nothing ever arrives at,
 // and records what the grouped GEMM's roles record when a wait gives up.  No TMA, no TMEM.
 __global__ void mbar_wait_probe_kernel(int32_t* header, uint64_t limit_ns) {
@@ -549,7 +555,7 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         continue;
       }
       if constexpr (epi_prefetches<Epi>::value) epi.prefetch_tile(row, n0, min(BN, p.N - n0));
-      if (!mbar_wait(smem_u32(&bar_tmem_full[acc]), acc_phase, &abort_flag)) {
+      if (!mbar_wait_warp(smem_u32(&bar_tmem_full[acc]), acc_phase, &abort_flag)) {
         abort_flag = 1;
         atomicMax(p.header + kHdrStatus, (int)kStatusEpilogueTimeout);
         break;

@@ -385,6 +385,15 @@ __device__ __forceinline__ void tma_store_wait_read() { asm volatile("cp.async.b
 __device__ __forceinline__ void tma_store_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 __device__ __forceinline__ void group_sync(int id) { asm volatile("bar.sync %0, 128;" ::"r"(id) : "memory"); }
 
+// One outcome for the four warps of a group: they meet in group_sync for every chunk, where a warp whose wait gave
+// up would be missing for good.
+__device__ __forceinline__ bool group_all(int id, bool ok) {
+  uint32_t all;
+  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %2, 0;\n\tbar.red.and.pred q, %1, 128, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+               : "=r"(all) : "r"(id), "r"((uint32_t)ok) : "memory");
+  return all != 0;
+}
+
 template <int MODE, class Epi>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
 umma_pair_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__ CUtensorMap tmN,
@@ -504,7 +513,7 @@ umma_pair_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant_
       const int row_k = MODE == kWgrad ? s_pad[e] : 0;
       for (int kb = 0; kb < kblocks; ++kb) {
         if ((stage & 1) == 0) {
-          ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_empty[stage >> 1]), phase ^ 1u, &abort_flag));
+          ok = mbar_wait_warp(smem_u32(&bar_empty[stage >> 1]), phase ^ 1u, &abort_flag);
           if (!ok) break;
         }
         if (elected) {
@@ -536,7 +545,7 @@ umma_pair_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant_
     }
     // the commits that free the last stages must have arrived here before this CTA ends
     for (int g = 0; g < kPairGroups && ok; ++g)
-      ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_empty[g]), 2 * g < stage ? phase : phase ^ 1u, &abort_flag));
+      ok = mbar_wait_warp(smem_u32(&bar_empty[g]), 2 * g < stage ? phase : phase ^ 1u, &abort_flag);
     if (!ok && lane == 0) {
       abort_flag = 1;
       atomicMax(p.header + kHdrStatus, (int)kStatusProducerTimeout);
@@ -566,12 +575,12 @@ umma_pair_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant_
         e_next = expert_of(id + n_clusters);
         if (kblocks == 0) continue;
         const uint32_t idesc = idesc_base | ((uint32_t)(width >> 3) << 17);
-        ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_tmem_empty[acc]), acc_phase ^ 1u, &abort_flag));
+        ok = mbar_wait_warp(smem_u32(&bar_tmem_empty[acc]), acc_phase ^ 1u, &abort_flag);
         if (!ok) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * kUmmaAccStride;
         for (int kb = 0; kb < kblocks; ++kb) {
-          ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_full[stage]), phase, &abort_flag));
+          ok = mbar_wait_warp(smem_u32(&bar_full[stage]), phase, &abort_flag);
           if (!ok) break;
           tc_fence_after();
           if (elected) {
@@ -641,12 +650,13 @@ umma_pair_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant_
         if (mine)
           for (int c = turn; c < nchunks; c += 2) epi.prefetch(m, n0 + c * 32, min(32, width - c * 32), lane);
       }
-      if (!mbar_wait(smem_u32(&bar_tmem_full[acc]), acc_phase, &abort_flag)) {
+      bool ok = mbar_wait_warp(smem_u32(&bar_tmem_full[acc]), acc_phase, &abort_flag);
+      if constexpr (kStore) ok = group_all(1 + turn, ok);
+      if (!ok) {
         abort_flag = 1;
         atomicMax(p.header + kHdrStatus, (int)kStatusEpilogueTimeout);
         break;
       }
-      __syncwarp();
       tc_fence_after();
       if (mine) {
         const uint32_t t_row = tmem_base + acc * kUmmaAccStride + ((uint32_t)(q * 32) << 16);
