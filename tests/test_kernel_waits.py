@@ -32,3 +32,11 @@ def test_warps_that_store_together_leave_together():
     agree = text.index("if constexpr (kStore) ok = group_all(1 + turn, ok);", wait)
     assert agree < text.index("if (!ok)", wait) < text.index("emit(c, v)", wait)
     assert "bar.red.and.pred q, %1, 128, p;" in text and "bar.sync %0, 128;" in text
+
+
+def test_commits_are_awaited_before_a_cta_ends():
+    """The leader's last commits arrive in both CTAs' shared memory: each barrier they reach is waited on after the
+    last tile, by the role that would use what they free."""
+    text = source("umma_f32.cuh")
+    for bar in ("bar_b_empty", "bar_a_empty"):
+        assert len(re.findall(r"mbar_wait\w*\(smem_u32\(&%s\[" % bar, text)) == 2, bar

@@ -776,6 +776,12 @@ umma_f32_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__
         if (slot == 0) phase ^= 1u;
       }
     }
+    // the commits that free the last operands must have arrived here before this CTA ends
+    for (int g = 0; g < 2 && ok; ++g) {
+      ok = mbar_wait_warp(smem_u32(&bar_a_empty[slot]), phase ^ 1u, &abort_flag);
+      slot ^= 1;
+      if (slot == 0) phase ^= 1u;
+    }
     if (!ok) give_up(kStatusMmaTimeout);
     __syncwarp();
   } else {
