@@ -122,6 +122,8 @@ int yamoe_b200_route_static(const int64_t *router_indices, int32_t *sorted_value
  *   expert_capacity   rows kept per expert: the first min(n_e, capacity) assignments of expert e
  *                     in stable sorted order (csrc/gather.cu:18-26, csrc/scatter.cu:78-96)
  * ------------------------------------------------------------------------------------------- */
+/* Besides the tables, per padded row (at most T*K + 128 min(E, T*K) + 127 of them) and column:
+ * bf16 6 bytes, fp32 12 where H is a multiple of 64 (rows as three bf16 planes) and 8 otherwise. */
 size_t yamoe_b200_forward_workspace_bytes(int64_t T, int H, int E, int K, int dtype);
 int yamoe_b200_experts_forward(const void *hidden_states, const int64_t *router_indices,
                                const void *routing_weights, int routing_cols,
@@ -144,6 +146,8 @@ int yamoe_b200_experts_forward(const void *hidden_states, const int64_t *router_
  *   d_gate_up_proj    dtype [E,H,2H];  d_gate_up_proj_bias dtype [E,2H]
  *   d_down_proj       dtype [E,H,H];   d_down_proj_bias    dtype [E,H]
  * ------------------------------------------------------------------------------------------- */
+/* Per padded row and column: bf16 14 bytes, fp32 50 where H is a multiple of 64 and 28 otherwise,
+ * whatever path is selected; bf16 also 4 T H bytes.  A buffer of the saving pair has the same size. */
 size_t yamoe_b200_backward_workspace_bytes(int64_t T, int H, int E, int K, int dtype);
 int yamoe_b200_experts_backward(const void *grad_out, int grad_out_per_slot,
                                 const void *hidden_states, const int64_t *router_indices,

@@ -47,6 +47,15 @@ def test_workspace_sizes(lib):
     assert lib.yamoe_b200_route_workspace_bytes(0, 8, 2) > 0
 
 
+@pytest.mark.parametrize("H,forward,backward", [(72, 8, 28), (128, 12, 50)])
+def test_fp32_workspace_bytes_per_row_and_column(lib, H, forward, backward):
+    """Rows of token operands are three bf16 planes at the widths of the tensor-core kernels only."""
+    T, E, K = 4096, 32, 4
+    rows = (T * K // 128 + E) * 128
+    for fn, want in ((lib.yamoe_b200_forward_workspace_bytes, forward), (lib.yamoe_b200_backward_workspace_bytes, backward)):
+        assert abs((fn(T, H + 64, E, K, 0) - fn(T, H, E, K, 0)) / (rows * 64) - want) < 1e-3
+
+
 def test_argument_checks_without_gpu(lib):
     # all rejected before any CUDA call is made
     assert lib.yamoe_b200_experts_forward(None, None, None, 8, None, None, None, None, None, 16, 64, 8, 2, 16, 0,

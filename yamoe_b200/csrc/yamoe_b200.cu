@@ -109,16 +109,20 @@ static void carve_tables(Bump& b, Plan& p, int64_t T, int E, int K, bool rows) {
   }
 }
 
+// fp32 at the widths that umma_f32.cuh serves: the operands that meet the tensor cores as token rows are three bf16
+// planes, 6 bytes per element; everything else is stored as itself.
+static bool planes_width(int dtype, int H) { return dtype == YAMOE_F32 && H % 64 == 0; }
+static size_t token_row_size(int dtype, int H) { return dtype == YAMOE_BF16 ? 2 : planes_width(dtype, H) ? 6 : 4; }
+
 static Plan plan_forward(void* ws, int64_t T, int H, int E, int K, int dtype) {
   Plan p;
   Bump b(ws);
   p.esize = dtype == YAMOE_BF16 ? 2 : 4;
   carve_tables(b, p, T, E, K, true);
-  // fp32: the operands that meet the tensor cores as token rows are three bf16 planes (umma_f32.cuh)
-  const size_t nsize = dtype == YAMOE_BF16 ? 2 : 6;
+  const size_t nsize = token_row_size(dtype, H);
   p.xs = b.take<char>((size_t)p.max_rows * H * nsize);
   p.act = b.take<char>((size_t)p.max_rows * H * nsize);
-  if (dtype == YAMOE_F32) p.yrows = b.take<char>((size_t)p.max_rows * H * p.esize);
+  if (planes_width(dtype, H)) p.yrows = p.xs;      // written by the down GEMM, which reads only `act`
   if (dtype == YAMOE_BF16) {
     // decode path: fp32 accumulator [T,H]; grouped-GEMM path: weighted rows [max_rows,H].
     // They are never live together, the larger one sizes the region.
@@ -144,13 +148,13 @@ static Plan plan_backward(void* ws, int64_t T, int H, int E, int K, int dtype) {
   Bump b(ws);
   p.esize = dtype == YAMOE_BF16 ? 2 : 4;
   carve_tables(b, p, T, E, K, true);
-  const size_t nsize = dtype == YAMOE_BF16 ? 2 : 6;      // see plan_forward
+  const size_t nsize = token_row_size(dtype, H);
   p.xs = b.take<char>((size_t)p.max_rows * (H + kBiasCols) * nsize);
   p.gys = b.take<char>((size_t)p.max_rows * H * p.esize);
   p.pre = b.take<char>((size_t)p.max_rows * 2 * H * p.esize);
   p.actw = b.take<char>((size_t)p.max_rows * (H + kBiasCols) * nsize);
   p.gpre = b.take<char>((size_t)p.max_rows * 2 * H * p.esize);
-  if (dtype == YAMOE_F32) {
+  if (planes_width(dtype, H)) {
     // (or the fp32 rows of actw, see saved_actw_rows)
     p.gys_planes = b.take<char>((size_t)p.max_rows * std::max(H * 6, (H + kBiasCols) * 4));
     p.gpre_planes = b.take<char>((size_t)p.max_rows * 2 * H * nsize);
@@ -188,7 +192,7 @@ static bool use_split_f32(int path, int H, const void* wgu, const void* wd) {
 // Layout of xs and actw in the buffer that the saving forward hands to the backward pass: planes for the widths
 // that umma_f32.cuh serves, rows otherwise.  Only the shape decides, since path, weight pointers and their
 // alignment may differ between the two calls; CUDA-core kernels convert (saved_xs_rows).
-static bool saves_planes(int dtype, int H) { return dtype == YAMOE_F32 && umma_available() && H % 64 == 0; }
+static bool saves_planes(int dtype, int H) { return planes_width(dtype, H) && umma_available(); }
 
 // Scratch for xs and actw as fp32 rows [max_rows, H + kBiasCols], in regions that only the tensor-core kernels use
 // (12 H and max(6 H, 4 H + 4 kBiasCols) bytes per row, H >= 64).
