@@ -75,7 +75,7 @@ __device__ __forceinline__ float ld_shared_cluster_f32(uint32_t cluster_addr) {
 }
 
 // ---- programmatic dependent launch -----------------------------------------------------------
-// A kernel launched with launch_pdl may start while its predecessor on the stream is still
+// A kernel launched with launch_pdl_opt may start while its predecessor on the stream is still
 // draining; it must execute pdl_wait() before touching any memory the predecessor writes or
 // reads.  A predecessor calls pdl_trigger() as early as it likes: the dependent's CTAs then
 // become resident as soon as SMs free up, and their set-up overlaps the predecessor's tail.
@@ -83,9 +83,10 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // Measured on B200: between the two decode GEMV kernels it saves about 2 us per call (T = 1: 52.0 us
-// against 53.8 us as a CUDA-graph replay).  The kernels of the expert pass use it as well (gather, the
-// grouped GEMMs of umma_pair.cuh and umma_f32.cuh, combine): their barrier and TMEM set-up and the launch
-// latency fall into the predecessor's tail.  The one-CTA GEMM does so only where it is gated.
+// against 53.8 us as a CUDA-graph replay).  Of the expert pass the grouped GEMMs of umma_pair.cuh and
+// umma_f32.cuh, the combine and the gather of the bf16 forward use it as well: their barrier and TMEM set-up and the
+// launch latency fall into the predecessor's tail.  The other gathers are plain launches, and the one-CTA
+// GEMM uses it only where it is gated.
 // YAMOE_B200_PDL=1 turns it on everywhere, YAMOE_B200_PDL=0 off everywhere.
 inline int pdl_setting() {
   static int v = []() {
@@ -128,12 +129,6 @@ inline cudaError_t launch_pdl_opt(bool default_on, void (*kern)(KArgs...), dim3 
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
-}
-
-template <typename... KArgs, typename... Args>
-inline cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
-                              Args&&... args) {
-  return launch_pdl_opt(false, kern, grid, block, smem, st, std::forward<Args>(args)...);
 }
 
 // Routing tables kept at the head of every workspace (all int32 unless noted).

@@ -361,12 +361,10 @@ ep_dispatch_fused_kernel(const EpDispatchArgs a, EpTables t) {
         atomicMax(t.rt.header + kHdrStatus, bad);
         t.rt.header[kHdrRowTiles] = 0;
         t.rt.header[kHdrRowsUsed] = 0;
-        t.rt.header[kHdrPairs] = 0;
         t.rt.header[kHdrDropped] = 0;
       }
       for (int le = tid; le <= per; le += nthr) {
         t.rt.pad_off[le] = 0;
-        t.rt.pair_off[le] = 0;
         t.rt.bins[le] = 0;
         if (le < per) t.rt.counts[le] = 0;
       }
@@ -376,26 +374,21 @@ ep_dispatch_fused_kernel(const EpDispatchArgs a, EpTables t) {
         t.seg_row[i] = segr[i];
       }
       if (tid == 0) {
-        int rows = 0, pairs = 0, cum = 0;
+        int rows = 0, cum = 0;
         for (int le = 0; le < per; ++le) {
           const int c = tot[rank * per + le];
           cum += c;
           t.rt.counts[le] = c;
           t.rt.bins[le] = cum;
           t.rt.pad_off[le] = rows;
-          t.rt.pair_off[le] = pairs;
           const int tiles = (c + kTileM - 1) / kTileM;
           for (int k = 0; k < tiles; ++k) t.rt.tile_expert[rows / kTileM + k] = le;
-          for (int k = 0; k < (tiles + 1) / 2; ++k) t.rt.pair_expert[pairs + k] = le;
           rows += tiles * kTileM;
-          pairs += (tiles + 1) / 2;
         }
         t.rt.bins[per] = 0;
         t.rt.pad_off[per] = rows;
-        t.rt.pair_off[per] = pairs;
         t.rt.header[kHdrRowTiles] = rows / kTileM;
         t.rt.header[kHdrRowsUsed] = rows;
-        t.rt.header[kHdrPairs] = pairs;
         t.rt.header[kHdrDropped] = 0;
       }
     }

@@ -39,7 +39,7 @@ struct GemmArgs {
   const int32_t* tile_expert;
   const int32_t* pad_off;
   const int32_t* header;
-  const int32_t* pair_expert = nullptr;   // tile-pair tables (256-row tcgen05 kernel only)
+  const int32_t* pair_expert = nullptr;   // tile-pair tables (CTA-pair kernel only)
   const int32_t* pair_off = nullptr;
   const int32_t* counts = nullptr;        // rows present per expert: lets the CUDA-core kernel skip all-padding tiles
   // row-tiled arrangements without tables (tile_expert == nullptr): one group (expert 0) owns the

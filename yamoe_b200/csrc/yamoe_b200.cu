@@ -550,14 +550,11 @@ __global__ void uniform_tables_kernel(RouteTables rt, int E, int C) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i <= E) rt.pad_off[i] = i * C;
   if (i < E) rt.counts[i] = C;
-  const int tiles = C / kTileM, pairs = (tiles + 1) / 2;
+  const int tiles = C / kTileM;
   if (i < E * tiles) rt.tile_expert[i] = i / tiles;
-  if (i <= E) rt.pair_off[i] = i * pairs;
-  if (i < E * pairs) rt.pair_expert[i] = i / pairs;
   if (i == 0) {
     rt.header[kHdrRowTiles] = E * tiles;
     rt.header[kHdrRowsUsed] = E * C;
-    rt.header[kHdrPairs] = E * pairs;
   }
 }
 
@@ -577,19 +574,16 @@ static int batch_mm_impl(const void* x, const void* w, void* out, int E, int C, 
   if (mode == kWgrad) {
     EpiStore<T> epi{reinterpret_cast<T*>(out), M, N};
     GemmArgs g{x, M, w, N, 0, M, N, 0, E, p.rt.tile_expert, p.rt.pad_off, p.rt.header};
-      g.pair_expert = p.rt.pair_expert; g.pair_off = p.rt.pair_off;
     if (tc) { if constexpr (sizeof(T) == 2) rc = launch_umma_gemm<kWgrad>(g, epi, rows, rows / kTileM, st); }
     else launch_simt_gemm<T, kWgrad>(g, epi, rows, st);
   } else {
     EpiStoreRows<T> epi{reinterpret_cast<T*>(out), N};
     if (mode == kFwd) {
       GemmArgs g{x, K, w, N, (int64_t)K * N, 0, N, K, E, p.rt.tile_expert, p.rt.pad_off, p.rt.header};
-      g.pair_expert = p.rt.pair_expert; g.pair_off = p.rt.pair_off;
       if (tc) { if constexpr (sizeof(T) == 2) rc = launch_umma_gemm<kFwd>(g, epi, rows, rows / kTileM, st); }
       else launch_simt_gemm<T, kFwd>(g, epi, rows, st);
     } else {
       GemmArgs g{x, K, w, K, (int64_t)K * N, 0, N, K, E, p.rt.tile_expert, p.rt.pad_off, p.rt.header};
-      g.pair_expert = p.rt.pair_expert; g.pair_off = p.rt.pair_off;
       if (tc) { if constexpr (sizeof(T) == 2) rc = launch_umma_gemm<kDgrad>(g, epi, rows, rows / kTileM, st); }
       else launch_simt_gemm<T, kDgrad>(g, epi, rows, st);
     }
@@ -621,9 +615,7 @@ static EpPlan plan_ep(void* ws, int64_t max_rows, int H, int E, int G, int dtype
   rt.counts = b.take<int32_t>(per);
   rt.bins = b.take<int32_t>(per + 1);
   rt.pad_off = b.take<int32_t>(per + 1);
-  rt.pair_off = b.take<int32_t>(per + 1);
   rt.tile_expert = b.take<int32_t>(max_tiles);
-  rt.pair_expert = b.take<int32_t>(max_tiles);
   rt.row_token = b.take<int32_t>(max_rows);
   rt.row_weight = b.take<float>(max_rows);
   p.t.dest_row = b.take<int32_t>(E);
@@ -662,18 +654,16 @@ static int ep_local_forward_impl(const void* recv_x, const void* wgu, const void
   const bool fused = yrows == nullptr;     // results go straight to the source ranks
   GemmArgs g1{recv_x, H, wgu, 2 * (int64_t)H, (int64_t)H * 2 * H, 0, 2 * H, H, per, rt.tile_expert, rt.pad_off,
               rt.header};
-  g1.pair_expert = rt.pair_expert; g1.pair_off = rt.pair_off; g1.counts = rt.counts;
+  g1.counts = rt.counts;
   g1.gate = gate;
   GemmArgs g2{p.act, H, wd, H, (int64_t)H * H, 0, H, H, per, rt.tile_expert, rt.pad_off, rt.header};
-  g2.pair_expert = rt.pair_expert; g2.pair_off = rt.pair_off; g2.counts = rt.counts;
+  g2.counts = rt.counts;
   int rc = YAMOE_OK;
   if (use_tcgen05(current_path(), dtype, H)) {
     if constexpr (sizeof(T) == 2) {
       {
         StageTimer tm(kStageGateUp, st);
-        // the gate is a feature of the one-CTA kernel
-        rc = gate.prep != nullptr ? launch_umma_gemm<kFwd>(g1, glu, max_rows, max_tiles, st)
-                                  : launch_umma_gemm<kFwd>(g1, glu, max_rows, max_tiles, st);
+        rc = launch_umma_gemm<kFwd>(g1, glu, max_rows, max_tiles, st);
       }
       if (rc) return rc;
       StageTimer tm(kStageDown, st);
@@ -701,27 +691,27 @@ static int ep_local_backward_impl(const void* recv_x, const void* recv_g, const 
                                   const GemmGate& gate = GemmGate{}) {
   const RouteTables& rt = p.t.rt;
   const int64_t max_tiles = max_rows / kTileM;
-  auto with_pairs = [&](GemmArgs g) { g.pair_expert = rt.pair_expert; g.pair_off = rt.pair_off; g.counts = rt.counts; return g; };
+  auto with_counts = [&](GemmArgs g) { g.counts = rt.counts; return g; };
   // p.act receives the activations times the routing weight; the weights are taken from the
   // receive buffer itself (row_weight is filled from it only after this GEMM)
   EpiGlu<T> glu{reinterpret_cast<const T*>(bgu), nullptr, reinterpret_cast<T*>(p.act), reinterpret_cast<T*>(p.pre),
                 rt.row_token, recv_w, H, 0};
-  GemmArgs g1 = with_pairs(GemmArgs{recv_x, H, wgu, 2 * (int64_t)H, (int64_t)H * 2 * H, 0, 2 * H, H, per,
-                                    rt.tile_expert, rt.pad_off, rt.header});
+  GemmArgs g1 = with_counts(GemmArgs{recv_x, H, wgu, 2 * (int64_t)H, (int64_t)H * 2 * H, 0, 2 * H, H, per,
+                                     rt.tile_expert, rt.pad_off, rt.header});
   g1.gate = gate;
   EpiGluBackward<T> glub{reinterpret_cast<const T*>(p.pre), reinterpret_cast<T*>(p.gpre), p.gw_row, rt.row_token,
                          rt.row_weight, H};
-  const GemmArgs g2 = with_pairs(GemmArgs{p.gys, H, wd, H, (int64_t)H * H, 0, H, H, per, rt.tile_expert, rt.pad_off,
-                                          rt.header});
+  const GemmArgs g2 = with_counts(GemmArgs{p.gys, H, wd, H, (int64_t)H * H, 0, H, H, per, rt.tile_expert, rt.pad_off,
+                                           rt.header});
   EpiStore<T> st_wd{reinterpret_cast<T*>(d_wd), H, H};
-  const GemmArgs g3 = with_pairs(GemmArgs{p.act, H, p.gys, H, 0, H, H, 0, per, rt.tile_expert, rt.pad_off,
-                                          rt.header});
+  const GemmArgs g3 = with_counts(GemmArgs{p.act, H, p.gys, H, 0, H, H, 0, per, rt.tile_expert, rt.pad_off,
+                                           rt.header});
   EpiPeerRows<T> prows{nullptr, p.t.row_dest, rt.row_token, H};
-  const GemmArgs g4 = with_pairs(GemmArgs{p.gpre, 2 * (int64_t)H, wgu, 2 * (int64_t)H, (int64_t)H * 2 * H, 0, H,
-                                          2 * H, per, rt.tile_expert, rt.pad_off, rt.header});
+  const GemmArgs g4 = with_counts(GemmArgs{p.gpre, 2 * (int64_t)H, wgu, 2 * (int64_t)H, (int64_t)H * 2 * H, 0, H,
+                                           2 * H, per, rt.tile_expert, rt.pad_off, rt.header});
   EpiStore<T> st_wgu{reinterpret_cast<T*>(d_wgu), H, 2 * H};
-  const GemmArgs g5 = with_pairs(GemmArgs{recv_x, H, p.gpre, 2 * (int64_t)H, 0, H, 2 * H, 0, per, rt.tile_expert,
-                                          rt.pad_off, rt.header});
+  const GemmArgs g5 = with_counts(GemmArgs{recv_x, H, p.gpre, 2 * (int64_t)H, 0, H, 2 * H, 0, per, rt.tile_expert,
+                                           rt.pad_off, rt.header});
   int rc = YAMOE_OK;
   const bool tc = use_tcgen05(current_path(), dtype, H);
   // The recomputed gate_up GEMM needs only the token rows: it goes first, and with a gate it runs
