@@ -326,11 +326,17 @@ struct F32Glu {                     // see PairGlu
       }
     }
     if constexpr (TRAIN) {
-      if (m == lane)               // columns 0..31: this warp also fills the columns behind H with (w, 0, 0, ...)
-        for (int t = 0; t < nvalid; ++t) {
-          const float w = __shfl_sync(0xffffffffu, w_lane, t);
-          for (int c = H + 4 * lane; c < actw.ld; c += 128) actw.store4(row + t, c, {c == H ? w : 0.f, 0.f, 0.f, 0.f});
+      if (m - lane < 128) {        // these warps also fill the 64 columns behind H (see PairGlu), four rows each
+        const int t = 4 * ((m - lane) >> 5) + (lane >> 3);
+        const uint3 s = split3_special(__shfl_sync(0xffffffffu, w_lane, t));
+        const bool first = (lane & 7) == 0;
+        if (t < nvalid) {
+          __nv_bfloat16* d = actw.p + (size_t)(row + t) * actw.ld + H + 8 * (lane & 7);
+          *reinterpret_cast<uint4*>(d) = make_uint4(first ? s.x >> 16 : 0u, 0u, 0u, 0u);
+          *reinterpret_cast<uint4*>(d + actw.stride) = make_uint4(first ? s.y >> 16 : 0u, 0u, 0u, 0u);
+          *reinterpret_cast<uint4*>(d + 2 * actw.stride) = make_uint4(first ? s.z >> 16 : 0u, 0u, 0u, 0u);
         }
+      }
     }
   }
 };

@@ -127,7 +127,7 @@ __device__ __forceinline__ void pair_columns(const float (&v)[32], bool odd, flo
 
 // + bias, clamped SwiGLU of the interleaved (gate, up) columns; reference: csrc/moe.cpp:163-180.
 // Outputs: `act` (activation) and, for a backward pass, `pre` (biased pre-activations) and `actw`
-// (activation times routing weight, rows actw_ld apart; the columns behind the H activations are
+// (activation times routing weight, rows actw_ld = H + 64 apart; the columns behind the H activations are
 // (w, 0, 0, ...), see EpiGlu).  The backward outputs of padding rows are exact zeros.
 template <bool TRAIN>
 struct PairGlu {
@@ -168,21 +168,27 @@ struct PairGlu {
         const float w = __shfl_sync(0xffffffffu, w_lane, t);
         const bool ok = (have >> t) & 1u;
         const uint32_t packed = ok ? pack_bf16x2(g[i], u[i]) : 0u;
-        // the backward pass re-derives the activation from the stored (rounded) pre-activations
-        const float a = ok ? glu_act(__uint_as_float(packed << 16), __uint_as_float(packed & 0xffff0000u)) : 0.f;
+        // the backward pass re-derives the activation from the stored (rounded) pre-activations; 0 for (0, 0)
+        const float a = glu_act(__uint_as_float(packed << 16), __uint_as_float(packed & 0xffff0000u));
         if (t < nvalid) {
           const size_t r = row + t;
           *reinterpret_cast<uint32_t*>(pre + r * 2 * H + (m & ~1)) = packed;
           if (act != nullptr) act[r * H + j] = __float2bfloat16_rn(a);
-          actw[r * actw_ld + j] = __float2bfloat16_rn(ok ? a * w : 0.f);
+          actw[r * actw_ld + j] = __float2bfloat16_rn(a * w);
         }
       }
-      if (actw_ld > H && m == lane) {            // this warp has columns 0..31: it also fills the columns behind H
-        for (int t = 0; t < nvalid; ++t) {
+      // The warps with columns 0..127 also fill the 64 columns behind H, eight rows each, eight columns to a lane.  As a
+      // loop of one warp over all rows with 4 bytes to a lane this was half of the kernel (gate_up at T = 2000,
+      // E = 32: H = 512 68 us, now 39; H = 1024 96 and 69), and the backward pass at H <= 512 slower than with the
+      // one-CTA kernel.
+      if (m - lane < 128) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const int t = 8 * ((m - lane) >> 5) + 4 * i + (lane >> 3);
           const float w = __shfl_sync(0xffffffffu, w_lane, t);
-          for (int c = H + 2 * lane; c < actw_ld; c += 64)
-            *reinterpret_cast<uint32_t*>(actw + (size_t)(row + t) * actw_ld + c) =
-                c == H ? pack_bf16x2(w, 0.f) : 0u;
+          if (t < nvalid)
+            *reinterpret_cast<uint4*>(actw + (size_t)(row + t) * actw_ld + H + 8 * (lane & 7)) =
+                make_uint4((lane & 7) == 0 ? pack_bf16x2(w, 0.f) : 0u, 0u, 0u, 0u);
         }
       }
     }
