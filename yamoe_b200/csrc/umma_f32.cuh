@@ -730,11 +730,12 @@ umma_f32_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__
         tc_fence_after();
         const uint8_t* tile = smem_raw + (smem_base - smem_u32(smem_raw)) + ws * kF32WBytes;
         const uint32_t t = tmem_base + kF32TmemA + slot * kF32TmemAStride + khalf * 16 + ((uint32_t)(q * 32) << 16);
+        // MODE kDgrad: 32 k of row mrow are 128 bytes, 16-byte pieces swizzled by the row
+        const uint8_t* rowp = tile + khalf * (kF32WBytes / 2) + mrow * 128;
+        const float* colp = reinterpret_cast<const float*>(tile) + khalf * 32 * kF32M + mrow;
+        float bad = 0.f;
 #pragma unroll
         for (int h = 0; h < 2; ++h) {                // 16 k at a time
-          // MODE kDgrad: 32 k of row mrow are 128 bytes, 16-byte pieces swizzled by the row
-          const uint8_t* rowp = tile + khalf * (kF32WBytes / 2) + mrow * 128;
-          const float* colp = reinterpret_cast<const float*>(tile) + (khalf * 32 + h * 16) * kF32M + mrow;
           float x[16];
           if constexpr (MODE == kDgrad) {
 #pragma unroll
@@ -744,31 +745,31 @@ umma_f32_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__
             }
           } else {
 #pragma unroll
-            for (int i = 0; i < 16; ++i) x[i] = colp[i * kF32M];
+            for (int i = 0; i < 16; ++i) x[i] = colp[(h * 16 + i) * kF32M];
           }
           uint32_t p0[8], p1[8], p2[8];
-          const float bad = split3_finite<16>(x, p0, p1, p2);
+          bad += split3_finite<16>(x, p0, p1, p2);
           tc_st_32x8(t + h * 8, p0);
           tc_st_32x8(t + h * 8 + 32, p1);
           tc_st_32x8(t + h * 8 + 64, p2);
-          if (__any_sync(0xffffffffu, bad != bad)) {
-            tc_st_wait();
+        }
+        if (__any_sync(0xffffffffu, bad != bad)) {
+          tc_st_wait();
 #pragma unroll 1
-            for (int i = 0; i < 8; ++i) {            // rolled, from memory again: rare, and hot code stays short
-              float y0, y1;
-              if constexpr (MODE == kDgrad) {
-                const uint8_t* q = rowp + (((h * 4 + (i >> 1)) ^ (mrow & 7)) << 4) + 8 * (i & 1);
-                y0 = *reinterpret_cast<const float*>(q);
-                y1 = *reinterpret_cast<const float*>(q + 4);
-              } else {
-                y0 = colp[2 * i * kF32M];
-                y1 = colp[(2 * i + 1) * kF32M];
-              }
-              const uint3 s0 = split3_special(y0), s1 = split3_special(y1);
-              tc_st_32x1(t + h * 8 + i, __byte_perm(s0.x, s1.x, 0x7632));
-              tc_st_32x1(t + h * 8 + i + 32, __byte_perm(s0.y, s1.y, 0x7632));
-              tc_st_32x1(t + h * 8 + i + 64, __byte_perm(s0.z, s1.z, 0x7632));
+          for (int i = 0; i < 16; ++i) {             // rolled, from memory again: rare, and the hot code stays short
+            float y0, y1;
+            if constexpr (MODE == kDgrad) {
+              const uint8_t* piece = rowp + (((i >> 1) ^ (mrow & 7)) << 4) + 8 * (i & 1);
+              y0 = *reinterpret_cast<const float*>(piece);
+              y1 = *reinterpret_cast<const float*>(piece + 4);
+            } else {
+              y0 = colp[2 * i * kF32M];
+              y1 = colp[(2 * i + 1) * kF32M];
             }
+            const uint3 s0 = split3_special(y0), s1 = split3_special(y1);
+            tc_st_32x1(t + i, __byte_perm(s0.x, s1.x, 0x7632));
+            tc_st_32x1(t + i + 32, __byte_perm(s0.y, s1.y, 0x7632));
+            tc_st_32x1(t + i + 64, __byte_perm(s0.z, s1.z, 0x7632));
           }
         }
         __syncwarp();
