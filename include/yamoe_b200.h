@@ -35,12 +35,13 @@ typedef enum {
 
 typedef enum { YAMOE_F32 = 0, YAMOE_BF16 = 1 } yamoe_dtype_t;
 
-/* Path selection for the GEMMs.  AUTO picks tcgen05 for bf16 when shapes allow, the GEMV path
- * for decode-sized bf16 token counts, and the SIMT path otherwise (fp32 always). */
+/* Path selection for the GEMMs.  AUTO picks tcgen05 where H is a multiple of 64 (fp32: and the
+ * weights are 16-byte aligned), the GEMV path for decode-sized bf16 token counts, and the SIMT
+ * path otherwise. */
 typedef enum {
   YAMOE_PATH_AUTO = 0,
   YAMOE_PATH_SIMT = 1,     /* CUDA-core FFMA grouped GEMM, fp32 accumulate (any dtype)     */
-  YAMOE_PATH_TCGEN05 = 2,  /* tcgen05 / TMEM / TMA grouped GEMM (bf16 only)                */
+  YAMOE_PATH_TCGEN05 = 2,  /* tcgen05 / TMEM / TMA grouped GEMM (fp32 as three bf16 parts) */
   YAMOE_PATH_GEMV = 3      /* weight-streaming GEMV path for small token counts (bf16)     */
 } yamoe_path_t;
 

@@ -27,13 +27,13 @@
 // is short, 2.1e-7 against 2.5e-7.
 //
 // Measured: gate_up of the README forward (T = 512, H = 2880, E = 8, K = 2) 213 us = 160 TFLOP/s of the
-// original product; the whole forward 412 us against 1797, a training step of 600 tokens 412 against 1191.
+// original product; the whole forward 412 us against 1797, a training step of 600 tokens 400 against 1191.
 //
 // Infinities and NaN behave as in fp32 arithmetic: see split3_special.
 //
 // Two CTAs share a tile (cta_group::2), 128 weight columns each: the planes are the larger half of what
 // L2 has to deliver (48 KB per 64-deep block against 32 KB of weights), and a pair needs them once.
-// With one CTA per tile the README forward took 485 us and the training step 463; now 422 and 405.
+// With one CTA per tile the README forward took 485 us and the training step 463, by pairs 422 and 405.
 //
 // A CTA has 20 warps: TMA producer, MMA issuer (of the leader only), two that only complete the
 // warpgroup, eight converters (two per TMEM lane quarter, 32 k each) and eight accumulator / epilogue

@@ -181,8 +181,8 @@ static bool use_tcgen05(int path, int dtype, int H) {
 }
 
 // fp32 through umma_f32.cuh (three bf16 parts per operand): README forward (T = 512, E = 8, H = 2880)
-// 422 us against 1797 us with the CUDA-core kernel, training step of 600 tokens (E = 16, H = 1024)
-// 405 against 1191 us.  The CUDA-core kernel keeps the widths that are no multiple of 64 and the
+// 412 us against 1797 us with the CUDA-core kernel, training step of 600 tokens (E = 16, H = 1024)
+// 400 against 1191 us.  The CUDA-core kernel keeps the widths that are no multiple of 64 and the
 // weights that TMA cannot address.
 static bool use_split_f32(int path, int H, const void* wgu, const void* wd) {
   return umma_available() && H % 64 == 0 && ((reinterpret_cast<uintptr_t>(wgu) | reinterpret_cast<uintptr_t>(wd)) & 15) == 0 &&
