@@ -124,7 +124,8 @@ int yamoe_b200_route_static(const int64_t *router_indices, int32_t *sorted_value
  *                     in stable sorted order (csrc/gather.cu:18-26, csrc/scatter.cu:78-96)
  * ------------------------------------------------------------------------------------------- */
 /* Besides the tables, per padded row (at most T*K + 128 min(E, T*K) + 127 of them) and column:
- * bf16 6 bytes, fp32 12 where H is a multiple of 64 (rows as three bf16 planes) and 8 otherwise. */
+ * bf16 6 bytes (up to 8 for K = 1), fp32 12 where H is a multiple of 64 (rows as three bf16 planes)
+ * and 8 otherwise. */
 size_t yamoe_b200_forward_workspace_bytes(int64_t T, int H, int E, int K, int dtype);
 int yamoe_b200_experts_forward(const void *hidden_states, const int64_t *router_indices,
                                const void *routing_weights, int routing_cols,
