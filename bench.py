@@ -469,7 +469,7 @@ class Case:
     def uses_gemv(self):
         """The library's rule for decode-sized bf16 calls of these widths (gemv_preferred in csrc/gemv.cuh)."""
         S = self.T * self.K
-        return self.decode and S <= min(256, 4 * self.E) and (S < 2 * self.E or S * self.H <= 80 * 1024)
+        return self.decode and S <= min(256, 4 * self.E) and (S < self.E or S * self.H <= 80 * 1024)
 
     def launches(self):
         if self.uses_gemv():

@@ -343,14 +343,15 @@ inline bool decode_sized(int64_t S, int E) { return S <= kGemvMaxS && S <= 4 * (
 
 // These kernels read an expert's weights once per 4 rows, the grouped GEMM (umma_pair.cuh) once whatever
 // its number of rows, after some 25 us of routing, gather and combine.  So the grouped GEMM takes the calls
-// with two or more rows per expert, from S * H = 80 K on.  Measured per call with L2 flushed, gemv / grouped,
-// H = 2880: E = 32 T = 16 298 / 266 us, T = 32 466 / 287, E = 128 T = 64 1004 / 870;  H = 2048, E = 64, K = 8:
-// T = 16 298 / 264, T = 32 446 / 283;  H = 1024, E = 32: T = 16 60 / 64, T = 32 85 / 72.  Between one and two
-// rows per expert it would be 5 to 9 % faster too (E = 128 T = 32 718 / 662, E = 32 T = 8 224 / 205); there the
-// sums keep the order that they have in these kernels.
+// with one or more rows per expert, from S * H = 80 K on.  Measured per call with L2 flushed, gemv / grouped,
+// H = 2880: E = 32 T = 8 224 / 205 us, T = 16 298 / 266, T = 32 466 / 287, E = 128 T = 32 718 / 662, T = 64
+// 1004 / 870;  H = 2048, E = 64, K = 8: T = 8 216 / 207, T = 16 298 / 264, T = 32 446 / 283;  H = 1024, E = 32:
+// T = 16 60 / 64, T = 32 85 / 72.  Where a few experts get most of the rows the difference is larger.  Below one row
+// per expert most experts that are hit have a single row, which these kernels are made for (E = 128 T = 4 is
+// 144 us; at T = 16 the grouped GEMM would take 424 us instead of 446).
 inline bool gemv_preferred(int64_t T, int H, int E, int K, bool tensor_cores) {
   const int64_t S = T * K;
-  return decode_sized(S, E) && (!tensor_cores || S < 2 * (int64_t)E || S * H <= 80 * 1024);
+  return decode_sized(S, E) && (!tensor_cores || S < E || S * H <= 80 * 1024);
 }
 
 template <int STAGE, int NB>
