@@ -3,7 +3,7 @@ import pytest
 import torch
 
 from oracle import experts_oracle as orc
-from helpers import SMALL_CASES, load_golden
+from helpers import RTOL_BF16, RTOL_F32, SMALL_CASES, load_golden
 
 pytestmark = pytest.mark.gpu
 
@@ -62,3 +62,22 @@ def test_sort_and_bincount_cumsum_ops():
     yamoe_b200.bincount_cumsum(x_out, bins, 32)
     ref = torch.cumsum(torch.bincount(x.cpu().long(), minlength=32), 0)
     assert torch.equal(bins[:32].cpu().long(), ref) and int(bins[32]) == 0
+
+
+@pytest.mark.parametrize("T,H,K,E,capacity", [(3, 72, 2, 4, 100), (61, 320, 9, 16, 100), (700, 64, 5, 8, 390),
+                                             (2500, 128, 9, 32, 5000), (5000, 64, 3, 8, 1700)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32], ids=["bf16", "fp32"])
+def test_gathers_by_token(T, H, K, E, capacity, dtype):
+    """One to eight warps to a token, more slots than one pass takes, dropped assignments, ragged last pieces."""
+    import yamoe_b200
+    inp = orc.make_inputs(T, H, E, K, seed=T + K, weight_std=H ** -0.5, bias_std=0.2, dtype=dtype, with_grad=True)
+    args = [inp[k] for k in ("hidden_states", "router_indices", "routing_weights", "gate_up_proj", "gate_up_proj_bias",
+                             "down_proj", "down_proj_bias")]
+    dev = [a.cuda() for a in args]
+    rtol = RTOL_BF16 if dtype == torch.bfloat16 else RTOL_F32
+    out = yamoe_b200.experts(*dev, capacity, E, K)
+    orc.check_close(out.float().cpu(), orc.experts_forward_oracle(*args, capacity, E, K), rtol, "forward")
+    got = yamoe_b200.experts_backward(inp["grad_out"].cuda(), *dev, capacity, E, K)
+    ref = orc.experts_backward_oracle(inp["grad_out"], *args, capacity, E, K)
+    for g, r, name in zip(got, ref, ["d_hidden", "d_routing", "d_wgu", "d_bgu", "d_wd", "d_bd"]):
+        orc.check_close(g.float().cpu(), r, rtol, name)

@@ -43,6 +43,12 @@ inline int64_t max_row_tiles(int64_t S, int E) {
   return ceil_div(S, kTileM) + ne;
 }
 
+// The grouped GEMMs cover an expert's rows up to this end: its assignments as far as the padded layout holds them,
+// rounded up to `row_round` rows.  Where the capacity drops some, that is more than the kept rows.
+__device__ __forceinline__ int covered_rows(int count, int padded, int row_round) {
+  return (min(count, padded) + row_round - 1) / row_round * row_round;
+}
+
 // Clamped SwiGLU of one (gate, up) pre-activation pair.  reference: csrc/moe.cpp:167-180.
 __device__ __forceinline__ float glu_act(float g, float u) {
   g = fminf(g, kLimit);
@@ -84,9 +90,8 @@ __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.lau
 
 // Measured on B200: between the two decode GEMV kernels it saves about 2 us per call (T = 1: 52.0 us
 // against 53.8 us as a CUDA-graph replay).  Of the expert pass the grouped GEMMs of umma_pair.cuh and
-// umma_f32.cuh, the combine and the gather of the bf16 forward use it as well: their barrier and TMEM set-up and the
-// launch latency fall into the predecessor's tail.  The other gathers are plain launches, and the one-CTA
-// GEMM uses it only where it is gated.
+// umma_f32.cuh, the gathers and the combine use it as well: their barrier and TMEM set-up and the
+// launch latency fall into the predecessor's tail.  The one-CTA GEMM uses it only where it is gated.
 // YAMOE_B200_PDL=1 turns it on everywhere, YAMOE_B200_PDL=0 off everywhere.
 inline int pdl_setting() {
   static int v = []() {

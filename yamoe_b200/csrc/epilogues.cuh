@@ -313,7 +313,7 @@ struct EpiStore {
 };
 
 // ---- weight gradient with the bias gradient riding along ------------------------------------
-// The transposed operand of the GEMM carries one extra column (see gather_rows_kernel / EpiGlu),
+// The transposed operand of the GEMM carries one extra column (see gather_tokens_kernel / EpiGlu),
 // so output row M holds the bias gradient: rows < M go to C, row M to bias_out, later rows nowhere.
 template <typename T>
 struct EpiStoreBias {

@@ -9,31 +9,89 @@ namespace yb {
 
 constexpr int kRowWarps = 8;  // rows per CTA in the warp-per-row kernels
 
-// dst[row, 0:H] = src[row_token[row], :], zeros for padding rows.  One warp per row, 16-byte
-// accesses.  reference: csrc/gather.cu:6-66 (which writes a padded [E,C,H] buffer instead).
-// Rows of dst are dst_ld elements apart; when dst_ld > H the columns behind the copy get
-// (1, 0, 0, ...) for token rows and zeros for padding rows: a weight-gradient GEMM that takes dst as
-// its transposed operand then yields, in output row H, the column sums of its other operand
-// (the bias gradient, reference: csrc/experts_backward.cu:308).
+// Where the gathers put 16-byte pieces of token rows: rows of T, or three bf16 planes (umma_f32.cuh).
 template <typename T>
+struct RowDst {
+  using Piece = uint4;
+  T* p;
+  int ld;
+  __device__ __forceinline__ Piece piece(const uint4& q) const { return q; }
+  __device__ __forceinline__ void put(size_t row, int vec, const Piece& q) const {
+    reinterpret_cast<uint4*>(p + row * ld)[vec] = q;
+  }
+  __device__ __forceinline__ uint4 one() const { return make_uint4(sizeof(T) == 2 ? 0x3f80u : 0x3f800000u, 0u, 0u, 0u); }
+};
+
+// The padding among the rows that the weight-gradient GEMMs cover (covered_rows) as zeros.  It lies in the last row tile
+// of an expert: CTA `cta` of kPadCtas per expert looks at eight rows of that tile, one to a warp.
+constexpr int kPadCtas = kTileM / kRowWarps;
+template <class Dst>
+__device__ __forceinline__ void zero_padding(const Dst& dst, const RouteTables& rt, int cta, int row_round, int nvec) {
+  const int lane = threadIdx.x & 31, e = cta / kPadCtas;
+  const int first = rt.pad_off[e], padded = rt.pad_off[e + 1] - first, count = rt.counts[e];
+  const int local = padded - kTileM + (cta % kPadCtas) * kRowWarps + (threadIdx.x >> 5);
+  if (local < 0 || local >= covered_rows(count, padded, row_round) || rt.row_token[first + local] >= 0) return;
+  const typename Dst::Piece zero = dst.piece(make_uint4(0, 0, 0, 0));
+  for (int i = lane; i < nvec; i += 32) dst.put((size_t)(first + local), i, zero);
+}
+
+// dst[row of assignment (t, k), 0:H] = src[t, :] for every kept assignment (reference: csrc/gather.cu:6-66, which
+// fills a padded [E,C,H] buffer).  Rows of dst are dst.ld elements apart; when dst.ld > H the columns behind the copy
+// get (1, 0, 0, ...) for token rows and zeros for padding rows: a weight-gradient GEMM that takes dst as its transposed
+// operand then yields, in output row H, the column sums of its other operand (the bias gradient,
+// reference: csrc/experts_backward.cu:308).
+//
+// HBM bound, so a token's row is read once and written K times: a warp takes 32 16-byte pieces of one token, the pieces
+// of a token side by side in the grid.  Walked by padded row, a warp per row, each token was read K times, from HBM once
+// the tokens exceed what L2 keeps.  H = 2880, K = 4, row by row / by token: T = 64 5.4 / 1.7 us, T = 4096 26 / 21,
+// T = 16384 120 / 75 (472 MB, 6.3 TB/s).
+// The first pad_ctas CTAs zero padding rows (zero_padding); the forward on the tensor cores, where no result depends on
+// them, has none.
+template <class Dst, int KB>
 __global__ void __launch_bounds__(kRowWarps * 32)
-gather_rows_kernel(const T* __restrict__ src, T* __restrict__ dst, const int32_t* __restrict__ row_token,
-                   const int32_t* __restrict__ header, int H, int dst_ld) {
+gather_tokens_kernel(const void* __restrict__ src, const Dst dst, const RouteTables rt, int64_t Tn, int nvec, int ld_vec,
+                     int K, unsigned pad_ctas, int row_round) {
   pdl_wait();
   pdl_trigger();
-  const int row = blockIdx.x * kRowWarps + (threadIdx.x >> 5);
-  if (row >= header[kHdrRowsUsed]) return;
   const int lane = threadIdx.x & 31;
-  const int tok = row_token[row];
-  const int nvec = H * (int)sizeof(T) / 16;
-  uint4* d = reinterpret_cast<uint4*>(dst + (size_t)row * dst_ld);
-  if (tok < 0) {
-    for (int i = lane; i < nvec; i += 32) d[i] = make_uint4(0, 0, 0, 0);
-  } else {
-    const uint4* s = reinterpret_cast<const uint4*>(src + (size_t)tok * H);
-    for (int i = lane; i < nvec; i += 32) d[i] = __ldg(s + i);
+  if (blockIdx.x < pad_ctas) {
+    zero_padding(dst, rt, (int)blockIdx.x, row_round, ld_vec);
+    return;
   }
-  for (int j = H + lane; j < dst_ld; j += 32) DT<T>::st(dst + (size_t)row * dst_ld + j, (j == H && tok >= 0) ? 1.f : 0.f);
+  const unsigned chunks = (unsigned)(nvec + 31) / 32;
+  const unsigned piece = (blockIdx.x - pad_ctas) * kRowWarps + (threadIdx.x >> 5);   // 2^32 pieces are 2 TB
+  const int64_t t = piece / chunks;
+  const int i = (int)(piece - (unsigned)t * chunks) * 32 + lane;
+  if (t >= Tn) return;
+  const bool real = i < nvec;
+  uint4 q = make_uint4(0, 0, 0, 0);
+  if (real) q = __ldg(reinterpret_cast<const uint4*>(src) + t * nvec + i);
+  // the columns behind H: the lanes of the last warp once more
+  const bool last = ld_vec > nvec && i - lane + 32 >= nvec;
+  typename Dst::Piece x;
+  for (int k0 = 0; k0 < K; k0 += KB) {
+    int32_t r[KB];
+#pragma unroll
+    for (int k = 0; k < KB; ++k) r[k] = k0 + k < K ? __ldg(rt.flat_row + t * K + k0 + k) : -1;
+    if (k0 == 0) x = dst.piece(q);
+#pragma unroll
+    for (int k = 0; k < KB; ++k)
+      if (r[k] >= 0) {
+        if (real) dst.put((size_t)r[k], i, x);
+        if (last && lane < ld_vec - nvec)
+          dst.put((size_t)r[k], nvec + lane, dst.piece(lane == 0 ? dst.one() : make_uint4(0, 0, 0, 0)));
+      }
+  }
+}
+
+template <class Dst>
+inline cudaError_t launch_gather_tokens(const void* src, const Dst& dst, const RouteTables& rt, int64_t Tn, int H,
+                                        int esize, int E, int K, int row_round, cudaStream_t st) {
+  const int nvec = H * esize / 16, ld_vec = dst.ld * esize / 16;
+  const int64_t token_ctas = ceil_div(Tn * ceil_div(nvec, 32), kRowWarps), pad_ctas = row_round > 0 ? (int64_t)E * kPadCtas : 0;
+  auto kern = K <= 4 ? gather_tokens_kernel<Dst, 4> : gather_tokens_kernel<Dst, 8>;
+  return launch_pdl_opt(true, kern, dim3((unsigned)(pad_ctas + token_ctas)), dim3(kRowWarps * 32), 0, st, src, dst, rt, Tn,
+                        nvec, ld_vec, K, (unsigned)pad_ctas, row_round);
 }
 
 // Backward gather: gys[row, :] = grad_y[token, :] where grad_y is grad_out, or the sum of its K
@@ -77,6 +135,96 @@ gather_grad_kernel(const T* __restrict__ grad_out, int slots, const T* __restric
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
   if (lane == 0) gw_row[row] = dot;
+}
+
+// The same from the tokens' side (see gather_tokens_kernel): the K rows of a token take its gradient, which is read
+// once, and the dot products with K experts' biases are accumulated beside each other (T = 8192, H = 2880, K = 4: 101 us
+// by row, 79 by token).  `wpt` warps (1, 2, 4 or 8) share a token, so that few tokens also fill the GPU.
+template <typename T, class Dst, int KB>
+__global__ void __launch_bounds__(kRowWarps * 32)
+gather_grad_tokens_kernel(const T* __restrict__ grad_out, int slots, const T* __restrict__ down_bias, const Dst dst,
+                          float* __restrict__ gw_row, const RouteTables rt, int64_t Tn, int H, int K, int wpt,
+                          unsigned pad_ctas, int row_round) {
+  pdl_wait();
+  pdl_trigger();
+  constexpr int VE = 16 / (int)sizeof(T);
+  const int nvec = H / VE;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  if (blockIdx.x < pad_ctas) {
+    zero_padding(dst, rt, (int)blockIdx.x, row_round, nvec);
+    return;
+  }
+  __shared__ float s_dot[kRowWarps][KB];
+  const int64_t t = (int64_t)(blockIdx.x - pad_ctas) * (kRowWarps / wpt) + w / wpt;
+  const int part = w % wpt;
+  for (int k0 = 0; k0 < K; k0 += KB) {
+    int32_t r[KB];
+    const T* bias[KB];
+    float dot[KB];
+#pragma unroll
+    for (int k = 0; k < KB; ++k) r[k] = t < Tn && k0 + k < K ? __ldg(rt.flat_row + t * K + k0 + k) : -1;
+#pragma unroll
+    for (int k = 0; k < KB; ++k) {
+      bias[k] = down_bias + (r[k] >= 0 ? (size_t)__ldg(rt.tile_expert + r[k] / kTileM) * H : 0);
+      dot[k] = 0.f;
+    }
+    if (t < Tn) {
+#pragma unroll 2
+      for (int i = lane + 32 * part; i < nvec; i += 32 * wpt) {
+        float g[VE];
+        load_vec<T, VE>(grad_out + (size_t)t * slots * H + (size_t)i * VE, g);
+        for (int s = 1; s < slots; ++s) {
+          float g2[VE];
+          load_vec<T, VE>(grad_out + ((size_t)t * slots + s) * H + (size_t)i * VE, g2);
+#pragma unroll
+          for (int j = 0; j < VE; ++j) g[j] += g2[j];
+        }
+        uint4 q;
+        store_vec<T, VE>(reinterpret_cast<T*>(&q), g);
+        const typename Dst::Piece x = dst.piece(q);
+#pragma unroll
+        for (int k = 0; k < KB; ++k)
+          if (r[k] >= 0) {
+            dst.put((size_t)r[k], i, x);
+            float b[VE];
+            load_vec<T, VE>(bias[k] + (size_t)i * VE, b);
+#pragma unroll
+            for (int j = 0; j < VE; ++j) dot[k] = fmaf(g[j], b[j], dot[k]);
+          }
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < KB; ++k) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) dot[k] += __shfl_xor_sync(0xffffffffu, dot[k], o);
+      if (lane == 0) s_dot[w][k] = dot[k];
+    }
+    __syncthreads();
+    if (part == 0 && lane < KB) {
+      int32_t row = -1;
+#pragma unroll
+      for (int k = 0; k < KB; ++k) row = lane == k ? r[k] : row;
+      if (row >= 0) {
+        float sum = 0.f;
+        for (int o = 0; o < wpt; ++o) sum += s_dot[w + o][lane];
+        gw_row[row] = sum;
+      }
+    }
+    __syncthreads();
+  }
+}
+
+template <typename T, class Dst>
+inline cudaError_t launch_gather_grad_tokens(const T* grad_out, int slots, const T* down_bias, const Dst& dst, float* gw_row,
+                                             const RouteTables& rt, int64_t Tn, int H, int E, int K, int row_round,
+                                             cudaStream_t st) {
+  // at least 32 warps per SM, while each has a piece of the row
+  int wpt = 1;
+  while (wpt < kRowWarps && Tn * wpt < 148 * 32 && H * (int)sizeof(T) / 16 > 32 * wpt) wpt *= 2;
+  const int64_t token_ctas = ceil_div(Tn * wpt, kRowWarps), pad_ctas = (int64_t)E * kPadCtas;
+  auto kern = K <= 4 ? gather_grad_tokens_kernel<T, Dst, 4> : gather_grad_tokens_kernel<T, Dst, 8>;
+  return launch_pdl_opt(true, kern, dim3((unsigned)(pad_ctas + token_ctas)), dim3(kRowWarps * 32), 0, st, grad_out, slots,
+                        down_bias, dst, gw_row, rt, Tn, H, K, wpt, (unsigned)pad_ctas, row_round);
 }
 
 // out[i] = (T) acc[i]
@@ -167,7 +315,9 @@ __global__ void routing_grad_kernel(const float* __restrict__ gw_row, const int3
 // order, one rounding, every output element written exactly once (no zero-fill, no atomics).
 // One warp per token and 32 16-byte pieces of its row, with the loads of up to KB slots in flight: latency bounds the
 // few-token calls (a warp per token left most SMs idle and walked the columns one after the
-// other: 30 us at T = 64 and 512 with H = 2880, now about 5).
+// other: 30 us at T = 64 and 512 with H = 2880, now 3 to 5), HBM the others.  The pieces of a row are neighbours in
+// the grid, so that its 512-byte parts are read at about the same time (T = 4096 44 us with the tokens as
+// neighbours, now 30; T = 16384 166 and 116).
 // Rows of another type than the output (fp32 rows of a bf16 call) lie at their flat positions p = t*K + k.
 template <typename TY, typename T, int KB>
 __global__ void __launch_bounds__(kRowWarps * 32)
@@ -176,8 +326,10 @@ combine_padded_kernel(const TY* __restrict__ y, const int32_t* __restrict__ flat
   pdl_wait();
   constexpr bool kFlat = !std::is_same<TY, T>::value;
   constexpr int VE = 16 / (int)sizeof(TY);
-  const int64_t t = (int64_t)blockIdx.x * kRowWarps + (threadIdx.x >> 5);
-  const int i = blockIdx.y * 32 + (threadIdx.x & 31);
+  const unsigned chunks = (unsigned)(H / VE + 31) / 32;
+  const unsigned piece = blockIdx.x * kRowWarps + (threadIdx.x >> 5);
+  const int64_t t = piece / chunks;
+  const int i = (int)(piece - (unsigned)t * chunks) * 32 + (threadIdx.x & 31);
   if (t >= Tn || i >= H / VE) return;
   float acc[VE];
 #pragma unroll
@@ -202,7 +354,7 @@ combine_padded_kernel(const TY* __restrict__ y, const int32_t* __restrict__ flat
 
 template <typename TY, typename T>
 inline int launch_combine(const TY* y, const int32_t* flat_row, T* out, int64_t Tn, int H, int K, cudaStream_t st) {
-  const dim3 grid((unsigned)ceil_div(Tn, kRowWarps), (unsigned)ceil_div(H, 32 * (16 / (int)sizeof(TY))));
+  const dim3 grid((unsigned)ceil_div(Tn * ceil_div(H, 32 * (16 / (int)sizeof(TY))), kRowWarps));
   auto kern = K <= 4 ? combine_padded_kernel<TY, T, 4> : combine_padded_kernel<TY, T, 8>;
   const cudaError_t rc = launch_pdl_opt(true, kern, grid, dim3(kRowWarps * 32), 0, st, y, flat_row, out, Tn, H, K);
   return rc == cudaSuccess && cudaGetLastError() == cudaSuccess ? YAMOE_OK : YAMOE_ERR_CUDA;

@@ -163,25 +163,26 @@ struct Planes {
   }
 };
 
-// Gather of the token rows into the padded layout, as planes (see gather_rows_kernel; the columns
-// from H to ld are (1, 0, 0, ...) for token rows).
-__global__ void __launch_bounds__(kRowWarps * 32)
-gather_split_kernel(const float* __restrict__ src, Planes dst, const int32_t* __restrict__ row_token,
-                    const int32_t* __restrict__ header, int H) {
-  const int row = blockIdx.x * kRowWarps + (threadIdx.x >> 5);
-  if (row >= header[kHdrRowsUsed]) return;
-  const int lane = threadIdx.x & 31;
-  const int tok = row_token[row];
-  const float4* s = reinterpret_cast<const float4*>(src + (size_t)(tok < 0 ? 0 : tok) * H);
-  for (int i = lane; i < dst.ld / 4; i += 32) {
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (tok >= 0) {
-      if (4 * i < H) v = __ldg(s + i);
-      else if (4 * i == H) v.x = 1.f;
-    }
-    dst.store4(row, 4 * i, {v.x, v.y, v.z, v.w});
+// The gathers' destinations as planes (see RowDst): a piece, four adjacent columns, is split once for all K rows.  With
+// `rows` the fp32 values are written as well, H apart (upstream gradient: M operand of the down weight gradient).
+struct PlaneDst {
+  struct Piece { uint4 x; uint2 p[3]; };
+  Planes planes;
+  int ld;
+  float* rows;
+  __device__ __forceinline__ Piece piece(const uint4& q) const {
+    uint32_t p0[2], p1[2], p2[2];
+    split3<4>({__uint_as_float(q.x), __uint_as_float(q.y), __uint_as_float(q.z), __uint_as_float(q.w)}, p0, p1, p2);
+    return Piece{q, {make_uint2(p0[0], p0[1]), make_uint2(p1[0], p1[1]), make_uint2(p2[0], p2[1])}};
   }
-}
+  __device__ __forceinline__ void put(size_t row, int vec, const Piece& q) const {
+    __nv_bfloat16* d = planes.p + row * ld + 4 * vec;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) *reinterpret_cast<uint2*>(d + i * planes.stride) = q.p[i];
+    if (rows != nullptr) reinterpret_cast<uint4*>(rows + row * ld)[vec] = q.x;
+  }
+  __device__ __forceinline__ uint4 one() const { return make_uint4(0x3f800000u, 0u, 0u, 0u); }
+};
 
 // Between fp32 rows and planes of the same pitch: the buffer of the saving forward holds planes whichever kernels
 // fill and read it, and the CUDA-core kernels (weights that TMA cannot address, the validation path) work on rows.
@@ -209,40 +210,6 @@ join_rows_kernel(Planes src, float* __restrict__ dst, const int32_t* __restrict_
     for (int j = 0; j < 4; ++j) a[j] += b[j] + c[j];          // exact: see split3_special
     store_vec<float, 4>(dst + (size_t)row * src.ld + i, a);
   }
-}
-
-// Gather of the upstream gradient: fp32 rows (M operand of the down weight gradient) and planes (N
-// operand of the data gradient); seeds the routing-weight gradient as gather_grad_kernel does.
-__global__ void __launch_bounds__(kRowWarps * 32)
-gather_grad_split_kernel(const float* __restrict__ grad_out, int slots, const float* __restrict__ down_bias,
-                         float* __restrict__ gys, Planes dst, float* __restrict__ gw_row,
-                         const int32_t* __restrict__ row_token, const int32_t* __restrict__ tile_expert,
-                         const int32_t* __restrict__ header, int H) {
-  const int row = blockIdx.x * kRowWarps + (threadIdx.x >> 5);
-  if (row >= header[kHdrRowsUsed]) return;
-  const int lane = threadIdx.x & 31;
-  const int tok = row_token[row];
-  const float* bias = down_bias + (size_t)tile_expert[row / kTileM] * H;
-  float dot = 0.f;
-  for (int i = lane; i < H / 4; i += 32) {
-    float g[4] = {0.f, 0.f, 0.f, 0.f};
-    if (tok >= 0) {
-      float g2[4], b[4];
-      for (int s = 0; s < slots; ++s) {
-        load_vec<float, 4>(grad_out + ((size_t)tok * slots + s) * H + 4 * (size_t)i, g2);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) g[j] = s == 0 ? g2[j] : g[j] + g2[j];
-      }
-      load_vec<float, 4>(bias + 4 * (size_t)i, b);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) dot += g[j] * b[j];
-    }
-    store_vec<float, 4>(gys + (size_t)row * H + 4 * (size_t)i, g);
-    dst.store4(row, 4 * i, g);
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
-  if (lane == 0) gw_row[row] = dot;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -543,8 +510,7 @@ umma_f32_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__
     const int p0 = p.pad_off[i];
     s_pad[i] = p0;
     if (i < p.E) {
-      const int have = min(p.counts[i], p.pad_off[i + 1] - p0);
-      s_rows[i] = (have + p.row_round - 1) & ~(p.row_round - 1);
+      s_rows[i] = covered_rows(p.counts[i], p.pad_off[i + 1] - p0, p.row_round);
     }
   }
   __syncthreads();

@@ -449,8 +449,7 @@ umma_pair_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant_
     s_pad[i] = p0;
     if (MODE != kWgrad) s_pair[i] = p.pair_off[i];
     if (i < p.E) {
-      const int have = min(p.counts[i], p.pad_off[i + 1] - p0);    // at least the rows the capacity keeps
-      s_rows[i] = (have + p.row_round - 1) & ~(p.row_round - 1);
+      s_rows[i] = covered_rows(p.counts[i], p.pad_off[i + 1] - p0, p.row_round);
     }
   }
   __syncthreads();

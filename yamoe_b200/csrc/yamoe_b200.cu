@@ -211,8 +211,8 @@ static int forward_f32_split(const Plan& p, const float* hidden, const float* wg
   const Planes xs = p.planes(p.xs, H), act = p.planes(p.act, H);
   {
     StageTimer tm(kStageGather, st);
-    gather_split_kernel<<<(unsigned)ceil_div(p.max_rows, kRowWarps), kRowWarps * 32, 0, st>>>(
-        hidden, xs, p.rt.row_token, p.rt.header, H);
+    if (launch_gather_tokens(hidden, PlaneDst{xs, H, nullptr}, p.rt, Tn, H, 4, E, K, 0, st) != cudaSuccess)
+      return YAMOE_ERR_CUDA;
   }
   int rc;
   {
@@ -263,12 +263,10 @@ static int forward_impl(const void* hidden, const int64_t* ridx, const void* rw,
                                reinterpret_cast<const T*>(bgu), reinterpret_cast<const T*>(wd),
                                reinterpret_cast<const T*>(bd), reinterpret_cast<T*>(out), Tn, H, E, K, st);
   }
-  const unsigned row_blocks = (unsigned)ceil_div(p.max_rows, kRowWarps);
   {
     StageTimer tm(kStageGather, st);
-    if (launch_pdl_opt(true, gather_rows_kernel<T>, dim3(row_blocks), dim3(kRowWarps * 32), 0, st,
-                   reinterpret_cast<const T*>(hidden), reinterpret_cast<T*>(p.xs),
-                   (const int32_t*)p.rt.row_token, (const int32_t*)p.rt.header, H, H) != cudaSuccess)
+    if (launch_gather_tokens(hidden, RowDst<T>{reinterpret_cast<T*>(p.xs), H}, p.rt, Tn, H, sizeof(T), E, K,
+                             tc ? 0 : kTileM, st) != cudaSuccess)
       return YAMOE_ERR_CUDA;
   }
   EpiGluAct<T> glu{reinterpret_cast<const T*>(bgu), reinterpret_cast<T*>(p.act), p.rt.row_token, H};
@@ -343,8 +341,8 @@ static int forward_train_impl(const void* hidden, const int64_t* ridx, const voi
   if constexpr (sizeof(T) == 4) {
     if (use_split_f32(current_path(), H, wgu, wd)) {
       const Planes xs = p.planes(p.xs, Hp), actw = p.planes(p.actw, Hp), act = p.planes(p.gpre_planes, H);
-      gather_split_kernel<<<row_blocks, kRowWarps * 32, 0, st>>>(reinterpret_cast<const T*>(hidden), xs, p.rt.row_token,
-                                                                 p.rt.header, H);
+      if (launch_gather_tokens(hidden, PlaneDst{xs, Hp, nullptr}, p.rt, Tn, H, 4, E, K, 64, st) != cudaSuccess)
+        return YAMOE_ERR_CUDA;
       const F32Glu<true> glu{reinterpret_cast<const T*>(bgu), act, actw, reinterpret_cast<T*>(p.pre), p.rt.row_token,
                              p.rt.row_weight, H};
       T* yrows = reinterpret_cast<T*>(p.gys);
@@ -361,8 +359,9 @@ static int forward_train_impl(const void* hidden, const int64_t* ridx, const voi
   const bool convert = saves_planes(dtype, H);
   T* xs = reinterpret_cast<T*>(convert ? (void*)saved_xs_rows(p) : p.xs);
   T* actw = reinterpret_cast<T*>(convert ? (void*)saved_actw_rows(p) : p.actw);
-  gather_rows_kernel<T><<<row_blocks, kRowWarps * 32, 0, st>>>(reinterpret_cast<const T*>(hidden), xs, p.rt.row_token,
-                                                              p.rt.header, H, Hp);
+  const bool tc = use_tcgen05(current_path(), dtype, H);
+  if (launch_gather_tokens(hidden, RowDst<T>{xs, Hp}, p.rt, Tn, H, sizeof(T), E, K, tc ? 64 : kTileM, st) != cudaSuccess)
+    return YAMOE_ERR_CUDA;
   T* act = reinterpret_cast<T*>(p.gpre);
   T* yrows = reinterpret_cast<T*>(p.gys);
   EpiGlu<T> glu{reinterpret_cast<const T*>(bgu), act, actw, reinterpret_cast<T*>(p.pre),
@@ -373,7 +372,7 @@ static int forward_train_impl(const void* hidden, const int64_t* ridx, const voi
   g1.pair_expert = p.rt.pair_expert; g1.pair_off = p.rt.pair_off; g1.counts = p.rt.counts;
   GemmArgs g2{act, H, wd, H, (int64_t)H * H, 0, H, H, E, p.rt.tile_expert, p.rt.pad_off, p.rt.header};
   g2.pair_expert = p.rt.pair_expert; g2.pair_off = p.rt.pair_off; g2.counts = p.rt.counts;
-  if (use_tcgen05(current_path(), dtype, H)) {
+  if (tc) {
     if constexpr (sizeof(T) == 2) {
       const PairGlu<true> pglu{glu.bias, act, glu.actw, glu.pre, p.rt.row_token, p.rt.row_weight, H, Hp};
       const PairWeightedRows pw{wrows.bias, yrows, p.rt.row_token, p.rt.row_weight, H};
@@ -396,8 +395,8 @@ static int forward_train_impl(const void* hidden, const int64_t* ridx, const voi
 // Input, weight and bias gradients in fp32 (the routing-weight gradients are left in p.gw_row); `acc` is zeroed.
 static int backward_f32_split(const Plan& p, const float* grad_out, int slots, const float* hidden, const float* wgu,
                               const float* bgu, const float* wd, const float* bd, float* acc, float* d_wgu,
-                              float* d_bgu, float* d_wd, float* d_bd, int H, int E, bool saved, cudaStream_t st) {
-  const unsigned row_blocks = (unsigned)ceil_div(p.max_rows, kRowWarps);
+                              float* d_bgu, float* d_wd, float* d_bd, int64_t Tn, int H, int E, int K, bool saved,
+                              cudaStream_t st) {
   const int Hp = H + kBiasCols, H2 = 2 * H;
   const int64_t HH = (int64_t)H * H;
   const Planes xs = p.planes(p.xs, Hp), actw = p.planes(p.actw, Hp), gys = p.planes(p.gys_planes, H),
@@ -405,10 +404,11 @@ static int backward_f32_split(const Plan& p, const float* grad_out, int slots, c
   float* gys32 = reinterpret_cast<float*>(p.gys);
   float* gpre32 = reinterpret_cast<float*>(p.gpre);
   float* pre = reinterpret_cast<float*>(p.pre);
-  if (!saved)
-    gather_split_kernel<<<row_blocks, kRowWarps * 32, 0, st>>>(hidden, xs, p.rt.row_token, p.rt.header, H);
-  gather_grad_split_kernel<<<row_blocks, kRowWarps * 32, 0, st>>>(grad_out, slots, bd, gys32, gys, p.gw_row,
-                                                                  p.rt.row_token, p.rt.tile_expert, p.rt.header, H);
+  if (!saved && launch_gather_tokens(hidden, PlaneDst{xs, Hp, nullptr}, p.rt, Tn, H, 4, E, K, 64, st) != cudaSuccess)
+    return YAMOE_ERR_CUDA;
+  if (launch_gather_grad_tokens(grad_out, slots, bd, PlaneDst{gys, H, gys32}, p.gw_row, p.rt, Tn, H, E, K, 64, st) !=
+      cudaSuccess)
+    return YAMOE_ERR_CUDA;
   const F32Glu<true> glu{bgu, Planes{}, actw, pre, p.rt.row_token, p.rt.row_weight, H};
   const F32GluBackward glub{pre, gpre32, gpre, p.gw_row, p.rt.row_token, p.rt.row_weight, H};
   const F32StoreBias st_wd{d_wd, d_bd, H, H}, st_wgu{d_wgu, d_bgu, H, H2};
@@ -464,7 +464,7 @@ static int backward_impl(const void* grad_out, int per_slot, const void* hidden,
                               reinterpret_cast<const T*>(wgu), reinterpret_cast<const T*>(bgu),
                               reinterpret_cast<const T*>(wd), reinterpret_cast<const T*>(bd), acc,
                               reinterpret_cast<T*>(d_wgu), reinterpret_cast<T*>(d_bgu), reinterpret_cast<T*>(d_wd),
-                              reinterpret_cast<T*>(d_bd), H, E, saved, st);
+                              reinterpret_cast<T*>(d_bd), Tn, H, E, K, saved, st);
       if (rc) return rc;
       routing_grad_kernel<T><<<(unsigned)ceil_div(p.max_rows, 256), 256, 0, st>>>(
           p.gw_row, p.rt.row_token, p.rt.row_flat, p.rt.tile_expert, p.rt.header, reinterpret_cast<T*>(d_routing),
@@ -482,12 +482,14 @@ static int backward_impl(const void* grad_out, int per_slot, const void* hidden,
       join_rows_kernel<<<row_blocks, kRowWarps * 32, 0, st>>>(p.planes(p.actw, Hp), actw, p.rt.header);
     }
   }
-  if (!saved)
-    gather_rows_kernel<T><<<row_blocks, kRowWarps * 32, 0, st>>>(reinterpret_cast<const T*>(hidden), xs,
-                                                                p.rt.row_token, p.rt.header, H, Hp);
-  gather_grad_kernel<T><<<row_blocks, kRowWarps * 32, 0, st>>>(
-      reinterpret_cast<const T*>(grad_out), per_slot ? K : 1, reinterpret_cast<const T*>(bd),
-      reinterpret_cast<T*>(p.gys), p.gw_row, p.rt.row_token, p.rt.tile_expert, p.rt.header, H);
+  const int row_round = use_tcgen05(path, dtype, H) ? 64 : kTileM;
+  if (!saved &&
+      launch_gather_tokens(hidden, RowDst<T>{xs, Hp}, p.rt, Tn, H, sizeof(T), E, K, row_round, st) != cudaSuccess)
+    return YAMOE_ERR_CUDA;
+  if (launch_gather_grad_tokens(reinterpret_cast<const T*>(grad_out), per_slot ? K : 1, reinterpret_cast<const T*>(bd),
+                                RowDst<T>{reinterpret_cast<T*>(p.gys), H}, p.gw_row, p.rt, Tn, H, E, K, row_round,
+                                st) != cudaSuccess)
+    return YAMOE_ERR_CUDA;
 
   // 1. recompute: pre = xs W_gu + b_gu,  actw = w * glu(pre)
   EpiGlu<T> glu{reinterpret_cast<const T*>(bgu), nullptr, actw, reinterpret_cast<T*>(p.pre), p.rt.row_token,
