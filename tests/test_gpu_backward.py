@@ -110,3 +110,16 @@ def test_saved_activation_pair_matches_recompute(dtype):
         for i, r, name in zip((0, 2, 3, 4, 5, 6), ref_g, GRADS):
             orc.check_close(dev[i].grad.float().cpu(), r, tol, f"saved-mode {name} (capacity {cap})",
                             rel_l2=None if dtype == torch.float32 else 2e-2)
+
+
+@pytest.mark.parametrize("H,E", [(64, 3), (128, 5), (256, 4), (320, 6), (64, 150), (128, 300)])
+def test_weight_gradients_of_few_rows(H, E):
+    """Output rows and columns at the edges of the parked boxes, the bias row in a box of its own or behind others, experts
+    without rows, and more experts than leave space for two parking buffers."""
+    T, K = 130, 2
+    inp = orc.make_inputs(T, H, E, K, seed=H + E, weight_std=H ** -0.5, bias_std=0.2, dtype=torch.bfloat16, with_grad=True)
+    args = [inp[k] for k in ("hidden_states", "router_indices", "routing_weights", "gate_up_proj", "gate_up_proj_bias",
+                             "down_proj", "down_proj_bias")]
+    ref = orc.experts_backward_oracle(inp["grad_out"], *args, T, E, K)
+    for a, b, key in zip(run_backward(inp["grad_out"], args, T, E, K), ref, GRADS):
+        orc.check_close(a.float(), b, RTOL_BF16, key, rel_l2=2e-2)

@@ -700,7 +700,7 @@ inline bool umma_available() {
 // Encoding a map is a driver call that costs some tens of microseconds of host time; the same
 // (pointer, shape, box) comes back call after call (weights, persistent buffers, workspaces that the
 // caching allocator hands out again), so the last maps are kept in a small table.
-enum MapKind { kMapBf16 = 0, kMapF32 = 1, kMapF32Swizzled = 2, kMapBf16Plain = 3 };   // plain: no swizzle
+enum MapKind { kMapBf16 = 0, kMapF32 = 1, kMapF32Swizzled = 2 };
 struct TensorMapKey {
   const void* base;
   int rank, kind;
@@ -739,9 +739,9 @@ inline bool make_map(CUtensorMap* m, const void* base, int rank, const uint64_t*
   cuuint32_t bx[4], es[4] = {1, 1, 1, 1};
   for (int i = 0; i < rank; ++i) { gd[i] = dims[i]; bx[i] = box[i]; }
   for (int i = 0; i + 1 < rank; ++i) gs[i] = strides[i];
-  CUresult r = encode_tiled_fn()(m, kind == kMapBf16 || kind == kMapBf16Plain ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32,
+  CUresult r = encode_tiled_fn()(m, kind == kMapBf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32,
                                  (cuuint32_t)rank, const_cast<void*>(base), gd, gs, bx, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                                 kind == kMapF32 || kind == kMapBf16Plain ? CU_TENSOR_MAP_SWIZZLE_NONE : CU_TENSOR_MAP_SWIZZLE_128B,
+                                 kind == kMapF32 ? CU_TENSOR_MAP_SWIZZLE_NONE : CU_TENSOR_MAP_SWIZZLE_128B,
                                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return false;
   std::lock_guard<std::mutex> lock(mu);

@@ -51,6 +51,7 @@ constexpr int kPairStageBytes = kPairABytes + kPairBBytes;
 constexpr int kPairStages = 6;
 constexpr int kPairGroups = kPairStages / 2;   // stages are freed two at a time
 constexpr int kPairSmem = kPairStages * kPairStageBytes + 1024;   // + slack for 1024-byte alignment
+constexpr int kPairParkBytes = 32 * 128 * 2;   // parked output rows of four epilogue warps (PairStoreBias)
 
 __device__ __forceinline__ void mbar_expect_tx_cluster(uint32_t bar_cluster_addr, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cluster.b64 _, [%0], %1;" ::"r"(bar_cluster_addr), "r"(bytes)
@@ -106,6 +107,7 @@ struct PairParams {
   const int32_t* pad_off;
   const int32_t* counts;
   int32_t* header;
+  int bufs;                     // parking buffers of a group (kTmaStore)
 };
 
 // ---------------------------------------------------------------------------------------------
@@ -347,30 +349,64 @@ struct PairGluBackward {
   }
 };
 
+// 32 M indices x 32 N indices of an accumulator: two TMEM loads of 16 lanes x 32 columns leave in a thread pairs of
+// neighbouring N of the M indices lane / 4 + 8 i, which is how stmatrix takes the rows of 8 x 8 matrices.
+__device__ __forceinline__ void tc_ld_16x256_issue(uint32_t taddr, uint32_t (&r)[32]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x4.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr) : "memory");
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x4.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
+        "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(taddr + (16u << 16)) : "memory");
+}
+__device__ __forceinline__ void stmatrix_x4_trans(uint32_t addr, uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};"
+               ::"r"(addr), "r"(r0), "r"(r1), "r"(r2), "r"(r3) : "memory");
+}
+
 // Weight gradient: output row n = `row` + i of C[e] ([H, ld]); row H is the bias gradient (the operand
 // in N carries a column of ones or routing weights behind its H columns), later rows do not exist.
 // With few rows per expert this GEMM is bound by its output (3 H^2 values per expert for as little
-// as one k-block), so the tile leaves by TMA: four warps park 32 rows of 128 columns in shared memory,
-// one copy stores them (whole 256-byte rows, clipped at the matrix edge) while the warps go on.
+// as one k-block), so the tile leaves by TMA: four warps park 32 rows of 128 columns in shared memory (two boxes of 64
+// columns, swizzled so that the eight rows of a matrix fall on different banks), and copies clipped at the matrix edge
+// store them while the warps go on.  The transposition is stmatrix's: with shuffles and 4-byte stores the epilogue of a
+// tile took longer still.  192 rows per expert (E = 64, H = 2048): gate_up 395 -> 350 us, down 205 -> 185 (1.07 and 0.54 GB of
+// output, 145 and 73 us at the rate of a fill; without the copies 250, without any epilogue 169).  Meeting once for two
+// chunks in a single buffer of twice the size: 363.
 struct PairStoreBias {
   static constexpr bool kTmaStore = true;
   __nv_bfloat16* C;                // [E, H, ld]
   __nv_bfloat16* bias_out;         // [E, ld]
   int H, ld;
 
-  // parks rows t0 .. t0+15 (even lanes) or 16.. (odd lanes) of the columns (m & ~1, +1); the bias row goes out directly
-  __device__ __forceinline__ void park(int e, int m, int row, int q, int lane, const float (&v)[32], uint8_t* buf) const {
-    const bool odd = lane & 1;
-    float lo[16], hi[16];
-    pair_columns(v, odd, lo, hi);
-    const int t0 = odd ? 16 : 0;
-    uint32_t* dst = reinterpret_cast<uint32_t*>(buf + t0 * 256 + q * 64) + (lane >> 1);
+  // accumulator values (tc_ld_16x256_issue) as bf16 pairs along N: p[4 j + h] holds N 8 j .. 8 j + 7 of M 8 h .. 8 h + 7
+  static __device__ __forceinline__ void pack(const uint32_t (&r)[32], uint32_t (&p)[16]) {
 #pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      const uint32_t x = pack_bf16x2(lo[i], hi[i]);
-      dst[i * 64] = x;
-      if (row + t0 + i == H && m < ld) *reinterpret_cast<uint32_t*>(bias_out + (size_t)e * ld + (m & ~1)) = x;
-    }
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int h = 0; h < 4; ++h) {
+        const int i = 16 * (h >> 1) + 4 * j + 2 * (h & 1);
+        p[4 * j + h] = pack_bf16x2(__uint_as_float(r[i]), __uint_as_float(r[i + 1]));
+      }
+  }
+  static __device__ __forceinline__ void park(const uint32_t (&p)[16], int q, int lane, uint32_t buf) {
+    const uint32_t row = lane & 7, piece = 4 * (q & 1) + (lane >> 3);
+    const uint32_t dst = buf + (q >> 1) * (kPairParkBytes / 2) + row * 128 + ((piece ^ row) << 4);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) stmatrix_x4_trans(dst + j * 8 * 128, p[4 * j], p[4 * j + 1], p[4 * j + 2], p[4 * j + 3]);
+  }
+  // parked row i is the bias gradient: one column to a thread of the group
+  __device__ __forceinline__ void bias_row(int e, int cta_m, int i, int q, int lane, const uint8_t* buf) const {
+    const int col = q * 32 + lane, c = col & 63;
+    if (cta_m + col < ld)
+      bias_out[(size_t)e * ld + cta_m + col] = *reinterpret_cast<const __nv_bfloat16*>(
+          buf + (q >> 1) * (kPairParkBytes / 2) + i * 128 + (((c >> 3) ^ (i & 7)) << 4) + 2 * (c & 7));
   }
 };
 
@@ -379,15 +415,23 @@ struct epi_tma_store : std::false_type {};
 template <class E>
 struct epi_tma_store<E, std::enable_if_t<E::kTmaStore>> : std::true_type {};
 
-constexpr int kPairParkBytes = 32 * 128 * 2;                    // parked rows of one group of four epilogue warps
-constexpr int kPairSmemStore = kPairSmem + 2 * kPairParkBytes;
+// Shared memory: ring, parking space (`bufs` buffers for either group of four warps), expert tables.  Two buffers, so that
+// a group parks a chunk while the copy of the one before is read, fit beside the tables of up to some 140 experts.
+constexpr int kMaxDynamicSmem = 227 * 1024 - 256;               // the barriers are static
+inline int pair_smem(bool store, int E, int bufs) {
+  return kPairSmem + (store ? 2 * bufs * kPairParkBytes : 0) + (3 * E + 2) * 4;
+}
 
 __device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, int c0, int c1, int c2, uint32_t src) {
   asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];"
                ::"l"(map), "r"(src), "r"(c0), "r"(c1), "r"(c2) : "memory");
-  asm volatile("cp.async.bulk.commit_group;" ::: "memory");
 }
-__device__ __forceinline__ void tma_store_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void tma_store_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+// until the copies of all groups, or of all but the last, have read their shared memory
+__device__ __forceinline__ void tma_store_wait_read(bool all) {
+  if (all) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+  else asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+}
 __device__ __forceinline__ void tma_store_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 __device__ __forceinline__ void group_sync(int id) { asm volatile("bar.sync %0, 128;" ::"r"(id) : "memory"); }
 
@@ -413,14 +457,14 @@ umma_pair_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant_
   __shared__ __align__(8) uint64_t bar_tmem_empty[2];           // used in the leader CTA
   __shared__ uint32_t tmem_base_slot;
   __shared__ int abort_flag;
-  __shared__ int32_t s_pad[kUmmaMaxExperts + 1];    // first padded row of each expert
-  __shared__ int32_t s_pair[kUmmaMaxExperts + 1];   // row-tiled: first 256-row tile of each expert
-  __shared__ int32_t s_rows[kUmmaMaxExperts];       // rows to cover
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
   const bool leader = rank == 0;
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  int32_t* s_pad = reinterpret_cast<int32_t*>(smem_raw + kPairSmem + (kStore ? 2 * p.bufs * kPairParkBytes : 0));
+  int32_t* s_pair = s_pad + p.E + 1;   // [E + 1] row-tiled: first 256-row tile of each expert; s_pad [E + 1]: first padded row
+  int32_t* s_rows = s_pair + p.E + 1;  // [E] rows to cover
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kPairStages; ++s) mbar_init(smem_u32(&bar_full[s]), 2);   // arrive.expect_tx of both producers
@@ -616,6 +660,8 @@ umma_pair_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant_
     // =========================== epilogue (warps 2..9 of both CTAs) ==========================
     const int q = warp & 3;                    // TMEM lane quarter this warp may read
     const int turn = (warp - 2) >> 2;          // takes the 32-column chunks turn, turn + 2, ...
+    [[maybe_unused]] const uint32_t park0 = smem_base + kPairStages * kPairStageBytes + turn * p.bufs * kPairParkBytes;
+    [[maybe_unused]] uint32_t park = park0;
     int acc = 0;
     uint32_t acc_phase = 0;
     int e_next = expert_of(cluster_id);
@@ -628,27 +674,36 @@ umma_pair_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant_
       // M is a multiple of 32.  (Stored by TMA, the four warps of a group stay together and the copy clips.)
       const bool mine = kStore ? cta_m < p.M : m - lane < p.M;
       const int nchunks = (width + 31) >> 5;
-      auto emit = [&](int c, const float (&v)[32]) {
+      // 32 columns of the accumulator: as fp32 by M index, or (kStore) packed for stmatrix
+      auto emit = [&](int c, const auto& v) {
         const int row = n0 + c * 32;
         if constexpr (kStore) {
-          uint8_t* buf = smem_raw + (smem_base - smem_u32(smem_raw)) + kPairStages * kPairStageBytes + turn * kPairParkBytes;
           const bool issuer = q == 0 && lane == 0;
-          if (issuer) tma_store_wait_read();
+          if (issuer) tma_store_wait_read(p.bufs == 1);
           group_sync(1 + turn);
-          epi.park(e, m, row, q, lane, v, buf);
+          epi.park(v, q, lane, park);
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the parked rows are read by the copy
           group_sync(1 + turn);
-          if (issuer && row < epi.H) tma_store_3d(&tmOut, cta_m, row, e, smem_u32(buf));
+          if (issuer) {
+            if (row < epi.H) {
+              tma_store_3d(&tmOut, cta_m, row, e, park);
+              if (cta_m + 64 < epi.ld) tma_store_3d(&tmOut, cta_m + 64, row, e, park + kPairParkBytes / 2);
+            }
+            tma_store_commit();                  // also without a copy: the groups count the buffers
+          }
+          if (row <= epi.H && epi.H < row + 32)
+            epi.bias_row(e, cta_m, epi.H - row, q, lane, smem_raw + (park - smem_u32(smem_raw)));
+          if (p.bufs == 2) park = park0 + (park == park0 ? kPairParkBytes : 0);
         } else {
           epi.apply(e, m, row, min(32, width - c * 32), lane, v);
         }
       };
       if (kblocks == 0) {                      // kWgrad of an expert without rows
-        float z[32];
-#pragma unroll
-        for (int i = 0; i < 32; ++i) z[i] = 0.f;
-        if (mine)
-          for (int c = turn; c < nchunks; c += 2) emit(c, z);
+        if constexpr (kStore) {
+          const uint32_t z[16] = {};
+          if (mine)
+            for (int c = turn; c < nchunks; c += 2) emit(c, z);
+        }
         continue;
       }
       if constexpr (epi_prefetches<Epi>::value) {
@@ -668,12 +723,20 @@ umma_pair_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant_
 #pragma unroll 1
         for (int c = turn; c < nchunks; c += 2) {
           uint32_t r[32];
-          tc_ld_32x32_issue(t_row + c * 32, r);
-          tc_ld_wait(r);
-          float v[32];
+          if constexpr (kStore) {
+            tc_ld_16x256_issue(t_row + c * 32, r);
+            tc_ld_wait(r);
+            uint32_t v[16];
+            epi.pack(r, v);
+            emit(c, v);
+          } else {
+            tc_ld_32x32_issue(t_row + c * 32, r);
+            tc_ld_wait(r);
+            float v[32];
 #pragma unroll
-          for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
-          emit(c, v);
+            for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
+            emit(c, v);
+          }
         }
       }
       tc_fence_before();
@@ -761,21 +824,22 @@ inline int launch_umma_pair(const GemmArgs& g, const Epi& epi, int64_t max_rows,
     }
   }
   constexpr bool kStore = epi_tma_store<Epi>::value;
-  constexpr int smem = kStore ? kPairSmemStore : kPairSmem;
+  const int bufs = pair_smem(kStore, g.E, 2) <= kMaxDynamicSmem ? 2 : 1;
+  const int smem = pair_smem(kStore, g.E, bufs);
   CUtensorMap tmOut = tmM;               // not used
   if constexpr (kStore) {
     const uint64_t d[3] = {(uint64_t)epi.ld, (uint64_t)epi.H, (uint64_t)g.E};
     const uint64_t st[2] = {(uint64_t)epi.ld * 2, (uint64_t)epi.ld * epi.H * 2};
-    const uint32_t b[3] = {128, 32, 1};
-    ok = ok && make_map(&tmOut, epi.C, 3, d, st, b, kMapBf16Plain);
+    const uint32_t b[3] = {64, 32, 1};
+    ok = ok && make_map(&tmOut, epi.C, 3, d, st, b);
   }
   if (!ok) return YAMOE_ERR_CUDA;
   auto kern = umma_pair_kernel<MODE, Epi>;
   static PerDevice<int> resident;    // per template instantiation and device
-  const int pairs = resident_pairs(kern, kPairThreads, smem, resident);
+  const int pairs = resident_pairs(kern, kPairThreads, kMaxDynamicSmem, resident);
   if (pairs <= 0) return YAMOE_ERR_CUDA;
   const PairParams p{g.N, g.M, g.K, g.E, row_round, g.pair_expert, g.pair_off, g.pad_off, g.counts,
-                     const_cast<int32_t*>(g.header)};
+                     const_cast<int32_t*>(g.header), bufs};
   const int64_t MT = ceil_div(g.N, kPairM);
   // the tables bound the number of row tiles by max_tiles (128-row tiles)
   const int64_t total_max = MODE == kWgrad ? (int64_t)g.E * MT * ceil_div(g.M, kPairN) : max_tiles * MT;
