@@ -123,3 +123,20 @@ def test_weight_gradients_of_few_rows(H, E):
     ref = orc.experts_backward_oracle(inp["grad_out"], *args, T, E, K)
     for a, b, key in zip(run_backward(inp["grad_out"], args, T, E, K), ref, GRADS):
         orc.check_close(a.float(), b, RTOL_BF16, key, rel_l2=2e-2)
+
+
+@pytest.mark.parametrize("dense", [True, False])
+@pytest.mark.parametrize("T,E,K,capacity", [(9, 40, 33, 4), (70, 70, 5, 3), (33, 8, 8, 100)])
+def test_routing_gradient_of_every_column(T, E, K, capacity, dense):
+    """d_routing is written whole: more slots than a warp has lanes, several rounds of columns, dropped assignments; nothing
+    of it was set before (the allocator is made to hand out used memory)."""
+    inp = orc.make_inputs(T, 64, E, K, seed=E + K, weight_std=0.125, bias_std=0.2, dtype=torch.float32, with_grad=True)
+    args = [inp[k] for k in ("hidden_states", "router_indices", "routing_weights", "gate_up_proj", "gate_up_proj_bias",
+                             "down_proj", "down_proj_bias")]
+    if not dense:
+        args[2] = torch.gather(args[2], 1, args[1]).contiguous()
+    ref = orc.experts_backward_oracle(inp["grad_out"], *args, capacity, E, K)
+    used = [torch.full((n,), float("nan"), device="cuda") for n in (T * E, T * K, T * 64) for _ in range(4)]
+    del used
+    for a, b, key in zip(run_backward(inp["grad_out"], args, capacity, E, K), ref, GRADS):
+        orc.check_close(a, b, RTOL_F32, key)

@@ -140,11 +140,13 @@ gather_grad_kernel(const T* __restrict__ grad_out, int slots, const T* __restric
 // The same from the tokens' side (see gather_tokens_kernel): the K rows of a token take its gradient, which is read
 // once, and the dot products with K experts' biases are accumulated beside each other (T = 8192, H = 2880, K = 4: 101 us
 // by row, 79 by token).  `wpt` warps (1, 2, 4 or 8) share a token, so that few tokens also fill the GPU.
+// The warps of a token also zero its row of `acc`, the fp32 sums of the hidden states' gradient: stores run at 7 TB/s
+// where a memset does 3.9, and a launch is saved (T = 8192, H = 2880: memset 22 us + gather 64, together 77).
 template <typename T, class Dst, int KB>
 __global__ void __launch_bounds__(kRowWarps * 32)
 gather_grad_tokens_kernel(const T* __restrict__ grad_out, int slots, const T* __restrict__ down_bias, const Dst dst,
-                          float* __restrict__ gw_row, const RouteTables rt, int64_t Tn, int H, int K, int wpt,
-                          unsigned pad_ctas, int row_round) {
+                          float* __restrict__ gw_row, float* __restrict__ acc, const RouteTables rt, int64_t Tn, int H,
+                          int K, int wpt, unsigned pad_ctas, int row_round) {
   pdl_wait();
   pdl_trigger();
   constexpr int VE = 16 / (int)sizeof(T);
@@ -178,6 +180,11 @@ gather_grad_tokens_kernel(const T* __restrict__ grad_out, int slots, const T* __
           load_vec<T, VE>(grad_out + ((size_t)t * slots + s) * H + (size_t)i * VE, g2);
 #pragma unroll
           for (int j = 0; j < VE; ++j) g[j] += g2[j];
+        }
+        if (k0 == 0) {
+#pragma unroll
+          for (int j = 0; j < VE; j += 4)
+            *reinterpret_cast<float4*>(acc + (size_t)t * H + (size_t)i * VE + j) = make_float4(0.f, 0.f, 0.f, 0.f);
         }
         uint4 q;
         store_vec<T, VE>(reinterpret_cast<T*>(&q), g);
@@ -216,15 +223,15 @@ gather_grad_tokens_kernel(const T* __restrict__ grad_out, int slots, const T* __
 
 template <typename T, class Dst>
 inline cudaError_t launch_gather_grad_tokens(const T* grad_out, int slots, const T* down_bias, const Dst& dst, float* gw_row,
-                                             const RouteTables& rt, int64_t Tn, int H, int E, int K, int row_round,
-                                             cudaStream_t st) {
+                                             float* acc, const RouteTables& rt, int64_t Tn, int H, int E, int K,
+                                             int row_round, cudaStream_t st) {
   // at least 32 warps per SM, while each has a piece of the row
   int wpt = 1;
   while (wpt < kRowWarps && Tn * wpt < 148 * 32 && H * (int)sizeof(T) / 16 > 32 * wpt) wpt *= 2;
   const int64_t token_ctas = ceil_div(Tn * wpt, kRowWarps), pad_ctas = (int64_t)E * kPadCtas;
   auto kern = K <= 4 ? gather_grad_tokens_kernel<T, Dst, 4> : gather_grad_tokens_kernel<T, Dst, 8>;
   return launch_pdl_opt(true, kern, dim3((unsigned)(pad_ctas + token_ctas)), dim3(kRowWarps * 32), 0, st, grad_out, slots,
-                        down_bias, dst, gw_row, rt, Tn, H, K, wpt, (unsigned)pad_ctas, row_round);
+                        down_bias, dst, gw_row, acc, rt, Tn, H, K, wpt, (unsigned)pad_ctas, row_round);
 }
 
 // out[i] = (T) acc[i]
@@ -295,19 +302,59 @@ colsum_kernel(const T* __restrict__ src, const float* __restrict__ row_weight,
   }
 }
 
-// d_routing[t, e] (dense) or d_routing[t, slot] = gw_row[row] for every kept row.
-// reference: csrc/experts_backward.cu:266-274 (placement), with the sort permutation applied once.
+// The last step of a backward pass.  CTAs below cast_ctas: d_hidden = (T) acc (acc null: it is d_hidden itself).  The others:
+// d_routing[t, e] (dense) or d_routing[t, slot] = gw_row of the assignment's row, 0 where there is none, a warp per token
+// (reference: csrc/experts_backward.cu:266-274, with the sort permutation applied once).  In one launch and by token, so
+// that nothing has to be zeroed before: a memset, this scatter by row and the cast were three (T = 1531, E = 64: 18 us,
+// now 7).
 template <typename T>
-__global__ void routing_grad_kernel(const float* __restrict__ gw_row, const int32_t* __restrict__ row_token,
-                                    const int32_t* __restrict__ row_flat, const int32_t* __restrict__ tile_expert,
-                                    const int32_t* __restrict__ header, T* __restrict__ d_routing,
-                                    int routing_cols, int E) {
-  const int row = blockIdx.x * blockDim.x + threadIdx.x;
-  if (row >= header[kHdrRowsUsed]) return;
-  const int tok = row_token[row];
-  if (tok < 0) return;
-  const size_t idx = (routing_cols == E) ? (size_t)tok * E + tile_expert[row / kTileM] : (size_t)row_flat[row];
-  DT<T>::st(d_routing + idx, gw_row[row]);
+__global__ void __launch_bounds__(256)
+finish_grads_kernel(const float* __restrict__ acc, T* __restrict__ d_hidden, int64_t n_vec4, unsigned cast_ctas,
+                    const float* __restrict__ gw_row, const RouteTables rt, T* __restrict__ d_routing, int64_t Tn,
+                    int routing_cols, int E, int K) {
+  pdl_wait();
+  if (blockIdx.x < cast_ctas) {
+    for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n_vec4; i += (int64_t)cast_ctas * 256) {
+      const float4 q = __ldcs(reinterpret_cast<const float4*>(acc) + i);
+      const float v[4] = {q.x, q.y, q.z, q.w};
+      store_vec<T, 4>(d_hidden + i * 4, v);
+    }
+    return;
+  }
+  const int lane = threadIdx.x & 31;
+  const int64_t t = (int64_t)(blockIdx.x - cast_ctas) * 8 + (threadIdx.x >> 5);
+  if (t >= Tn) return;
+  for (int k0 = 0; k0 < K; k0 += 32) {
+    const int n = min(32, K - k0);
+    const int32_t r = lane < n ? rt.flat_row[t * K + k0 + lane] : -1;
+    const float g = r >= 0 ? gw_row[r] : 0.f;
+    if (routing_cols != E) {
+      if (lane < n) DT<T>::st(d_routing + (size_t)t * K + k0 + lane, g);
+      continue;
+    }
+    const int e = r >= 0 ? rt.tile_expert[r / kTileM] : -1;
+    for (int c = lane; c - lane < E; c += 32) {
+      float v = 0.f;
+      bool set = k0 == 0;                 // columns without an assignment are zero
+      for (int k = 0; k < n; ++k) {
+        const int ek = __shfl_sync(0xffffffffu, e, k);
+        const float gk = __shfl_sync(0xffffffffu, g, k);
+        if (ek == c) { v = gk; set = true; }
+      }
+      if (c < E && set) DT<T>::st(d_routing + (size_t)t * E + c, v);
+    }
+  }
+}
+
+// acc: null where the sums are d_hidden itself
+template <typename T>
+inline int launch_finish_grads(const float* acc, T* d_hidden, const float* gw_row, const RouteTables& rt, T* d_routing,
+                               int64_t Tn, int H, int routing_cols, int E, int K, cudaStream_t st) {
+  const int64_t nv = Tn * H / 4;
+  const unsigned cast_ctas = acc != nullptr ? (unsigned)std::min<int64_t>(ceil_div(nv, 256), 148 * 8) : 0u;
+  const cudaError_t rc = launch_pdl_opt(true, finish_grads_kernel<T>, dim3(cast_ctas + (unsigned)ceil_div(Tn, 8)), dim3(256), 0,
+                                        st, acc, d_hidden, nv, cast_ctas, gw_row, rt, d_routing, Tn, routing_cols, E, K);
+  return rc == cudaSuccess && cudaGetLastError() == cudaSuccess ? YAMOE_OK : YAMOE_ERR_CUDA;
 }
 
 // out[t, :] = sum over the kept slots k of y[flat_row[t*K + k], :]   (rows already weighted).

@@ -392,7 +392,7 @@ static int forward_train_impl(const void* hidden, const int64_t* ridx, const voi
   return launch_combine(yrows, p.rt.flat_row, reinterpret_cast<T*>(out), Tn, H, K, st);
 }
 
-// Input, weight and bias gradients in fp32 (the routing-weight gradients are left in p.gw_row); `acc` is zeroed.
+// Input, weight and bias gradients in fp32 (the routing-weight gradients are left in p.gw_row).
 static int backward_f32_split(const Plan& p, const float* grad_out, int slots, const float* hidden, const float* wgu,
                               const float* bgu, const float* wd, const float* bd, float* acc, float* d_wgu,
                               float* d_bgu, float* d_wd, float* d_bd, int64_t Tn, int H, int E, int K, bool saved,
@@ -406,7 +406,7 @@ static int backward_f32_split(const Plan& p, const float* grad_out, int slots, c
   float* pre = reinterpret_cast<float*>(p.pre);
   if (!saved && launch_gather_tokens(hidden, PlaneDst{xs, Hp, nullptr}, p.rt, Tn, H, 4, E, K, 64, st) != cudaSuccess)
     return YAMOE_ERR_CUDA;
-  if (launch_gather_grad_tokens(grad_out, slots, bd, PlaneDst{gys, H, gys32}, p.gw_row, p.rt, Tn, H, E, K, 64, st) !=
+  if (launch_gather_grad_tokens(grad_out, slots, bd, PlaneDst{gys, H, gys32}, p.gw_row, acc, p.rt, Tn, H, E, K, 64, st) !=
       cudaSuccess)
     return YAMOE_ERR_CUDA;
   const F32Glu<true> glu{bgu, Planes{}, actw, pre, p.rt.row_token, p.rt.row_weight, H};
@@ -442,8 +442,6 @@ static int backward_impl(const void* grad_out, int per_slot, const void* hidden,
   const int path = current_path();
   const size_t es = sizeof(T);
   float* acc = p.acc32 ? p.acc32 : reinterpret_cast<float*>(d_hidden);
-  YB_CUDA_OK(cudaMemsetAsync(acc, 0, (size_t)Tn * H * sizeof(float), st));
-  YB_CUDA_OK(cudaMemsetAsync(d_routing, 0, (size_t)Tn * rcols * es, st));
   if (Tn == 0) {
     YB_CUDA_OK(cudaMemsetAsync(d_wgu, 0, (size_t)E * H * 2 * H * es, st));
     YB_CUDA_OK(cudaMemsetAsync(d_bgu, 0, (size_t)E * 2 * H * es, st));
@@ -466,10 +464,8 @@ static int backward_impl(const void* grad_out, int per_slot, const void* hidden,
                               reinterpret_cast<T*>(d_wgu), reinterpret_cast<T*>(d_bgu), reinterpret_cast<T*>(d_wd),
                               reinterpret_cast<T*>(d_bd), Tn, H, E, K, saved, st);
       if (rc) return rc;
-      routing_grad_kernel<T><<<(unsigned)ceil_div(p.max_rows, 256), 256, 0, st>>>(
-          p.gw_row, p.rt.row_token, p.rt.row_flat, p.rt.tile_expert, p.rt.header, reinterpret_cast<T*>(d_routing),
-          rcols, E);
-      return cudaGetLastError() == cudaSuccess ? YAMOE_OK : YAMOE_ERR_CUDA;
+      return launch_finish_grads<T>(nullptr, reinterpret_cast<T*>(d_hidden), p.gw_row, p.rt, reinterpret_cast<T*>(d_routing),
+                                    Tn, H, rcols, E, K, st);
     }
   }
   T* xs = reinterpret_cast<T*>(p.xs);
@@ -487,7 +483,7 @@ static int backward_impl(const void* grad_out, int per_slot, const void* hidden,
       launch_gather_tokens(hidden, RowDst<T>{xs, Hp}, p.rt, Tn, H, sizeof(T), E, K, row_round, st) != cudaSuccess)
     return YAMOE_ERR_CUDA;
   if (launch_gather_grad_tokens(reinterpret_cast<const T*>(grad_out), per_slot ? K : 1, reinterpret_cast<const T*>(bd),
-                                RowDst<T>{reinterpret_cast<T*>(p.gys), H}, p.gw_row, p.rt, Tn, H, E, K, row_round,
+                                RowDst<T>{reinterpret_cast<T*>(p.gys), H}, p.gw_row, acc, p.rt, Tn, H, E, K, row_round,
                                 st) != cudaSuccess)
     return YAMOE_ERR_CUDA;
 
@@ -535,16 +531,9 @@ static int backward_impl(const void* grad_out, int per_slot, const void* hidden,
     launch_simt_gemm<T, kDgrad>(g4, sc_dh, p.max_rows, st);
     launch_simt_gemm<T, kWgrad>(g5, st_wgu, p.max_rows, st);
   }
-  // routing-weight gradients (the bias gradients came out of the weight-gradient GEMMs)
-  routing_grad_kernel<T><<<(unsigned)ceil_div(p.max_rows, 256), 256, 0, st>>>(
-      p.gw_row, p.rt.row_token, p.rt.row_flat, p.rt.tile_expert, p.rt.header, reinterpret_cast<T*>(d_routing),
-      rcols, E);
-  if (p.acc32) {
-    const int64_t nv = Tn * H / 4;
-    cast_kernel<T><<<(unsigned)std::min<int64_t>(ceil_div(nv, 256), 148 * 8), 256, 0, st>>>(
-        p.acc32, reinterpret_cast<T*>(d_hidden), nv);
-  }
-  return cudaGetLastError() == cudaSuccess ? YAMOE_OK : YAMOE_ERR_CUDA;
+  // routing-weight gradients and the cast (the bias gradients came out of the weight-gradient GEMMs)
+  return launch_finish_grads<T>(p.acc32, reinterpret_cast<T*>(d_hidden), p.gw_row, p.rt, reinterpret_cast<T*>(d_routing), Tn,
+                                H, rcols, E, K, st);
 }
 
 // Uniform layout for the batched-matmul sub-operator: expert e owns rows [e*C, (e+1)*C).
