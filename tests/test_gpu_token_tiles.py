@@ -198,3 +198,17 @@ def test_fp32_parts_of_special_values(value):
     for a, b in zip(res["auto"], res["simt"]):
         assert torch.equal(a.isnan(), b.isnan())
         assert torch.equal(a.isinf() & (a > 0), b.isinf() & (b > 0)) and torch.equal(a.isinf(), b.isinf())
+
+
+@pytest.mark.parametrize("counts", [[79, 80, 81, 0, 95, 97], [112, 113, 127, 129, 144], [145, 159, 160, 161], [320, 321, 1, 480],
+                                    [1] * 400 + [0] * 500 + [161, 33]], ids=["80", "128", "160", "320", "many experts"])
+def test_fp32_tile_sizes(counts):
+    """Rows around the tile sizes that the fp32 kernel chooses from, and more experts than leave room for four stages."""
+    import yamoe_b200
+    args, grad, T, E = _problem(counts, 64, torch.float32, seed=len(counts))
+    dev = [a.cuda() for a in args]
+    ref = orc.experts_forward_oracle(*args, T, E, 1)
+    orc.check_close(yamoe_b200.experts(*dev, T, E, 1).cpu(), ref, RTOL_F32, "forward")
+    ref_g = orc.experts_backward_oracle(grad, *args, T, E, 1)
+    for a, b, n in zip(yamoe_b200.experts_backward(grad.cuda(), *dev, T, E, 1), ref_g, GRADS):
+        orc.check_close(a.cpu(), b, RTOL_F32, n)

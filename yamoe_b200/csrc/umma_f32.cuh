@@ -5,7 +5,7 @@
 // every product.)  Splitting into bf16 parts for the tensor cores: G. Henry, P. T. P. Tang and A. Heinecke,
 // "Leveraging the bfloat16 artificial intelligence datatype for higher-precision computations", ARITH 2019.
 //
-//   arrangement   M operand (256), fp32, split on the way       N operand (up to 128), three bf16 planes
+//   arrangement   M operand (256), fp32, split on the way       N operand (up to 160), three bf16 planes
 //   kFwd          W[e][k][m]   weight columns                   rows of the expert, K-major
 //   kDgrad        W[e][m][k]   weight rows                      rows of the expert, K-major
 //   kWgrad        grad[r][m]   columns, k = rows                act[r][n] columns, MN-major
@@ -26,8 +26,8 @@
 // sum is 1.6e-6, the gradients of 600 tokens (H = 1024) at most 2.7e-7 against 1.1e-6; at H = 64, where the serial sum
 // is short, 2.1e-7 against 2.5e-7.
 //
-// Measured: gate_up of the README forward (T = 512, H = 2880, E = 8, K = 2) 213 us = 160 TFLOP/s of the
-// original product; the whole forward 412 us against 1797, a training step of 600 tokens 400 against 1191.
+// Measured: gate_up of the README forward (T = 512, H = 2880, E = 8, K = 2) 177 us = 192 TFLOP/s of the
+// original product; the whole forward 313 us, a training step of 600 tokens 387 (CUDA cores: 1797 and 1191).
 //
 // Infinities and NaN behave as in fp32 arithmetic: see split3_special.
 //
@@ -35,27 +35,38 @@
 // L2 has to deliver (48 KB per 64-deep block against 32 KB of weights), and a pair needs them once.
 // With one CTA per tile the README forward took 485 us and the training step 463, by pairs 422 and 405.
 //
-// A CTA has 20 warps: TMA producer, MMA issuer (of the leader only), two that only complete the
-// warpgroup, eight converters (two per TMEM lane quarter, 32 k each) and eight accumulator / epilogue
-// warps (two per lane quarter, 64 columns each).  Shared memory: three stages of weights (32 KB) and four
-// of activations (24 KB); TMEM: two accumulators of 128 columns, two A operands of 96.  Signals between
+// A CTA has 24 warps: TMA producer, MMA issuer (of the leader only), two that only complete the
+// warpgroup, eight converters (two per TMEM lane quarter, 32 k each) and twelve accumulator / epilogue
+// warps (three per lane quarter, which take 16-column chunks in turn).  Shared memory: three stages of weights (32 KB) and
+// four of activations (30 KB); TMEM, all 512 columns: two accumulators of 160, two A operands of 96.  Signals between
 // the CTAs as in umma_pair.cuh, every wait bounded as in umma_gemm.cuh.
+//
+// Tiles of up to 160 rows, of a size that the kernel picks for the launch (see `consider`): a tile's weights are converted
+// for its rows alone, and with 128 rows at most half of the experts of the README forward (128 rows each on average) took
+// two tiles: 276 tiles in four waves of 74 pairs, now 184 in three.  gate_up 216 -> 177 us, the whole forward
+// 348 -> 313, with the waits looked at side by side included: a look at a barrier that is ready takes some 120 clocks, of
+// which a k-block had three in the issuer and two in the converters.
 #pragma once
 #include "misc_kernels.cuh"
 #include "umma_pair.cuh"
 
 namespace yb {
 
-constexpr int kF32Threads = 640;
-constexpr int kF32ConvWarps = 8, kF32AccWarps = 8;
-constexpr int kF32M = 128, kF32N = 128, kF32K = 64;      // M per CTA, N per pair
+constexpr int kF32ConvWarps = 8, kF32AccWarps = 12;
+constexpr int kF32Threads = 32 * (4 + kF32ConvWarps + kF32AccWarps);
+constexpr int kF32M = 128, kF32K = 64;                   // M per CTA
+constexpr int kF32N = 160, kF32WgradN = 128;             // most N of a pair: rows of an expert, columns of the activations
 constexpr int kF32WBytes = kF32M * kF32K * 4;            // 32 KB: fp32 tile of the M operand
-constexpr int kF32PlaneBytes = kF32N / 2 * kF32K * 2;    // 8 KB: this CTA's half of one part of the N operand
-constexpr int kF32BBytes = 3 * kF32PlaneBytes;
-constexpr int kF32WStages = 3, kF32BStages = 4;
-constexpr int kF32Smem = kF32WStages * kF32WBytes + kF32BStages * kF32BBytes + 1024;
-constexpr int kF32TmemA = 256;                           // first TMEM column of the A operands
+constexpr int kF32BBytes = 3 * (kF32N / 2) * kF32K * 2;  // 30 KB: this CTA's half of the N operand, three planes
+constexpr int kF32WStages = 3, kF32BStages = 4;          // (three of activations where the tables of many experts need room)
+constexpr int kF32TmemA = 2 * kF32N;                     // first TMEM column of the A operands
 constexpr int kF32TmemAStride = 96;                      // 3 parts x 32 columns (64 bf16)
+// Registers of a thread: all warps start with a 768th of the SM's file; issuers give up some, accumulators get them.
+constexpr int kF32RegsIssue = 48, kF32RegsConv = 72, kF32RegsAcc = 96;
+static_assert(128 * (kF32RegsIssue + 2 * kF32RegsConv + 3 * kF32RegsAcc) <= kF32Threads * 80, "more than the launch brings");
+inline int f32_smem(int E, int b_stages) {
+  return kF32WStages * kF32WBytes + b_stages * kF32BBytes + 1024 + (3 * E + 2) * 4;
+}
 
 // The three parts of a number: a = bf16(x), b = bf16(x - a), c = x - a - b, each rounded to nearest (halves away from
 // zero).  They sum to x exactly for |x| >= 2^-110 (below that c falls short of the last bits), with |b| <= 2^-8
@@ -423,10 +434,10 @@ struct F32StoreBias {               // see PairStoreBias
 struct F32Params {
   int M, N, K, E;
   int row_round;                   // see PairParams
-  const int32_t* tile_expert;
   const int32_t* pad_off;
   const int32_t* counts;
   int32_t* header;
+  int b_stages;
 };
 
 // tcgen05.mma with the A operand in TMEM (each CTA of the pair holds its own 128 rows)
@@ -455,12 +466,17 @@ __device__ __forceinline__ void tc_ld_32x16(uint32_t taddr, uint32_t (&r)[16]) {
         "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
       : "r"(taddr) : "memory");
 }
+// whether an mbarrier phase is over, for a first look at several: each look takes some 100 clocks, side by side once
+__device__ __forceinline__ bool mbar_ready(uint32_t bar, uint32_t parity) { return mbar_try_wait(bar, parity) != 0; }
+template <int N> __device__ __forceinline__ void more_registers() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N> __device__ __forceinline__ void fewer_registers() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 __device__ __forceinline__ void tc_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 template <int MODE, class Epi>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kF32Threads, 1)
 umma_f32_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__ CUtensorMap tmN,
-                const __grid_constant__ CUtensorMap tmNsmall, const F32Params p, const Epi epi) {
+                const __grid_constant__ CUtensorMap tmN64, const __grid_constant__ CUtensorMap tmN32, const F32Params p,
+                const Epi epi) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t bar_w_full[kF32WStages], bar_w_empty[kF32WStages];
   __shared__ __align__(8) uint64_t bar_b_full[kF32BStages], bar_b_empty[kF32BStages];
@@ -468,14 +484,15 @@ umma_f32_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__
   __shared__ __align__(8) uint64_t bar_acc_full[2], bar_acc_empty[2];
   __shared__ uint32_t tmem_base_slot;
   __shared__ int abort_flag;
-  __shared__ int32_t s_pad[kUmmaMaxExperts + 1];
-  __shared__ int32_t s_rows[kUmmaMaxExperts];
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
   const bool leader = rank == 0;
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t smem_b = smem_base + kF32WStages * kF32WBytes;
+  int32_t* s_pad = reinterpret_cast<int32_t*>(smem_raw + kF32WStages * kF32WBytes + p.b_stages * kF32BBytes + 1024);
+  int32_t* s_first = s_pad + p.E + 1;  // [E + 1] row-tiled: first tile of each expert; s_pad [E + 1]: first padded row
+  int32_t* s_rows = s_first + p.E + 1; // [E] rows to cover
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kF32WStages; ++s) {
@@ -517,32 +534,66 @@ umma_f32_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__
   const uint32_t tmem_base = tmem_base_slot;
 
   const int MT = (p.M + 2 * kF32M - 1) / (2 * kF32M);
-  const int NT = (p.N + kF32N - 1) / kF32N;       // kWgrad
-  const int total = MODE == kWgrad ? p.E * MT * NT : p.header[kHdrRowTiles] * MT;
   const int cluster_id = blockIdx.x >> 1, n_clusters = gridDim.x >> 1;
-  auto expert_of = [&](int id) -> int {
-    if constexpr (MODE == kWgrad) return 0;
-    return id < total ? __ldg(p.tile_expert + id / MT) : 0;
-  };
-  // as in umma_pair.cuh, with tiles of up to 128 rows / columns
-  auto decode = [&](int id, int e_hint, int& e, int& m0, int& n0, int& width, int& kblocks) {
+  if (MODE != kWgrad && warp == 4) {
+    // Most rows of a tile: the candidate with the smallest product of waves and clocks of its widest k-block, 12 per row
+    // on the tensor core (24 instructions) but no less than kConvClocks for the weights' conversion.
+    constexpr int kConvClocks = 1200;
+    int best = 0x7fffffff, tile = kF32N;
+    auto consider = [&](auto cap) {
+      constexpr int C = decltype(cap)::value;
+      int n = 0, widest = 0;
+      for (int e = lane; e < p.E; e += 32) {
+        const int rows = s_rows[e], cnt = (rows + C - 1) / C;
+        n += cnt;
+        if (cnt > 0) widest = max(widest, cnt == 1 ? rows : (rows / cnt + 16) & ~15);
+      }
+      n = __reduce_add_sync(0xffffffffu, n);
+      widest = __reduce_max_sync(0xffffffffu, widest);
+      const int cost = (n * MT + n_clusters - 1) / n_clusters * max(12 * widest, kConvClocks);
+      if (cost < best) { best = cost; tile = C; }
+    };
+    consider(std::integral_constant<int, 160>{});
+    consider(std::integral_constant<int, 144>{});
+    consider(std::integral_constant<int, 128>{});
+    consider(std::integral_constant<int, 112>{});
+    consider(std::integral_constant<int, 96>{});
+    consider(std::integral_constant<int, 80>{});
+    int before = 0;
+    for (int e0 = 0; e0 < p.E; e0 += 32) {
+      const int n = e0 + lane < p.E ? (s_rows[e0 + lane] + tile - 1) / tile : 0;
+      int inc = n;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += v;
+      }
+      if (e0 + lane < p.E) s_first[e0 + lane] = before + inc - n;
+      before += __shfl_sync(0xffffffffu, inc, 31);
+    }
+    if (lane == 0) s_first[p.E] = before;
+  }
+  __syncthreads();
+  const int NT = (p.N + kF32WgradN - 1) / kF32WgradN;       // kWgrad
+  const int total = (MODE == kWgrad ? p.E * NT : s_first[p.E]) * MT;
+  // as in umma_pair.cuh; e: expert of an earlier item of the same role, moved on
+  auto decode = [&](int id, int& e, int& m0, int& n0, int& width, int& kblocks) {
     if constexpr (MODE == kWgrad) {
       e = id / (MT * NT);
       const int rem = id - e * (MT * NT);
       const int nt = rem / MT;
       m0 = (rem - nt * MT) * 2 * kF32M + (int)rank * kF32M;
-      n0 = nt * kF32N;
+      n0 = nt * kF32WgradN;
       const int left = p.N - n0;
-      width = left > 64 ? kF32N : (left + 15) & ~15;        // a 64-column box per CTA, or both halves in one box
+      width = left > 64 ? kF32WgradN : (left + 15) & ~15;   // a 64-column box per CTA, or both halves in one box
       kblocks = s_rows[e] / kF32K;
     } else {
-      e = e_hint;
-      const int first = s_pad[e] / kTileM;
-      const int cnt = s_pad[e + 1] / kTileM - first;
-      const int local = id - first * MT;
-      const int mt = local / cnt;
+      while (s_first[e + 1] * MT <= id) ++e;
+      const int cnt = s_first[e + 1] - s_first[e];
+      const int local = id - s_first[e] * MT;
+      const int mt = cnt == 1 ? local : local / cnt;
       const int rows = s_rows[e];
-      const int step = ((rows + cnt - 1) / cnt + 15) & ~15;
+      const int step = cnt == 1 ? rows : ((rows + cnt - 1) / cnt + 15) & ~15;
       const int off = (local - mt * cnt) * step;
       m0 = mt * 2 * kF32M + (int)rank * kF32M;
       n0 = s_pad[e] + off;
@@ -556,6 +607,7 @@ umma_f32_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__
   };
 
   if (warp < 4) {
+  fewer_registers<kF32RegsIssue>();
   if (warp == 0) {
     // =========================== TMA producer ================================================
     if (lane == 0) {
@@ -567,7 +619,7 @@ umma_f32_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__
       int w_e = 0, w_m0 = 0, w_n0 = 0, w_width = 0, w_kblocks = 0;
       auto w_open = [&]() {                         // next work item that has k-blocks
         while (w_id < total) {
-          decode(w_id, expert_of(w_id), w_e, w_m0, w_n0, w_width, w_kblocks);
+          decode(w_id, w_e, w_m0, w_n0, w_width, w_kblocks);
           if (w_kblocks > 0) return;
           w_id += n_clusters;
         }
@@ -597,13 +649,14 @@ umma_f32_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__
       };
       w_open();
       ok = w_issue();
+      int e = 0;
       for (int id = cluster_id; id < total && ok; id += n_clusters) {
-        int e, m0, n0, width, kblocks;
-        decode(id, expert_of(id), e, m0, n0, width, kblocks);
+        int m0, n0, width, kblocks;
+        decode(id, e, m0, n0, width, kblocks);
         const int half = width >> 1;
-        // this CTA's rows (columns) of the N operand: one box of 64, or of 32
-        const bool big = MODE == kWgrad || half > 32;
-        const uint32_t bytes = big ? kF32BBytes : kF32BBytes / 2;
+        // this CTA's rows (columns) of the N operand: one box of 80, 64 or 32
+        const int box = MODE == kWgrad ? 64 : half > 64 ? 80 : half > 32 ? 64 : 32;
+        const uint32_t bytes = (uint32_t)box * (3 * kF32K * 2);
         const int my_n = n0 + (int)rank * half;
         for (int kb = 0; kb < kblocks; ++kb) {
           ok = w_issue() && mbar_wait(smem_u32(&bar_b_empty[bs]), bph ^ 1u, &abort_flag);
@@ -612,14 +665,14 @@ umma_f32_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__
           const uint32_t sb = smem_b + bs * kF32BBytes;
           mbar_expect_tx_cluster(full, bytes);
           if constexpr (MODE == kWgrad) tma2_load_4d(sb, &tmN, my_n & 63, s_pad[e] + kb * kF32K, my_n >> 6, 0, full);
-          else tma2_load_3d(sb, big ? &tmN : &tmNsmall, kb * kF32K, my_n, 0, full);
-          if (++bs == kF32BStages) { bs = 0; bph ^= 1u; }
+          else tma2_load_3d(sb, box == 80 ? &tmN : box == 64 ? &tmN64 : &tmN32, kb * kF32K, my_n, 0, full);
+          if (++bs == p.b_stages) { bs = 0; bph ^= 1u; }
         }
       }
       // the commits that free the last stages must have arrived here before this CTA ends
-      for (int g = 0; g < kF32BStages && ok; ++g) {
+      for (int g = 0; g < p.b_stages && ok; ++g) {
         ok = mbar_wait(smem_u32(&bar_b_empty[bs]), bph ^ 1u, &abort_flag);
-        if (++bs == kF32BStages) { bs = 0; bph ^= 1u; }
+        if (++bs == p.b_stages) { bs = 0; bph ^= 1u; }
       }
       if (!ok) give_up(kStatusProducerTimeout);
     }
@@ -638,17 +691,18 @@ umma_f32_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__
       int slot = 0, bs = 0;                          // A operand and accumulator: two of each; B stage
       uint32_t phase = 0, bph = 0;
       bool ok = true;
-      int e_next = expert_of(cluster_id);
+      int e = 0;
       for (int id = cluster_id; id < total && ok; id += n_clusters) {
-        int e, m0, n0, width, kblocks;
-        decode(id, e_next, e, m0, n0, width, kblocks);
-        e_next = expert_of(id + n_clusters);
+        int m0, n0, width, kblocks;
+        decode(id, e, m0, n0, width, kblocks);
         const uint32_t idesc = idesc_base | ((uint32_t)(width >> 3) << 17);
-        const uint32_t plane = (MODE == kWgrad || width > 64 ? kF32PlaneBytes : kF32PlaneBytes / 2) >> 4;
+        const uint32_t plane = (uint32_t)((MODE == kWgrad ? 64 : width > 128 ? 80 : width > 64 ? 64 : 32) * kF32K * 2) >> 4;
         for (int kb = 0; kb < kblocks; ++kb) {
-          ok = mbar_wait(smem_u32(&bar_acc_empty[slot]), phase ^ 1u, &abort_flag) &&
-               mbar_wait(smem_u32(&bar_b_full[bs]), bph, &abort_flag) &&
-               mbar_wait(smem_u32(&bar_a_full[slot]), phase, &abort_flag);
+          const bool r0 = mbar_ready(smem_u32(&bar_acc_empty[slot]), phase ^ 1u), r1 = mbar_ready(smem_u32(&bar_b_full[bs]), bph),
+                     r2 = mbar_ready(smem_u32(&bar_a_full[slot]), phase);
+          ok = (r0 || mbar_wait(smem_u32(&bar_acc_empty[slot]), phase ^ 1u, &abort_flag)) &&
+               (r1 || mbar_wait(smem_u32(&bar_b_full[bs]), bph, &abort_flag)) &&
+               (r2 || mbar_wait(smem_u32(&bar_a_full[slot]), phase, &abort_flag));
           ok = __all_sync(0xffffffffu, ok);
           if (!ok) break;
           tc_fence_after();
@@ -669,7 +723,7 @@ umma_f32_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__
           __syncwarp();
           slot ^= 1;
           if (slot == 0) phase ^= 1u;
-          if (++bs == kF32BStages) { bs = 0; bph ^= 1u; }
+          if (++bs == p.b_stages) { bs = 0; bph ^= 1u; }
         }
       }
       if (!ok && lane == 0) give_up(kStatusMmaTimeout);
@@ -678,21 +732,23 @@ umma_f32_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__
   }
   } else if (warp < 4 + kF32ConvWarps) {
     // =========================== converters: fp32 tile -> three parts in TMEM ================
+    fewer_registers<kF32RegsConv>();
     const int q = warp & 3, khalf = (warp - 4) >> 2;
     const int mrow = q * 32 + lane;
     int ws = 0, slot = 0;
     uint32_t wph = 0, phase = 0;
     bool ok = true;
-    int e_next = expert_of(cluster_id);
+    int e = 0;
     for (int id = cluster_id; id < total && ok; id += n_clusters) {
-      int e, m0, n0, width, kblocks;
-      decode(id, e_next, e, m0, n0, width, kblocks);
-      e_next = expert_of(id + n_clusters);
+      int m0, n0, width, kblocks;
+      decode(id, e, m0, n0, width, kblocks);
       for (int kb = 0; kb < kblocks; ++kb) {
-        ok = mbar_wait_warp(smem_u32(&bar_w_full[ws]), wph, &abort_flag);
-        if (!ok) break;
-        ok = mbar_wait_warp(smem_u32(&bar_a_empty[slot]), phase ^ 1u, &abort_flag);
-        if (!ok) break;
+        const bool r0 = mbar_ready(smem_u32(&bar_w_full[ws]), wph), r1 = mbar_ready(smem_u32(&bar_a_empty[slot]), phase ^ 1u);
+        if (!__all_sync(0xffffffffu, r0 && r1)) {
+          ok = mbar_wait_warp(smem_u32(&bar_w_full[ws]), wph, &abort_flag) &&
+               mbar_wait_warp(smem_u32(&bar_a_empty[slot]), phase ^ 1u, &abort_flag);
+          if (!ok) break;
+        }
         tc_fence_after();
         const uint8_t* tile = smem_raw + (smem_base - smem_u32(smem_raw)) + ws * kF32WBytes;
         const uint32_t t = tmem_base + kF32TmemA + slot * kF32TmemAStride + khalf * 16 + ((uint32_t)(q * 32) << 16);
@@ -759,16 +815,15 @@ umma_f32_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__
     __syncwarp();
   } else {
     // =========================== accumulators and epilogue ===================================
-    const int q = warp & 3, nhalf = (warp - 4 - kF32ConvWarps) >> 2;
+    more_registers<kF32RegsAcc>();
+    const int q = warp & 3, third = (warp - 4 - kF32ConvWarps) >> 2;   // takes the 16-column chunks third, third + 3, ...
     int slot = 0;
     uint32_t phase = 0;
     bool ok = true;
-    int e_next = expert_of(cluster_id);
+    int e = 0;
     for (int id = cluster_id; id < total && ok; id += n_clusters) {
-      int e, m0, n0, width, kblocks;
-      decode(id, e_next, e, m0, n0, width, kblocks);
-      e_next = expert_of(id + n_clusters);
-      const int cols = min(64, width - nhalf * 64);  // of this warp; <= 0: none
+      int m0, n0, width, kblocks;
+      decode(id, e, m0, n0, width, kblocks);
       float acc[64];
 #pragma unroll
       for (int i = 0; i < 64; ++i) acc[i] = 0.f;
@@ -776,12 +831,12 @@ umma_f32_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__
         ok = mbar_wait_warp(smem_u32(&bar_acc_full[slot]), phase, &abort_flag);
         if (!ok) break;
         tc_fence_after();
-        const uint32_t t = tmem_base + slot * kF32N + nhalf * 64 + ((uint32_t)(q * 32) << 16);
+        const uint32_t t = tmem_base + slot * kF32N + third * 16 + ((uint32_t)(q * 32) << 16);
 #pragma unroll
         for (int c = 0; c < 4; ++c)
-          if (c * 16 < cols) {
+          if ((third + 3 * c) * 16 < width) {
             uint32_t r[16];
-            tc_ld_32x16(t + c * 16, r);
+            tc_ld_32x16(t + c * 48, r);
 #pragma unroll
             for (int i = 0; i < 16; ++i) acc[c * 16 + i] += __uint_as_float(r[i]);
           }
@@ -796,11 +851,11 @@ umma_f32_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__
       if (m - lane < p.M) {                          // M is a multiple of 32
 #pragma unroll
         for (int c = 0; c < 4; ++c)
-          if (c * 16 < cols) {
+          if (const int n = (third + 3 * c) * 16; n < width) {
             float v[16];
 #pragma unroll
             for (int i = 0; i < 16; ++i) v[i] = acc[c * 16 + i];
-            epi.apply(e, m, n0 + nhalf * 64 + c * 16, min(16, cols - c * 16), lane, v);
+            epi.apply(e, m, n0 + n, min(16, width - n), lane, v);
           }
       }
     }
@@ -824,28 +879,31 @@ umma_f32_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__
   }
 }
 
+// Most tiles of at least 80 rows (the smallest candidate) that the padded rows make.
+inline int64_t f32_max_tiles(int64_t max_rows, int E) { return max_rows / 80 + E; }
+
 // GemmArgs as for launch_umma_pair: A / lda describe the planes (N operand; `a_plane` elements
 // between planes), B / ldb the fp32 operand.  All widths and pitches are multiples of 64.
 template <int MODE, class Epi>
-inline int launch_umma_f32(const GemmArgs& g, int64_t a_plane, const Epi& epi, int64_t max_rows, int64_t max_tiles,
-                           int row_round, cudaStream_t stream) {
+inline int launch_umma_f32(const GemmArgs& g, int64_t a_plane, const Epi& epi, int64_t max_rows, int row_round,
+                           cudaStream_t stream) {
   if (!umma_available() || g.E > kUmmaMaxExperts) return YAMOE_ERR_UNSUPPORTED;
-  CUtensorMap tmM, tmN, tmNs;
+  CUtensorMap tmM, tmN, tmN64, tmN32;
   bool ok = true;
   if (MODE == kWgrad) {
     const uint64_t dn[4] = {64, (uint64_t)max_rows, (uint64_t)g.lda / 64, 3};
     const uint64_t sn[3] = {(uint64_t)g.lda * 2, 128, (uint64_t)a_plane * 2};
     const uint32_t b1[4] = {64, 64, 1, 3};
     ok = make_map(&tmN, g.A, 4, dn, sn, b1);
-    tmNs = tmN;                          // not used
+    tmN64 = tmN32 = tmN;                 // not used
     const uint64_t dm[2] = {(uint64_t)g.N, (uint64_t)max_rows}, sm[1] = {(uint64_t)g.ldb * 4};
     const uint32_t bm[2] = {kF32M, kF32K};
     ok = ok && make_map(&tmM, g.B, 2, dm, sm, bm, kMapF32);
   } else {
     const uint64_t dn[3] = {(uint64_t)g.K, (uint64_t)max_rows, 3};
     const uint64_t sn[2] = {(uint64_t)g.lda * 2, (uint64_t)a_plane * 2};
-    const uint32_t b64[3] = {64, 64, 3}, b32[3] = {64, 32, 3};
-    ok = make_map(&tmN, g.A, 3, dn, sn, b64) && make_map(&tmNs, g.A, 3, dn, sn, b32);
+    const uint32_t b80[3] = {64, 80, 3}, b64[3] = {64, 64, 3}, b32[3] = {64, 32, 3};
+    ok = make_map(&tmN, g.A, 3, dn, sn, b80) && make_map(&tmN64, g.A, 3, dn, sn, b64) && make_map(&tmN32, g.A, 3, dn, sn, b32);
     const uint64_t sm[2] = {(uint64_t)g.ldb * 4, (uint64_t)g.b_expert_stride * 4};
     if (MODE == kFwd) {
       const uint64_t dm[3] = {(uint64_t)g.N, (uint64_t)g.K, (uint64_t)g.E};
@@ -860,14 +918,15 @@ inline int launch_umma_f32(const GemmArgs& g, int64_t a_plane, const Epi& epi, i
   if (!ok) return YAMOE_ERR_CUDA;
   auto kern = umma_f32_kernel<MODE, Epi>;
   static PerDevice<int> resident;    // per template instantiation and device
-  const int pairs = resident_pairs(kern, kF32Threads, kF32Smem, resident);
+  const int pairs = resident_pairs(kern, kF32Threads, kMaxDynamicSmem, resident);
   if (pairs <= 0) return YAMOE_ERR_CUDA;
-  const F32Params p{g.N, g.M, g.K, g.E, row_round, g.tile_expert, g.pad_off, g.counts, const_cast<int32_t*>(g.header)};
+  const int b_stages = f32_smem(g.E, kF32BStages) <= kMaxDynamicSmem ? kF32BStages : kF32BStages - 1;
+  const F32Params p{g.N, g.M, g.K, g.E, row_round, g.pad_off, g.counts, const_cast<int32_t*>(g.header), b_stages};
   const int64_t MT = ceil_div(g.N, 2 * kF32M);
-  const int64_t total_max = MODE == kWgrad ? (int64_t)g.E * MT * ceil_div(g.M, kF32N) : max_tiles * MT;
+  const int64_t total_max = MODE == kWgrad ? (int64_t)g.E * MT * ceil_div(g.M, kF32WgradN) : f32_max_tiles(max_rows, g.E) * MT;
   const int grid = (int)(2 * std::min<int64_t>(total_max, pairs));
   if (grid <= 0) return YAMOE_OK;
-  if (launch_pdl_opt(true, kern, dim3(grid), dim3(kF32Threads), kF32Smem, stream, tmM, tmN, tmNs, p, epi) != cudaSuccess)
+  if (launch_pdl_opt(true, kern, dim3(grid), dim3(kF32Threads), f32_smem(g.E, b_stages), stream, tmM, tmN, tmN64, tmN32, p, epi) != cudaSuccess)
     return YAMOE_ERR_CUDA;
   return cudaGetLastError() == cudaSuccess ? YAMOE_OK : YAMOE_ERR_CUDA;
 }

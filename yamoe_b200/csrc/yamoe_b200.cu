@@ -219,14 +219,13 @@ static int forward_f32_split(const Plan& p, const float* hidden, const float* wg
     StageTimer tm(kStageGateUp, st);
     const F32Glu<false> glu{bgu, act, Planes{}, nullptr, p.rt.row_token, nullptr, H};
     rc = launch_umma_f32<kFwd>(pair_args(p, xs.p, H, wgu, 2 * (int64_t)H, (int64_t)H * 2 * H, 0, 2 * H, H, E), xs.stride,
-                               glu, p.max_rows, p.max_tiles, 16, st);
+                               glu, p.max_rows, 16, st);
   }
   if (rc) return rc;
   {
     StageTimer tm(kStageDown, st);
     const F32WeightedRows wrows{bd, reinterpret_cast<float*>(p.yrows), p.rt.row_token, p.rt.row_weight, H};
-    rc = launch_umma_f32<kFwd>(pair_args(p, act.p, H, wd, H, (int64_t)H * H, 0, H, H, E), act.stride, wrows, p.max_rows,
-                               p.max_tiles, 16, st);
+    rc = launch_umma_f32<kFwd>(pair_args(p, act.p, H, wd, H, (int64_t)H * H, 0, H, H, E), act.stride, wrows, p.max_rows, 16, st);
   }
   if (rc) return rc;
   StageTimer tm(kStageCombine, st);
@@ -348,10 +347,10 @@ static int forward_train_impl(const void* hidden, const int64_t* ridx, const voi
       T* yrows = reinterpret_cast<T*>(p.gys);
       const F32WeightedRows wrows{reinterpret_cast<const T*>(bd), yrows, p.rt.row_token, p.rt.row_weight, H};
       if ((rc = launch_umma_f32<kFwd>(pair_args(p, xs.p, Hp, wgu, 2 * (int64_t)H, (int64_t)H * 2 * H, 0, 2 * H, H, E),
-                                      xs.stride, glu, p.max_rows, p.max_tiles, 64, st)))
+                                      xs.stride, glu, p.max_rows, 64, st)))
         return rc;
       if ((rc = launch_umma_f32<kFwd>(pair_args(p, act.p, H, wd, H, (int64_t)H * H, 0, H, H, E), act.stride, wrows,
-                                      p.max_rows, p.max_tiles, 16, st)))
+                                      p.max_rows, 16, st)))
         return rc;
       return launch_combine(yrows, p.rt.flat_row, reinterpret_cast<T*>(out), Tn, H, K, st);
     }
@@ -415,19 +414,15 @@ static int backward_f32_split(const Plan& p, const float* grad_out, int slots, c
   const F32ScatterAdd sc{acc, p.rt.row_token, H};
   int rc;
   if (!saved && (rc = launch_umma_f32<kFwd>(pair_args(p, xs.p, Hp, wgu, H2, 2 * HH, 0, H2, H, E), xs.stride, glu,
-                                            p.max_rows, p.max_tiles, 64, st)))
+                                            p.max_rows, 64, st)))
     return rc;
-  if ((rc = launch_umma_f32<kDgrad>(pair_args(p, gys.p, H, wd, H, HH, 0, H, H, E), gys.stride, glub, p.max_rows,
-                                    p.max_tiles, 64, st)))
+  if ((rc = launch_umma_f32<kDgrad>(pair_args(p, gys.p, H, wd, H, HH, 0, H, H, E), gys.stride, glub, p.max_rows, 64, st)))
     return rc;
-  if ((rc = launch_umma_f32<kWgrad>(pair_args(p, actw.p, Hp, gys32, H, 0, H + 1, H, 0, E), actw.stride, st_wd, p.max_rows,
-                                    p.max_tiles, 64, st)))
+  if ((rc = launch_umma_f32<kWgrad>(pair_args(p, actw.p, Hp, gys32, H, 0, H + 1, H, 0, E), actw.stride, st_wd, p.max_rows, 64, st)))
     return rc;
-  if ((rc = launch_umma_f32<kDgrad>(pair_args(p, gpre.p, H2, wgu, H2, 2 * HH, 0, H, H2, E), gpre.stride, sc, p.max_rows,
-                                    p.max_tiles, 16, st)))
+  if ((rc = launch_umma_f32<kDgrad>(pair_args(p, gpre.p, H2, wgu, H2, 2 * HH, 0, H, H2, E), gpre.stride, sc, p.max_rows, 16, st)))
     return rc;
-  return launch_umma_f32<kWgrad>(pair_args(p, xs.p, Hp, gpre32, H2, 0, H + 1, H2, 0, E), xs.stride, st_wgu, p.max_rows,
-                                 p.max_tiles, 64, st);
+  return launch_umma_f32<kWgrad>(pair_args(p, xs.p, Hp, gpre32, H2, 0, H + 1, H2, 0, E), xs.stride, st_wgu, p.max_rows, 64, st);
 }
 
 template <typename T>
