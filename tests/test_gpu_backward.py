@@ -112,11 +112,12 @@ def test_saved_activation_pair_matches_recompute(dtype):
                             rel_l2=None if dtype == torch.float32 else 2e-2)
 
 
-@pytest.mark.parametrize("H,E", [(64, 3), (128, 5), (256, 4), (320, 6), (64, 150), (128, 300)])
-def test_weight_gradients_of_few_rows(H, E):
+@pytest.mark.parametrize("T,H,E", [(130, 64, 3), (130, 128, 5), (130, 256, 4), (130, 320, 6), (130, 64, 150), (130, 128, 300),
+                                   (600, 192, 2), (1100, 320, 3)])
+def test_weight_gradients_of_few_rows(T, H, E):
     """Output rows and columns at the edges of the parked boxes, the bias row in a box of its own or behind others, experts
-    without rows, and more experts than leave space for two parking buffers."""
-    T, K = 130, 2
+    without rows, more experts than leave space to park for four groups of warps, and enough rows for two groups."""
+    K = 2
     inp = orc.make_inputs(T, H, E, K, seed=H + E, weight_std=H ** -0.5, bias_std=0.2, dtype=torch.bfloat16, with_grad=True)
     args = [inp[k] for k in ("hidden_states", "router_indices", "routing_weights", "gate_up_proj", "gate_up_proj_bias",
                              "down_proj", "down_proj_bias")]

@@ -42,8 +42,6 @@
 
 namespace yb {
 
-constexpr int kPairThreads = 352;
-constexpr int kPairEpiWarps = 8;
 constexpr int kPairM = 256, kPairN = 256;
 constexpr int kPairABytes = 128 * 128;     // this CTA's 128 M rows x 64 bf16
 constexpr int kPairBBytes = 128 * 128;     // this CTA's half of the N rows (up to 128) x 64 bf16
@@ -107,7 +105,7 @@ struct PairParams {
   const int32_t* pad_off;
   const int32_t* counts;
   int32_t* header;
-  int bufs;                     // parking buffers of a group (kTmaStore)
+  int groups;                   // of four epilogue warps, which take the chunks of a tile in turn
 };
 
 // ---------------------------------------------------------------------------------------------
@@ -376,11 +374,13 @@ __device__ __forceinline__ void stmatrix_x4_trans(uint32_t addr, uint32_t r0, ui
 // as one k-block), so the tile leaves by TMA: four warps park 32 rows of 128 columns in shared memory (two boxes of 64
 // columns, swizzled so that the eight rows of a matrix fall on different banks), and copies clipped at the matrix edge
 // store them while the warps go on.  The transposition is stmatrix's: with shuffles and 4-byte stores the epilogue of a
-// tile took longer still.  192 rows per expert (E = 64, H = 2048): gate_up 395 -> 350 us, down 205 -> 185 (1.07 and 0.54 GB of
-// output, 145 and 73 us at the rate of a fill; without the copies 250, without any epilogue 169).  Meeting once for two
-// chunks in a single buffer of twice the size: 363.
+// tile took longer still.  192 rows per expert (E = 64, H = 2048): gate_up 395 us with shuffles, 360 by stmatrix, 306 with
+// sixteen epilogue warps instead of eight; down 205, 190, 160 (1.07 and 0.54 GB of output, 145 and 73 us at the rate of a
+// fill).  Eight warps with two buffers each took 350 and 185, meeting once for two chunks 363.
+template <int WARPS>
 struct PairStoreBias {
   static constexpr bool kTmaStore = true;
+  static constexpr int kWarps = WARPS;      // see pair_wgrad_warps
   __nv_bfloat16* C;                // [E, H, ld]
   __nv_bfloat16* bias_out;         // [E, ld]
   int H, ld;
@@ -415,23 +415,30 @@ struct epi_tma_store : std::false_type {};
 template <class E>
 struct epi_tma_store<E, std::enable_if_t<E::kTmaStore>> : std::true_type {};
 
-// Shared memory: ring, parking space (`bufs` buffers for either group of four warps), expert tables.  Two buffers, so that
-// a group parks a chunk while the copy of the one before is read, fit beside the tables of up to some 140 experts.
+// Shared memory: ring, parking space for each group of four epilogue warps (kTmaStore), expert tables.  Beside the tables of
+// more than some 140 experts there is space for two groups; the others then have no chunks.
 constexpr int kMaxDynamicSmem = 227 * 1024 - 256;               // the barriers are static
-inline int pair_smem(bool store, int E, int bufs) {
-  return kPairSmem + (store ? 2 * bufs * kPairParkBytes : 0) + (3 * E + 2) * 4;
+inline int pair_smem(int park_groups, int E) { return kPairSmem + park_groups * kPairParkBytes + (3 * E + 2) * 4; }
+
+// Epilogue warps.
+template <class Epi>
+constexpr int pair_epi_warps() {
+  if constexpr (epi_tma_store<Epi>::value) return Epi::kWarps;
+  else return 8;
 }
+// Of the weight gradients: sixteen while a tile's epilogue is longer than its main loop, eight above some 512 rows per
+// expert, where they only wait (8 / 16 warps: 192 rows, H = 2048 gate_up 359 / 306 us, down 190 / 160; 1024 rows, H = 2880
+// 788 / 806 and 396 / 407).
+inline bool pair_wgrad_16_warps(int64_t S, int E) { return S <= 512 * (int64_t)E; }
+template <class Epi>
+constexpr int pair_threads() { return 32 * (3 + pair_epi_warps<Epi>()); }
 
 __device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, int c0, int c1, int c2, uint32_t src) {
   asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];"
                ::"l"(map), "r"(src), "r"(c0), "r"(c1), "r"(c2) : "memory");
 }
 __device__ __forceinline__ void tma_store_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-// until the copies of all groups, or of all but the last, have read their shared memory
-__device__ __forceinline__ void tma_store_wait_read(bool all) {
-  if (all) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-  else asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-}
+__device__ __forceinline__ void tma_store_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 __device__ __forceinline__ void tma_store_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 __device__ __forceinline__ void group_sync(int id) { asm volatile("bar.sync %0, 128;" ::"r"(id) : "memory"); }
 
@@ -445,11 +452,12 @@ __device__ __forceinline__ bool group_all(int id, bool ok) {
 }
 
 template <int MODE, class Epi>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair_threads<Epi>(), 1)
 umma_pair_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__ CUtensorMap tmN,
                  const __grid_constant__ CUtensorMap tmNsmall, const __grid_constant__ CUtensorMap tmOut,
                  const PairParams p, const Epi epi) {
   constexpr bool kStore = epi_tma_store<Epi>::value;
+  constexpr int kEpiWarps = pair_epi_warps<Epi>();
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t bar_full[kPairStages];       // used in the leader CTA
   __shared__ __align__(8) uint64_t bar_empty[kPairGroups];      // per CTA
@@ -462,7 +470,7 @@ umma_pair_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant_
   const uint32_t rank = cluster_ctarank();
   const bool leader = rank == 0;
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  int32_t* s_pad = reinterpret_cast<int32_t*>(smem_raw + kPairSmem + (kStore ? 2 * p.bufs * kPairParkBytes : 0));
+  int32_t* s_pad = reinterpret_cast<int32_t*>(smem_raw + kPairSmem + (kStore ? p.groups * kPairParkBytes : 0));
   int32_t* s_pair = s_pad + p.E + 1;   // [E + 1] row-tiled: first 256-row tile of each expert; s_pad [E + 1]: first padded row
   int32_t* s_rows = s_pair + p.E + 1;  // [E] rows to cover
 
@@ -471,7 +479,7 @@ umma_pair_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant_
     for (int s = 0; s < kPairGroups; ++s) mbar_init(smem_u32(&bar_empty[s]), 1);
     for (int a = 0; a < 2; ++a) {
       mbar_init(smem_u32(&bar_tmem_full[a]), 1);
-      mbar_init(smem_u32(&bar_tmem_empty[a]), 2 * kPairEpiWarps);
+      mbar_init(smem_u32(&bar_tmem_empty[a]), 2 * kEpiWarps);
     }
     abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -488,7 +496,7 @@ umma_pair_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant_
   const uint32_t tmem_base = tmem_base_slot;
   pdl_trigger();
   pdl_wait();
-  for (int i = threadIdx.x; i <= p.E; i += kPairThreads) {
+  for (int i = threadIdx.x; i <= p.E; i += pair_threads<Epi>()) {
     const int p0 = p.pad_off[i];
     s_pad[i] = p0;
     if (MODE != kWgrad) s_pair[i] = p.pair_off[i];
@@ -536,7 +544,7 @@ umma_pair_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant_
     }
   };
 
-  if (warp == 0 || warp == 2 + kPairEpiWarps) {
+  if (warp == 0 || warp == 2 + kEpiWarps) {
     // =========================== TMA producers (both CTAs) ===================================
     // One warp for the M operand, which also announces the bytes of both, and one for the N operand: a
     // warp that issues everything is slower than the tensor core.  The whole warp walks the loop (see
@@ -659,9 +667,9 @@ umma_pair_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant_
   } else {
     // =========================== epilogue (warps 2..9 of both CTAs) ==========================
     const int q = warp & 3;                    // TMEM lane quarter this warp may read
-    const int turn = (warp - 2) >> 2;          // takes the 32-column chunks turn, turn + 2, ...
-    [[maybe_unused]] const uint32_t park0 = smem_base + kPairStages * kPairStageBytes + turn * p.bufs * kPairParkBytes;
-    [[maybe_unused]] uint32_t park = park0;
+    const int turn = (warp - 2) >> 2;          // takes the 32-column chunks turn, turn + groups, ...
+    const int groups = kStore ? p.groups : kEpiWarps / 4;
+    [[maybe_unused]] const uint32_t park = smem_base + kPairStages * kPairStageBytes + turn * kPairParkBytes;
     int acc = 0;
     uint32_t acc_phase = 0;
     int e_next = expert_of(cluster_id);
@@ -672,14 +680,14 @@ umma_pair_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant_
       const int cta_m = m0 + (int)rank * 128;
       const int m = cta_m + q * 32 + lane;
       // M is a multiple of 32.  (Stored by TMA, the four warps of a group stay together and the copy clips.)
-      const bool mine = kStore ? cta_m < p.M : m - lane < p.M;
+      const bool mine = kStore ? cta_m < p.M && turn < groups : m - lane < p.M;
       const int nchunks = (width + 31) >> 5;
       // 32 columns of the accumulator: as fp32 by M index, or (kStore) packed for stmatrix
       auto emit = [&](int c, const auto& v) {
         const int row = n0 + c * 32;
         if constexpr (kStore) {
           const bool issuer = q == 0 && lane == 0;
-          if (issuer) tma_store_wait_read(p.bufs == 1);
+          if (issuer) tma_store_wait_read();
           group_sync(1 + turn);
           epi.park(v, q, lane, park);
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the parked rows are read by the copy
@@ -689,11 +697,10 @@ umma_pair_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant_
               tma_store_3d(&tmOut, cta_m, row, e, park);
               if (cta_m + 64 < epi.ld) tma_store_3d(&tmOut, cta_m + 64, row, e, park + kPairParkBytes / 2);
             }
-            tma_store_commit();                  // also without a copy: the groups count the buffers
+            tma_store_commit();
           }
           if (row <= epi.H && epi.H < row + 32)
             epi.bias_row(e, cta_m, epi.H - row, q, lane, smem_raw + (park - smem_u32(smem_raw)));
-          if (p.bufs == 2) park = park0 + (park == park0 ? kPairParkBytes : 0);
         } else {
           epi.apply(e, m, row, min(32, width - c * 32), lane, v);
         }
@@ -702,13 +709,13 @@ umma_pair_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant_
         if constexpr (kStore) {
           const uint32_t z[16] = {};
           if (mine)
-            for (int c = turn; c < nchunks; c += 2) emit(c, z);
+            for (int c = turn; c < nchunks; c += groups) emit(c, z);
         }
         continue;
       }
       if constexpr (epi_prefetches<Epi>::value) {
         if (mine)
-          for (int c = turn; c < nchunks; c += 2) epi.prefetch(m, n0 + c * 32, min(32, width - c * 32), lane);
+          for (int c = turn; c < nchunks; c += groups) epi.prefetch(m, n0 + c * 32, min(32, width - c * 32), lane);
       }
       bool ok = mbar_wait_warp(smem_u32(&bar_tmem_full[acc]), acc_phase, &abort_flag);
       if constexpr (kStore) ok = group_all(1 + turn, ok);
@@ -721,7 +728,7 @@ umma_pair_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant_
       if (mine) {
         const uint32_t t_row = tmem_base + acc * kUmmaAccStride + ((uint32_t)(q * 32) << 16);
 #pragma unroll 1
-        for (int c = turn; c < nchunks; c += 2) {
+        for (int c = turn; c < nchunks; c += groups) {
           uint32_t r[32];
           if constexpr (kStore) {
             tc_ld_16x256_issue(t_row + c * 32, r);
@@ -824,8 +831,9 @@ inline int launch_umma_pair(const GemmArgs& g, const Epi& epi, int64_t max_rows,
     }
   }
   constexpr bool kStore = epi_tma_store<Epi>::value;
-  const int bufs = pair_smem(kStore, g.E, 2) <= kMaxDynamicSmem ? 2 : 1;
-  const int smem = pair_smem(kStore, g.E, bufs);
+  constexpr int kThreads = pair_threads<Epi>();
+  const int groups = !kStore || pair_smem(4, g.E) <= kMaxDynamicSmem ? pair_epi_warps<Epi>() / 4 : 2;
+  const int smem = pair_smem(kStore ? groups : 0, g.E);
   CUtensorMap tmOut = tmM;               // not used
   if constexpr (kStore) {
     const uint64_t d[3] = {(uint64_t)epi.ld, (uint64_t)epi.H, (uint64_t)g.E};
@@ -836,16 +844,16 @@ inline int launch_umma_pair(const GemmArgs& g, const Epi& epi, int64_t max_rows,
   if (!ok) return YAMOE_ERR_CUDA;
   auto kern = umma_pair_kernel<MODE, Epi>;
   static PerDevice<int> resident;    // per template instantiation and device
-  const int pairs = resident_pairs(kern, kPairThreads, kMaxDynamicSmem, resident);
+  const int pairs = resident_pairs(kern, kThreads, kMaxDynamicSmem, resident);
   if (pairs <= 0) return YAMOE_ERR_CUDA;
   const PairParams p{g.N, g.M, g.K, g.E, row_round, g.pair_expert, g.pair_off, g.pad_off, g.counts,
-                     const_cast<int32_t*>(g.header), bufs};
+                     const_cast<int32_t*>(g.header), groups};
   const int64_t MT = ceil_div(g.N, kPairM);
   // the tables bound the number of row tiles by max_tiles (128-row tiles)
   const int64_t total_max = MODE == kWgrad ? (int64_t)g.E * MT * ceil_div(g.M, kPairN) : max_tiles * MT;
   const int grid = (int)(2 * std::min<int64_t>(total_max, pairs));
   if (grid <= 0) return YAMOE_OK;
-  if (launch_pdl_opt(true, kern, dim3(grid), dim3(kPairThreads), smem, stream, tmM, tmN, tmNs, tmOut, p, epi) != cudaSuccess)
+  if (launch_pdl_opt(true, kern, dim3(grid), dim3(kThreads), smem, stream, tmM, tmN, tmNs, tmOut, p, epi) != cudaSuccess)
     return YAMOE_ERR_CUDA;
   return cudaGetLastError() == cudaSuccess ? YAMOE_OK : YAMOE_ERR_CUDA;
 }

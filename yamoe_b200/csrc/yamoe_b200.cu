@@ -511,13 +511,17 @@ static int backward_impl(const void* grad_out, int per_slot, const void* hidden,
     if constexpr (sizeof(T) == 2) {
       const PairGlu<true> pglu{glu.bias, nullptr, glu.actw, glu.pre, p.rt.row_token, p.rt.row_weight, H, Hp};
       const PairGluBackward pglub{glub.pre, glub.g_pre, p.gw_row, p.rt.row_token, p.rt.row_weight, H};
-      const PairStoreBias pwd{st_wd.C, st_wd.bias_out, H, H}, pwgu{st_wgu.C, st_wgu.bias_out, H, 2 * H};
+      auto wgrad = [&](const GemmArgs& g, const EpiStoreBias<T>& o, int ld) {
+        if (pair_wgrad_16_warps(p.S, E))
+          return launch_umma_pair<kWgrad>(g, PairStoreBias<16>{o.C, o.bias_out, H, ld}, p.max_rows, p.max_tiles, 64, st);
+        return launch_umma_pair<kWgrad>(g, PairStoreBias<8>{o.C, o.bias_out, H, ld}, p.max_rows, p.max_tiles, 64, st);
+      };
       const PairScatterAdd pdh{acc, p.rt.row_token, H};
       if (!saved && (rc = launch_umma_pair<kFwd>(g1, pglu, p.max_rows, p.max_tiles, 64, st))) return rc;
       if ((rc = launch_umma_pair<kDgrad>(g2, pglub, p.max_rows, p.max_tiles, 64, st))) return rc;
-      if ((rc = launch_umma_pair<kWgrad>(g3, pwd, p.max_rows, p.max_tiles, 64, st))) return rc;
+      if ((rc = wgrad(g3, st_wd, H))) return rc;
       if ((rc = launch_umma_pair<kDgrad>(g4, pdh, p.max_rows, p.max_tiles, 16, st))) return rc;
-      if ((rc = launch_umma_pair<kWgrad>(g5, pwgu, p.max_rows, p.max_tiles, 64, st))) return rc;
+      if ((rc = wgrad(g5, st_wgu, 2 * H))) return rc;
     }
   } else {
     if (!saved) launch_simt_gemm<T, kFwd>(g1, glu, p.max_rows, st);
