@@ -364,10 +364,24 @@ inline int launch_finish_grads(const float* acc, T* d_hidden, const float* gw_ro
 // few-token calls (a warp per token left most SMs idle and walked the columns one after the
 // other: 30 us at T = 64 and 512 with H = 2880, now 3 to 5), HBM the others.  The pieces of a row are neighbours in
 // the grid, so that its 512-byte parts are read at about the same time (T = 4096 44 us with the tokens as
-// neighbours, now 30; T = 16384 166 and 116).
+// neighbours, 30 with the pieces, 24 since the loads wait unconverted; T = 1531, K = 8, H = 2048 23 and 11).
 // Rows of another type than the output (fp32 rows of a bf16 call) lie at their flat positions p = t*K + k.
+template <typename T>
+__device__ __forceinline__ void unpack_vec(const uint4& q, float (&v)[16 / sizeof(T)]) {
+  const uint32_t u[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    if constexpr (sizeof(T) == 4) {
+      v[j] = __uint_as_float(u[j]);
+    } else {
+      v[2 * j] = __uint_as_float(u[j] << 16);
+      v[2 * j + 1] = __uint_as_float(u[j] & 0xffff0000u);
+    }
+  }
+}
+
 template <typename TY, typename T, int KB>
-__global__ void __launch_bounds__(kRowWarps * 32)
+__global__ void __launch_bounds__(kRowWarps * 32, KB > 4 ? 4 : 5)
 combine_padded_kernel(const TY* __restrict__ y, const int32_t* __restrict__ flat_row, T* __restrict__ out,
                       int64_t Tn, int H, int K) {
   pdl_wait();
@@ -383,17 +397,22 @@ combine_padded_kernel(const TY* __restrict__ y, const int32_t* __restrict__ flat
   for (int j = 0; j < VE; ++j) acc[j] = 0.f;
   for (int k0 = 0; k0 < K; k0 += KB) {
     int32_t r[KB];
-    float v[KB][VE];
+    uint4 q[KB];                           // as loaded: as fp32 they took 105 registers at KB = 8, now 56, and half the warps
 #pragma unroll
     for (int k = 0; k < KB; ++k) r[k] = k0 + k < K ? __ldg(flat_row + t * K + k0 + k) : -1;
 #pragma unroll
-    for (int k = 0; k < KB; ++k)
-      if (r[k] >= 0) load_vec<TY, VE>(y + (kFlat ? (size_t)(t * K + k0 + k) : (size_t)r[k]) * H + (size_t)i * VE, v[k]);
+    for (int k = 0; k < KB; ++k) {
+      q[k] = make_uint4(0, 0, 0, 0);
+      if (r[k] >= 0)
+        q[k] = __ldg(reinterpret_cast<const uint4*>(y + (kFlat ? (size_t)(t * K + k0 + k) : (size_t)r[k]) * H) + i);
+    }
 #pragma unroll
     for (int k = 0; k < KB; ++k)
       if (r[k] >= 0) {
+        float v[VE];
+        unpack_vec<TY>(q[k], v);
 #pragma unroll
-        for (int j = 0; j < VE; ++j) acc[j] += v[k][j];
+        for (int j = 0; j < VE; ++j) acc[j] += v[j];
       }
   }
   store_vec<T, VE>(out + (size_t)t * H + (size_t)i * VE, acc);
