@@ -377,10 +377,8 @@ __device__ __forceinline__ void stmatrix_x4_trans(uint32_t addr, uint32_t r0, ui
 // tile took longer still.  192 rows per expert (E = 64, H = 2048): gate_up 395 us with shuffles, 360 by stmatrix, 306 with
 // sixteen epilogue warps instead of eight; down 205, 190, 160 (1.07 and 0.54 GB of output, 145 and 73 us at the rate of a
 // fill).  Eight warps with two buffers each took 350 and 185, meeting once for two chunks 363.
-template <int WARPS>
 struct PairStoreBias {
   static constexpr bool kTmaStore = true;
-  static constexpr int kWarps = WARPS;      // see pair_wgrad_warps
   __nv_bfloat16* C;                // [E, H, ld]
   __nv_bfloat16* bias_out;         // [E, ld]
   int H, ld;
@@ -420,18 +418,15 @@ struct epi_tma_store<E, std::enable_if_t<E::kTmaStore>> : std::true_type {};
 constexpr int kMaxDynamicSmem = 227 * 1024 - 256;               // the barriers are static
 inline int pair_smem(int park_groups, int E) { return kPairSmem + park_groups * kPairParkBytes + (3 * E + 2) * 4; }
 
-// Epilogue warps.
-template <class Epi>
-constexpr int pair_epi_warps() {
-  if constexpr (epi_tma_store<Epi>::value) return Epi::kWarps;
-  else return 8;
-}
-// Of the weight gradients: sixteen while a tile's epilogue is longer than its main loop, eight above some 512 rows per
-// expert, where they only wait (8 / 16 warps: 192 rows, H = 2048 gate_up 359 / 306 us, down 190 / 160; 1024 rows, H = 2880
-// 788 / 806 and 396 / 407).
+// Epilogue warps: eight, or sixteen where the epilogue of a tile is long beside its main loop, as hidden behind the next
+// tile it is not, or where the last one of a CTA counts; else the additional warps only wait and take power (T = 4096,
+// H = 2880: 735 us with eight, 755 with sixteen).
+// Weight gradients: up to some 512 rows per expert (8 / 16 warps: 192 rows, H = 2048 gate_up 359 / 306 us, down 190 / 160;
+// 1024 rows, H = 2880 788 / 806 and 396 / 407).
 inline bool pair_wgrad_16_warps(int64_t S, int E) { return S <= 512 * (int64_t)E; }
-template <class Epi>
-constexpr int pair_threads() { return 32 * (3 + pair_epi_warps<Epi>()); }
+// The others: main loops of up to 16 k-blocks (T = 2048, E = 16, H = 1024 67.0 / 63.7 us), with the longer epilogue
+// of the GLU's backward up to 32 (192 rows per expert, H = 2048 180 / 168).
+inline bool pair_16_warps(int kblocks, bool glu_backward) { return kblocks <= (glu_backward ? 32 : 16); }
 
 __device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, int c0, int c1, int c2, uint32_t src) {
   asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];"
@@ -451,13 +446,12 @@ __device__ __forceinline__ bool group_all(int id, bool ok) {
   return all != 0;
 }
 
-template <int MODE, class Epi>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair_threads<Epi>(), 1)
+template <int MODE, class Epi, int kEpiWarps>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(32 * (3 + kEpiWarps), 1)
 umma_pair_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__ CUtensorMap tmN,
                  const __grid_constant__ CUtensorMap tmNsmall, const __grid_constant__ CUtensorMap tmOut,
                  const PairParams p, const Epi epi) {
   constexpr bool kStore = epi_tma_store<Epi>::value;
-  constexpr int kEpiWarps = pair_epi_warps<Epi>();
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t bar_full[kPairStages];       // used in the leader CTA
   __shared__ __align__(8) uint64_t bar_empty[kPairGroups];      // per CTA
@@ -496,7 +490,7 @@ umma_pair_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant_
   const uint32_t tmem_base = tmem_base_slot;
   pdl_trigger();
   pdl_wait();
-  for (int i = threadIdx.x; i <= p.E; i += pair_threads<Epi>()) {
+  for (int i = threadIdx.x; i <= p.E; i += 32 * (3 + kEpiWarps)) {
     const int p0 = p.pad_off[i];
     s_pad[i] = p0;
     if (MODE != kWgrad) s_pair[i] = p.pair_off[i];
@@ -803,9 +797,9 @@ inline int resident_pairs(void (*kern)(KArgs...), int threads, int smem, PerDevi
 // H % 64 == 0 holds on every path here: all pitches and widths are multiples of 64.
 // `row_round`: 16 where rows beyond an expert's own are never read again, 64 where a weight-gradient
 // GEMM will reduce over them (its k-blocks).
-template <int MODE, class Epi>
-inline int launch_umma_pair(const GemmArgs& g, const Epi& epi, int64_t max_rows, int64_t max_tiles, int row_round,
-                            cudaStream_t stream) {
+template <int MODE, int kEpiWarps, class Epi>
+inline int launch_umma_pair_warps(const GemmArgs& g, const Epi& epi, int64_t max_rows, int64_t max_tiles, int row_round,
+                                  cudaStream_t stream) {
   if (!umma_available() || g.E > kUmmaMaxExperts) return YAMOE_ERR_UNSUPPORTED;
   CUtensorMap tmM, tmN, tmNs;
   bool ok = true;
@@ -831,8 +825,8 @@ inline int launch_umma_pair(const GemmArgs& g, const Epi& epi, int64_t max_rows,
     }
   }
   constexpr bool kStore = epi_tma_store<Epi>::value;
-  constexpr int kThreads = pair_threads<Epi>();
-  const int groups = !kStore || pair_smem(4, g.E) <= kMaxDynamicSmem ? pair_epi_warps<Epi>() / 4 : 2;
+  constexpr int kThreads = 32 * (3 + kEpiWarps);
+  const int groups = !kStore || pair_smem(kEpiWarps / 4, g.E) <= kMaxDynamicSmem ? kEpiWarps / 4 : 2;
   const int smem = pair_smem(kStore ? groups : 0, g.E);
   CUtensorMap tmOut = tmM;               // not used
   if constexpr (kStore) {
@@ -842,7 +836,7 @@ inline int launch_umma_pair(const GemmArgs& g, const Epi& epi, int64_t max_rows,
     ok = ok && make_map(&tmOut, epi.C, 3, d, st, b);
   }
   if (!ok) return YAMOE_ERR_CUDA;
-  auto kern = umma_pair_kernel<MODE, Epi>;
+  auto kern = umma_pair_kernel<MODE, Epi, kEpiWarps>;
   static PerDevice<int> resident;    // per template instantiation and device
   const int pairs = resident_pairs(kern, kThreads, kMaxDynamicSmem, resident);
   if (pairs <= 0) return YAMOE_ERR_CUDA;
@@ -856,6 +850,13 @@ inline int launch_umma_pair(const GemmArgs& g, const Epi& epi, int64_t max_rows,
   if (launch_pdl_opt(true, kern, dim3(grid), dim3(kThreads), smem, stream, tmM, tmN, tmNs, tmOut, p, epi) != cudaSuccess)
     return YAMOE_ERR_CUDA;
   return cudaGetLastError() == cudaSuccess ? YAMOE_OK : YAMOE_ERR_CUDA;
+}
+
+template <int MODE, class Epi>
+inline int launch_umma_pair(const GemmArgs& g, const Epi& epi, int64_t max_rows, int64_t max_tiles, int row_round,
+                            bool sixteen, cudaStream_t stream) {
+  return sixteen ? launch_umma_pair_warps<MODE, 16>(g, epi, max_rows, max_tiles, row_round, stream)
+                 : launch_umma_pair_warps<MODE, 8>(g, epi, max_rows, max_tiles, row_round, stream);
 }
 
 }  // namespace yb

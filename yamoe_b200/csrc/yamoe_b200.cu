@@ -281,7 +281,7 @@ static int forward_impl(const void* hidden, const int64_t* ridx, const void* rw,
         StageTimer tm(kStageGateUp, st);
         const PairGlu<false> pglu{reinterpret_cast<const T*>(bgu), reinterpret_cast<T*>(p.act), nullptr, nullptr,
                                   nullptr, nullptr, H, 0};
-        rc = launch_umma_pair<kFwd>(g1, pglu, p.max_rows, p.max_tiles, 16, st);
+        rc = launch_umma_pair<kFwd>(g1, pglu, p.max_rows, p.max_tiles, 16, pair_16_warps(H / kUmmaBK, false), st);
       }
       if (rc) return rc;
       // two-step combine: weighted rows out of the GEMM epilogue, then one gather-sum pass; decode-sized calls
@@ -292,11 +292,11 @@ static int forward_impl(const void* hidden, const int64_t* ridx, const void* rw,
         if (flat) {
           const PairWeightedFlat wflat{reinterpret_cast<const T*>(bd), reinterpret_cast<float*>(p.yrows), p.rt.row_token,
                                        p.rt.row_flat, p.rt.row_weight, H};
-          rc = launch_umma_pair<kFwd>(g2, wflat, p.max_rows, p.max_tiles, 16, st);
+          rc = launch_umma_pair<kFwd>(g2, wflat, p.max_rows, p.max_tiles, 16, pair_16_warps(H / kUmmaBK, false), st);
         } else {
           const PairWeightedRows wrows{reinterpret_cast<const T*>(bd), reinterpret_cast<T*>(p.yrows), p.rt.row_token,
                                        p.rt.row_weight, H};
-          rc = launch_umma_pair<kFwd>(g2, wrows, p.max_rows, p.max_tiles, 16, st);
+          rc = launch_umma_pair<kFwd>(g2, wrows, p.max_rows, p.max_tiles, 16, pair_16_warps(H / kUmmaBK, false), st);
         }
       }
       if (rc) return rc;
@@ -375,8 +375,8 @@ static int forward_train_impl(const void* hidden, const int64_t* ridx, const voi
     if constexpr (sizeof(T) == 2) {
       const PairGlu<true> pglu{glu.bias, act, glu.actw, glu.pre, p.rt.row_token, p.rt.row_weight, H, Hp};
       const PairWeightedRows pw{wrows.bias, yrows, p.rt.row_token, p.rt.row_weight, H};
-      if ((rc = launch_umma_pair<kFwd>(g1, pglu, p.max_rows, p.max_tiles, 64, st))) return rc;
-      if ((rc = launch_umma_pair<kFwd>(g2, pw, p.max_rows, p.max_tiles, 16, st))) return rc;
+      if ((rc = launch_umma_pair<kFwd>(g1, pglu, p.max_rows, p.max_tiles, 64, pair_16_warps(H / kUmmaBK, false), st))) return rc;
+      if ((rc = launch_umma_pair<kFwd>(g2, pw, p.max_rows, p.max_tiles, 16, pair_16_warps(H / kUmmaBK, false), st))) return rc;
     }
   } else {
     launch_simt_gemm<T, kFwd>(g1, glu, p.max_rows, st);
@@ -511,17 +511,14 @@ static int backward_impl(const void* grad_out, int per_slot, const void* hidden,
     if constexpr (sizeof(T) == 2) {
       const PairGlu<true> pglu{glu.bias, nullptr, glu.actw, glu.pre, p.rt.row_token, p.rt.row_weight, H, Hp};
       const PairGluBackward pglub{glub.pre, glub.g_pre, p.gw_row, p.rt.row_token, p.rt.row_weight, H};
-      auto wgrad = [&](const GemmArgs& g, const EpiStoreBias<T>& o, int ld) {
-        if (pair_wgrad_16_warps(p.S, E))
-          return launch_umma_pair<kWgrad>(g, PairStoreBias<16>{o.C, o.bias_out, H, ld}, p.max_rows, p.max_tiles, 64, st);
-        return launch_umma_pair<kWgrad>(g, PairStoreBias<8>{o.C, o.bias_out, H, ld}, p.max_rows, p.max_tiles, 64, st);
-      };
+      const PairStoreBias pwd{st_wd.C, st_wd.bias_out, H, H}, pwgu{st_wgu.C, st_wgu.bias_out, H, 2 * H};
+      const bool w16 = pair_wgrad_16_warps(p.S, E);
       const PairScatterAdd pdh{acc, p.rt.row_token, H};
-      if (!saved && (rc = launch_umma_pair<kFwd>(g1, pglu, p.max_rows, p.max_tiles, 64, st))) return rc;
-      if ((rc = launch_umma_pair<kDgrad>(g2, pglub, p.max_rows, p.max_tiles, 64, st))) return rc;
-      if ((rc = wgrad(g3, st_wd, H))) return rc;
-      if ((rc = launch_umma_pair<kDgrad>(g4, pdh, p.max_rows, p.max_tiles, 16, st))) return rc;
-      if ((rc = wgrad(g5, st_wgu, 2 * H))) return rc;
+      if (!saved && (rc = launch_umma_pair<kFwd>(g1, pglu, p.max_rows, p.max_tiles, 64, pair_16_warps(H / kUmmaBK, false), st))) return rc;
+      if ((rc = launch_umma_pair<kDgrad>(g2, pglub, p.max_rows, p.max_tiles, 64, pair_16_warps(H / kUmmaBK, true), st))) return rc;
+      if ((rc = launch_umma_pair<kWgrad>(g3, pwd, p.max_rows, p.max_tiles, 64, w16, st))) return rc;
+      if ((rc = launch_umma_pair<kDgrad>(g4, pdh, p.max_rows, p.max_tiles, 16, pair_16_warps(2 * H / kUmmaBK, false), st))) return rc;
+      if ((rc = launch_umma_pair<kWgrad>(g5, pwgu, p.max_rows, p.max_tiles, 64, w16, st))) return rc;
     }
   } else {
     if (!saved) launch_simt_gemm<T, kFwd>(g1, glu, p.max_rows, st);
