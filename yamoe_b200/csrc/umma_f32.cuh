@@ -537,8 +537,10 @@ umma_f32_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__
   const int cluster_id = blockIdx.x >> 1, n_clusters = gridDim.x >> 1;
   if (MODE != kWgrad && warp == 4) {
     // Most rows of a tile: the candidate with the smallest product of waves and clocks of its widest k-block, 12 per row
-    // on the tensor core (24 instructions) but no less than kConvClocks for the weights' conversion.
-    constexpr int kConvClocks = 1200;
+    // on the tensor core (24 instructions) but no less than kConvClocks for the weights' conversion and the chain of signals
+    // around it.  (With 1200 it cuts too finely: T = 900, E = 8, H = 2880 510 us against 487; with 900 T = 512 382 against 316;
+    // 2000 is the same as 1600.)
+    constexpr int kConvClocks = 1600;
     int best = 0x7fffffff, tile = kF32N;
     auto consider = [&](auto cap) {
       constexpr int C = decltype(cap)::value;
