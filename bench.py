@@ -74,13 +74,13 @@ TRAFFIC = {
 
 # kernels of this library launched by one call (memsets not counted):
 #   fwd     routing + row gather + gate_up GEMM + down GEMM + combine
-#   bwd     routing + 2 gathers + 5 GEMMs (bias gradients ride along) + routing gradient + cast
+#   bwd     routing + 2 gathers + 5 GEMMs (bias gradients ride along) + cast and routing gradients
 #           (one more in either where more than 32768 assignments take the two-launch routing)
 #   decode  2 GEMV kernels, or the kernels of fwd where the grouped GEMM takes the call
 #   ep_fwd  2 routing + publish + dispatch + 2 GEMMs + signal + combine
 #   ep_bwd  2 routing + publish + dispatch + weights + gather + 5 GEMMs + 2 column sums +
 #           scalar return + signal + combine + routing gradient
-LAUNCHES = {"fwd": 5, "fwd_fp32": 5, "bwd": 10, "train": 15, "decode": 2, "ep_fwd": 8, "ep_bwd": 17}
+LAUNCHES = {"fwd": 5, "fwd_fp32": 5, "bwd": 9, "train": 14, "decode": 2, "ep_fwd": 8, "ep_bwd": 17}
 
 
 def measured_peaks():

@@ -22,8 +22,11 @@
 // 64).  The weights' last M tile may be partly empty: 2880 columns take 12 pairs of which the last
 // has 64 columns, 6.7 %; 5760 take 23, 2.2 %.
 //
-// A CTA has 11 warps: two TMA producers, MMA issuer (of the leader only), eight epilogue warps (two per
-// TMEM lane quarter, which take 32-column chunks in turn).  Six stages of 32 KB; two accumulators of
+// A CTA has 11 or 19 warps: two TMA producers, MMA issuer (of the leader only), eight or sixteen epilogue warps (two or four
+// per TMEM lane quarter, which take 32-column chunks in turn; see pair_16_warps).  A larger item, 512 rows in two accumulators
+// that share the weight slab, was no gain: 25 % fewer operand bytes, but the rings that it needs cost the issuer a second
+// wait per k-block (7 to 10 % of any launch), and an accumulator must be drained while the other is filled (T = 4096
+// 715 -> 768 .. 868 us in four forms).  Six stages of 32 KB; two accumulators of
 // 256 TMEM columns, so that the epilogue of a tile overlaps the main loop of the next.  The
 // epilogue thread of lane m holds 32 rows' values of ONE weight column: bias and column sums are per
 // thread, and the rows of the output are written by the lanes of a warp side by side.
