@@ -41,7 +41,7 @@
 // four of activations (30 KB); TMEM, all 512 columns: two accumulators of 160, two A operands of 96.  Signals between
 // the CTAs as in umma_pair.cuh, every wait bounded as in umma_gemm.cuh.
 //
-// Tiles of up to 160 rows, of a size that the kernel picks for the launch (see `consider`): a tile's weights are converted
+// Tiles of up to 160 rows, of a size that the kernel picks for the launch (see s_cost): a tile's weights are converted
 // for its rows alone, and with 128 rows at most half of the experts of the README forward (128 rows each on average) took
 // two tiles: 276 tiles in four waves of 74 pairs, now 184 in three.  gate_up 216 -> 177 us, the whole forward
 // 348 -> 313, with the waits looked at side by side included: a look at a barrier that is ready takes some 120 clocks, of
@@ -56,6 +56,7 @@ constexpr int kF32ConvWarps = 8, kF32AccWarps = 12;
 constexpr int kF32Threads = 32 * (4 + kF32ConvWarps + kF32AccWarps);
 constexpr int kF32M = 128, kF32K = 64;                   // M per CTA
 constexpr int kF32N = 160, kF32WgradN = 128;             // most N of a pair: rows of an expert, columns of the activations
+constexpr int kF32Tiles = 6;                             // candidates for the rows of a tile: 160, 144, ... 80
 constexpr int kF32WBytes = kF32M * kF32K * 4;            // 32 KB: fp32 tile of the M operand
 constexpr int kF32BBytes = 3 * (kF32N / 2) * kF32K * 2;  // 30 KB: this CTA's half of the N operand, three planes
 constexpr int kF32WStages = 3, kF32BStages = 4;          // (three of activations where the tables of many experts need room)
@@ -483,7 +484,7 @@ umma_f32_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__
   __shared__ __align__(8) uint64_t bar_a_full[2], bar_a_empty[2];
   __shared__ __align__(8) uint64_t bar_acc_full[2], bar_acc_empty[2];
   __shared__ uint32_t tmem_base_slot;
-  __shared__ int abort_flag;
+  __shared__ int abort_flag, s_cost[kF32Tiles];
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
@@ -535,32 +536,30 @@ umma_f32_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__
 
   const int MT = (p.M + 2 * kF32M - 1) / (2 * kF32M);
   const int cluster_id = blockIdx.x >> 1, n_clusters = gridDim.x >> 1;
-  if (MODE != kWgrad && warp == 4) {
-    // Most rows of a tile: the candidate with the smallest product of waves and clocks of its widest k-block, 12 per row
-    // on the tensor core (24 instructions) but no less than kConvClocks for the weights' conversion and the chain of signals
-    // around it.  (With 1200 it cuts too finely: T = 900, E = 8, H = 2880 510 us against 487; with 900 T = 512 382 against 316;
-    // 2000 is the same as 1600.)
+  if (MODE != kWgrad && warp >= 4 && warp < 4 + kF32Tiles) {
+    // Most rows of a tile: the candidate (one to a warp) with the smallest product of waves and clocks of its widest k-block, 12
+    // per row on the tensor core (24 instructions) but no less than kConvClocks for the weights' conversion and the chain of
+    // signals around it.  (With 1200 it cuts too finely: T = 900, E = 8, H = 2880 510 us against 487; with 900 T = 512 382
+    // against 316; 2000 is the same as 1600.)  By one warp after the other this stood before the first load of every launch:
+    // training step of 600 tokens 379 us, now 364.
     constexpr int kConvClocks = 1600;
-    int best = 0x7fffffff, tile = kF32N;
-    auto consider = [&](auto cap) {
-      constexpr int C = decltype(cap)::value;
-      int n = 0, widest = 0;
-      for (int e = lane; e < p.E; e += 32) {
-        const int rows = s_rows[e], cnt = (rows + C - 1) / C;
-        n += cnt;
-        if (cnt > 0) widest = max(widest, cnt == 1 ? rows : (rows / cnt + 16) & ~15);
-      }
-      n = __reduce_add_sync(0xffffffffu, n);
-      widest = __reduce_max_sync(0xffffffffu, widest);
-      const int cost = (n * MT + n_clusters - 1) / n_clusters * max(12 * widest, kConvClocks);
-      if (cost < best) { best = cost; tile = C; }
-    };
-    consider(std::integral_constant<int, 160>{});
-    consider(std::integral_constant<int, 144>{});
-    consider(std::integral_constant<int, 128>{});
-    consider(std::integral_constant<int, 112>{});
-    consider(std::integral_constant<int, 96>{});
-    consider(std::integral_constant<int, 80>{});
+    const int cap = kF32N - 16 * (warp - 4);
+    int n = 0, widest = 0;
+    for (int e = lane; e < p.E; e += 32) {
+      const int rows = s_rows[e], cnt = (rows + cap - 1) / cap;
+      n += cnt;
+      if (cnt > 0) widest = max(widest, cnt == 1 ? rows : (rows / cnt + 16) & ~15);
+    }
+    n = __reduce_add_sync(0xffffffffu, n);
+    widest = __reduce_max_sync(0xffffffffu, widest);
+    if (lane == 0) s_cost[warp - 4] = (n * MT + n_clusters - 1) / n_clusters * max(12 * widest, kConvClocks);
+  }
+  __syncthreads();
+  if (MODE != kWgrad && warp == 4) {
+    int tile = kF32N, best = s_cost[0];
+#pragma unroll
+    for (int i = 1; i < kF32Tiles; ++i)
+      if (s_cost[i] < best) { best = s_cost[i]; tile = kF32N - 16 * i; }
     int before = 0;
     for (int e0 = 0; e0 < p.E; e0 += 32) {
       const int n = e0 + lane < p.E ? (s_rows[e0 + lane] + tile - 1) / tile : 0;
