@@ -1,6 +1,6 @@
-"""Bounded waits of the tensor-core kernels, by reading their source: a wait that runs out must take every thread
-that later meets in one barrier or one warp-wide instruction the same way.  (On a GPU this shows only when
-a wait runs out for some threads and ends well for others.)"""
+"""Waits of the kernels, by reading their source.  Bounded waits: one that runs out must take every thread that later meets
+in one barrier or one warp-wide instruction the same way.  (On a GPU this shows only when a wait runs out for some
+threads and ends well for others.)  Waits for the kernel before: nothing that it wrote is loaded as read-only data."""
 import os
 import re
 
@@ -40,3 +40,47 @@ def test_commits_are_awaited_before_a_cta_ends():
     text = source("umma_f32.cuh")
     for bar in ("bar_b_empty", "bar_a_empty"):
         assert len(re.findall(r"mbar_wait\w*\(smem_u32\(&%s\[" % bar, text)) == 2, bar
+
+
+#: kernels that may start before the one before them has ended (launch_pdl_opt), and what each may load by __ldg or take as
+#: `const __restrict__`: tensors of the caller that no kernel of the same call writes, read behind another kernel of that call
+EARLY = {"misc_kernels.cuh": {"gather_tokens_kernel": ["src"], "gather_grad_tokens_kernel": [], "finish_grads_kernel": [],
+                              "combine_padded_kernel": []},
+         "gemv.cuh": {"gemv_kernel": []}, "umma_gemm.cuh": {"umma_gemm_kernel": []}, "umma_pair.cuh": {"umma_pair_kernel": []},
+         "umma_f32.cuh": {"umma_f32_kernel": []}}
+
+
+def kernel(text, name):
+    start = text.index("\n%s(" % name)
+    return text[start:text.index("\n}\n", start)]
+
+
+def test_early_kernels_are_known():
+    for name in sorted(os.listdir(CSRC)):
+        if name.endswith((".cuh", ".cu")) and name != "common.cuh":
+            calls = len(re.findall(r"\blaunch_pdl_opt\(", source(name)))
+            assert calls == len(EARLY.get(name, {})), name
+
+
+@pytest.mark.parametrize("name,kern", [(f, k) for f in sorted(EARLY) for k in EARLY[f]])
+def test_early_kernels_load_what_others_wrote_behind_the_wait(name, kern):
+    body = kernel(source(name), kern)
+    wait = body.index("pdl_wait()")
+    read_only = re.findall(r"const\s+\w+\s*\*\s*__restrict__\s+(\w+)", body)
+    assert read_only == EARLY[name][kern], read_only
+    for load in re.findall(r"__ldg\(([^;]*);", body):
+        assert any(re.search(r"\b%s\b" % allowed, load) for allowed in EARLY[name][kern]), load
+    # pointers are taken behind the wait, and what is loaded past this kernel's own stores comes from one of them
+    taken = re.findall(r"(\w+) = after_wait\(", body)
+    assert all(m.start() > wait for m in re.finditer(r"after_wait\(", body))
+    for load in re.findall(r"ld_written\(reinterpret_cast<const uint4\*>\((\w+)", body):
+        assert load in taken, load
+    for call in re.findall(r"load_vec<([^;]*);", body):
+        assert ", true>(" in call, call
+
+
+def test_epilogues_of_early_kernels_load_no_read_only_data():
+    """Pre-activations come from an earlier GEMM of the same pass."""
+    for name in ("umma_pair.cuh", "umma_f32.cuh", "umma_gemm.cuh", "gemv.cuh"):
+        assert "__ldg(" not in source(name), name
+    assert re.findall(r"load_vec<([^>]*)>\(pre\b", source("epilogues.cuh")) == ["T, 2 * NV, true"]

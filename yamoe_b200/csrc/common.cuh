@@ -88,6 +88,27 @@ __device__ __forceinline__ float ld_shared_cluster_f32(uint32_t cluster_addr) {
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// Loads of what an earlier kernel on the stream has written, in a kernel that may start before that one has ended.  Not
+// __ldg, which wants memory that nobody writes while the kernel runs, and whose loads the compiler may move past the
+// wait: ordinary loads, from a pointer that after_wait() hands out behind pdl_wait().  ld_written is one that may
+// still move past this kernel's own stores, for memory that it does not write itself.
+template <typename P>
+__device__ __forceinline__ P* after_wait(P* p) {
+  uint64_t a = reinterpret_cast<uint64_t>(p);
+  asm volatile("" : "+l"(a) : : "memory");
+  return reinterpret_cast<P*>(a);
+}
+__device__ __forceinline__ uint4 ld_written(const uint4* p) {
+  uint4 q;
+  asm("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(q.x), "=r"(q.y), "=r"(q.z), "=r"(q.w) : "l"(p));
+  return q;
+}
+__device__ __forceinline__ float2 ld_written(const float2* p) {
+  float2 q;
+  asm("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(q.x), "=f"(q.y) : "l"(p));
+  return q;
+}
+
 // Measured on B200: between the two decode GEMV kernels it saves about 2 us per call (T = 1: 52.0 us
 // against 53.8 us as a CUDA-graph replay).  Of the expert pass the grouped GEMMs of umma_pair.cuh and
 // umma_f32.cuh, the gathers and the combine use it as well: their barrier and TMEM set-up and the

@@ -12,16 +12,20 @@
 namespace yb {
 
 // ---- small vector load / store helpers (fp32 <-> storage dtype) ------------------------------
-template <typename T, int N>
+// WRITTEN: `src` was written by an earlier kernel on the stream (see ld_written)
+template <typename T, int N, bool WRITTEN = false>
 __device__ __forceinline__ void load_vec(const T* __restrict__ src, float (&out)[N]) {
   if constexpr (sizeof(T) == 4) {
     if constexpr (N % 4 == 0) {
 #pragma unroll
       for (int i = 0; i < N / 4; ++i) {
-        float4 q = __ldg(reinterpret_cast<const float4*>(src) + i);
-        out[4 * i] = q.x; out[4 * i + 1] = q.y; out[4 * i + 2] = q.z; out[4 * i + 3] = q.w;
+        const uint4* p = reinterpret_cast<const uint4*>(src) + i;
+        const uint4 q = WRITTEN ? ld_written(p) : __ldg(p);
+        out[4 * i] = __uint_as_float(q.x); out[4 * i + 1] = __uint_as_float(q.y);
+        out[4 * i + 2] = __uint_as_float(q.z); out[4 * i + 3] = __uint_as_float(q.w);
       }
     } else {
+      static_assert(!WRITTEN, "16 bytes at a time");
 #pragma unroll
       for (int i = 0; i < N; ++i) out[i] = __ldg(reinterpret_cast<const float*>(src) + i);
     }
@@ -29,7 +33,8 @@ __device__ __forceinline__ void load_vec(const T* __restrict__ src, float (&out)
     if constexpr (N % 8 == 0) {
 #pragma unroll
       for (int i = 0; i < N / 8; ++i) {
-        uint4 q = __ldg(reinterpret_cast<const uint4*>(src) + i);
+        const uint4* p = reinterpret_cast<const uint4*>(src) + i;
+        const uint4 q = WRITTEN ? ld_written(p) : __ldg(p);
         const uint32_t u[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -38,6 +43,7 @@ __device__ __forceinline__ void load_vec(const T* __restrict__ src, float (&out)
         }
       }
     } else if constexpr (N % 2 == 0) {
+      static_assert(!WRITTEN, "16 bytes at a time");
 #pragma unroll
       for (int i = 0; i < N / 2; ++i) {
         uint32_t u = __ldg(reinterpret_cast<const uint32_t*>(src) + i);
@@ -273,7 +279,7 @@ struct EpiGluBackward {
       for (int i = 0; i < 2 * NV; ++i) out[i] = 0.f;
     } else {
       float p[2 * NV];
-      load_vec<T, 2 * NV>(pre + (size_t)row * 2 * H + 2 * n0, p);
+      load_vec<T, 2 * NV, true>(pre + (size_t)row * 2 * H + 2 * n0, p);
       const float w = row_weight[row];
       float dot = 0.f;
 #pragma unroll

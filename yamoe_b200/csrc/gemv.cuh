@@ -244,6 +244,7 @@ gemv_kernel(const GemvArgs g) {
   const __nv_bfloat16* wp = g.W + ((size_t)e * g.Kdim + k0) * g.N + n;
   // everything above read only the caller's inputs; below come act / out32 / slab counters
   if constexpr (STAGE == kDown) pdl_wait();
+  const __nv_bfloat16* x = after_wait(g.x);
   const int part = w * RPW + lane / LPR;
 
   for (int r0 = 0; r0 < n_rows; r0 += kGemvMT) {
@@ -255,7 +256,7 @@ gemv_kernel(const GemvArgs g) {
       const int p = rows[r0 + m];
       const size_t src_row = (STAGE == kGateUp) ? (size_t)(p / g.K) : (size_t)p;
       reinterpret_cast<uint4*>(xs + (size_t)m * klen)[c] =
-          __ldg(reinterpret_cast<const uint4*>(g.x + src_row * g.Kdim + k0) + c);
+          ld_written(reinterpret_cast<const uint4*>(x + src_row * g.Kdim + k0) + c);
     }
     __syncthreads();
     float acc[kGemvMT][8];

@@ -68,11 +68,12 @@ gather_tokens_kernel(const void* __restrict__ src, const Dst dst, const RouteTab
   if (real) q = __ldg(reinterpret_cast<const uint4*>(src) + t * nvec + i);
   // the columns behind H: the lanes of the last warp once more
   const bool last = ld_vec > nvec && i - lane + 32 >= nvec;
+  const int32_t* flat_row = after_wait(rt.flat_row);
   typename Dst::Piece x;
   for (int k0 = 0; k0 < K; k0 += KB) {
     int32_t r[KB];
 #pragma unroll
-    for (int k = 0; k < KB; ++k) r[k] = k0 + k < K ? __ldg(rt.flat_row + t * K + k0 + k) : -1;
+    for (int k = 0; k < KB; ++k) r[k] = k0 + k < K ? flat_row[t * K + k0 + k] : -1;
     if (k0 == 0) x = dst.piece(q);
 #pragma unroll
     for (int k = 0; k < KB; ++k)
@@ -144,11 +145,16 @@ gather_grad_kernel(const T* __restrict__ grad_out, int slots, const T* __restric
 // where a memset does 3.9, and a launch is saved (T = 8192, H = 2880: memset 22 us + gather 64, together 77).
 template <typename T, class Dst, int KB>
 __global__ void __launch_bounds__(kRowWarps * 32)
-gather_grad_tokens_kernel(const T* __restrict__ grad_out, int slots, const T* __restrict__ down_bias, const Dst dst,
-                          float* __restrict__ gw_row, float* __restrict__ acc, const RouteTables rt, int64_t Tn, int H,
-                          int K, int wpt, unsigned pad_ctas, int row_round) {
+gather_grad_tokens_kernel(const T* grad_out, int slots, const T* down_bias, const Dst dst, float* __restrict__ gw_row,
+                          float* __restrict__ acc, const RouteTables rt, int64_t Tn, int H, int K, int wpt,
+                          unsigned pad_ctas, int row_round) {
   pdl_wait();
   pdl_trigger();
+  // after a saving forward this is the first kernel of the call: what wrote the caller's tensors may still have been running
+  grad_out = after_wait(grad_out);
+  down_bias = after_wait(down_bias);
+  const int32_t* flat_row = after_wait(rt.flat_row);
+  const int32_t* tile_expert = after_wait(rt.tile_expert);
   constexpr int VE = 16 / (int)sizeof(T);
   const int nvec = H / VE;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -164,20 +170,20 @@ gather_grad_tokens_kernel(const T* __restrict__ grad_out, int slots, const T* __
     const T* bias[KB];
     float dot[KB];
 #pragma unroll
-    for (int k = 0; k < KB; ++k) r[k] = t < Tn && k0 + k < K ? __ldg(rt.flat_row + t * K + k0 + k) : -1;
+    for (int k = 0; k < KB; ++k) r[k] = t < Tn && k0 + k < K ? flat_row[t * K + k0 + k] : -1;
 #pragma unroll
     for (int k = 0; k < KB; ++k) {
-      bias[k] = down_bias + (r[k] >= 0 ? (size_t)__ldg(rt.tile_expert + r[k] / kTileM) * H : 0);
+      bias[k] = down_bias + (r[k] >= 0 ? (size_t)tile_expert[r[k] / kTileM] * H : 0);
       dot[k] = 0.f;
     }
     if (t < Tn) {
 #pragma unroll 2
       for (int i = lane + 32 * part; i < nvec; i += 32 * wpt) {
         float g[VE];
-        load_vec<T, VE>(grad_out + (size_t)t * slots * H + (size_t)i * VE, g);
+        load_vec<T, VE, true>(grad_out + (size_t)t * slots * H + (size_t)i * VE, g);
         for (int s = 1; s < slots; ++s) {
           float g2[VE];
-          load_vec<T, VE>(grad_out + ((size_t)t * slots + s) * H + (size_t)i * VE, g2);
+          load_vec<T, VE, true>(grad_out + ((size_t)t * slots + s) * H + (size_t)i * VE, g2);
 #pragma unroll
           for (int j = 0; j < VE; ++j) g[j] += g2[j];
         }
@@ -194,7 +200,7 @@ gather_grad_tokens_kernel(const T* __restrict__ grad_out, int slots, const T* __
           if (r[k] >= 0) {
             dst.put((size_t)r[k], i, x);
             float b[VE];
-            load_vec<T, VE>(bias[k] + (size_t)i * VE, b);
+            load_vec<T, VE, true>(bias[k] + (size_t)i * VE, b);
 #pragma unroll
             for (int j = 0; j < VE; ++j) dot[k] = fmaf(g[j], b[j], dot[k]);
           }
@@ -309,10 +315,11 @@ colsum_kernel(const T* __restrict__ src, const float* __restrict__ row_weight,
 // now 7).
 template <typename T>
 __global__ void __launch_bounds__(256)
-finish_grads_kernel(const float* __restrict__ acc, T* __restrict__ d_hidden, int64_t n_vec4, unsigned cast_ctas,
-                    const float* __restrict__ gw_row, const RouteTables rt, T* __restrict__ d_routing, int64_t Tn,
-                    int routing_cols, int E, int K) {
+finish_grads_kernel(const float* acc, T* __restrict__ d_hidden, int64_t n_vec4, unsigned cast_ctas, const float* gw_row,
+                    const RouteTables rt, T* __restrict__ d_routing, int64_t Tn, int routing_cols, int E, int K) {
   pdl_wait();
+  acc = after_wait(acc);
+  gw_row = after_wait(gw_row);
   if (blockIdx.x < cast_ctas) {
     for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n_vec4; i += (int64_t)cast_ctas * 256) {
       const float4 q = __ldcs(reinterpret_cast<const float4*>(acc) + i);
@@ -382,9 +389,10 @@ __device__ __forceinline__ void unpack_vec(const uint4& q, float (&v)[16 / sizeo
 
 template <typename TY, typename T, int KB>
 __global__ void __launch_bounds__(kRowWarps * 32, KB > 4 ? 4 : 5)
-combine_padded_kernel(const TY* __restrict__ y, const int32_t* __restrict__ flat_row, T* __restrict__ out,
-                      int64_t Tn, int H, int K) {
+combine_padded_kernel(const TY* y, const int32_t* flat_row, T* __restrict__ out, int64_t Tn, int H, int K) {
   pdl_wait();
+  y = after_wait(y);
+  flat_row = after_wait(flat_row);
   constexpr bool kFlat = !std::is_same<TY, T>::value;
   constexpr int VE = 16 / (int)sizeof(TY);
   const unsigned chunks = (unsigned)(H / VE + 31) / 32;
@@ -399,12 +407,12 @@ combine_padded_kernel(const TY* __restrict__ y, const int32_t* __restrict__ flat
     int32_t r[KB];
     uint4 q[KB];                           // as loaded: as fp32 they took 105 registers at KB = 8, now 56, and half the warps
 #pragma unroll
-    for (int k = 0; k < KB; ++k) r[k] = k0 + k < K ? __ldg(flat_row + t * K + k0 + k) : -1;
+    for (int k = 0; k < KB; ++k) r[k] = k0 + k < K ? flat_row[t * K + k0 + k] : -1;
 #pragma unroll
     for (int k = 0; k < KB; ++k) {
       q[k] = make_uint4(0, 0, 0, 0);
       if (r[k] >= 0)
-        q[k] = __ldg(reinterpret_cast<const uint4*>(y + (kFlat ? (size_t)(t * K + k0 + k) : (size_t)r[k]) * H) + i);
+        q[k] = ld_written(reinterpret_cast<const uint4*>(y + (kFlat ? (size_t)(t * K + k0 + k) : (size_t)r[k]) * H) + i);
     }
 #pragma unroll
     for (int k = 0; k < KB; ++k)

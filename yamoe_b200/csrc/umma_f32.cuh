@@ -376,7 +376,7 @@ struct F32GluBackward {             // see PairGluBackward; the gradient leaves 
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
       const bool ok = (have >> i) & 1u;
-      const float2 q = ok ? __ldg(src + (size_t)i * H) : make_float2(0.f, 0.f);
+      const float2 q = ok ? ld_written(src + (size_t)i * H) : make_float2(0.f, 0.f);
       const float w = __shfl_sync(0xffffffffu, w_lane, i);
       const float pg = q.x, pu = q.y;
       const float gc = fminf(pg, kLimit);

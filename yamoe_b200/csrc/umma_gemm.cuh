@@ -347,7 +347,7 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   auto expert_of = [&](int id) -> int {
     if constexpr (MODE == kWgrad) return 0;
     if (uniform) return 0;
-    return id < total ? __ldg(p.tile_expert + id / NT) : 0;
+    return id < total ? p.tile_expert[id / NT] : 0;
   };
   auto decode = [&](int id, int e_hint, int& e, int& row0, int& n0, int& kb_begin_row, int& kblocks) {
     if constexpr (MODE == kWgrad) {

@@ -510,7 +510,7 @@ umma_pair_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant_
   // expert of a work item: the one entry that comes from global memory, asked for one item ahead
   auto expert_of = [&](int id) -> int {
     if constexpr (MODE == kWgrad) return 0;
-    return id < total ? __ldg(p.pair_expert + id / MT) : 0;
+    return id < total ? p.pair_expert[id / MT] : 0;
   };
   // work item -> expert, first M index, first N index (row or column), width (multiple of 16), k-blocks.
   // The tiles of one M slab follow each other: the CTAs running at any moment share the weight slab in L2.
