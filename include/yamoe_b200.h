@@ -9,6 +9,9 @@
  *
  * Every entry point returns YAMOE_OK (0) or a negative yamoe_status_t.
  *
+ * Tensors of the expert passes start on 16-byte boundaries where nothing else is said; integer ones and biases
+ * of the weights in fp32 need no more than their element's size.
+ *
  * The comments cite the interface of the reference project (drbh/yamoe) that each entry
  * point replaces, as path:line within that project.
  */
@@ -24,7 +27,7 @@ extern "C" {
 
 typedef enum {
   YAMOE_OK = 0,
-  YAMOE_ERR_BAD_ARG = -1,        /* null pointer, non-positive size, H not a multiple of 8, ... */
+  YAMOE_ERR_BAD_ARG = -1,        /* null pointer, non-positive size, H not a multiple of 8, d_hidden misaligned, ... */
   YAMOE_ERR_WORKSPACE = -2,      /* workspace pointer null / misaligned / too small          */
   YAMOE_ERR_DTYPE = -3,          /* dtype is not YAMOE_F32 or YAMOE_BF16                      */
   YAMOE_ERR_CUDA = -4,           /* a CUDA runtime / driver call failed (launch, tensor map)  */
@@ -141,7 +144,7 @@ int yamoe_b200_experts_forward(const void *hidden_states, const int64_t *router_
  *
  *   grad_out          dtype, T*H elements, or T*K*H elements (grad_out_per_slot != 0) that are
  *                     summed over K first (csrc/experts_backward.cu:224-228)
- *   d_hidden          dtype [T,H]
+ *   d_hidden          dtype [T,H]; 8-byte aligned (16 in fp32 on the SIMT path), otherwise YAMOE_ERR_BAD_ARG
  *   d_routing         dtype [T,routing_cols]; zero outside selected, kept entries.  The value is
  *                     the autograd gradient <grad_out[t], y_e[t]>; the reference applies the sort
  *                     permutation twice here (csrc/experts_backward.cu:261-264) and is not followed.

@@ -4,7 +4,7 @@ import pytest
 import torch
 
 from oracle import experts_oracle as orc
-from helpers import RTOL_BF16, RTOL_F32, SMALL_CASES, golden_inputs, load_golden
+from helpers import RTOL_BF16, RTOL_F32, SMALL_CASES, backward_by_c_abi, golden_inputs, load_golden
 
 pytestmark = pytest.mark.gpu
 GRADS = ["d_hidden", "d_routing", "d_wgu", "d_bgu", "d_wd", "d_bd"]
@@ -141,3 +141,27 @@ def test_routing_gradient_of_every_column(T, E, K, capacity, dense):
     del used
     for a, b, key in zip(run_backward(inp["grad_out"], args, capacity, E, K), ref, GRADS):
         orc.check_close(a, b, RTOL_F32, key)
+
+
+@pytest.mark.parametrize("saved", [False, True])
+@pytest.mark.parametrize("dtype,H,path,offset,accepted", [
+    (torch.float32, 64, "auto", 2, True), (torch.float32, 64, "auto", 1, False), (torch.float32, 64, "simt", 2, False),
+    (torch.float32, 72, "auto", 2, False), (torch.float32, 72, "auto", 4, True), (torch.bfloat16, 64, "auto", 4, True),
+    (torch.bfloat16, 64, "auto", 2, False), (torch.bfloat16, 64, "simt", 4, True)])
+def test_alignment_of_d_hidden(dtype, H, path, offset, accepted, saved):
+    """In fp32 the sums of d_hidden are the caller's buffer.  What the kernels can address is served, the rest refused."""
+    import yamoe_b200
+    T, E, K = 130, 4, 2
+    inp = orc.make_inputs(T, H, E, K, seed=H + offset, weight_std=H ** -0.5, bias_std=0.2, dtype=dtype, with_grad=True)
+    args = [inp[k] for k in ("hidden_states", "router_indices", "routing_weights", "gate_up_proj", "gate_up_proj_bias",
+                             "down_proj", "down_proj_bias")]
+    yamoe_b200.set_path(path)
+    try:
+        status, got = backward_by_c_abi(inp["grad_out"], args, T, E, K, saved=saved, d_hidden_offset=offset)
+    finally:
+        yamoe_b200.set_path("auto")
+    assert status == (0 if accepted else -1)
+    if accepted:
+        ref = orc.experts_backward_oracle(inp["grad_out"], *args, T, E, K)
+        for a, b, key in zip(got, ref, GRADS):
+            orc.check_close(a.float(), b, RTOL_F32 if dtype == torch.float32 else RTOL_BF16, key)

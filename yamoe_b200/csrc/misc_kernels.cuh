@@ -188,9 +188,14 @@ gather_grad_tokens_kernel(const T* grad_out, int slots, const T* down_bias, cons
           for (int j = 0; j < VE; ++j) g[j] += g2[j];
         }
         if (k0 == 0) {
+          float* a = acc + (size_t)t * H + (size_t)i * VE;
+          if (sizeof(T) == 4 && (reinterpret_cast<uintptr_t>(acc) & 15) != 0) {   // the caller's d_hidden, 8-byte aligned
 #pragma unroll
-          for (int j = 0; j < VE; j += 4)
-            *reinterpret_cast<float4*>(acc + (size_t)t * H + (size_t)i * VE + j) = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int j = 0; j < VE; j += 2) *reinterpret_cast<float2*>(a + j) = make_float2(0.f, 0.f);
+          } else {
+#pragma unroll
+            for (int j = 0; j < VE; j += 4) *reinterpret_cast<float4*>(a + j) = make_float4(0.f, 0.f, 0.f, 0.f);
+          }
         }
         uint4 q;
         store_vec<T, VE>(reinterpret_cast<T*>(&q), g);

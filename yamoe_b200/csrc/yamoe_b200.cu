@@ -444,6 +444,9 @@ static int backward_impl(const void* grad_out, int per_slot, const void* hidden,
     YB_CUDA_OK(cudaMemsetAsync(d_bd, 0, (size_t)E * H * es, st));
     return YAMOE_OK;
   }
+  // d_hidden leaves by 8-byte stores or atomics, in fp32 on the CUDA cores by 16-byte atomics
+  const bool wide = sizeof(T) == 4 && !use_split_f32(path, H, wgu, wd);
+  if ((reinterpret_cast<uintptr_t>(d_hidden) & (wide ? 15 : 7)) != 0) return YAMOE_ERR_BAD_ARG;
   int rc = YAMOE_OK;
   const int Hp = H + kBiasCols;     // row pitch of xs and actw (see kBiasCols)
   const unsigned row_blocks = (unsigned)ceil_div(p.max_rows, kRowWarps);
