@@ -441,6 +441,11 @@ struct F32Params {
   int b_stages;
 };
 
+// Rows of a tile where an expert's rows (a multiple of 16) are cut into cnt >= 1 tiles; the last one takes the rest.
+__device__ __forceinline__ int f32_tile_rows(int rows, int cnt) {
+  return cnt == 1 ? rows : (int)(((unsigned)(rows + cnt - 1) / (unsigned)cnt + 15u) & ~15u);
+}
+
 // tcgen05.mma with the A operand in TMEM (each CTA of the pair holds its own 128 rows)
 __device__ __forceinline__ void tc2_mma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
                                                 uint32_t accumulate) {
@@ -539,16 +544,18 @@ umma_f32_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__
   if (MODE != kWgrad && warp >= 4 && warp < 4 + kF32Tiles) {
     // Most rows of a tile: the candidate (one to a warp) with the smallest product of waves and clocks of its widest k-block, 12
     // per row on the tensor core (24 instructions) but no less than kConvClocks for the weights' conversion and the chain of
-    // signals around it.  (With 1200 it cuts too finely: T = 900, E = 8, H = 2880 510 us against 487; with 900 T = 512 382
-    // against 316; 2000 is the same as 1600.)  By one warp after the other this stood before the first load of every launch:
-    // training step of 600 tokens 379 us, now 364.
-    constexpr int kConvClocks = 1600;
+    // signals around it; of equals the one of fewest rows (by most rows, skewed routing, H = 1024, E = 16: T = 600 122 us, now 112;
+    // T = 800 128, now 122).  kConvClocks, H = 2880, E = 8, skewed: with 1400 it cuts too finely (T = 333 296 us against 271, T = 1100
+    // 688 against 655), with 2000 too coarsely (T = 800 512 against 482); with 1600 H = 2048, E = 16, K = 4, T = 1000 takes 576, now 558.
+    // By one warp after the other this stood before the first load of every launch: training step of 600 tokens 379 us, now 364.
+    constexpr int kConvClocks = 1800;
     const int cap = kF32N - 16 * (warp - 4);
     int n = 0, widest = 0;
+#pragma unroll 1
     for (int e = lane; e < p.E; e += 32) {
-      const int rows = s_rows[e], cnt = (rows + cap - 1) / cap;
+      const int rows = s_rows[e], cnt = (int)((unsigned)(rows + cap - 1) / (unsigned)cap);
       n += cnt;
-      if (cnt > 0) widest = max(widest, cnt == 1 ? rows : (rows / cnt + 16) & ~15);
+      if (cnt > 0) widest = max(widest, f32_tile_rows(rows, cnt));
     }
     n = __reduce_add_sync(0xffffffffu, n);
     widest = __reduce_max_sync(0xffffffffu, widest);
@@ -559,8 +566,9 @@ umma_f32_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__
     int tile = kF32N, best = s_cost[0];
 #pragma unroll
     for (int i = 1; i < kF32Tiles; ++i)
-      if (s_cost[i] < best) { best = s_cost[i]; tile = kF32N - 16 * i; }
+      if (s_cost[i] <= best) { best = s_cost[i]; tile = kF32N - 16 * i; }
     int before = 0;
+#pragma unroll 1
     for (int e0 = 0; e0 < p.E; e0 += 32) {
       const int n = e0 + lane < p.E ? (s_rows[e0 + lane] + tile - 1) / tile : 0;
       int inc = n;
@@ -594,7 +602,7 @@ umma_f32_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__
       const int local = id - s_first[e] * MT;
       const int mt = cnt == 1 ? local : local / cnt;
       const int rows = s_rows[e];
-      const int step = cnt == 1 ? rows : ((rows + cnt - 1) / cnt + 15) & ~15;
+      const int step = f32_tile_rows(rows, cnt);
       const int off = (local - mt * cnt) * step;
       m0 = mt * 2 * kF32M + (int)rank * kF32M;
       n0 = s_pad[e] + off;
