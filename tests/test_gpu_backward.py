@@ -165,3 +165,28 @@ def test_alignment_of_d_hidden(dtype, H, path, offset, accepted, saved):
         ref = orc.experts_backward_oracle(inp["grad_out"], *args, T, E, K)
         for a, b, key in zip(got, ref, GRADS):
             orc.check_close(a.float(), b, RTOL_F32 if dtype == torch.float32 else RTOL_BF16, key)
+
+
+@pytest.mark.parametrize("saved", [False, True])
+@pytest.mark.parametrize("T,E,K,capacity,dense", [(130, 4, 2, 37, True), (300, 16, 8, 90, False), (5, 8, 2, 1, True),
+                                                  (700, 3, 2, 300, False)])
+@pytest.mark.parametrize("dtype,H,path", [(torch.float32, 64, "auto"), (torch.float32, 72, "auto"), (torch.float32, 128, "simt"),
+                                          (torch.bfloat16, 64, "auto"), (torch.bfloat16, 192, "auto"), (torch.bfloat16, 72, "auto")])
+def test_dropped_rows_among_unset_memory(dtype, H, path, T, E, K, capacity, dense, saved):
+    """A capacity that drops, on outputs and workspace full of NaN: every element of a gradient is written, and nothing that a
+    kernel reads without having written it (padding behind the kept rows, rows of dropped assignments) reaches one."""
+    import yamoe_b200
+    inp = orc.make_inputs(T, H, E, K, seed=T + H, weight_std=H ** -0.5, bias_std=0.2, dtype=dtype, with_grad=True)
+    args = [inp[k] for k in ("hidden_states", "router_indices", "routing_weights", "gate_up_proj", "gate_up_proj_bias",
+                             "down_proj", "down_proj_bias")]
+    if not dense:
+        args[2] = torch.gather(args[2], 1, args[1]).contiguous()
+    yamoe_b200.set_path(path)
+    try:
+        status, got = backward_by_c_abi(inp["grad_out"], args, capacity, E, K, saved=saved)
+    finally:
+        yamoe_b200.set_path("auto")
+    assert status == 0
+    ref = orc.experts_backward_oracle(inp["grad_out"], *args, capacity, E, K)
+    for a, b, key in zip(got, ref, GRADS):
+        orc.check_close(a.float(), b, RTOL_F32 if dtype == torch.float32 else RTOL_BF16, key)
