@@ -170,7 +170,7 @@ def make_workload(name, weights_on=None, token_seed=None, weights=None):
     (the four weight tensors of an earlier workload of the same shape) skips drawing them again;
     routing and activations are what `make_inputs` draws first from the same seed."""
     import torch
-    from yamoe_b200 import workloads
+    from oracle.experts_oracle import workloads      # without the package and its libraries
     w = WORKLOADS[name]
     dtype = torch.float32 if w.get("fp32") else torch.bfloat16
     if weights is not None:

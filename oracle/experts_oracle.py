@@ -24,6 +24,9 @@ Reference lines each function follows (paths are within the reference project):
 """
 from __future__ import annotations
 
+import importlib.util
+import os
+
 import torch
 
 ALPHA = 1.702  # csrc/moe.cpp:179, reference.py:15
@@ -157,9 +160,18 @@ def experts_backward_oracle(grad_out, hidden_states, router_indices, routing_wei
     return d_hidden, d_routing, d_wgu, d_bgu, d_wd, d_bd
 
 
-# Seeded synthetic workloads live in the package (they are inputs, not a checker) and are
-# re-exported here for the tests.
-from yamoe_b200.workloads import make_inputs, make_readme_inputs, make_routing  # noqa: E402,F401
+def _workloads():
+    """Seeded synthetic workloads live in the package (they are inputs, not a checker) and are re-exported here.  Loaded by
+    path: importing the package loads its CUDA libraries, which have no place in a process that times the CPU code."""
+    path = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "yamoe_b200", "workloads.py")
+    spec = importlib.util.spec_from_file_location("yamoe_b200_workloads", path)
+    module = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(module)
+    return module
+
+
+workloads = _workloads()
+make_inputs, make_readme_inputs, make_routing = workloads.make_inputs, workloads.make_readme_inputs, workloads.make_routing
 
 
 def binned_gather_oracle(x, indices, bins, num_experts, capacity, top_k):
@@ -229,7 +241,6 @@ def reference_forward_from(path: str):
     the signature of `experts_forward_oracle`, running the sparse (training) branch
     (reference.py:38-59).  The reference has no expert capacity: the wrapper is only valid when the
     capacity drops nothing, which holds for every benchmark workload."""
-    import importlib.util
     import types
     spec = importlib.util.spec_from_file_location("yamoe_reference_py", path)
     mod = importlib.util.module_from_spec(spec)

@@ -1,6 +1,8 @@
 """Host-side pieces of bench.py that need no GPU: the clock-sample parser and the launch counts."""
 import datetime
+import json
 import os
+import subprocess
 import sys
 import time
 
@@ -72,3 +74,15 @@ def test_launch_counts_cover_every_mode():
     assert bench.LAUNCHES["train"] == bench.LAUNCHES["fwd"] + bench.LAUNCHES["bwd"]
     for name, w in bench.WORKLOADS.items():
         assert w["mode"] in ("fwd", "bwd", "train"), name
+
+
+def test_reference_arm_loads_none_of_the_library():
+    """The arm that times the reference's CPU code runs in a process of its own, without this project's package."""
+    code = ("import sys, types, bench\n"
+            "bench.WORKLOADS['tiny'] = dict(T=16, H=64, E=4, K=2, mode='fwd')\n"
+            "bench.run_reference(types.SimpleNamespace(workload='tiny', steps=1, warmup=0, gpus=1))\n"
+            "assert 'yamoe_b200' not in sys.modules\n"
+            "assert 'libyamoe' not in open('/proc/self/maps').read()\n")
+    done = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True, timeout=300)
+    assert done.returncode == 0, done.stderr
+    assert json.loads(done.stdout)["impl"] == "reference"
