@@ -1,5 +1,7 @@
 """Shared helpers for the tests: golden loading and tolerance rules."""
+import importlib
 import os
+import pickle
 
 import numpy as np
 import torch
@@ -13,6 +15,30 @@ INPUT_KEYS = ["hidden_states", "router_indices", "routing_weights", "gate_up_pro
 RTOL_F32 = 1e-4
 RTOL_BF16 = 2e-2
 REL_L2_BF16 = 1e-2
+
+
+class _Whole:
+    """Arrives at the other end of a queue as the object that was put, tensors by value."""
+
+    def __init__(self, obj):
+        self.data = pickle.dumps(obj)
+
+    def __reduce__(self):
+        return pickle.loads, (self.data,)
+
+
+class _WholeQueue:
+    def __init__(self, queue):
+        self.queue = queue
+
+    def put(self, obj):
+        self.queue.put(_Whole(obj))
+
+
+def run_rank(module, worker, *args):
+    """`worker` of a test module as a process, its queue (the last argument) passing tensors by value: by torch's own way a
+    tensor goes as a file handle, which its reader has to fetch while the sending process still lives."""
+    getattr(importlib.import_module(module), worker)(*args[:-1], _WholeQueue(args[-1]))
 
 
 def load_golden(name):
