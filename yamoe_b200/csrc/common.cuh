@@ -43,6 +43,9 @@ inline int64_t max_row_tiles(int64_t S, int E) {
   return ceil_div(S, kTileM) + ne;
 }
 
+// SMs of a B200, for what only sizes a grid or a split; what relies on CTAs being resident asks the device.
+constexpr int kSMs = 148;
+
 // The grouped GEMMs cover an expert's rows up to this end: its assignments as far as the padded layout holds them,
 // rounded up to `row_round` rows.  Where the capacity drops some, that is more than the kept rows.
 __device__ __forceinline__ int covered_rows(int count, int padded, int row_round) {

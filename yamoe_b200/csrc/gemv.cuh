@@ -98,11 +98,14 @@ __device__ __forceinline__ void gemv_accumulate(const __nv_bfloat16* __restrict_
 
 // Weights of stage two that stage one asks L2 for: the first rows of each expert hit.  HBM would idle through the last
 // reductions, the kernel boundary and the set-up of stage two; now it works on, and stage two begins in L2.  Asked by the CTAs
-// of the last wave, when they have issued their own loads.  Each call on other experts than the one before (weights
-// not in L2), H = 2880, K = 4: T = 1 49.0 -> 47.0 us, T = 2 82.8 -> 80.5; H = 2048, K = 8, T = 1 55.4 -> 51.7.  Asked at the
-// start of stage one, 64 MB: 49.0 and 82.8 (stage one takes as much longer); 64 MB at this place: 49.4.
+// of the last wave, when they have issued their own loads.  Without / with it, calls in a row as a graph replay, us.  Each on
+// other experts than the one before (weights not in L2): H = 2880, K = 4, E = 128 T = 1 44.2 / 44.1, T = 2 77.8 / 77.4, T = 4
+// 141.3 / 139.3, T = 8 249.7 / 247.2, T = 16 434 / 432; E = 32 T = 1 43.9 / 43.3, T = 4 132.5 / 129.8; H = 2048, K = 8, T = 1
+// 49.0 / 48.0; H = 1024, E = 32 T = 1 no difference, T = 8 34.6 / 33.0.  On the same experts again: H = 2880, T = 1 43.4 / 41.7.  So one
+// token's call gains next to nothing where its experts are new, others about 1 %, and none loses.  64 MB, or asked at the
+// start of stage one, was no better (stage one takes as much longer).
 constexpr int64_t kGemvAheadBytes = (int64_t)32 << 20;
-constexpr int kGemvWave = 3 * 148;           // CTAs that run at a time
+constexpr int kGemvWave = 3 * kSMs;           // CTAs that run at a time
 __device__ __forceinline__ void gemv_ask_ahead(const GemvArgs& g, int e, int touched) {
   const int askers = min((int)gridDim.y, (kGemvWave + touched - 1) / touched);
   const int i = (int)(blockIdx.y - gridDim.y) + askers;
@@ -340,7 +343,7 @@ inline int gemv_gate_up_slab(int64_t S, int E, int N) {
   }();
   if (forced) return forced;
   const int64_t slots = E < S ? E : S;
-  return slots * ceil_div(N, 128) < 4 * 148 ? 64 : 128;
+  return slots * ceil_div(N, 128) < 4 * kSMs ? 64 : 128;
 }
 
 // Number of CTAs that share the reduction dimension of one (expert, column slab) in the down
@@ -355,7 +358,7 @@ inline int gemv_down_ksplit(int64_t S, int E, int N) {
   }();
   if (forced) return forced;
   const int64_t ctas = (E < S ? E : S) * ceil_div(N, 64);
-  return ctas <= 2 * 148 ? 2 : 1;     // measured: 53.6 / 55.0 / 55.6 us with 2 / 1 / 4 parts at T = 1; no gain beyond
+  return ctas <= 2 * kSMs ? 2 : 1;     // measured: 53.6 / 55.0 / 55.6 us with 2 / 1 / 4 parts at T = 1; no gain beyond
 }
 
 // Decode-sized calls, at most about 4 rows per expert.  A token's K weighted rows are summed in fp32 there,
@@ -427,7 +430,7 @@ inline int launch_gemv_forward(const void* hidden, const int64_t* ridx, const vo
     }();
     // 128-column slabs pay only when they still give every SM about eight CTAs (T = 64: 1006 us
     // against 1018 us; T = 16: 465 us against 457 us)
-    const bool wide = down_nb ? down_nb == 128 : (E < S ? E : S) * ceil_div(H, 128) >= 8 * 148;
+    const bool wide = down_nb ? down_nb == 128 : (E < S ? E : S) * ceil_div(H, 128) >= 8 * kSMs;
     rc = wide ? launch_gemv_stage<kDown, 128>(g2, st, 1)
               : launch_gemv_stage<kDown, 64>(g2, st, gemv_down_ksplit(S, E, H));
   }

@@ -1,6 +1,7 @@
-// Memory-bound helper kernels around the grouped GEMMs: row gathers into the padded,
-// expert-sorted layout, the fp32 -> storage cast of the combined output, bias-gradient column
-// sums and the placement of routing-weight gradients.
+// Memory-bound helper kernels around the grouped GEMMs: gathers of token rows and of gradients into the padded,
+// expert-sorted layout (by token; by row for expert parallelism) with the zeroing of its padding, the combine of a
+// token's K rows, the fp32 -> storage cast, bias-gradient column sums, the last step of a backward pass (cast and
+// routing gradients), the rows that expert parallelism sends, and the reference's small sub-operators.
 #pragma once
 #include "common.cuh"
 #include "epilogues.cuh"
@@ -95,14 +96,13 @@ inline cudaError_t launch_gather_tokens(const void* src, const Dst& dst, const R
                         nvec, ld_vec, K, (unsigned)pad_ctas, row_round);
 }
 
-// Backward gather: gys[row, :] = grad_y[token, :] where grad_y is grad_out, or the sum of its K
-// slot slices (reference: csrc/experts_backward.cu:224-228); also seeds the routing-weight
-// gradient of the row with <grad_y[token], b_down[e]>, the bias part of <grad_y, y_e>
+// Backward gather of the expert-parallel path, by row: gys[row, :] = grad_out[token, :]; also seeds the
+// routing-weight gradient of the row with <grad_out[token], b_down[e]>, the bias part of <grad_out, y_e>
 // (reference: csrc/experts_backward.cu:83-88).
 template <typename T>
 __global__ void __launch_bounds__(kRowWarps * 32)
-gather_grad_kernel(const T* __restrict__ grad_out, int slots, const T* __restrict__ down_bias,
-                   T* __restrict__ gys, float* __restrict__ gw_row, const int32_t* __restrict__ row_token,
+gather_grad_kernel(const T* __restrict__ grad_out, const T* __restrict__ down_bias, T* __restrict__ gys,
+                   float* __restrict__ gw_row, const int32_t* __restrict__ row_token,
                    const int32_t* __restrict__ tile_expert, const int32_t* __restrict__ header, int H) {
   const int row = blockIdx.x * kRowWarps + (threadIdx.x >> 5);
   if (row >= header[kHdrRowsUsed]) return;
@@ -121,13 +121,7 @@ gather_grad_kernel(const T* __restrict__ grad_out, int slots, const T* __restric
   float dot = 0.f;
   for (int i = lane; i < nvec; i += 32) {
     float g[VE], bb[VE];
-    load_vec<T, VE>(grad_out + ((size_t)tok * slots) * H + (size_t)i * VE, g);
-    for (int s = 1; s < slots; ++s) {
-      float g2[VE];
-      load_vec<T, VE>(grad_out + ((size_t)tok * slots + s) * H + (size_t)i * VE, g2);
-#pragma unroll
-      for (int j = 0; j < VE; ++j) g[j] += g2[j];
-    }
+    load_vec<T, VE>(grad_out + (size_t)tok * H + (size_t)i * VE, g);
     store_vec<T, VE>(d + (size_t)i * VE, g);
     load_vec<T, VE>(b + (size_t)i * VE, bb);
 #pragma unroll
@@ -138,8 +132,8 @@ gather_grad_kernel(const T* __restrict__ grad_out, int slots, const T* __restric
   if (lane == 0) gw_row[row] = dot;
 }
 
-// The same from the tokens' side (see gather_tokens_kernel): the K rows of a token take its gradient, which is read
-// once, and the dot products with K experts' biases are accumulated beside each other (T = 8192, H = 2880, K = 4: 101 us
+// The same from the tokens' side (see gather_tokens_kernel), where the gradient may also be the sum of K slot slices
+// (reference: csrc/experts_backward.cu:224-228): the K rows of a token take its gradient, which is read once, and the dot products with K experts' biases are accumulated beside each other (T = 8192, H = 2880, K = 4: 101 us
 // by row, 79 by token).  `wpt` warps (1, 2, 4 or 8) share a token, so that few tokens also fill the GPU.
 // The warps of a token also zero its row of `acc`, the fp32 sums of the hidden states' gradient: stores run at 7 TB/s
 // where a memset does 3.9, and a launch is saved (T = 8192, H = 2880: memset 22 us + gather 64, together 77).
@@ -238,7 +232,7 @@ inline cudaError_t launch_gather_grad_tokens(const T* grad_out, int slots, const
                                              int row_round, cudaStream_t st) {
   // at least 32 warps per SM, while each has a piece of the row
   int wpt = 1;
-  while (wpt < kRowWarps && Tn * wpt < 148 * 32 && H * (int)sizeof(T) / 16 > 32 * wpt) wpt *= 2;
+  while (wpt < kRowWarps && Tn * wpt < kSMs * 32 && H * (int)sizeof(T) / 16 > 32 * wpt) wpt *= 2;
   const int64_t token_ctas = ceil_div(Tn * wpt, kRowWarps), pad_ctas = (int64_t)E * kPadCtas;
   auto kern = K <= 4 ? gather_grad_tokens_kernel<T, Dst, 4> : gather_grad_tokens_kernel<T, Dst, 8>;
   return launch_pdl_opt(true, kern, dim3((unsigned)(pad_ctas + token_ctas)), dim3(kRowWarps * 32), 0, st, grad_out, slots,
@@ -363,21 +357,13 @@ template <typename T>
 inline int launch_finish_grads(const float* acc, T* d_hidden, const float* gw_row, const RouteTables& rt, T* d_routing,
                                int64_t Tn, int H, int routing_cols, int E, int K, cudaStream_t st) {
   const int64_t nv = Tn * H / 4;
-  const unsigned cast_ctas = acc != nullptr ? (unsigned)std::min<int64_t>(ceil_div(nv, 256), 148 * 8) : 0u;
+  const unsigned cast_ctas = acc != nullptr ? (unsigned)std::min<int64_t>(ceil_div(nv, 256), kSMs * 8) : 0u;
   const cudaError_t rc = launch_pdl_opt(true, finish_grads_kernel<T>, dim3(cast_ctas + (unsigned)ceil_div(Tn, 8)), dim3(256), 0,
                                         st, acc, d_hidden, nv, cast_ctas, gw_row, rt, d_routing, Tn, routing_cols, E, K);
   return rc == cudaSuccess && cudaGetLastError() == cudaSuccess ? YAMOE_OK : YAMOE_ERR_CUDA;
 }
 
-// out[t, :] = sum over the kept slots k of y[flat_row[t*K + k], :]   (rows already weighted).
-// Second half of the combine (reference: csrc/scatter.cu:67-108): fp32 accumulation in slot
-// order, one rounding, every output element written exactly once (no zero-fill, no atomics).
-// One warp per token and 32 16-byte pieces of its row, with the loads of up to KB slots in flight: latency bounds the
-// few-token calls (a warp per token left most SMs idle and walked the columns one after the
-// other: 30 us at T = 64 and 512 with H = 2880, now 3 to 5), HBM the others.  The pieces of a row are neighbours in
-// the grid, so that its 512-byte parts are read at about the same time (T = 4096 44 us with the tokens as
-// neighbours, 30 with the pieces, 24 since the loads wait unconverted; T = 1531, K = 8, H = 2048 23 and 11).
-// Rows of another type than the output (fp32 rows of a bf16 call) lie at their flat positions p = t*K + k.
+// the elements of 16 bytes, as fp32
 template <typename T>
 __device__ __forceinline__ void unpack_vec(const uint4& q, float (&v)[16 / sizeof(T)]) {
   const uint32_t u[4] = {q.x, q.y, q.z, q.w};
@@ -392,6 +378,15 @@ __device__ __forceinline__ void unpack_vec(const uint4& q, float (&v)[16 / sizeo
   }
 }
 
+// out[t, :] = sum over the kept slots k of y[flat_row[t*K + k], :]   (rows already weighted).
+// Second half of the combine (reference: csrc/scatter.cu:67-108): fp32 accumulation in slot
+// order, one rounding, every output element written exactly once (no zero-fill, no atomics).
+// One warp per token and 32 16-byte pieces of its row, with the loads of up to KB slots in flight: latency bounds the
+// few-token calls (a warp per token left most SMs idle and walked the columns one after the
+// other: 30 us at T = 64 and 512 with H = 2880, now 3 to 5), HBM the others.  The pieces of a row are neighbours in
+// the grid, so that its 512-byte parts are read at about the same time (T = 4096 44 us with the tokens as
+// neighbours, 30 with the pieces, 24 since the loads wait unconverted; T = 1531, K = 8, H = 2048 23 and 11).
+// Rows of another type than the output (fp32 rows of a bf16 call) lie at their flat positions p = t*K + k.
 template <typename TY, typename T, int KB>
 __global__ void __launch_bounds__(kRowWarps * 32, KB > 4 ? 4 : 5)
 combine_padded_kernel(const TY* y, const int32_t* flat_row, T* __restrict__ out, int64_t Tn, int H, int K) {

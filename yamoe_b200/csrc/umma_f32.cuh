@@ -27,7 +27,8 @@
 // is short, 2.1e-7 against 2.5e-7.
 //
 // Measured: gate_up of the README forward (T = 512, H = 2880, E = 8, K = 2) 177 us = 192 TFLOP/s of the
-// original product; the whole forward 313 us, a training step of 600 tokens 387 (CUDA cores: 1797 and 1191).
+// original product; the whole forward 355 us among others of its kind, 300 to 315 on a cool GPU (the power cap lowers the
+// clock), a training step of 600 tokens 366 (CUDA cores: 1797 and 1191).
 //
 // Infinities and NaN behave as in fp32 arithmetic: see split3_special.
 //
@@ -44,8 +45,8 @@
 // Tiles of up to 160 rows, of a size that the kernel picks for the launch (see s_cost): a tile's weights are converted
 // for its rows alone, and with 128 rows at most half of the experts of the README forward (128 rows each on average) took
 // two tiles: 276 tiles in four waves of 74 pairs, now 184 in three.  gate_up 216 -> 177 us, the whole forward
-// 348 -> 313, with the waits looked at side by side included: a look at a barrier that is ready takes some 120 clocks, of
-// which a k-block had three in the issuer and two in the converters.
+// 348 -> 313 (both on a cool GPU), with the waits looked at side by side included: a look at a barrier that is ready takes
+// some 120 clocks, of which a k-block had three in the issuer and two in the converters.
 #pragma once
 #include "misc_kernels.cuh"
 #include "umma_pair.cuh"
@@ -91,7 +92,7 @@ __device__ __forceinline__ uint3 split3_special(float x) {
 
 // The parts of N numbers as bf16 pairs (the first of a pair in the low half).  Returns NaN where one of them is special;
 // the caller then has it done again.  One look at all N: a branch for each pair keeps the loads of the next from
-// being issued ahead (README forward 513 us, now 412; 511 with cvt.rn.bf16x2 instead of integer arithmetic).
+// being issued ahead (README forward of that time 513 us and 412 without; 511 with cvt.rn.bf16x2 instead of integer arithmetic).
 template <int N>
 __device__ __forceinline__ float split3_finite(const float (&x)[N], uint32_t (&p0)[N / 2], uint32_t (&p1)[N / 2],
                                                uint32_t (&p2)[N / 2]) {
@@ -472,7 +473,7 @@ __device__ __forceinline__ void tc_ld_32x16(uint32_t taddr, uint32_t (&r)[16]) {
         "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
       : "r"(taddr) : "memory");
 }
-// whether an mbarrier phase is over, for a first look at several: each look takes some 100 clocks, side by side once
+// whether an mbarrier phase is over, for a first look at several: a look takes some 120 clocks, several side by side no more
 __device__ __forceinline__ bool mbar_ready(uint32_t bar, uint32_t parity) { return mbar_try_wait(bar, parity) != 0; }
 template <int N> __device__ __forceinline__ void more_registers() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 template <int N> __device__ __forceinline__ void fewer_registers() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }

@@ -756,7 +756,7 @@ inline int umma_sm_count() {
   const int dev = current_device_index();
   int n = count.get(dev);
   if (n == 0) {
-    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = kSMs;
     count.set(dev, n);
   }
   return n;

@@ -425,10 +425,12 @@ inline int pair_smem(int park_groups, int E) { return kPairSmem + park_groups * 
 // tile it is not, or where the last one of a CTA counts; else the additional warps only wait and take power (T = 4096,
 // H = 2880: 735 us with eight, 755 with sixteen).
 // Weight gradients: up to some 512 rows per expert (8 / 16 warps: 192 rows, H = 2048 gate_up 359 / 306 us, down 190 / 160;
-// 1024 rows, H = 2880 788 / 806 and 396 / 407).
+// 1024 rows, H = 2880 788 / 806 and 396 / 407; a whole backward of 16 experts, H = 2048: 100 rows 340 / 297, 320 460 / 439, 400
+// 507 / 492, 512 585 / 583, 600 663 / 669, 700 767 / 783; H = 1024: 100 rows 146 / 135, 512 237 / 236, 600 253 / 254).
 inline bool pair_wgrad_16_warps(int64_t S, int E) { return S <= 512 * (int64_t)E; }
-// The others: main loops of up to 16 k-blocks (T = 2048, E = 16, H = 1024 67.0 / 63.7 us), with the longer epilogue
-// of the GLU's backward up to 32 (192 rows per expert, H = 2048 180 / 168).
+// The others: main loops of up to 16 k-blocks (a forward of 16 experts, H = 1024: 192 rows 51.4 / 48.1 us, 1000 rows 115 / 110;
+// 24 k-blocks, H = 1536: 192 rows 78.5 / 76.0, 512 126.1 / 126.5, 1000 201.7 / 203.9; 32, H = 2048: 192 rows 112 / 108, 512 202.0 / 202.6),
+// with the longer epilogue of the GLU's backward up to 32 (192 rows, H = 2048 180 / 168; a whole backward of 1024 rows 1000 / 974).
 inline bool pair_16_warps(int kblocks, bool glu_backward) { return kblocks <= (glu_backward ? 32 : 16); }
 
 __device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, int c0, int c1, int c2, uint32_t src) {
@@ -662,7 +664,7 @@ umma_pair_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant_
     }
     __syncwarp();
   } else {
-    // =========================== epilogue (warps 2..9 of both CTAs) ==========================
+    // =========================== epilogue (warps 2 .. 1 + kEpiWarps of both CTAs) ============
     const int q = warp & 3;                    // TMEM lane quarter this warp may read
     const int turn = (warp - 2) >> 2;          // takes the 32-column chunks turn, turn + groups, ...
     const int groups = kStore ? p.groups : kEpiWarps / 4;

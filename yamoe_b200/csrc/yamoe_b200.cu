@@ -181,8 +181,8 @@ static bool use_tcgen05(int path, int dtype, int H) {
 }
 
 // fp32 through umma_f32.cuh (three bf16 parts per operand): README forward (T = 512, E = 8, H = 2880)
-// 412 us against 1797 us with the CUDA-core kernel, training step of 600 tokens (E = 16, H = 1024)
-// 400 against 1191 us.  The CUDA-core kernel keeps the widths that are no multiple of 64 and the
+// 355 us against 1797 us with the CUDA-core kernel, training step of 600 tokens (E = 16, H = 1024)
+// 366 against 1191 us.  The CUDA-core kernel keeps the widths that are no multiple of 64 and the
 // weights that TMA cannot address.
 static bool use_split_f32(int path, int H, const void* wgu, const void* wd) {
   return umma_available() && H % 64 == 0 && ((reinterpret_cast<uintptr_t>(wgu) | reinterpret_cast<uintptr_t>(wd)) & 15) == 0 &&
@@ -317,7 +317,7 @@ static int forward_impl(const void* hidden, const int64_t* ridx, const void* rw,
   }
   if (p.acc32) {
     const int64_t nv = Tn * H / 4;
-    cast_kernel<T><<<(unsigned)std::min<int64_t>(ceil_div(nv, 256), 148 * 8), 256, 0, st>>>(
+    cast_kernel<T><<<(unsigned)std::min<int64_t>(ceil_div(nv, 256), kSMs * 8), 256, 0, st>>>(
         p.acc32, reinterpret_cast<T*>(out), nv);
   }
   return cudaGetLastError() == cudaSuccess ? YAMOE_OK : YAMOE_ERR_CUDA;
@@ -716,7 +716,7 @@ static int ep_local_backward_impl(const void* recv_x, const void* recv_g, const 
   }
   ep_load_weights_kernel<<<(unsigned)ceil_div(max_rows, 256), 256, 0, st>>>(p.t, recv_w, max_rows);
   gather_grad_kernel<T><<<(unsigned)ceil_div(max_rows, kRowWarps), kRowWarps * 32, 0, st>>>(
-      reinterpret_cast<const T*>(recv_g), 1, reinterpret_cast<const T*>(bd), reinterpret_cast<T*>(p.gys), p.gw_row,
+      reinterpret_cast<const T*>(recv_g), reinterpret_cast<const T*>(bd), reinterpret_cast<T*>(p.gys), p.gw_row,
       rt.row_token, rt.tile_expert, rt.header, H);
   if (tc) {
     if constexpr (sizeof(T) == 2) {
