@@ -13,10 +13,11 @@ import shutil
 import sys
 
 HERE = os.path.dirname(os.path.abspath(__file__))
+BESIDE = os.path.join(os.path.dirname(os.path.dirname(HERE)), "reference")      # the reference tree beside this one
 REL = os.path.join("build", "torch28-cxx11-cu129-x86_64-linux", "yamoe", "reference.py")
 
 
-def make_ref(root: str = os.environ.get("YAMOE_REFERENCE_ROOT", "/root/reference")) -> str | None:
+def make_ref(root: str = os.environ.get("YAMOE_REFERENCE_ROOT", BESIDE)) -> str | None:
     src = os.path.join(root, REL)
     if not os.path.exists(src):
         return None
