@@ -9,8 +9,8 @@
  *
  * Every entry point returns YAMOE_OK (0) or a negative yamoe_status_t.
  *
- * Tensors of the expert passes start on 16-byte boundaries where nothing else is said; integer ones and biases
- * of the weights in fp32 need no more than their element's size.
+ * Tensors of the expert passes start on 16-byte boundaries where nothing else is said; integer ones and the weight
+ * matrices in fp32 (CUDA-core kernels, where TMA cannot address them) need no more than their element's size.
  *
  * The comments cite the interface of the reference project (drbh/yamoe) that each entry
  * point replaces, as path:line within that project.
